@@ -53,7 +53,7 @@ def listed():
              bounces=8, out="image", estimator=1, guide="fixed"),
         # the first waves of a guided render: the guide is trained, not yet sampled
         dict(name="guide_warmup", kind="render", scene="hard_indirect", size=7, width=512, height=512, spp=16, bounces=8,
-             out="image", estimator=0, guide="warmup"),
+             out="image", estimator=1, guide="warmup"),
         # several uneven scenes served by one renderer
         dict(name="batch", kind="render", scene="batch", size=12, width=0, height=256, spp=32, bounces=0, out="images"),
         # closest hits against a soup that is new on every call (no allocation, BVH built in place)
