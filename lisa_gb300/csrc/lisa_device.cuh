@@ -585,28 +585,51 @@ __device__ __forceinline__ bool emit_may_hit(const SceneDev& sc, V3 o, V3 d) {
   return box_may_hit(r, sc.emit_lo, sc.emit_hi, RAY_TMIN, RAY_TMAX);
 }
 
-// Conservative emit_may_hit for a hemisphere draw (x, y, z) of
-// shoot_ray_hemisphere before it is normalised and flipped.  The draw,
-// flipped by the sign of dot(N, draw), points along the same ray as the
-// exact direction (a positive multiple, up to the direction's own
-// rounding, which the slab padding covers); testing it on (0, inf) covers
-// every point of (RAY_TMIN, RAY_TMAX) along the exact direction.  Where
-// dot(N, draw) is too near zero for its sign to be certain (a few ulp of
-// the exact dot would be), or not a number, the answer is "may hit".
-__device__ __forceinline__ bool emit_may_hit_draw(const SceneDev& sc, V3 o, V3 N, float x, float y, float z) {
-  if (!sc.has_emit_box) return false;
-  const float s = N.x * x + N.y * y + N.z * z;
-  if (!(fabsf(s) > 1e-5f * (fabsf(x) + fabsf(y) + fabsf(z)))) return true;
-  const float f = s > 0.0f ? 1.0f : -1.0f;
-  const float dx = f * x, dy = f * y, dz = f * z;
-  RayPre r;
-  r.ox = o.x;
-  r.oy = o.y;
-  r.oz = o.z;
-  r.ix = fabsf(dx) > 1e-30f ? __fdividef(1.0f, dx) : copysignf(1e30f, dx);
-  r.iy = fabsf(dy) > 1e-30f ? __fdividef(1.0f, dy) : copysignf(1e30f, dy);
-  r.iz = fabsf(dz) > 1e-30f ? __fdividef(1.0f, dz) : copysignf(1e30f, dz);
-  return box_may_hit(r, sc.emit_lo, sc.emit_hi, 0.0f, 3.0e38f);
+// The tries of a vertex's emitter search that may reach an emitter, as a bit
+// mask (bit j = try j; `seed` is the stream's state before try 0).  Try j is
+// the hemisphere draw q = (x, y, z) of shoot_ray_hemisphere, not normalised:
+// the exact direction is a positive multiple of q, flipped by the sign of
+// dot(N, q), each component with one more rounding.  A try is left out when
+// its line misses the padded bounds of the emissive triangles (one of the
+// three cross-product axes separates them; the axes do not depend on the
+// flip) or when all of the bounds lie behind the ray; where dot(N, q) is too
+// near zero for its sign to be certain, only the line is tested.  The bounds
+// relative to the origin (centre c, half extent h) grow by 2^-19 of |c| + |h|,
+// four times the roundings of c, h, the products and the direction.  Every
+// comparison rejects on a definite answer, so a NaN leaves the try in.  The
+// last try always stays: the search ends there.
+//
+// Divisions would cost more than the rest of the test (three reciprocals and
+// their guards a try); the separating axes need none: about 40 instructions a
+// try, all lanes busy, for a vertex of their own each.
+__device__ __forceinline__ uint32_t emit_candidates(const SceneDev& sc, V3 o, V3 N, uint32_t seed) {
+  constexpr uint32_t LAST = 1u << (NEE_TRIES - 1);
+  if (!sc.has_emit_box) return LAST;
+  const float lx = sc.emit_lo[0] - o.x, ly = sc.emit_lo[1] - o.y, lz = sc.emit_lo[2] - o.z;
+  const float ux = sc.emit_hi[0] - o.x, uy = sc.emit_hi[1] - o.y, uz = sc.emit_hi[2] - o.z;
+  const float cx = 0.5f * (lx + ux), cy = 0.5f * (ly + uy), cz = 0.5f * (lz + uz);
+  float hx = 0.5f * (ux - lx), hy = 0.5f * (uy - ly), hz = 0.5f * (uz - lz);
+  const float pad = 1.9073486328125e-6f * (((fabsf(cx) + fabsf(cy)) + fabsf(cz)) + ((hx + hy) + hz));
+  hx += pad;
+  hy += pad;
+  hz += pad;
+  uint32_t mask = LAST;
+#pragma unroll 2
+  for (int j = 0; j < NEE_TRIES - 1; ++j) {
+    const float x = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+    const float y = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+    const float z = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+    const float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
+    const bool off = fabsf(fmaf(y, cz, -(z * cy))) > fmaf(hy, az, hz * ay) ||
+                     fabsf(fmaf(z, cx, -(x * cz))) > fmaf(hz, ax, hx * az) ||
+                     fabsf(fmaf(x, cy, -(y * cx))) > fmaf(hx, ay, hy * ax);
+    const float s = fmaf(N.x, x, fmaf(N.y, y, N.z * z));
+    const float e = fmaf(cx, x, fmaf(cy, y, cz * z));
+    const bool behind = fabsf(s) > 1e-5f * ((ax + ay) + az) &&
+                        copysignf(1.0f, s) * e < -fmaf(hx, ax, fmaf(hy, ay, hz * az));
+    if (!off && !behind) mask |= 1u << j;
+  }
+  return mask;
 }
 
 // Whether the ray (o, d) may meet the box [lo, hi] inside (tmin, tmax),

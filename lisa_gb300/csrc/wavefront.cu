@@ -408,6 +408,14 @@ __global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
 // appends the continuation ray and takes the next vertex.  Lanes advance
 // independently, so a warp stays full while its vertices need between 1 and
 // 30 rays of different lengths.
+//
+// Bound by issue: most tries are decided without a traversal, so the kernel
+// is the arithmetic around the queue.  A warp therefore prepares 32 vertices
+// at a time, each lane testing all tries of its own vertex, and keeps the
+// answers as a bit mask.  (One warp-wide search per vertex and per
+// traversal, 32 lanes on the tries of one vertex, took 13.3 ms of the
+// 1.31 M-triangle icosphere step's 59 M vertices; this takes 10.3 ms, and
+// 2.5 instead of 3.3 ms on the Cornell box frame.)
 
 // Guided bounce at an opaque vertex with roughness 1, where the reference
 // draws hemi(N) (lambertian.cu:7-13): one-sample MIS between that sampler
@@ -430,6 +438,14 @@ __device__ __forceinline__ V3 guided_bounce(const float* o, V3 N, uint32_t& seed
   return w;
 }
 
+// Queue entries a warp of k_nee has prepared (shared memory).
+struct NeeVertices {
+  float4 p[32];         // position, slot
+  float4 n[32];         // normal, material
+  uint4 s[32];          // stream state, emitter flag, candidate tries, scene
+  uint32_t entry[32];
+};
+
 template <bool COUNT, bool GUIDED = false>
 __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, int depth) {
   const int q = depth & 1;
@@ -449,8 +465,13 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
   uint32_t shadow = 0, walked = 0, visits = 0, tests = 0;
   bool pending = false;  // a finished shadow ray not yet evaluated
   bool emit_pass = false;  // the finished traversal was of the emitters' own BVH
-  // LCG jumps over j tries (3 draws each), j = 0..31, for the warp's
-  // search of the next try that needs a traversal
+  uint32_t cand = 0;       // the vertex's tries that may reach an emitter (emit_candidates)
+  // vertices the warp has taken from the queue and prepared, not yet started
+  __shared__ NeeVertices vertex_buf[4];
+  NeeVertices& vb = vertex_buf[threadIdx.x >> 5];
+  uint32_t vb_next = 0, vb_count = 0;  // (the same in every lane)
+  bool queue_empty = false;
+  // LCG jumps over j tries (3 draws each), j = 0..31
   __shared__ uint2 s_jump[32];
   if (threadIdx.x < 32) {
     const LcgJump j = lcg_jump(3u * threadIdx.x);
@@ -531,33 +552,58 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
         b.ro[q ^ 1][ri] = make_float4(s.r.ox, s.r.oy, s.r.oz, __uint_as_float(slot));
         b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float((uint32_t)(sc - b.scenes)));
       }
-      const bool need = !have && !exhausted;
-      const uint32_t nmask = __ballot_sync(FULL, need);
-      if (nmask) {
-        const int leader = __ffs(nmask) - 1;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&b.ctrl->head[HEAD_NEE], (uint32_t)__popc(nmask));
-        base = __shfl_sync(FULL, base, leader);
-        if (need) {
-          entry = base + __popc(nmask & lt);
-          if (entry < count) {
-            const float4 a4 = b.nee_a[entry], b4 = b.nee_b[entry];
-            s.r.ox = a4.x;
-            s.r.oy = a4.y;
-            s.r.oz = a4.z;
-            slot = __float_as_uint(a4.w);
-            N = ld3(b4);
-            mat_idx = __float_as_int(b4.w);
-            stale = __float_as_int(b.ps_att[slot].w);
-            seed = b.ps_rng[slot];
-            sc = b.scenes + __float_as_uint(__ldg(&b.nee_c[entry].w));
-            ts = trace_scene(*sc);
-            tries = 0;
-            have = true;
-          } else {
-            exhausted = true;
+      // Idle lanes take their next vertices from the warp's buffer.  An empty
+      // buffer is filled by the whole warp: 32 consecutive queue entries at
+      // once, so that their loads coalesce and the test of their tries
+      // (emit_candidates) runs on 32 lanes.
+      while (__any_sync(FULL, !have && !exhausted)) {
+        if (vb_next == vb_count) {
+          uint32_t base = 0;
+          if (!queue_empty) {
+            if (lane == 0) base = atomicAdd(&b.ctrl->head[HEAD_NEE], 32u);
+            base = __shfl_sync(FULL, base, 0);
           }
+          if (queue_empty || base >= count) {
+            queue_empty = true;
+            if (!have) exhausted = true;
+            break;
+          }
+          vb_next = 0;
+          vb_count = min(32u, count - base);
+          if (lane < (int)vb_count) {
+            const float4 a4 = b.nee_a[base + lane], b4 = b.nee_b[base + lane];
+            const uint32_t vslot = __float_as_uint(a4.w);
+            const uint32_t scene = __float_as_uint(__ldg(&b.nee_c[base + lane].w));
+            const uint32_t flag = __float_as_uint(b.ps_att[vslot].w), vseed = b.ps_rng[vslot];
+            vb.p[lane] = a4;
+            vb.n[lane] = b4;
+            vb.s[lane] = make_uint4(vseed, flag, emit_candidates(b.scenes[scene], ld3(a4), ld3(b4), vseed), scene);
+            vb.entry[lane] = base + lane;
+          }
+          __syncwarp();
         }
+        const bool need = !have && !exhausted;
+        const uint32_t nmask = __ballot_sync(FULL, need);
+        const uint32_t k = vb_next + __popc(nmask & lt);
+        vb_next = min(vb_next + (uint32_t)__popc(nmask), vb_count);
+        if (need && k < vb_count) {
+          const float4 a4 = vb.p[k], b4 = vb.n[k];
+          const uint4 s4 = vb.s[k];
+          entry = vb.entry[k];
+          s.r.ox = a4.x;
+          s.r.oy = a4.y;
+          s.r.oz = a4.z;
+          slot = __float_as_uint(a4.w);
+          N = ld3(b4);
+          mat_idx = __float_as_int(b4.w);
+          seed = s4.x;
+          stale = (int)s4.y;
+          cand = s4.z;
+          sc = b.scenes + s4.w;
+          tries = 0;
+          have = true;
+        }
+        __syncwarp();
       }
       if (!__any_sync(FULL, have)) break;
       // The next try of a vertex.  A ray that cannot reach an emitter can
@@ -570,42 +616,14 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
       // with the flag's emitter, a miss clears it); a ray that may reach one
       // is traced to its closest hit.
       //
-      // For the vertices whose flag is unset, the warp finds the next try
-      // that may reach an emitter together: the LCG jumps to the state
-      // before each later try, so lane j tests try `tries + j` of one
-      // vertex (a conservative test on the unnormalised draw), and the first
-      // lane that may (or the vertex's last try) sets where the vertex goes
-      // on.  The tries before it are passed over without their directions.
-      const bool search = have && !ray_active && !pending && stale < 0;
-      uint32_t smask = __ballot_sync(FULL, search);
+      // The next try of a vertex whose flag is unset is its next candidate:
+      // the LCG jumps over the tries before it.
       uint32_t skipped = 0;
-      while (smask) {
-        const int owner = __ffs(smask) - 1;
-        smask &= smask - 1;
-        const uint32_t s0 = __shfl_sync(FULL, seed, owner);
-        const uint32_t t0 = __shfl_sync(FULL, tries, owner);
-        const V3 po = v3(__shfl_sync(FULL, s.r.ox, owner), __shfl_sync(FULL, s.r.oy, owner),
-                         __shfl_sync(FULL, s.r.oz, owner));
-        const V3 no = v3(__shfl_sync(FULL, N.x, owner), __shfl_sync(FULL, N.y, owner), __shfl_sync(FULL, N.z, owner));
-        const SceneDev* so = (const SceneDev*)__shfl_sync(FULL, (unsigned long long)sc, owner);
-        const uint32_t t = t0 + (uint32_t)lane;
-        bool cand = t + 1 == (uint32_t)NEE_TRIES;
-        if (t + 1 < (uint32_t)NEE_TRIES) {
-          const uint2 j = s_jump[lane];
-          uint32_t st = j.x * s0 + j.y;
-          const float hx = rng11(st);
-          const float hy = rng11(st);
-          const float hz = rng11(st);
-          cand = emit_may_hit_draw(*so, po, no, hx, hy, hz);
-        }
-        // the vertex's last try is always a candidate, so a lane is found
-        const int first = __ffs(__ballot_sync(FULL, cand)) - 1;
-        if (lane == owner) {
-          const uint2 j = s_jump[first];
-          seed = j.x * seed + j.y;
-          tries = t0 + (uint32_t)first;
-          skipped = (uint32_t)first;
-        }
+      if (have && !ray_active && !pending && stale < 0) {
+        skipped = (uint32_t)__ffs((int)(cand >> tries)) - 1u;  // (the last try is always a candidate)
+        const uint2 j = s_jump[skipped];
+        seed = j.x * seed + j.y;
+        tries += skipped;
       }
       if (have && !ray_active && !pending) {
         const V3 p = v3(s.r.ox, s.r.oy, s.r.oz);
