@@ -389,8 +389,8 @@ __global__ void k_emit_of_prim(int32_t* m, uint32_t n, const int32_t* em, uint32
 // scene-wide indices).
 __global__ void k_emit_global_ids(float4* tris, uint32_t n, const int32_t* __restrict__ global) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int local = __float_as_int(tris[3ull * k].w);
-    tris[3ull * k].w = __int_as_float(global[local]);
+    float4& v0 = tris[(TRI_BYTES / 16) * (size_t)k];
+    v0.w = __int_as_float(global[__float_as_int(v0.w)]);
   }
 }
 

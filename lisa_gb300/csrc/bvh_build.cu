@@ -689,10 +689,24 @@ __device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restric
     node_box(cand[nc], a.vals, a.plo, a.phi, a.ilo, a.ihi, clo[nc], chi[nc]);
     ++nc;
   }
+  // internal children take the first slots
   uint32_t num_int = 0, num_tri = 0;
   for (int k = 0; k < nc; ++k) {
     const uint32_t cnt = sub_count(a, cand[k]);
-    if (cnt > 3u) ++num_int; else num_tri += cnt;
+    if (cnt <= 3u) {
+      num_tri += cnt;
+      continue;
+    }
+    const int j = (int)num_int++;
+    if (j == k) continue;
+    const uint32_t c = cand[k];
+    const float4 lo = clo[k], hi = chi[k];
+    cand[k] = cand[j];
+    clo[k] = clo[j];
+    chi[k] = chi[j];
+    cand[j] = c;
+    clo[j] = lo;
+    chi[j] = hi;
   }
   const uint32_t child_base = num_int ? atomicAdd(&a.counters[0], num_int) : 0u;
   const uint32_t tri_base = num_tri ? atomicAdd(&a.counters[1], num_tri) : 0u;
@@ -710,10 +724,9 @@ __device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restric
   const float ph[3] = {nhi.x, nhi.y, nhi.z};
   int e[3];
   for (int ax = 0; ax < 3; ++ax) e[ax] = grid_exponent((double)ph[ax] - (double)p[ax]);
-  uint8_t qlo[3][8], qhi[3][8], meta[8];
-  uint32_t imask = 0, rank = 0, toff = 0;
+  uint8_t qlo[3][8], qhi[3][8];
+  uint32_t leaves = 0, toff = 0;
   for (int k = 0; k < 8; ++k) {
-    meta[k] = 0;
     for (int ax = 0; ax < 3; ++ax) {
       qlo[ax][k] = 0;
       qhi[ax][k] = 0;
@@ -735,13 +748,10 @@ __device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restric
     }
     const uint32_t cnt = sub_count(a, cand[k]);
     if (cnt > 3u) {
-      imask |= 1u << k;
-      meta[k] = (uint8_t)rank;
       const uint32_t slot = atomicAdd(next_count, 1u);
-      next[slot] = make_uint2(child_base + rank, cand[k]);
-      ++rank;
+      next[slot] = make_uint2(child_base + (uint32_t)k, cand[k]);
     } else {
-      meta[k] = (uint8_t)((cnt << 5) | toff);
+      leaves |= ((1u << cnt) - 1u) << (3 * k);
       // the (at most 3) primitives below, left to right
       uint32_t leaves[3], st[4];
       int nlv = 0, sp = 0;
@@ -758,10 +768,11 @@ __device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restric
       for (uint32_t q = 0; q < cnt; ++q) {
         const uint32_t prim = a.vals[leaves[q]];
         const float* t = a.verts + 9ull * prim;
-        float4* o = a.tris + 3ull * (tri_base + toff + q);
+        float4* o = a.tris + (size_t)(TRI_BYTES / 16) * (tri_base + toff + q);
         o[0] = make_float4(t[0], t[1], t[2], __int_as_float((int)prim));
         o[1] = make_float4(t[3], t[4], t[5], __int_as_float(a.mats ? a.mats[prim] : 0));
         o[2] = make_float4(t[6], t[7], t[8], 0.0f);
+        o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
       toff += cnt;
     }
@@ -769,14 +780,14 @@ __device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restric
   auto pack4 = [](const uint8_t* b) {
     return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
   };
-  uint4* np = a.nodes + 5ull * dst;
-  np[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]),
-                     (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) | ((uint32_t)(e[2] + 127) << 16) |
-                         (imask << 24));
-  np[1] = make_uint4(child_base, tri_base, pack4(meta), pack4(meta + 4));
+  auto scale = [&](int ax) { return (uint32_t)(e[ax] + 127) << 23; };  // 2^e
+  uint4* np = a.nodes + (size_t)(NODE_BYTES / 16) * dst;
+  np[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), scale(0));
+  np[1] = make_uint4(scale(1), scale(2), child_base, tri_base);
   np[2] = make_uint4(pack4(qlo[0]), pack4(qlo[0] + 4), pack4(qlo[1]), pack4(qlo[1] + 4));
   np[3] = make_uint4(pack4(qlo[2]), pack4(qlo[2] + 4), pack4(qhi[0]), pack4(qhi[0] + 4));
   np[4] = make_uint4(pack4(qhi[1]), pack4(qhi[1] + 4), pack4(qhi[2]), pack4(qhi[2] + 4));
+  np[5] = make_uint4(leaves | (((1u << num_int) - 1u) << 24), 0u, 0u, 0u);
 }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -836,7 +847,16 @@ size_t bvh_temp_bytes(uint32_t n) {
   return (size_t)b;
 }
 
-size_t bvh_output_bytes(uint32_t n) { return (size_t)(al256(80ull * (n + 1)) + al256(48ull * n)); }
+// Most 8-wide nodes that n triangles can give.  A node with an internal
+// child has eight children (the collapse opens candidates until there are
+// eight or none is left to open), the others (T, below F such nodes) hold at
+// least four triangles; the F nodes' own leaves number 8 F - (F + T - 1), so
+// n >= 4 T + 7 F - T + 1 >= 3 (F + T) + 1.
+static uint32_t max_nodes(uint32_t n) { return n / 3 + 1; }
+
+size_t bvh_output_bytes(uint32_t n) {
+  return (size_t)(al256((uint64_t)NODE_BYTES * max_nodes(n)) + al256((uint64_t)TRI_BYTES * n));
+}
 
 Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
                  uint4** d_nodes, float4** d_tris, BvhBuildResult* info, const int32_t* d_mat, bool refine) {
@@ -906,8 +926,8 @@ Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource
   // outputs
   uint4* nodes = nullptr;
   float4* tris = nullptr;
-  LISA_TRY(take(out, &nodes, 5ull * (n + 1), "bvh nodes"));
-  LISA_TRY(take(out, &tris, 3ull * n, "bvh triangles"));
+  LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), "bvh nodes"));
+  LISA_TRY(take(out, &tris, (uint64_t)(TRI_BYTES / 16) * n, "bvh triangles"));
   const uint2 root = make_uint2(0u, n > 1 ? 0u : LEAF_BIT);
   k_collapse_init<<<1, 1, 0, s>>>(counters, levels, work0, root);
   LISA_CUDA(cudaGetLastError());

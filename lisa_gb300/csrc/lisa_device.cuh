@@ -2,19 +2,20 @@
 //
 // HBM layout of one scene (all arrays 16-byte aligned, read with 128-bit
 // loads):
-//   nodes  : 8-wide compressed BVH nodes, 80 B = 5 x uint4 each
-//              uint4 0: origin p.xyz (f32) | exponents ex,ey,ez (u8), imask (u8)
-//              uint4 1: child_base | tri_base | meta[0..3] | meta[4..7]
-//              uint4 2: qlo.x[8] | qlo.y[8]
-//              uint4 3: qlo.z[8] | qhi.x[8]
-//              uint4 4: qhi.y[8] | qhi.z[8]
-//            child box = p + 2^(e-127) * q (per axis); imask bit i marks an
-//            internal child at node child_base + meta[i]; a leaf child has
-//            meta[i] = count<<5 | offset (count 1..3 triangles at
-//            tri_base + offset); meta 0 and imask 0 = empty slot.
-//   tris   : 3 x float4 per leaf triangle slot, in leaf order:
+//   nodes  : 8-wide compressed BVH nodes, 96 B each, three 32-byte loads
+//              0: origin x, y, z | scale x | scale y, z | child_base | tri_base
+//              1: qlo.x[8] qlo.y[8] qlo.z[8] qhi.x[8] (bytes)
+//              2: qhi.y[8] qhi.z[8] | leaf triangles (24 bits), imask (8 bits) | 0 0 0
+//            child box = origin + scale * q (per axis; the scales are powers
+//            of two).  Internal children come first: imask = 2^k - 1 for k of
+//            them, at nodes child_base + slot.  Bit 3 c + q of the leaf
+//            triangles says that leaf child c has a q-th triangle (at most
+//            3); the node's triangles lie one after another from tri_base.
+//            An empty slot has none of these bits.
+//   tris   : 4 x float4 per leaf triangle slot, in leaf order:
 //            (v0.xyz, original triangle id as int bits),
-//            (v1, its material if that is an emitter, else -1), (v2, 0)
+//            (v1, its material if that is an emitter, else -1), (v2, 0), 0
+//            -- 64 B, so a triangle is a 32- and a 16-byte load
 //   prims  : 5 x float4 per original triangle (shading record):
 //            (v0, n0.x) (v1, n0.y) (v2, n0.z) (n1, n2.x) (n2.y, n2.z, mat, 0)
 //   mats   : DevMaterial, 48 B each
@@ -155,39 +156,35 @@ struct WaveCtrl {
 struct RayPre {
   float ox, oy, oz;
   float ix, iy, iz;  // 1/d per axis
-  uint32_t k;        // shear axes: kx | ky << 2 | kz << 4
+  float slack;       // absolute slack on the best distance, in t units
+};
+// The shear of the triangle test, along the axis kz of the largest |d|.
+struct RayShear {
   float Sx, Sy, Sz;
-  float slack;  // absolute slack on the best distance, in t units
-  __device__ __forceinline__ int kx() const { return (int)(k & 3u); }
-  __device__ __forceinline__ int ky() const { return (int)((k >> 2) & 3u); }
-  __device__ __forceinline__ int kz() const { return (int)((k >> 4) & 3u); }
+  int kz;
 };
 
-__device__ __forceinline__ float sel3(float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); }
+// Components of a vector on the shear's axes: kx = kz + 1, ky = kz + 2
+// (mod 3).  The published test swaps kx and ky for a negative d[kz] to keep
+// the winding; that negates U, V, W, det and T exactly (each is a
+// difference or a sum of products) and leaves t as it is, so here they stay.
+__device__ __forceinline__ float on_kx(float x, float y, float z, int kz) { return kz == 0 ? y : (kz == 1 ? z : x); }
+__device__ __forceinline__ float on_ky(float x, float y, float z, int kz) { return kz == 0 ? z : (kz == 1 ? x : y); }
+__device__ __forceinline__ float on_kz(float x, float y, float z, int kz) { return kz == 0 ? x : (kz == 1 ? y : z); }
 
-__device__ __forceinline__ RayPre ray_prepare(V3 o, V3 d, float extent) {
-  RayPre r;
+__device__ __forceinline__ void ray_prepare(V3 o, V3 d, float extent, RayPre& r, RayShear& h) {
   r.ox = o.x;
   r.oy = o.y;
   r.oz = o.z;
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-  int kz = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
-  int kx = kz + 1;
-  if (kx == 3) kx = 0;
-  int ky = kx + 1;
-  if (ky == 3) ky = 0;
-  const float dz = sel3(d.x, d.y, d.z, kz);
-  if (dz < 0.0f) {
-    const int t = kx;
-    kx = ky;
-    ky = t;
-  }
-  r.k = (uint32_t)kx | ((uint32_t)ky << 2) | ((uint32_t)kz << 4);
-  r.Sx = fdiv(sel3(d.x, d.y, d.z, kx), dz);
-  r.Sy = fdiv(sel3(d.x, d.y, d.z, ky), dz);
+  const int kz = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
+  const float dz = on_kz(d.x, d.y, d.z, kz);
+  h.kz = kz;
+  h.Sx = fdiv(on_kx(d.x, d.y, d.z, kz), dz);
+  h.Sy = fdiv(on_ky(d.x, d.y, d.z, kz), dz);
   // __frcp_rn is the correctly rounded 1/x, the same value as 1.0f/x: the
   // shear's 1/dz, and the node-culling reciprocal of that (dominant) axis
-  r.Sz = __frcp_rn(dz);
+  h.Sz = __frcp_rn(dz);
   // The other two axes' reciprocals serve node culling only; __fdividef is
   // within 2 ulp there, which the slab padding covers (see trav_node).  A
   // zero or vanishing component takes a huge finite reciprocal of its sign
@@ -197,28 +194,25 @@ __device__ __forceinline__ RayPre ray_prepare(V3 o, V3 d, float extent) {
   const float qx = ax > 1e-30f ? __fdividef(1.0f, d.x) : copysignf(1e30f, d.x);
   const float qy = ay > 1e-30f ? __fdividef(1.0f, d.y) : copysignf(1e30f, d.y);
   const float qz = az > 1e-30f ? __fdividef(1.0f, d.z) : copysignf(1e30f, d.z);
-  r.ix = kz == 0 ? r.Sz : qx;
-  r.iy = kz == 1 ? r.Sz : qy;
-  r.iz = kz == 2 ? r.Sz : qz;
+  r.ix = kz == 0 ? h.Sz : qx;
+  r.iy = kz == 1 ? h.Sz : qy;
+  r.iz = kz == 2 ? h.Sz : qz;
   // 2^-18 * extent / |d|max; a margin, so an approximate quotient will do
   r.slack = __fdividef(3.814697265625e-6f * extent, fmaxf(ax, fmaxf(ay, az)));
-  return r;
 }
 
 // Returns t of the hit (or +inf).  prim_t < tbest test is the caller's.
-__device__ __forceinline__ float intersect_tri(const RayPre& r, float4 a4, float4 b4, float4 c4, float tmin) {
+__device__ __forceinline__ float intersect_tri(V3 o, const RayShear& h, V3 va, V3 vb, V3 vc, float tmin) {
   // translate to the ray origin
-  const float ax_ = fsub(a4.x, r.ox), ay_ = fsub(a4.y, r.oy), az_ = fsub(a4.z, r.oz);
-  const float bx_ = fsub(b4.x, r.ox), by_ = fsub(b4.y, r.oy), bz_ = fsub(b4.z, r.oz);
-  const float cx_ = fsub(c4.x, r.ox), cy_ = fsub(c4.y, r.oy), cz_ = fsub(c4.z, r.oz);
-  const int kx = r.kx(), ky = r.ky(), kz = r.kz();
-  const float Akx = sel3(ax_, ay_, az_, kx), Aky = sel3(ax_, ay_, az_, ky), Akz = sel3(ax_, ay_, az_, kz);
-  const float Bkx = sel3(bx_, by_, bz_, kx), Bky = sel3(bx_, by_, bz_, ky), Bkz = sel3(bx_, by_, bz_, kz);
-  const float Ckx = sel3(cx_, cy_, cz_, kx), Cky = sel3(cx_, cy_, cz_, ky), Ckz = sel3(cx_, cy_, cz_, kz);
+  const V3 a = va - o, b = vb - o, c = vc - o;
+  const int kz = h.kz;
+  const float Akx = on_kx(a.x, a.y, a.z, kz), Aky = on_ky(a.x, a.y, a.z, kz), Akz = on_kz(a.x, a.y, a.z, kz);
+  const float Bkx = on_kx(b.x, b.y, b.z, kz), Bky = on_ky(b.x, b.y, b.z, kz), Bkz = on_kz(b.x, b.y, b.z, kz);
+  const float Ckx = on_kx(c.x, c.y, c.z, kz), Cky = on_ky(c.x, c.y, c.z, kz), Ckz = on_kz(c.x, c.y, c.z, kz);
   // shear
-  const float Axs = fsub(Akx, fmul(r.Sx, Akz)), Ays = fsub(Aky, fmul(r.Sy, Akz));
-  const float Bxs = fsub(Bkx, fmul(r.Sx, Bkz)), Bys = fsub(Bky, fmul(r.Sy, Bkz));
-  const float Cxs = fsub(Ckx, fmul(r.Sx, Ckz)), Cys = fsub(Cky, fmul(r.Sy, Ckz));
+  const float Axs = fsub(Akx, fmul(h.Sx, Akz)), Ays = fsub(Aky, fmul(h.Sy, Akz));
+  const float Bxs = fsub(Bkx, fmul(h.Sx, Bkz)), Bys = fsub(Bky, fmul(h.Sy, Bkz));
+  const float Cxs = fsub(Ckx, fmul(h.Sx, Ckz)), Cys = fsub(Cky, fmul(h.Sy, Ckz));
   // scaled barycentrics (edge functions)
   const float U = fsub(fmul(Cxs, Bys), fmul(Cys, Bxs));
   const float V = fsub(fmul(Axs, Cys), fmul(Ays, Cxs));
@@ -226,7 +220,7 @@ __device__ __forceinline__ float intersect_tri(const RayPre& r, float4 a4, float
   if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return __int_as_float(0x7f800000);
   const float det = fadd(fadd(U, V), W);
   if (det == 0.0f) return __int_as_float(0x7f800000);
-  const float Az = fmul(r.Sz, Akz), Bz = fmul(r.Sz, Bkz), Cz = fmul(r.Sz, Ckz);
+  const float Az = fmul(h.Sz, Akz), Bz = fmul(h.Sz, Bkz), Cz = fmul(h.Sz, Ckz);
   const float T = fadd(fadd(fmul(U, Az), fmul(V, Bz)), fmul(W, Cz));
   const float t = fdiv(T, det);
   if (!(t > tmin)) return __int_as_float(0x7f800000);
@@ -245,12 +239,19 @@ __device__ __forceinline__ float intersect_tri(const RayPre& r, float4 a4, float
 // Together with the lowest-index tie rule the result equals a brute-force
 // scan with the same triangle test.
 //
-// The traversal is resumable: trav_step() processes one node -- its eight
-// child boxes, then, in one flat loop, the triangles of the leaf children it
-// hit -- and moves to the nearest internal child, pushing the others sorted
-// by entry distance.  Kernels call it once per loop trip, so a lane whose
-// ray finished can start another ray while the rest of its warp is still
-// traversing.
+// The traversal is resumable: trav_step_warp() processes one node -- its
+// eight child boxes, then the triangles of the leaf children it hit -- and
+// moves to the nearest internal child, the others pushed sorted by entry
+// distance.  Kernels call it once per loop trip, so a lane whose ray finished
+// can start another ray while the rest of its warp is still traversing.
+//
+// What bounds it: issue slots, the ALU pipe above all (selects, byte
+// extraction, min/max), and the wavefronts of scattered loads through L1.
+// So a node is three 32-byte loads instead of five of 16, the boxes are
+// tested two at a time with packed FP32 operations, the hit children are
+// ordered in registers by their distance bits (the nearest never goes
+// through the stack), and the leaf triangles follow from the hit mask by a
+// bit spread.
 
 struct TraceScene {
   const uint4* nodes;
@@ -288,7 +289,30 @@ __device__ __forceinline__ TraceScene trace_scene_emit(const SceneDev& sc) {
   return t;
 }
 
-constexpr uint32_t NODE_NONE = 0xffffffffu;
+constexpr int NODE_BYTES = 96;
+constexpr int TRI_BYTES = 64;
+
+// 32 bytes of read-only global memory, 32-byte aligned, in one load.
+struct Words8 {
+  uint32_t v[8];
+};
+__device__ __forceinline__ Words8 load32(const void* p) {
+  Words8 w;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(w.v[0]), "=r"(w.v[1]), "=r"(w.v[2]), "=r"(w.v[3]), "=r"(w.v[4]), "=r"(w.v[5]), "=r"(w.v[6]), "=r"(w.v[7])
+      : "l"(p));
+  return w;
+}
+
+// Per-warp scratch of the traversal (shared memory): what a lane needs to
+// test another lane's triangle, and the exchange of the triangle passes.
+struct TriPass {
+  float4 ray0[32];             // origin xyz, tmin
+  float4 ray1[32];             // shear Sx, Sy, Sz, kz (int bits)
+  unsigned long long key[32];  // (t bits << 32 | triangle id) of each lane's best hit
+  unsigned long long list[32]; // address of the pass's j-th triangle | lane that asks for it
+  int mat[32];
+};
 
 struct TravState {
   RayPre r;
@@ -304,14 +328,17 @@ struct TravState {
   bool any;  // stop at the first non-emitter hit found (see trav_pop)
 };
 
-__device__ __forceinline__ float byte_f(uint32_t w, int b) { return (float)((w >> (8 * b)) & 0xffu); }
+// Byte k of w as the float 2^23 + byte (exact; subtract 2^23 for the value).
+__device__ __forceinline__ float byte_biased(uint32_t w, int k) {
+  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7650u | (uint32_t)k));
+}
 
 // Starts a ray; returns false when there is nothing to traverse (empty
 // scene or zero direction), in which case the ray is a miss.  With `any`
 // the traversal ends at the first hit it finds: best_prim then says only
 // whether the segment (tmin, tmax) is blocked.
 __device__ __forceinline__ bool trav_begin(TravState& s, const TraceScene& sc, V3 o, V3 d, float tmin, float tmax,
-                                           bool any = false) {
+                                           TriPass& tp, bool any = false) {
   s.any = any;
   s.best_t = tmax;
   s.cull = tmax;
@@ -320,21 +347,32 @@ __device__ __forceinline__ bool trav_begin(TravState& s, const TraceScene& sc, V
   s.sp = 0;
   s.node = 0;
   if (sc.num_nodes == 0 || is_zero(d)) return false;
-  s.r = ray_prepare(o, d, sc.extent);
+  RayShear h;
+  ray_prepare(o, d, sc.extent, s.r, h);
+  const int lane = threadIdx.x & 31;
+  tp.ray0[lane] = make_float4(o.x, o.y, o.z, tmin);
+  tp.ray1[lane] = make_float4(h.Sx, h.Sy, h.Sz, __int_as_float(h.kz));
   return true;
 }
 
 // One node of the traversal, in three parts.  trav_node tests the node's
-// eight child boxes, pushes the internal children it hits (with their entry
-// distances) and returns, as a bitmask over the node's triangle slots, the
-// triangles of the leaf children it hits.  The triangles are then tested,
-// by the lane itself (trav_tris) or by its warp (trav_tris_warp), and
-// trav_pop orders the pushed children and moves to the next node.
+// eight child boxes, finds the nearest internal child it hits, pushes the
+// others and returns the triangles of the leaf children it hits.  The
+// triangles are then tested by the warp (trav_tris_warp), and trav_pop moves
+// to the next node.
 struct NodeWork {
-  uint32_t tmask;     // triangle slots tri_base + bit index still to test
+  uint32_t tmask;     // the node's leaf triangles still to test, as bits 3 c + q
+  uint32_t leaves;    // all of the node's leaf triangles
   uint32_t tri_base;
-  int sp0;            // stack depth before this node's pushes
+  uint32_t next;      // the nearest internal child hit
+  float next_t;       // its entry distance (rounded down; NaN when there is none)
 };
+
+// Near and far distances of children c and c + 1 on one axis, packed.
+__device__ __forceinline__ float2 slab2(uint32_t w, int k, float s, float c) {
+  const float2 q = __fadd2_rn(make_float2(byte_biased(w, k), byte_biased(w, k + 1)), make_float2(-8388608.0f, -8388608.0f));
+  return __ffma2_rn(q, make_float2(s, s), make_float2(c, c));
+}
 
 template <bool COUNT>
 __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc, uint2* stack, uint32_t& visits,
@@ -343,85 +381,84 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
 #ifdef LISA_BOUNDS
   if (s.node >= sc.num_nodes) {  // end the ray
     if (status) atomicOr(status, ST_BOUNDS);
-    NodeWork bad;
-    bad.tmask = 0;
-    bad.tri_base = 0;
-    bad.sp0 = 0;
     s.sp = 0;
-    return bad;
+    return NodeWork{0u, 0u, 0u, 0u, __int_as_float(0x7fffffff)};
   }
 #endif
   if (COUNT) ++visits;
-  const uint4* np = sc.nodes + 5ull * s.node;
-  const uint4 n0 = __ldg(np + 0);
-  const uint4 n1 = __ldg(np + 1);
-  const uint4 n2 = __ldg(np + 2);
-  const uint4 n3 = __ldg(np + 3);
-  const uint4 n4 = __ldg(np + 4);
-  const float sx = __int_as_float((n0.w & 0xffu) << 23) * r.ix;
-  const float sy = __int_as_float(((n0.w >> 8) & 0xffu) << 23) * r.iy;
-  const float sz = __int_as_float(((n0.w >> 16) & 0xffu) << 23) * r.iz;
-  const float cx = (__uint_as_float(n0.x) - r.ox) * r.ix;
-  const float cy = (__uint_as_float(n0.y) - r.oy) * r.iy;
-  const float cz = (__uint_as_float(n0.z) - r.oz) * r.iz;
-  const float gx = 9.5367431640625e-7f * (fabsf(cx) + 255.0f * fabsf(sx));
-  const float gy = 9.5367431640625e-7f * (fabsf(cy) + 255.0f * fabsf(sy));
-  const float gz = 9.5367431640625e-7f * (fabsf(cz) + 255.0f * fabsf(sz));
-  const float cnx = cx - gx, cfx = cx + gx;
-  const float cny = cy - gy, cfy = cy + gy;
-  const float cnz = cz - gz, cfz = cz + gz;
+  const char* np = (const char*)sc.nodes + (size_t)NODE_BYTES * s.node;
+  const Words8 A = load32(np), B = load32(np + 32), C = load32(np + 64);
+  const float sx = __uint_as_float(A.v[3]) * r.ix, sy = __uint_as_float(A.v[4]) * r.iy,
+              sz = __uint_as_float(A.v[5]) * r.iz;
+  const float cx = (__uint_as_float(A.v[0]) - r.ox) * r.ix;
+  const float cy = (__uint_as_float(A.v[1]) - r.oy) * r.iy;
+  const float cz = (__uint_as_float(A.v[2]) - r.oz) * r.iz;
+  const float gx = fmaf(255.0f, fabsf(sx), fabsf(cx));
+  const float gy = fmaf(255.0f, fabsf(sy), fabsf(cy));
+  const float gz = fmaf(255.0f, fabsf(sz), fabsf(cz));
+  constexpr float PAD = 9.5367431640625e-7f;
+  const float cnx = fmaf(-PAD, gx, cx), cfx = fmaf(PAD, gx, cx);
+  const float cny = fmaf(-PAD, gy, cy), cfy = fmaf(PAD, gy, cy);
+  const float cnz = fmaf(-PAD, gz, cz), cfz = fmaf(PAD, gz, cz);
   const bool negx = r.ix < 0.0f, negy = r.iy < 0.0f, negz = r.iz < 0.0f;
-  const uint32_t nx0 = negx ? n3.z : n2.x, nx1 = negx ? n3.w : n2.y;
-  const uint32_t fx0 = negx ? n2.x : n3.z, fx1 = negx ? n2.y : n3.w;
-  const uint32_t ny0 = negy ? n4.x : n2.z, ny1 = negy ? n4.y : n2.w;
-  const uint32_t fy0 = negy ? n2.z : n4.x, fy1 = negy ? n2.w : n4.y;
-  const uint32_t nz0 = negz ? n4.z : n3.x, nz1 = negz ? n4.w : n3.y;
-  const uint32_t fz0 = negz ? n3.x : n4.z, fz1 = negz ? n3.y : n4.w;
-  const uint32_t imask = n0.w >> 24;
-  const uint32_t child_base = n1.x;
-  NodeWork w;
-  w.tri_base = n1.y;
-  // child boxes: hit mask; internal children that are hit go straight onto
-  // the stack with their entry distance (predicated stores, no branches)
-  uint32_t hit = 0;
-  w.sp0 = s.sp;
-  int sp = w.sp0;
+  const uint32_t nx[2] = {negx ? B.v[6] : B.v[0], negx ? B.v[7] : B.v[1]};
+  const uint32_t fx[2] = {negx ? B.v[0] : B.v[6], negx ? B.v[1] : B.v[7]};
+  const uint32_t ny[2] = {negy ? C.v[0] : B.v[2], negy ? C.v[1] : B.v[3]};
+  const uint32_t fy[2] = {negy ? B.v[2] : C.v[0], negy ? B.v[3] : C.v[1]};
+  const uint32_t nz[2] = {negz ? C.v[2] : B.v[4], negz ? C.v[3] : B.v[5]};
+  const uint32_t fz[2] = {negz ? B.v[4] : C.v[2], negz ? B.v[5] : C.v[3]};
+  const uint32_t imask = C.v[4] >> 24;
+  // hit mask, and a sort key per internal child that is hit: its entry
+  // distance (positive, so the bits order as the float) with the slot in the
+  // low three bits, which rounds the distance down
+  uint32_t hit = 0, key[8];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const int b = c & 3;
-    const float a0 = fmaf(byte_f(c < 4 ? nx0 : nx1, b), sx, cnx);
-    const float a1 = fmaf(byte_f(c < 4 ? ny0 : ny1, b), sy, cny);
-    const float a2 = fmaf(byte_f(c < 4 ? nz0 : nz1, b), sz, cnz);
-    const float f0 = fmaf(byte_f(c < 4 ? fx0 : fx1, b), sx, cfx);
-    const float f1 = fmaf(byte_f(c < 4 ? fy0 : fy1, b), sy, cfy);
-    const float f2 = fmaf(byte_f(c < 4 ? fz0 : fz1, b), sz, cfz);
-    const float tn = fmaxf(fmaxf(a0, a1), fmaxf(a2, s.tmin));
-    const float tf = fminf(fminf(f0, f1), fminf(f2, s.cull));
-    const bool h = tn <= tf;
-    hit |= (h ? 1u : 0u) << c;
-    if (h && ((imask >> c) & 1u) && sp < TRAV_STACK) {
-      const uint32_t meta = ((c < 4 ? n1.z : n1.w) >> (8 * b)) & 0xffu;
-      stack[sp++] = make_uint2(child_base + meta, __float_as_uint(tn));
+  for (int p = 0; p < 4; ++p) {
+    const int w = p >> 1, k = 2 * (p & 1);
+    const float2 a0 = slab2(nx[w], k, sx, cnx), a1 = slab2(ny[w], k, sy, cny), a2 = slab2(nz[w], k, sz, cnz);
+    const float2 f0 = slab2(fx[w], k, sx, cfx), f1 = slab2(fy[w], k, sy, cfy), f2 = slab2(fz[w], k, sz, cfz);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = 2 * p + j;
+      const float tn = fmaxf(fmaxf(fmaxf(j ? a0.y : a0.x, j ? a1.y : a1.x), j ? a2.y : a2.x), s.tmin);
+      const float tf = fminf(fminf(fminf(j ? f0.y : f0.x, j ? f1.y : f1.x), j ? f2.y : f2.x), s.cull);
+      const bool h = tn <= tf;
+      if (h) hit |= 1u << c;
+      key[c] = (h && ((imask >> c) & 1u)) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)c) : 0xffffffffu;
     }
   }
-  if (status && (imask & hit) && sp == TRAV_STACK && __popc(imask & hit) > sp - w.sp0)
-    atomicOr(status, ST_STACK_OVERFLOW);
-  s.sp = sp;
-  // occupied slots: internal children and leaves with a non-zero meta byte
-  uint32_t leafmask = 0;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) leafmask |= ((((c < 4 ? n1.z : n1.w) >> (8 * (c & 3))) & 0xe0u) ? 1u : 0u) << c;
-  leafmask &= ~imask & hit;
-  // triangles of the hit leaves, as a bitmask over the node's triangle slots
-  w.tmask = 0;
-  while (leafmask) {
-    const int c = __ffs(leafmask) - 1;
-    leafmask &= leafmask - 1;
-    const uint32_t meta = ((c < 4 ? n1.z : n1.w) >> (8 * (c & 3))) & 0xffu;
-    w.tmask |= ((1u << (meta >> 5)) - 1u) << (meta & 31u);
+  uint32_t k = min(min(min(key[0], key[1]), min(key[2], key[3])), min(min(key[4], key[5]), min(key[6], key[7])));
+  const uint32_t child_base = A.v[6];
+  NodeWork w;
+  w.next = child_base + (k & 7u);
+  w.next_t = __uint_as_float(k & ~7u);
+  const int n = __popc(imask & hit);
+  if (n > 1) {
+    // the others, farthest first: the next larger key is the smallest of
+    // key - (k + 1) in unsigned arithmetic
+    const int sp0 = s.sp;
+    int at = sp0 + n - 2;
+    s.sp = at + 1;
+    if (s.sp > TRAV_STACK) {
+      if (status) atomicOr(status, ST_STACK_OVERFLOW);
+      s.sp = TRAV_STACK;
+    }
+    for (; at >= sp0; --at) {
+      const uint32_t o = k + 1u;
+      k = o + min(min(min(key[0] - o, key[1] - o), min(key[2] - o, key[3] - o)),
+                  min(min(key[4] - o, key[5] - o), min(key[6] - o, key[7] - o)));
+      if (at < TRAV_STACK) stack[at] = make_uint2(child_base + (k & 7u), k & ~7u);
+    }
   }
+  // bit c of the hit mask to bits 3 c .. 3 c + 2
+  uint32_t m = (hit | (hit << 8)) & 0x00f00fu;
+  m = (m | (m << 4)) & 0x0c30c3u;
+  m = (m | (m << 2)) & 0x249249u;
+  w.leaves = C.v[4] & 0xffffffu;
+  w.tmask = (m * 7u) & w.leaves;
+  w.tri_base = A.v[7];
 #ifdef LISA_BOUNDS
-  if (w.tmask && w.tri_base + (31u - (uint32_t)__clz(w.tmask)) >= sc.num_tris) {
+  if (w.tmask && w.tri_base + (uint32_t)__popc(w.leaves) > sc.num_tris) {
     if (status) atomicOr(status, ST_BOUNDS);
     w.tmask = 0;
   }
@@ -429,123 +466,112 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
   return w;
 }
 
-// Keeps the hit (t, prim) if it is nearer, or as near with a lower
-// triangle index (the brute-force tie rule).
-__device__ __forceinline__ void trav_take(TravState& s, float t, int prim, int mat) {
-  if (t < s.best_t || (t == s.best_t && prim < s.best_prim)) {
-    s.best_t = t;
-    s.best_prim = prim;
-    s.best_mat = mat;
-    s.cull = fmaf(t, 1.52587890625e-5f, t) + s.r.slack;
-  }
+// Address of the leaf triangle at the lowest bit of w.tmask.
+__device__ __forceinline__ const char* first_tri(const TraceScene& sc, const NodeWork& w) {
+  const uint32_t low = w.tmask & (0u - w.tmask);
+  return (const char*)sc.tris + (size_t)TRI_BYTES * (w.tri_base + (uint32_t)__popc(w.leaves & (low - 1u)));
 }
 
-// The lane tests its own triangles.
+// Tests the triangle at p with the ray (r0, r1) of TriPass.
+__device__ __forceinline__ float test_tri(const char* p, float4 r0, float4 r1, int& prim, int& mat) {
+  const Words8 t = load32(p);
+  const float4 c = __ldg((const float4*)(p + 32));
+  prim = (int)t.v[3];
+  mat = (int)t.v[7];
+  const RayShear h{r1.x, r1.y, r1.z, __float_as_int(r1.w)};
+  return intersect_tri(ld3(r0), h, v3(__uint_as_float(t.v[0]), __uint_as_float(t.v[1]), __uint_as_float(t.v[2])),
+                       v3(__uint_as_float(t.v[4]), __uint_as_float(t.v[5]), __uint_as_float(t.v[6])), ld3(c), r0.w);
+}
+
+// The lane tests its own triangles; keeps a hit if it is nearer, or as near
+// with a lower triangle index (the brute-force tie rule).
 template <bool COUNT>
-__device__ __forceinline__ void trav_tris(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests) {
+__device__ __forceinline__ void trav_tris(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests,
+                                          const TriPass& tp) {
+  const int lane = threadIdx.x & 31;
   while (w.tmask) {
-    const int j = __ffs(w.tmask) - 1;
-    w.tmask &= w.tmask - 1;
-    const float4* tp = sc.tris + 3ull * (w.tri_base + (uint32_t)j);
-    const float4 a = __ldg(tp + 0), bb = __ldg(tp + 1), cc = __ldg(tp + 2);
+    int prim, mat;
+    const float t = test_tri(first_tri(sc, w), tp.ray0[lane], tp.ray1[lane], prim, mat);
+    w.tmask &= w.tmask - 1u;
     if (COUNT) ++tests;
-    trav_take(s, intersect_tri(s.r, a, bb, cc, s.tmin), __float_as_int(a.w), __float_as_int(bb.w));
+    if (t < s.best_t || (t == s.best_t && prim < s.best_prim)) {
+      s.best_t = t;
+      s.best_prim = prim;
+      s.best_mat = mat;
+      s.cull = fmaf(t, 1.52587890625e-5f, t) + s.r.slack;
+    }
   }
 }
 
-// Per-warp scratch of trav_tris_warp (shared memory).
-struct TriPass {
-  unsigned long long key[32];  // (t bits << 32 | triangle id) of each lane's best hit
-  int mat[32];
-  int owner[32];               // lane whose triangles start at this position of a pass
-};
-
-// The warp tests the triangles of all its lanes together, 32 at a time:
-// the lanes' triangle lists are laid end to end (a prefix sum of their
-// counts) and lane j of a pass takes the j-th triangle of the pass, with
-// the owner's ray.  The owner's best hit is the minimum of the 64-bit keys
-// (t, triangle id) -- t is positive, so its bits order as the float -- the
-// same choice as the lane's own loop with its tie rule.  Called by all 32
-// lanes; lanes without a ray pass w.tmask = 0.
-template <bool COUNT>
+// The warp tests the triangles of all its lanes together, 32 at a time: the
+// lanes' triangles are laid end to end (a prefix sum of their counts), each
+// lane writes the addresses of its own into the pass's list, and lane j
+// takes the j-th with the asking lane's ray.  That lane's best hit is the
+// minimum of the 64-bit keys (t, triangle id) -- t is positive, so its bits
+// order as the float -- the same choice as the lane's own loop with its tie
+// rule.  Called by all 32 lanes; lanes without a ray pass w.tmask = 0.  MAT:
+// the hit's emitter material is wanted too.
+template <bool COUNT, bool MAT>
 __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests,
                                                TriPass& tp) {
   const int lane = threadIdx.x & 31;
   const uint32_t cnt = __popc(w.tmask);
-  uint32_t incl = cnt;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+  if (most == 0) return;
+  uint32_t incl = cnt, total = 0;
+  if (most > 1) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    total = __shfl_sync(0xffffffffu, incl, 31);
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  if (total == 0) return;
   // when no lane has more triangles than the passes a warp would need,
   // the lanes' own loops are cheaper than the exchange
-  if (__reduce_max_sync(0xffffffffu, cnt) <= ((total + 31u) >> 5)) {
-    if (cnt) trav_tris<COUNT>(s, sc, w, tests);
+  if (most <= 1 || most <= ((total + 31u) >> 5)) {
+    trav_tris<COUNT>(s, sc, w, tests, tp);
     return;
   }
-  const uint32_t excl = incl - cnt;
+  uint32_t pos = incl - cnt;
   const unsigned long long key0 =
       ((unsigned long long)__float_as_uint(s.best_t) << 32) | (uint32_t)s.best_prim;
   tp.key[lane] = key0;
   for (uint32_t k0 = 0; k0 < total; k0 += 32) {
-    // positions of this pass where a lane's list starts (the list holding
-    // position 0 starts there too)
-    const bool here = cnt && excl < k0 + 32 && excl + cnt > k0;
-    const uint32_t pos = excl > k0 ? excl - k0 : 0u;
-    if (here) tp.owner[pos] = lane;
-    const uint32_t starts = __reduce_or_sync(0xffffffffu, here ? 1u << pos : 0u);
+    while (w.tmask && pos < k0 + 32u) {
+      tp.list[pos - k0] = (unsigned long long)first_tri(sc, w) | (uint32_t)lane;
+      w.tmask &= w.tmask - 1u;
+      ++pos;
+    }
     __syncwarp();
-    const uint32_t k = k0 + (uint32_t)lane;
-    // the list holding position `lane`: the last start at or below it
-    const int first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
-    const int o = tp.owner[first];
-    const uint32_t o_excl = __shfl_sync(0xffffffffu, excl, o);
-    uint32_t m = __shfl_sync(0xffffffffu, w.tmask, o);
-    const uint32_t o_base = __shfl_sync(0xffffffffu, w.tri_base, o);
-    RayPre r;
-    r.ox = __shfl_sync(0xffffffffu, s.r.ox, o);
-    r.oy = __shfl_sync(0xffffffffu, s.r.oy, o);
-    r.oz = __shfl_sync(0xffffffffu, s.r.oz, o);
-    r.k = __shfl_sync(0xffffffffu, s.r.k, o);
-    r.Sx = __shfl_sync(0xffffffffu, s.r.Sx, o);
-    r.Sy = __shfl_sync(0xffffffffu, s.r.Sy, o);
-    r.Sz = __shfl_sync(0xffffffffu, s.r.Sz, o);
-    const float tmin = __shfl_sync(0xffffffffu, s.tmin, o);
-    const unsigned long long tris_p = __shfl_sync(0xffffffffu, (unsigned long long)sc.tris, o);
-    const unsigned long long okey = __shfl_sync(0xffffffffu, key0, o);
     bool better = false;
     unsigned long long key = 0;
-    int mat = 0;
-    if (k < total) {
-      // the (k - o_excl)-th remaining triangle of the owner's list
-      for (uint32_t i = k - o_excl; i > 0; --i) m &= m - 1;
-      const uint32_t j = (uint32_t)(__ffs(m) - 1);
-      const float4* tq = (const float4*)tris_p + 3ull * (o_base + j);
-      const float4 a = __ldg(tq + 0), bb = __ldg(tq + 1), cc = __ldg(tq + 2);
+    int mat = 0, o = 0;
+    if (k0 + (uint32_t)lane < total) {
+      const unsigned long long e = tp.list[lane];
+      o = (int)(e & 31u);
+      int prim;
+      const float t = test_tri((const char*)(e & ~31ull), tp.ray0[o], tp.ray1[o], prim, mat);
       if (COUNT) ++tests;
-      const float t = intersect_tri(r, a, bb, cc, tmin);
-      const int prim = __float_as_int(a.w);
+      const unsigned long long okey = *(volatile unsigned long long*)&tp.key[o];
       const float bt = __uint_as_float((uint32_t)(okey >> 32));
-      const int bp = (int)(uint32_t)okey;
-      if (t < bt || (t == bt && prim < bp)) {
+      if (t < bt || (t == bt && prim < (int)(uint32_t)okey)) {
         better = true;
         key = ((unsigned long long)__float_as_uint(t) << 32) | (uint32_t)prim;
-        mat = __float_as_int(bb.w);
         atomicMin(&tp.key[o], key);
       }
     }
     __syncwarp();
-    if (better && tp.key[o] == key) tp.mat[o] = mat;
-    __syncwarp();
+    if (MAT) {
+      if (better && tp.key[o] == key) tp.mat[o] = mat;
+      __syncwarp();
+    }
   }
   const unsigned long long best = tp.key[lane];
   if (best != key0) {
     s.best_t = __uint_as_float((uint32_t)(best >> 32));
     s.best_prim = (int)(uint32_t)best;
-    s.best_mat = tp.mat[lane];
+    if (MAT) s.best_mat = tp.mat[lane];
     s.cull = fmaf(s.best_t, 1.52587890625e-5f, s.best_t) + s.r.slack;
   }
   __syncwarp();
@@ -654,25 +680,17 @@ __device__ __forceinline__ bool box_may_hit_exact(V3 o, V3 d, const float* lo, c
   return tn <= tf;
 }
 
-// Orders the children trav_node pushed by entry distance (nearest on top)
-// and moves to the nearest child not culled.  Returns true when the
-// traversal is finished.
-__device__ __forceinline__ bool trav_pop(TravState& s, uint2* stack, int sp0) {
+// Moves to the nearest child not culled: the node's own, else the stack's
+// top.  Returns true when the traversal is finished.
+__device__ __forceinline__ bool trav_pop(TravState& s, uint2* stack, const NodeWork& w) {
   // an any-hit traversal ends at its first hit that is not an emitter's (a
   // ray that cannot reach an emitter only finds such hits; the emitter
   // search's scene pass starts from an emitter hit and looks for a nearer
   // triangle, which cannot be an emitter's)
   if (s.any && s.best_prim >= 0 && s.best_mat < 0) return true;
-  // (entry distances are positive, so their bit patterns order as floats)
-  const int sp = s.sp;
-  for (int i = sp0 + 1; i < sp; ++i) {
-    const uint2 e = stack[i];
-    int k = i;
-    while (k > sp0 && stack[k - 1].y < e.y) {
-      stack[k] = stack[k - 1];
-      --k;
-    }
-    stack[k] = e;
+  if (w.next_t <= s.cull) {
+    s.node = w.next;
+    return false;
   }
   while (s.sp > 0) {
     const uint2 e = stack[--s.sp];
@@ -684,43 +702,17 @@ __device__ __forceinline__ bool trav_pop(TravState& s, uint2* stack, int sp0) {
   return true;
 }
 
-// Processes one node with the lane's own triangle loop.  Returns true when
-// the traversal is finished (s.best_prim / s.best_t hold the result,
-// best_prim -1 on a miss).
-template <bool COUNT>
-__device__ __forceinline__ bool trav_step(TravState& s, const TraceScene& sc, uint2* stack, uint32_t& visits,
-                                          uint32_t& tests, uint32_t* status) {
-  const NodeWork w = trav_node<COUNT>(s, sc, stack, visits, status);
-  trav_tris<COUNT>(s, sc, w, tests);
-  return trav_pop(s, stack, w.sp0);
-}
-
-// The same step for a whole warp (all 32 lanes call it), the triangles
-// tested by trav_tris_warp.  Returns true for an active lane whose
-// traversal is finished; inactive lanes get false.
-template <bool COUNT>
+// Processes one node for each active lane of a warp (all 32 lanes call it).
+// Returns true for an active lane whose traversal is finished (s.best_prim /
+// s.best_t hold the result, best_prim -1 on a miss); inactive lanes get
+// false.
+template <bool COUNT, bool MAT>
 __device__ __forceinline__ bool trav_step_warp(bool active, TravState& s, const TraceScene& sc, uint2* stack,
                                                uint32_t& visits, uint32_t& tests, uint32_t* status, TriPass& tp) {
-  NodeWork w;
-  w.tmask = 0;
-  w.tri_base = 0;
-  w.sp0 = 0;
+  NodeWork w{0u, 0u, 0u, 0u, 0.0f};
   if (active) w = trav_node<COUNT>(s, sc, stack, visits, status);
-  trav_tris_warp<COUNT>(s, sc, w, tests, tp);
-  return active && trav_pop(s, stack, w.sp0);
-}
-
-template <bool COUNT>
-__device__ __forceinline__ void closest_hit(const TraceScene& sc, V3 o, V3 d, float tmin, float tmax, int& out_prim,
-                                            float& out_t, uint32_t& visits, uint32_t& tests, uint32_t* status) {
-  TravState s;
-  uint2 stack[TRAV_STACK];
-  if (trav_begin(s, sc, o, d, tmin, tmax)) {
-    while (!trav_step<COUNT>(s, sc, stack, visits, tests, status)) {
-    }
-  }
-  out_prim = s.best_prim;
-  out_t = s.best_prim >= 0 ? s.best_t : __int_as_float(0x7f800000);
+  trav_tris_warp<COUNT, MAT>(s, sc, w, tests, tp);
+  return active && trav_pop(s, stack, w);
 }
 
 // Brute-force scan in original triangle order with the same test and tie
@@ -730,13 +722,15 @@ __device__ __forceinline__ void brute_hit(const SceneDev& sc, V3 o, V3 d, float 
   out_prim = -1;
   out_t = __int_as_float(0x7f800000);
   if (is_zero(d)) return;
-  const RayPre r = ray_prepare(o, d, sc.extent);
+  RayPre r;
+  RayShear h;
+  ray_prepare(o, d, sc.extent, r, h);
   float best_t = tmax;
   int best = -1;
   for (uint32_t p = 0; p < sc.num_prims; ++p) {
     const float4* pr = sc.prims + 5ull * p;
     const float4 a = __ldg(pr + 0), b = __ldg(pr + 1), c = __ldg(pr + 2);
-    const float t = intersect_tri(r, a, b, c, tmin);
+    const float t = intersect_tri(o, h, ld3(a), ld3(b), ld3(c), tmin);
     if (t < best_t) {
       best_t = t;
       best = (int)p;

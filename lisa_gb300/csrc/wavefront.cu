@@ -256,7 +256,7 @@ __global__ void LISA_TRACE_BOUNDS k_trace(WaveBufs b, int depth) {
           if (ray < count) {
             const float4 o = b.ro[q][ray], d = b.rd[q][ray];
             ts = trace_scene(b.scenes[__float_as_uint(d.w)]);
-            active = trav_begin(s, ts, ld3(o), ld3(d), RAY_TMIN, RAY_TMAX);
+            active = trav_begin(s, ts, ld3(o), ld3(d), RAY_TMIN, RAY_TMAX, tp);
             if (!active) b.hit[ray] = make_int2(-1, 0x7f800000);
           } else {
             exhausted = true;
@@ -265,7 +265,7 @@ __global__ void LISA_TRACE_BOUNDS k_trace(WaveBufs b, int depth) {
       }
       if (!__any_sync(FULL, active || !exhausted)) break;
     }
-    if (trav_step_warp<COUNT>(active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
+    if (trav_step_warp<COUNT, false>(active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
       b.hit[ray] = make_int2(s.best_prim, s.best_prim >= 0 ? __float_as_int(s.best_t) : 0x7f800000);
       active = false;
     }
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
           const float te = s.best_t;
           const int pe = s.best_prim, me = s.best_mat;
           ts = trace_scene(*sc);
-          ray_active = trav_begin(s, ts, v3(s.r.ox, s.r.oy, s.r.oz), dir, RAY_TMIN, RAY_TMAX);
+          ray_active = trav_begin(s, ts, v3(s.r.ox, s.r.oy, s.r.oz), dir, RAY_TMIN, RAY_TMAX, tp);
           s.best_t = te;
           s.best_prim = pe;
           s.best_mat = me;
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
           // triangles; with a few, the bounds test above is as selective)
           emit_pass = stale < 0 && sc->num_etris >= EMIT_BVH_MIN_TRIS;
           ts = emit_pass ? trace_scene_emit(*sc) : trace_scene(*sc);
-          ray_active = trav_begin(s, ts, p, dir, RAY_TMIN, RAY_TMAX);
+          ray_active = trav_begin(s, ts, p, dir, RAY_TMIN, RAY_TMAX, tp);
           if (ray_active) {
             s.any = !capable;
             ++walked;
@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
         }
       }
     }
-    if (trav_step_warp<COUNT>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
+    if (trav_step_warp<COUNT, true>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
       ray_active = false;
       pending = true;
     }
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs
                 shadow = true;
                 ++nshadow;
                 // stop short of the emitter itself; any blocker will do
-                ray_active = trav_begin(s, ts, p, wi, RAY_TMIN, fmul(dist, 0.9990234375f), true);
+                ray_active = trav_begin(s, ts, p, wi, RAY_TMIN, fmul(dist, 0.9990234375f), tp, true);
               }
             }
             pending = !ray_active;  // no shadow ray, or nothing to traverse
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs
       }
       if (!__any_sync(FULL, have)) break;
     }
-    if (trav_step_warp<COUNT>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
+    if (trav_step_warp<COUNT, true>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
       ray_active = false;
       pending = true;
     }
@@ -1175,10 +1175,10 @@ __global__ void __launch_bounds__(128) k_trace_rays(const SceneDev* __restrict__
     bool active = false;
     if (i < n) {
       const float* r = rays + 8ull * i;
-      active = trav_begin(s, ts, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), r[3], r[7]);
+      active = trav_begin(s, ts, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), r[3], r[7], tp);
     }
     while (__any_sync(FULL, active))
-      if (trav_step_warp<COUNT>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) active = false;
+      if (trav_step_warp<COUNT, false>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) active = false;
     if (i < n) {
       if (prim) prim[i] = s.best_prim;
       if (tout) tout[i] = s.best_prim >= 0 ? s.best_t : __int_as_float(0x7f800000);
