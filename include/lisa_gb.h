@@ -107,7 +107,10 @@ typedef struct lisa_options {
   uint32_t blocks_per_sm;    /* persistent-kernel residency (0 = auto)         */
   uint32_t threads_per_block;/* persistent-kernel block size (0 = auto)        */
   uint32_t use_graph;        /* capture each launch sequence in a CUDA graph   */
-  uint32_t stage_timing;     /* record CUDA events around every stage launch   */
+  uint32_t stage_timing;     /* record CUDA events around every stage launch (small
+                                waves then run stage by stage too; otherwise they
+                                run whole paths in one kernel, counted among the
+                                trace launches)                               */
   uint32_t accum_fp64;       /* also accumulate the pixel mean in FP64         */
   float aperture;            /* thin-lens aperture radius; 0 = pinhole (ref.)  */
   float focal_distance;      /* 0 = |look_at - eye|                            */

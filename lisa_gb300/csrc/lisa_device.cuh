@@ -443,6 +443,7 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
       if (status) atomicOr(status, ST_STACK_OVERFLOW);
       s.sp = TRAV_STACK;
     }
+#pragma unroll 1
     for (; at >= sp0; --at) {
       const uint32_t o = k + 1u;
       k = o + min(min(min(key[0] - o, key[1] - o), min(key[2] - o, key[3] - o)),
@@ -483,34 +484,15 @@ __device__ __forceinline__ float test_tri(const char* p, float4 r0, float4 r1, i
                        v3(__uint_as_float(t.v[4]), __uint_as_float(t.v[5]), __uint_as_float(t.v[6])), ld3(c), r0.w);
 }
 
-// The lane tests its own triangles; keeps a hit if it is nearer, or as near
-// with a lower triangle index (the brute-force tie rule).
-template <bool COUNT>
-__device__ __forceinline__ void trav_tris(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests,
-                                          const TriPass& tp) {
-  const int lane = threadIdx.x & 31;
-  while (w.tmask) {
-    int prim, mat;
-    const float t = test_tri(first_tri(sc, w), tp.ray0[lane], tp.ray1[lane], prim, mat);
-    w.tmask &= w.tmask - 1u;
-    if (COUNT) ++tests;
-    if (t < s.best_t || (t == s.best_t && prim < s.best_prim)) {
-      s.best_t = t;
-      s.best_prim = prim;
-      s.best_mat = mat;
-      s.cull = fmaf(t, 1.52587890625e-5f, t) + s.r.slack;
-    }
-  }
-}
-
-// The warp tests the triangles of all its lanes together, 32 at a time: the
-// lanes' triangles are laid end to end (a prefix sum of their counts), each
-// lane writes the addresses of its own into the pass's list, and lane j
-// takes the j-th with the asking lane's ray.  That lane's best hit is the
-// minimum of the 64-bit keys (t, triangle id) -- t is positive, so its bits
-// order as the float -- the same choice as the lane's own loop with its tie
-// rule.  Called by all 32 lanes; lanes without a ray pass w.tmask = 0.  MAT:
-// the hit's emitter material is wanted too.
+// Tests the triangles of all lanes of the warp, up to 32 at a time.  Either
+// each lane its own, one per pass (when that takes no more passes), or the
+// lanes' triangles laid end to end (a prefix sum of their counts): each lane
+// writes the addresses of its own into the pass's list, and lane j takes the
+// j-th with the asking lane's ray.  A lane's best hit is the minimum of the
+// 64-bit keys (t, triangle id) -- t is positive, so its bits order as the
+// float -- which is the brute-force tie rule.  Called by all 32 lanes; lanes
+// without a ray pass w.tmask = 0.  MAT: the hit's emitter material is wanted
+// too.
 template <bool COUNT, bool MAT>
 __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests,
                                                TriPass& tp) {
@@ -527,29 +509,36 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
     }
     total = __shfl_sync(0xffffffffu, incl, 31);
   }
-  // when no lane has more triangles than the passes a warp would need,
-  // the lanes' own loops are cheaper than the exchange
-  if (most <= 1 || most <= ((total + 31u) >> 5)) {
-    trav_tris<COUNT>(s, sc, w, tests, tp);
-    return;
-  }
+  const bool own = most <= 1 || most <= ((total + 31u) >> 5);
   uint32_t pos = incl - cnt;
   const unsigned long long key0 =
       ((unsigned long long)__float_as_uint(s.best_t) << 32) | (uint32_t)s.best_prim;
   tp.key[lane] = key0;
-  for (uint32_t k0 = 0; k0 < total; k0 += 32) {
-    while (w.tmask && pos < k0 + 32u) {
-      tp.list[pos - k0] = (unsigned long long)first_tri(sc, w) | (uint32_t)lane;
+  const uint32_t passes = own ? most : (total + 31u) >> 5;
+#pragma unroll 1
+  for (uint32_t k = 0; k < passes; ++k) {
+    unsigned long long e = 0;
+    bool test;
+    if (own) {
+      test = w.tmask != 0u;
+      e = (unsigned long long)first_tri(sc, w) | (uint32_t)lane;
       w.tmask &= w.tmask - 1u;
-      ++pos;
+    } else {
+#pragma unroll 1
+      while (w.tmask && pos < 32u * k + 32u) {
+        tp.list[pos - 32u * k] = (unsigned long long)first_tri(sc, w) | (uint32_t)lane;
+        w.tmask &= w.tmask - 1u;
+        ++pos;
+      }
+      __syncwarp();
+      test = 32u * k + (uint32_t)lane < total;
+      if (test) e = tp.list[lane];
     }
-    __syncwarp();
     bool better = false;
     unsigned long long key = 0;
-    int mat = 0, o = 0;
-    if (k0 + (uint32_t)lane < total) {
-      const unsigned long long e = tp.list[lane];
-      o = (int)(e & 31u);
+    int mat = 0;
+    const int o = (int)(e & 31u);
+    if (test) {
       int prim;
       const float t = test_tri((const char*)(e & ~31ull), tp.ray0[o], tp.ray1[o], prim, mat);
       if (COUNT) ++tests;
@@ -611,50 +600,61 @@ __device__ __forceinline__ bool emit_may_hit(const SceneDev& sc, V3 o, V3 d) {
   return box_may_hit(r, sc.emit_lo, sc.emit_hi, RAY_TMIN, RAY_TMAX);
 }
 
-// The tries of a vertex's emitter search that may reach an emitter, as a bit
-// mask (bit j = try j; `seed` is the stream's state before try 0).  Try j is
-// the hemisphere draw q = (x, y, z) of shoot_ray_hemisphere, not normalised:
-// the exact direction is a positive multiple of q, flipped by the sign of
+// Bounds of the scene's emissive triangles relative to a vertex: centre c,
+// half extent h, grown by 2^-19 of |c| + |h|.
+struct EmitBounds {
+  V3 c, h;
+};
+__device__ __forceinline__ EmitBounds emit_bounds(const SceneDev& sc, V3 o) {
+  const float lx = sc.emit_lo[0] - o.x, ly = sc.emit_lo[1] - o.y, lz = sc.emit_lo[2] - o.z;
+  const float ux = sc.emit_hi[0] - o.x, uy = sc.emit_hi[1] - o.y, uz = sc.emit_hi[2] - o.z;
+  EmitBounds e;
+  e.c = v3(0.5f * (lx + ux), 0.5f * (ly + uy), 0.5f * (lz + uz));
+  const float hx = 0.5f * (ux - lx), hy = 0.5f * (uy - ly), hz = 0.5f * (uz - lz);
+  const float pad = 1.9073486328125e-6f * (((fabsf(e.c.x) + fabsf(e.c.y)) + fabsf(e.c.z)) + ((hx + hy) + hz));
+  e.h = v3(hx + pad, hy + pad, hz + pad);
+  return e;
+}
+
+// Whether the next try of a vertex's emitter search may reach an emitter
+// (`seed` is the stream's state before it, advanced past it).  The try is the
+// hemisphere draw q = (x, y, z) of shoot_ray_hemisphere, not normalised: the
+// exact direction is a positive multiple of q, flipped by the sign of
 // dot(N, q), each component with one more rounding.  A try is left out when
 // its line misses the padded bounds of the emissive triangles (one of the
 // three cross-product axes separates them; the axes do not depend on the
 // flip) or when all of the bounds lie behind the ray; where dot(N, q) is too
-// near zero for its sign to be certain, only the line is tested.  The bounds
-// relative to the origin (centre c, half extent h) grow by 2^-19 of |c| + |h|,
-// four times the roundings of c, h, the products and the direction.  Every
-// comparison rejects on a definite answer, so a NaN leaves the try in.  The
-// last try always stays: the search ends there.
+// near zero for its sign to be certain, only the line is tested.  The
+// bounds' padding is four times the roundings of c, h, the products and the
+// direction.  Every comparison rejects on a definite answer, so a NaN leaves
+// the try in.
 //
 // Divisions would cost more than the rest of the test (three reciprocals and
-// their guards a try); the separating axes need none: about 40 instructions a
-// try, all lanes busy, for a vertex of their own each.
+// their guards a try); the separating axes need none: about 40 instructions.
+__device__ __forceinline__ bool emit_candidate(const EmitBounds& e, V3 N, uint32_t& seed) {
+  const float x = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+  const float y = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+  const float z = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
+  const float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
+  const bool off = fabsf(fmaf(y, e.c.z, -(z * e.c.y))) > fmaf(e.h.y, az, e.h.z * ay) ||
+                   fabsf(fmaf(z, e.c.x, -(x * e.c.z))) > fmaf(e.h.z, ax, e.h.x * az) ||
+                   fabsf(fmaf(x, e.c.y, -(y * e.c.x))) > fmaf(e.h.x, ay, e.h.y * ax);
+  const float s = fmaf(N.x, x, fmaf(N.y, y, N.z * z));
+  const float f = fmaf(e.c.x, x, fmaf(e.c.y, y, e.c.z * z));
+  const bool behind = fabsf(s) > 1e-5f * ((ax + ay) + az) &&
+                      copysignf(1.0f, s) * f < -fmaf(e.h.x, ax, fmaf(e.h.y, ay, e.h.z * az));
+  return !off && !behind;
+}
+
+// All tries of a vertex, as a bit mask (bit j = try j; `seed` is the state
+// before try 0).  The last try always stays: the search ends there.
 __device__ __forceinline__ uint32_t emit_candidates(const SceneDev& sc, V3 o, V3 N, uint32_t seed) {
-  constexpr uint32_t LAST = 1u << (NEE_TRIES - 1);
-  if (!sc.has_emit_box) return LAST;
-  const float lx = sc.emit_lo[0] - o.x, ly = sc.emit_lo[1] - o.y, lz = sc.emit_lo[2] - o.z;
-  const float ux = sc.emit_hi[0] - o.x, uy = sc.emit_hi[1] - o.y, uz = sc.emit_hi[2] - o.z;
-  const float cx = 0.5f * (lx + ux), cy = 0.5f * (ly + uy), cz = 0.5f * (lz + uz);
-  float hx = 0.5f * (ux - lx), hy = 0.5f * (uy - ly), hz = 0.5f * (uz - lz);
-  const float pad = 1.9073486328125e-6f * (((fabsf(cx) + fabsf(cy)) + fabsf(cz)) + ((hx + hy) + hz));
-  hx += pad;
-  hy += pad;
-  hz += pad;
-  uint32_t mask = LAST;
+  uint32_t mask = 1u << (NEE_TRIES - 1);
+  if (!sc.has_emit_box) return mask;
+  const EmitBounds e = emit_bounds(sc, o);
 #pragma unroll 2
-  for (int j = 0; j < NEE_TRIES - 1; ++j) {
-    const float x = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
-    const float y = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
-    const float z = fmaf((float)lcg(seed), 1.1920928955078125e-7f, -1.0f);
-    const float ax = fabsf(x), ay = fabsf(y), az = fabsf(z);
-    const bool off = fabsf(fmaf(y, cz, -(z * cy))) > fmaf(hy, az, hz * ay) ||
-                     fabsf(fmaf(z, cx, -(x * cz))) > fmaf(hz, ax, hx * az) ||
-                     fabsf(fmaf(x, cy, -(y * cx))) > fmaf(hx, ay, hy * ax);
-    const float s = fmaf(N.x, x, fmaf(N.y, y, N.z * z));
-    const float e = fmaf(cx, x, fmaf(cy, y, cz * z));
-    const bool behind = fabsf(s) > 1e-5f * ((ax + ay) + az) &&
-                        copysignf(1.0f, s) * e < -fmaf(hx, ax, fmaf(hy, ay, hz * az));
-    if (!off && !behind) mask |= 1u << j;
-  }
+  for (int j = 0; j < NEE_TRIES - 1; ++j)
+    if (emit_candidate(e, N, seed)) mask |= 1u << j;
   return mask;
 }
 
@@ -692,6 +692,7 @@ __device__ __forceinline__ bool trav_pop(TravState& s, uint2* stack, const NodeW
     s.node = w.next;
     return false;
   }
+#pragma unroll 1
   while (s.sp > 0) {
     const uint2 e = stack[--s.sp];
     if (__uint_as_float(e.y) <= s.cull) {

@@ -63,6 +63,12 @@ constexpr uint32_t FULL = 0xffffffffu;
 #ifndef LISA_NEE_PB_MIN_BLOCKS
 #define LISA_NEE_PB_MIN_BLOCKS 7  // physically based emitter kernel: 7 x 128 threads per SM
 #endif
+#ifndef LISA_PATHS_MIN_BLOCKS
+#define LISA_PATHS_MIN_BLOCKS 5  // whole-path kernel: 5 x 128 threads per SM (96 registers; best of 4..6)
+#endif
+#ifndef LISA_PATHS_REFILL_IDLE
+#define LISA_PATHS_REFILL_IDLE 20  // idle lanes that trigger a round of k_paths (best of 8, 12, .. 28: its rounds are long)
+#endif
 #ifndef LISA_REFILL_IDLE
 #define LISA_REFILL_IDLE 12  // default: idle lanes (of 32) that trigger a refill round
 #endif
@@ -149,8 +155,53 @@ __device__ __forceinline__ int find_group(const WaveDesc& w, uint32_t key, bool 
 }
 
 // ---------------------------------------------------------------------------
-// raygen (shader.cu:126-152) -- also resets the counters of depth 0
+// raygen (shader.cu:126-152)
 
+// Scene, pixel, stream state and camera ray of the wave's path `slot`
+// (shader.cu:126-152).
+__device__ __forceinline__ void camera_ray(const WaveBufs& b, const WaveDesc& w, uint32_t slot, uint32_t& scene,
+                                           uint32_t& pix, uint32_t& seed, V3& org, V3& dir) {
+  const WaveGroup& g = w.groups[find_group(w, slot, false)];
+  const SceneDev& sc = b.scenes[g.scene];
+  const uint32_t off = slot - g.slot0;
+  const uint32_t m = off / g.npix;
+  scene = g.scene;
+  pix = g.pix0 + (off - m * g.npix);
+  const uint32_t sample = g.sample0 + m;
+  const uint32_t x = pix % sc.width, y = pix / sc.width;
+  if (w.rng_mode == LISA_RNG_PER_PIXEL) {
+    seed = sc.pix_rng[pix];
+  } else {
+    seed = tea<16>(pix, tea<4>(sample, w.seed));
+  }
+  const float jx = rng11(seed);
+  const float jy = rng11(seed);
+  const float dx = fsub(fdiv(fadd(fmul(2.0f, (float)x), jx), (float)sc.width), 1.0f);
+  const float dy = fsub(fdiv(fadd(fmul(2.0f, (float)y), jy), (float)sc.height), 1.0f);
+  const V3 U = v3(sc.U[0], sc.U[1], sc.U[2]), V = v3(sc.V[0], sc.V[1], sc.V[2]), W = v3(sc.W[0], sc.W[1], sc.W[2]);
+  dir = normalize((dx * U + dy * V) + W);
+  org = v3(sc.eye[0], sc.eye[1], sc.eye[2]);
+  if (sc.lens_radius > 0.0f) {
+    // Thin lens (not in the reference, whose camera is a pinhole): the
+    // pinhole ray meets the focal plane at distance focal_distance along
+    // the view axis; the origin moves to a uniform point of the lens disk,
+    // drawn by rejection from the square (trig-free, so the oracle draws
+    // the same point bit for bit).
+    const V3 wu = v3(sc.unitW[0], sc.unitW[1], sc.unitW[2]);
+    const float tf = fdiv(sc.focal_distance, dot(dir, wu));
+    const V3 focus = org + tf * dir;
+    float lu, lv;
+    do {
+      lu = rng11(seed);
+      lv = rng11(seed);
+    } while (fadd(fmul(lu, lu), fmul(lv, lv)) > 1.0f);
+    org = org + fmul(sc.lens_radius, lu) * v3(sc.unitU[0], sc.unitU[1], sc.unitU[2]) +
+          fmul(sc.lens_radius, lv) * v3(sc.unitV[0], sc.unitV[1], sc.unitV[2]);
+    dir = normalize(focus - org);
+  }
+}
+
+// One path per slot; also resets the counters of depth 0.
 __global__ void k_raygen(WaveBufs b, const WaveDesc* __restrict__ wave) {
   const WaveDesc& w = *wave;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -167,50 +218,15 @@ __global__ void k_raygen(WaveBufs b, const WaveDesc* __restrict__ wave) {
     b.ctrl->rays_primary += w.paths;
   }
   for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < w.paths; slot += gridDim.x * blockDim.x) {
-    const WaveGroup& g = w.groups[find_group(w, slot, false)];
-    const SceneDev& sc = b.scenes[g.scene];
-    const uint32_t off = slot - g.slot0;
-    const uint32_t m = off / g.npix;
-    const uint32_t pix = g.pix0 + (off - m * g.npix);
-    const uint32_t sample = g.sample0 + m;
-    const uint32_t x = pix % sc.width, y = pix / sc.width;
-    uint32_t seed;
-    if (w.rng_mode == LISA_RNG_PER_PIXEL) {
-      seed = sc.pix_rng[pix];
-    } else {
-      seed = tea<16>(pix, tea<4>(sample, w.seed));
-    }
-    const float jx = rng11(seed);
-    const float jy = rng11(seed);
-    const float dx = fsub(fdiv(fadd(fmul(2.0f, (float)x), jx), (float)sc.width), 1.0f);
-    const float dy = fsub(fdiv(fadd(fmul(2.0f, (float)y), jy), (float)sc.height), 1.0f);
-    const V3 U = v3(sc.U[0], sc.U[1], sc.U[2]), V = v3(sc.V[0], sc.V[1], sc.V[2]), W = v3(sc.W[0], sc.W[1], sc.W[2]);
-    V3 dir = normalize((dx * U + dy * V) + W);
-    V3 org = v3(sc.eye[0], sc.eye[1], sc.eye[2]);
-    if (sc.lens_radius > 0.0f) {
-      // Thin lens (not in the reference, whose camera is a pinhole): the
-      // pinhole ray meets the focal plane at distance focal_distance along
-      // the view axis; the origin moves to a uniform point of the lens disk,
-      // drawn by rejection from the square (trig-free, so the oracle draws
-      // the same point bit for bit).
-      const V3 wu = v3(sc.unitW[0], sc.unitW[1], sc.unitW[2]);
-      const float tf = fdiv(sc.focal_distance, dot(dir, wu));
-      const V3 focus = org + tf * dir;
-      float lu, lv;
-      do {
-        lu = rng11(seed);
-        lv = rng11(seed);
-      } while (fadd(fmul(lu, lu), fmul(lv, lv)) > 1.0f);
-      org = org + fmul(sc.lens_radius, lu) * v3(sc.unitU[0], sc.unitU[1], sc.unitU[2]) +
-            fmul(sc.lens_radius, lv) * v3(sc.unitV[0], sc.unitV[1], sc.unitV[2]);
-      dir = normalize(focus - org);
-    }
+    uint32_t scene, pix, seed;
+    V3 org, dir;
+    camera_ray(b, w, slot, scene, pix, seed, org, dir);
     b.ro[0][slot] = make_float4(org.x, org.y, org.z, __uint_as_float(slot));
-    b.rd[0][slot] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(g.scene));
+    b.rd[0][slot] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(scene));
     // w: the stale emitter flag (compat, -1 = none) or the pdf of the last
     // diffuse bounce (physically based, 0 = camera or specular)
     b.ps_att[slot] = make_float4(1.0f, 1.0f, 1.0f, b.physical ? 0.0f : __int_as_float(-1));
-    b.ps_col[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float((g.scene << 24) | pix));
+    b.ps_col[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float((scene << 24) | pix));
     b.ps_rng[slot] = seed;
   }
 }
@@ -279,6 +295,61 @@ __global__ void LISA_TRACE_BOUNDS k_trace(WaveBufs b, int depth) {
 // ---------------------------------------------------------------------------
 // shade: emitter / miss / dielectric / opaque (shader.cu:189-194,211-255)
 
+// What an emitter hit adds to a path: Le * throughput (shader.cu:216-218),
+// weighted in the physically based estimator when a diffuse bounce of density
+// att.w reached it (power heuristic against the emitter sampler's density
+// for this direction).
+template <bool PHYS>
+__device__ __forceinline__ V3 emitter_hit(const SceneDev& sc, const DevMaterial& m, int prim, float t, V3 d,
+                                          float4 att) {
+  V3 le = v3(m.emission[0], m.emission[1], m.emission[2]) * ld3(att);
+  if (PHYS && att.w > 0.0f) {
+    const float prev = att.w;
+    const float4* pr = sc.prims + 5ull * prim;
+    const V3 v0 = ld3(pr[0]);
+    const V3 cr = cross3(ld3(pr[1]) - v0, ld3(pr[2]) - v0);
+    const V3 n = cr * fdiv(1.0f, fsqrt(dot(cr, cr)));
+    const float cos_y = fabsf(dot(n, d));
+    float w = 0.0f;
+    if (cos_y > 0.0f) {
+      const float pl = fdiv(fmul(m.light_pdf, fmul(t, t)), cos_y);
+      w = fdiv(fmul(prev, prev), fadd(fmul(prev, prev), fmul(pl, pl)));
+    }
+    le = le * w;
+  }
+  return le;
+}
+
+// Continuation at a dielectric hit with shading normal N (shader.cu:226-247):
+// the direction (zero on total internal reflection in the reference
+// estimator, a miss), the throughput a and the stream updated.
+template <bool PHYS>
+__device__ __forceinline__ V3 dielectric_bounce(const DevMaterial& m, V3 d, V3 N, V3& a, uint32_t& seed) {
+  float cosI = dot(d, N);
+  float eta;
+  V3 nrm;
+  if (cosI < 0.0f) {
+    cosI = -cosI;
+    eta = fdiv(1.0f, m.ior);
+    nrm = N;
+  } else {
+    a = a * v3(m.albedo[0], m.albedo[1], m.albedo[2]);
+    eta = m.ior;
+    nrm = -N;
+  }
+  if (eta == 1.0f) return d;
+  if (PHYS) {
+    // total internal reflection reflects; Schlick's term takes the cosine on
+    // the less dense side (the transmitted one on exit)
+    const float cost2 = fsub(1.0f, fmul(fmul(eta, eta), fsub(1.0f, fmul(cosI, cosI))));
+    if (cost2 <= 0.0f) return reflect(d, nrm);
+    if (rnd(seed) <= bsdf::BTDF(eta > 1.0f ? fsqrt(cost2) : cosI, eta)) return reflect(d, nrm);
+    return bsdf::refract(cosI, d, nrm, eta);
+  }
+  if (rnd(seed) <= bsdf::BTDF(cosI, eta)) return reflect(d, nrm);
+  return bsdf::refract(cosI, d, nrm, eta);
+}
+
 template <bool PHYS>
 __global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
   const int q = depth & 1;
@@ -306,26 +377,8 @@ __global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
         const DevMaterial& m = sc.mats[mat_idx];
         float4 att = b.ps_att[slot];
         if (m.cls == MAT_EMIT) {
-          // color += Le * att; done (shader.cu:216-218)
           const float4 col = b.ps_col[slot];
-          V3 le = v3(m.emission[0], m.emission[1], m.emission[2]) * ld3(att);
-          if (PHYS && att.w > 0.0f) {
-            // reached by a diffuse bounce: power-heuristic weight against
-            // the emitter sampler's density for this direction
-            const float prev = att.w;
-            const float t = __int_as_float(h.y);
-            const float4* pr = sc.prims + 5ull * h.x;
-            const V3 v0 = ld3(pr[0]);
-            const V3 cr = cross3(ld3(pr[1]) - v0, ld3(pr[2]) - v0);
-            const V3 n = cr * fdiv(1.0f, fsqrt(dot(cr, cr)));
-            const float cos_y = fabsf(dot(n, ld3(d4)));
-            float w = 0.0f;
-            if (cos_y > 0.0f) {
-              const float pl = fdiv(fmul(m.light_pdf, fmul(t, t)), cos_y);
-              w = fdiv(fmul(prev, prev), fadd(fmul(prev, prev), fmul(pl, pl)));
-            }
-            le = le * w;
-          }
+          const V3 le = emitter_hit<PHYS>(sc, m, h.x, __int_as_float(h.y), ld3(d4), att);
           const V3 c = ld3(col) + le;
           b.ps_col[slot] = make_float4(c.x, c.y, c.z, col.w);
         } else if (!PHYS || depth < (int)sc.num_bounces) {
@@ -339,39 +392,9 @@ __global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
           // based one also the ray leaving its last vertex
           const bool last = !PHYS && depth + 1 >= (int)sc.num_bounces;
           if (m.cls == MAT_DIELECTRIC) {
-            float cosI = dot(d, N);
-            float eta;
-            V3 nrm;
             V3 a = ld3(att);
-            if (cosI < 0.0f) {
-              cosI = -cosI;
-              eta = fdiv(1.0f, m.ior);
-              nrm = N;
-            } else {
-              a = a * v3(m.albedo[0], m.albedo[1], m.albedo[2]);
-              eta = m.ior;
-              nrm = -N;
-            }
             uint32_t seed = b.ps_rng[slot];
-            if (eta == 1.0f) {
-              nd = d;
-            } else if (PHYS) {
-              // total internal reflection reflects; Schlick's term takes the
-              // cosine on the less dense side (the transmitted one on exit)
-              const float cost2 = fsub(1.0f, fmul(fmul(eta, eta), fsub(1.0f, fmul(cosI, cosI))));
-              if (cost2 <= 0.0f) {
-                nd = reflect(d, nrm);
-              } else if (rnd(seed) <= bsdf::BTDF(eta > 1.0f ? fsqrt(cost2) : cosI, eta)) {
-                nd = reflect(d, nrm);
-              } else {
-                nd = bsdf::refract(cosI, d, nrm, eta);
-              }
-            } else if (rnd(seed) <= bsdf::BTDF(cosI, eta)) {
-              nd = reflect(d, nrm);
-            } else {
-              // a zero direction (total internal reflection) is traced as a miss
-              nd = bsdf::refract(cosI, d, nrm, eta);
-            }
+            nd = dielectric_bounce<PHYS>(m, d, N, a, seed);
             b.ps_rng[slot] = seed;
             b.ps_att[slot] = make_float4(a.x, a.y, a.z, PHYS ? 0.0f : att.w);
             want_ray = !last && !is_zero(nd);
@@ -1007,10 +1030,300 @@ __global__ void __launch_bounds__(INFER_THREADS, INFER_BLOCKS_PER_SM) k_guided_i
 }
 
 // ---------------------------------------------------------------------------
+// whole paths in one kernel (plain sampling, small waves)
+//
+// A lane takes a path from camera to end: closest hit, shading, emitter
+// search and bounce, depth after depth, advancing one BVH node per loop trip
+// like the stage kernels, whose routines it calls in the same order -- the
+// paths are the same bit for bit.  Nothing passes through memory but the
+// path's final radiance.
+//
+// For small waves, whose time is the latency of the stages and not their
+// throughput: each stage launch ends with the wave's longest ray (up to a
+// hundred node visits of about a microsecond), and a frame is a chain of
+// three such launches per depth.  Here a path waits only for itself: a
+// 160 x 90 preview of the Cornell box takes 182 us instead of 397, a
+// 333 x 217 frame in eight one-sample waves 3.4 ms instead of 8.0.  It is
+// bound by issue (58 % of the slots) and by instruction fetch: the loop is
+// 42 KB of code, so a routine is written once and shared by the ray kinds
+// (two more copies of trav_begin and of the triangle test cost 10 %).
+template <bool PHYS>
+__global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b, const WaveDesc* __restrict__ wave,
+                                                                      uint32_t lanes) {
+  const WaveDesc& w = *wave;
+  const uint32_t count = w.paths;
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = lanemask_lt();
+  uint2 stack[TRAV_STACK];
+  TravState s;
+  TraceScene ts;
+  const SceneDev* sc = nullptr;
+  // a lane with a path traces a radiance ray, or (shadow) an emitter-search
+  // ray from the vertex p; its ray's origin is s.r.o
+  bool have = false, exhausted = (uint32_t)lane >= lanes, ray_active = false, pending = false, shadow = false;
+  bool emit_pass = false;  // the finished traversal was of the emitters' own BVH
+  uint32_t slot = 0, seed = 0, cand = 0;
+  int depth = 0, tries = 0, mat_idx = 0;
+  int stale = -1;             // reference estimator: stale emitter flag
+  float pdf = 0.0f;           // physically based: density of the last diffuse bounce
+  int em_m = 0;               // physically based: the sampled emitter's material, density and cosine
+  float pl = 0.0f, cos_x = 0.0f;
+  V3 att = v3(0.0f), col = v3(0.0f);
+  V3 N = v3(0.0f), D = v3(0.0f), dir = v3(0.0f);  // normal; radiance ray; current ray
+  s.r.ox = s.r.oy = s.r.oz = 0.0f;
+  uint32_t nbounce = 0, nshadow = 0, nwalked = 0, nvertex = 0;
+  uint32_t visits = 0, tests = 0;
+  __shared__ uint2 s_jump[32];
+  if (threadIdx.x < 32) {
+    const LcgJump j = lcg_jump(3u * threadIdx.x);
+    s_jump[threadIdx.x] = make_uint2(j.a, j.c);
+  }
+  __syncthreads();
+  __shared__ TriPass tri_pass[4];
+  TriPass& tp = tri_pass[threadIdx.x >> 5];
+  while (true) {
+    const uint32_t busy = __ballot_sync(FULL, ray_active);
+    if (__popc(busy) <= (int)b.refill_busy_max) {
+      bool vertex = false;   // a new opaque vertex
+      bool search = false;   // a vertex that needs its next try (reference estimator)
+      bool leave = false;    // a vertex whose emitter search is over: draw the bounce
+      bool lit = false, start = false, over = false;
+      bool nearer = false;   // look for a triangle nearer than the emitter hit
+      float tmax = RAY_TMAX;
+      V3 p = v3(s.r.ox, s.r.oy, s.r.oz);
+      if (pending && shadow) {
+        pending = false;
+        if (PHYS) {
+          lit = s.best_prim < 0;
+          leave = true;
+        } else if (emit_pass && s.best_prim >= 0) {
+          // the emitters' BVH gave the nearest emitter on the ray: the scene's
+          // keeps it unless a triangle is nearer (see k_nee)
+          emit_pass = false;
+          nearer = true;
+          start = true;
+        } else {
+          emit_pass = false;
+          // the occlusion programs: a hit marks only an emitter and otherwise
+          // leaves the flag as it was, a miss clears it (shader.cu:172-184)
+          if (s.best_prim < 0) stale = -1;
+          else if (s.best_mat >= 0) stale = s.best_mat;
+          lit = stale >= 0;
+          leave = lit || ++tries == NEE_TRIES;
+          search = !leave;
+        }
+      } else if (pending) {
+        pending = false;
+        over = true;
+        const int prim = s.best_prim;
+        if (prim >= 0) {  // a miss adds the background, 0, and ends the path
+          mat_idx = prim_material(*sc, prim);
+          const DevMaterial& m = sc->mats[mat_idx];
+          if (m.cls == MAT_EMIT) {
+            col = col + emitter_hit<PHYS>(*sc, m, prim, s.best_t, D, make_float4(att.x, att.y, att.z, pdf));
+          } else if (!PHYS || depth < (int)sc->num_bounces) {
+            p = p + s.best_t * D;
+            N = barycentric_normal(p, sc->prims + 5ull * prim);
+            if (m.cls == MAT_DIELECTRIC) {
+              const V3 nd = dielectric_bounce<PHYS>(m, D, N, att, seed);
+              if (PHYS) pdf = 0.0f;
+              start = (PHYS || depth + 1 < (int)sc->num_bounces) && !is_zero(nd);
+              if (PHYS && start && depth + 1 == (int)sc->num_bounces) start = final_ray_wanted(*sc, p, nd);
+              over = !start;
+              D = nd;
+            } else {
+              att = att * v3(m.albedo[0], m.albedo[1], m.albedo[2]);
+              over = false;
+              vertex = true;
+              ++nvertex;
+            }
+          }
+        }
+      }
+      if (PHYS) {
+        if (vertex) {
+          N = dot(N, D) < 0.0f ? N : -N;  // faces the incoming ray
+          leave = true;
+          if (sc->mats[mat_idx].roughness > 0.0f && sc->num_emit > 0) {
+            V3 y;
+            const uint32_t k = sample_emitter(*sc, seed, y);
+            const V3 to = y - p;
+            const float d2 = dot(to, to);
+            const float dist = fsqrt(d2);
+            dir = to * fdiv(1.0f, dist);
+            cos_x = dot(N, dir);
+            const float cos_y = fabsf(dot(ld3(__ldg(sc->emit + 4ull * k + 3)), dir));
+            if (cos_x > 0.0f && cos_y > 0.0f && dist > 0.0f) {
+              pl = fdiv(fmul(__ldg(sc->emit + 4ull * k).w, d2), cos_y);
+              em_m = __float_as_int(__ldg(sc->emit + 4ull * k + 1).w);
+              ++nshadow;
+              // stop short of the emitter itself; any blocker will do
+              tmax = fmul(dist, 0.9990234375f);
+              shadow = true;
+              start = true;
+              leave = false;
+            }
+          }
+        }
+      } else {
+        // the tries of each new vertex that may reach an emitter: lane j
+        // tests try j of one vertex after another
+        uint32_t vmask = __ballot_sync(FULL, vertex);
+        if (vmask) {
+          const EmitBounds e = vertex ? emit_bounds(*sc, p) : EmitBounds{};
+          while (vmask) {
+            const int owner = __ffs(vmask) - 1;
+            vmask &= vmask - 1;
+            EmitBounds o;
+            o.c = v3(__shfl_sync(FULL, e.c.x, owner), __shfl_sync(FULL, e.c.y, owner), __shfl_sync(FULL, e.c.z, owner));
+            o.h = v3(__shfl_sync(FULL, e.h.x, owner), __shfl_sync(FULL, e.h.y, owner), __shfl_sync(FULL, e.h.z, owner));
+            const V3 on = v3(__shfl_sync(FULL, N.x, owner), __shfl_sync(FULL, N.y, owner), __shfl_sync(FULL, N.z, owner));
+            const uint2 j = s_jump[lane];
+            uint32_t st = j.x * __shfl_sync(FULL, seed, owner) + j.y;
+            const uint32_t mask = __ballot_sync(FULL, emit_candidate(o, on, st));
+            if (lane == owner) cand = mask;
+          }
+          if (vertex) {
+            cand = (sc->has_emit_box ? cand & ((1u << (NEE_TRIES - 1)) - 1u) : 0u) | (1u << (NEE_TRIES - 1));
+            tries = 0;
+            shadow = true;
+            search = true;
+          }
+        }
+        // The next try that is traced (see k_nee): with the flag unset, tries
+        // that cannot reach an emitter are only counted.
+        while (search) {
+          if (stale < 0) {
+            const uint32_t skip = (uint32_t)__ffs((int)(cand >> tries)) - 1u;  // (the last try is always a candidate)
+            const uint2 j = s_jump[skip];
+            seed = j.x * seed + j.y;
+            tries += (int)skip;
+            nshadow += skip;
+          }
+          ++nshadow;
+          const float hx = rng11(seed);
+          const float hy = rng11(seed);
+          const float hz = rng11(seed);
+          dir = bsdf::hemisphere_direction(N, hx, hy, hz);
+          const bool capable = emit_may_hit(*sc, p, dir);
+          if (!capable && stale < 0) {
+            leave = ++tries == NEE_TRIES;
+            search = !leave;
+          } else {
+            emit_pass = stale < 0 && sc->num_etris >= EMIT_BVH_MIN_TRIS;
+            s.any = !capable;
+            start = true;
+            search = false;
+          }
+        }
+      }
+      if (leave) {
+        const DevMaterial& m = sc->mats[mat_idx];
+        V3 nd;
+        if (PHYS) {
+          const float r = m.roughness;
+          if (lit) {
+            const DevMaterial& em = sc->mats[em_m];
+            const float fcos = fmul(r, fdiv(cos_x, PI_F));
+            // power heuristic against the bounce
+            const float wl = fdiv(fmul(pl, pl), fadd(fmul(pl, pl), fmul(fcos, fcos)));
+            col = col + ((att * v3(em.emission[0], em.emission[1], em.emission[2])) * fdiv(fcos, pl)) * wl;
+          }
+          pdf = 0.0f;
+          if (r >= 1.0f || (r > 0.0f && rnd(seed) < r)) {
+            nd = cosine_dir(N, seed);
+            pdf = fmul(r, fdiv(dot(N, nd), PI_F));
+          } else {
+            nd = reflect(D, N);
+          }
+          start = !is_zero(nd);
+          if (start && depth + 1 == (int)sc->num_bounces) start = final_ray_wanted(*sc, p, nd);
+        } else {
+          if (lit) {
+            const DevMaterial& em = sc->mats[stale];
+            col = col + (v3(em.emission[0], em.emission[1], em.emission[2]) * bsdf::BRDF(N, dir, m)) * att;
+          }
+          nd = bsdf::bounce(D, N, seed, m);
+          start = depth + 1 < (int)sc->num_bounces && !is_zero(nd);
+        }
+        shadow = false;
+        over = !start;
+        D = nd;
+      }
+      if (over) {
+        b.ps_col[slot] = make_float4(col.x, col.y, col.z, 0.0f);
+        if (w.rng_mode == LISA_RNG_PER_PIXEL) b.ps_rng[slot] = seed;
+        have = false;
+      } else if (start && !shadow) {
+        ++depth;
+        ++nbounce;
+      }
+      const bool need = !have && !exhausted;
+      const uint32_t nmask = __ballot_sync(FULL, need);
+      if (nmask) {
+        const int leader = __ffs(nmask) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(&b.ctrl->head[HEAD_TRACE], (uint32_t)__popc(nmask));
+        base = __shfl_sync(FULL, base, leader);
+        if (need) {
+          slot = base + __popc(nmask & lt);
+          if (slot < count) {
+            uint32_t scene, pix;
+            camera_ray(b, w, slot, scene, pix, seed, p, D);
+            sc = b.scenes + scene;
+            att = v3(1.0f);
+            col = v3(0.0f);
+            stale = -1;
+            pdf = 0.0f;
+            depth = 0;
+            shadow = false;
+            have = true;
+            start = true;
+          } else {
+            exhausted = true;
+          }
+        }
+      }
+      if (!__any_sync(FULL, have)) break;
+      if (start) {
+        if (!shadow) dir = D;
+        const bool any = shadow && (PHYS || s.any || nearer);
+        const float te = s.best_t;
+        const int pe = s.best_prim, me = s.best_mat;
+        ts = emit_pass ? trace_scene_emit(*sc) : trace_scene(*sc);
+        ray_active = trav_begin(s, ts, p, dir, RAY_TMIN, tmax, tp, any);
+        s.r.ox = p.x;  // (kept when there is nothing to traverse)
+        s.r.oy = p.y;
+        s.r.oz = p.z;
+        if (!PHYS && nearer) {
+          s.best_t = te;
+          s.best_prim = pe;
+          s.best_mat = me;
+          s.cull = fmaf(te, 1.52587890625e-5f, te) + s.r.slack;
+        }
+        if (ray_active) nwalked += shadow ? 1u : 0u;
+        else emit_pass = false;
+        pending = !ray_active;
+      }
+    }
+    if (trav_step_warp<false, true>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
+      ray_active = false;
+      pending = true;
+    }
+  }
+  warp_add64(&b.ctrl->rays_bounce, nbounce);
+  warp_add64(&b.ctrl->rays_shadow, nshadow);
+  warp_add64(&b.ctrl->shadow_walked, nwalked);
+  warp_add64(&b.ctrl->nee_total, nvertex);
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->rays_primary += count;
+}
+
+// ---------------------------------------------------------------------------
 // accumulate: per pixel, the wave's samples in sample order
 
 __global__ void k_accumulate(WaveBufs b, const WaveDesc* __restrict__ wave) {
   const WaveDesc& w = *wave;
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->head[HEAD_TRACE] = 0;  // for a whole-path wave that follows
   for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < w.acc_items; item += gridDim.x * blockDim.x) {
     const WaveGroup& g = w.groups[find_group(w, item, true)];
     const SceneDev& sc = b.scenes[g.scene];
@@ -1205,6 +1518,20 @@ __global__ void k_brute_rays(const SceneDev* __restrict__ scd, const float* __re
 // ---------------------------------------------------------------------------
 // host side
 
+// Plain waves of at most this many paths run whole paths in one kernel
+// (k_paths), larger ones stage by stage.  Measured device times, k_paths
+// against the stages, by wave size (8 bounces; 12 for the 5,000-sphere soup):
+//   reference estimator     64 Ki         1 Mi          4 Mi
+//     Cornell box           0.25 / 0.60   1.41 / 1.62   4.99 / 4.90 ms
+//     icosphere box, 328 k  0.44 / 1.42   2.46 / 3.26   9.09 / 8.32 ms
+//     sphere soup           3.18 / 9.16   9.68 / 16.5   29.8 / 33.4 ms
+//   physically based        64 Ki         256 Ki        1 Mi
+//     hard indirect, 328 k  0.56 / 1.06   1.20 / 1.38   3.44 / 2.76 ms
+// The stages win on large waves by their occupancy (32 warps an SM against
+// 20) and by running each routine on full warps; the physically based
+// estimator's short searches leave less to win.
+constexpr uint32_t PATHS_MAX_WAVE = 1u << 21, PATHS_MAX_WAVE_PB = 1u << 18;
+
 // Host view of one planned wave.
 struct WaveLaunch {
   uint32_t bounces;  // depth of its deepest scene
@@ -1213,6 +1540,8 @@ struct WaveLaunch {
   bool train;        // guided wave: train the guide after it
   bool warm;         // guided wave: warm-up, sample the BSDF only
   uint32_t steps;    // guided wave: Adam steps after it, in proportion to its paths
+  uint32_t paths;
+  bool whole;        // rendered by k_paths, not stage by stage
 };
 
 namespace {
@@ -1230,6 +1559,7 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
                 std::vector<WaveDesc>& waves, std::vector<WaveLaunch>& wave_launch) {
   const uint32_t W = r.capacity;
   const bool per_pixel = r.opts.rng == LISA_RNG_PER_PIXEL;
+  const uint32_t max_whole = r.opts.estimator == LISA_ESTIMATOR_PHYSICAL ? PATHS_MAX_WAVE_PB : PATHS_MAX_WAVE;
   waves.clear();
   wave_launch.clear();
   WaveDesc cur;
@@ -1246,7 +1576,8 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
                                             1u, (uint32_t)(((uint64_t)cur.paths * r.opts.guide_steps_per_wave +
                                                             (1ull << 21)) >> 22)))
                                       : 0u;
-    wave_launch.push_back(WaveLaunch{cur_b, (int)cur.groups[0].scene, cur_guided, false, false, steps});
+    const bool whole = !cur_guided && cur.paths <= max_whole && !r.opts.stage_timing && !r.opts.count_traversal;
+    wave_launch.push_back(WaveLaunch{cur_b, (int)cur.groups[0].scene, cur_guided, false, false, steps, cur.paths, whole});
     std::memset(&cur, 0, sizeof(cur));
     cur_b = 0;
   };
@@ -1429,6 +1760,26 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
       train_src.count = &r.ctrl->train_count;
       train_src.n = r.guide_batch_cap;
     }
+    if (waves[wv].whole) {
+      // at least eight warps an SM, so that a small wave's paths spread over
+      // the GPU; then 32 paths a warp
+      const uint32_t wpb = (uint32_t)r.nee_threads / 32u, paths = waves[wv].paths;
+      const uint32_t few = (uint32_t)r.sm_count * ((8u + wpb - 1u) / wpb);
+      const uint32_t grid = std::min<uint32_t>((uint32_t)r.path_blocks, std::max<uint32_t>(few, (paths + 32u * wpb - 1u) / (32u * wpb)));
+      const uint32_t lanes = std::min<uint32_t>(32u, (paths + grid * wpb - 1u) / (grid * wpb));
+      LISA_TRY(stage(0, [&] {
+        WaveBufs bp = b;
+        if (r.opts.refill_idle == 0) bp.refill_busy_max = 32u - LISA_PATHS_REFILL_IDLE;
+        if (physical) k_paths<true><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
+        else k_paths<false><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
+        return Status();
+      }));
+      LISA_TRY(stage(3, [&] {
+        k_accumulate<<<acc_blocks, 256, 0, r.stream>>>(b, wd);
+        return Status();
+      }));
+      continue;
+    }
     LISA_TRY(stage(3, [&] {
       k_raygen<<<r.sm_count * 8, 256, 0, r.stream>>>(b, wd);
       return Status();
@@ -1573,9 +1924,11 @@ Status renderer_render(Renderer& r, uint32_t spp_req, bool progressive, lisa_ren
     // one graph per launch-sequence shape; the wave table it reads is
     // refreshed above, outside the graph
     std::vector<uint64_t> key;
-    for (const WaveLaunch& w : wb)
+    for (const WaveLaunch& w : wb) {
+      key.push_back(w.whole ? w.paths : 0u);  // (its launch shape)
       key.push_back(((uint64_t)w.steps << 40) | ((uint64_t)w.bounces << 32) | ((uint64_t)w.scene << 3) |
                     ((uint64_t)w.guided << 2) | ((uint64_t)w.warm << 1) | w.train);
+    }
     key.push_back(r.opts.count_traversal);
     key.push_back(r.opts.stage_timing);
     key.push_back((uint64_t)(uintptr_t)r.d_waves);
@@ -1849,6 +2202,9 @@ Status configure_launch(Renderer& r) {
   bps = r.opts.blocks_per_sm ? (int)r.opts.blocks_per_sm : std::max(occ, 1);
   bps = std::min(bps, std::max(occ, 1));
   r.nee_pb_blocks = r.sm_count * bps;
+  LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_paths<false>, tthreads, 0));
+  bps = r.opts.blocks_per_sm ? (int)r.opts.blocks_per_sm : std::max(occ, 1);
+  r.path_blocks = r.sm_count * std::min(bps, std::max(occ, 1));
   LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_shade<false>, 256, 0));
   r.shade_threads = 256;
   r.shade_blocks = r.sm_count * std::max(occ, 1);
