@@ -4,15 +4,18 @@
 // (src/LiSA/src/optix_wrapper.cc:92-145).  Pipeline, all on the device:
 //   1. per-triangle AABB and centroid, scene and centroid bounds
 //   2. 30-bit Morton code of each centroid
-//   3. stable LSD radix sort of (code, triangle) pairs: 4 passes of 8 bits,
-//      tile histograms -> exclusive scan -> stable scatter (warp match-any
-//      ranking), written here without a sort library
+//   3. stable LSD radix sort of (code, triangle) pairs: one histogram of all
+//      four digits, then 4 passes of 8 bits that rank a tile in shared memory
+//      (warp match-any) and find its place by looking back over the tiles
+//      before it (Adinets & Merrill, "Onesweep", 2022); written here without
+//      a sort library
 //   4. binary radix tree over the sorted codes (Karras, "Maximizing
 //      Parallelism in the Construction of BVHs, Octrees, and k-d Trees",
 //      HPG 2012), equal codes ordered by index
 //   5. bottom-up AABBs with one atomic arrival counter per node
-//   6. collapse into 8-wide nodes, level by level: each node adopts up to 8
-//      descendants by repeatedly opening the child of largest surface area
+//   6. collapse into 8-wide nodes, level by level in one cooperative launch,
+//      eight lanes per node: each node adopts up to 8 descendants by
+//      repeatedly opening the child of largest surface area
 //      (subtrees of <= 3 triangles become leaves), then stores its child
 //      boxes quantised to 8 bits against a per-axis power-of-two grid,
 //      rounded outward (compressed layout in the style of Ylitie, Karras,
@@ -36,19 +39,9 @@ __device__ __forceinline__ int f2ord(float f) {
   const int i = __float_as_int(f);
   return i >= 0 ? i : i ^ 0x7fffffff;
 }
-__host__ __device__ __forceinline__ float ord2f(int i) {
-#ifdef __CUDA_ARCH__
-  return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff);
-#else
-  const int j = i >= 0 ? i : i ^ 0x7fffffff;
-  float f;
-  std::memcpy(&f, &j, 4);
-  return f;
-#endif
-}
 
 // bounds[0..2] = min scene xyz, [3..5] = max scene xyz, [6..8] min centroid,
-// [9..11] max centroid, as order-preserving ints.
+// [9..11] max centroid, as order-preserving ints.  Blocks of 256.
 __global__ void k_prim_bounds(const float* __restrict__ v, uint32_t n, float4* __restrict__ lo,
                               float4* __restrict__ hi, int* bounds) {
   float mn[6], mx[6];
@@ -73,21 +66,28 @@ __global__ void k_prim_bounds(const float* __restrict__ v, uint32_t n, float4* _
     lo[i] = make_float4(a[0], a[1], a[2], 0.0f);
     hi[i] = make_float4(b[0], b[1], b[2], 0.0f);
   }
+  // one set of atomics per block (per warp, they took longer than the scan:
+  // 249 us of 1.31 M triangles, all on the same 12 words)
+  __shared__ float red[8][12];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
     for (int o = 16; o > 0; o >>= 1) {
       mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
       mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
     }
-  }
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      atomicMin(&bounds[k], f2ord(mn[k]));
-      atomicMax(&bounds[3 + k], f2ord(mx[k]));
-      atomicMin(&bounds[6 + k], f2ord(mn[3 + k]));
-      atomicMax(&bounds[9 + k], f2ord(mx[3 + k]));
+    if ((threadIdx.x & 31) == 0) {
+      red[threadIdx.x >> 5][k] = mn[k];
+      red[threadIdx.x >> 5][6 + k] = mx[k];
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 12) {
+    const int k = threadIdx.x;
+    float v = red[0][k];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = k < 6 ? fminf(v, red[w][k]) : fmaxf(v, red[w][k]);
+    // red: min scene, min centroid, max scene, max centroid
+    if (k < 6) atomicMin(&bounds[k < 3 ? k : k + 3], f2ord(v));
+    else atomicMax(&bounds[k < 9 ? k - 3 : k], f2ord(v));
   }
 }
 
@@ -142,72 +142,32 @@ __global__ void k_morton(const float4* __restrict__ lo, const float4* __restrict
 
 // ---- radix sort -----------------------------------------------------------
 constexpr int RS_THREADS = 256;
-constexpr int RS_ROUNDS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
+constexpr int RS_PASSES = 4;  // 8 bits each (BvhDeviceInfo has a ticket per pass)
+constexpr uint32_t RS_POLLS = 1u << 22;  // of a look-back wait, then the build fails
 
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
-                                                       uint32_t* __restrict__ hist, uint32_t num_tiles) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
+// Keys per thread of a tile: 16, but 4 for up to 256 Ki keys, which would
+// otherwise make too few tiles (8 of them at 30,000) to fill the GPU.
+inline int rs_rounds(uint32_t n) { return n <= (1u << 18) ? 4 : 16; }
+
+// Histograms of the four digits (hist: 4 x 256, zeroed before).
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n,
+                                                       uint32_t* __restrict__ hist) {
+  __shared__ uint32_t h[RS_PASSES][256];
+#pragma unroll
+  for (int d = 0; d < RS_PASSES; ++d) h[d][threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
-#pragma unroll 4
-  for (int k = 0; k < RS_ROUNDS; ++k) {
-    const uint64_t idx = base + (uint64_t)k * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1u);
+  for (uint32_t i = blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += gridDim.x * RS_THREADS) {
+    const uint32_t k = keys[i];
+#pragma unroll
+    for (int d = 0; d < RS_PASSES; ++d) atomicAdd(&h[d][(k >> (8 * d)) & 255u], 1u);
   }
   __syncthreads();
-  hist[(uint64_t)threadIdx.x * num_tiles + blockIdx.x] = h[threadIdx.x];
+#pragma unroll
+  for (int d = 0; d < RS_PASSES; ++d)
+    if (h[d][threadIdx.x]) atomicAdd(&hist[256 * d + threadIdx.x], h[d][threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                          uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                          uint32_t n, int shift, const uint32_t* __restrict__ offs,
-                                                          uint32_t num_tiles) {
-  __shared__ uint32_t s_base[256];
-  __shared__ uint32_t s_run[256];
-  __shared__ uint32_t s_wc[RS_THREADS / 32][256];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  s_base[tid] = offs[(uint64_t)tid * num_tiles + blockIdx.x];
-  s_run[tid] = 0;
-  const uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
-  const uint32_t lt = (1u << lane) - 1u;
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-#pragma unroll
-    for (int w = 0; w < RS_THREADS / 32; ++w) s_wc[w][tid] = 0;
-    __syncthreads();
-    const uint64_t idx = base + (uint64_t)r * RS_THREADS + tid;
-    const bool valid = idx < n;
-    const uint32_t key = valid ? kin[idx] : 0u;
-    const uint32_t d = valid ? ((key >> shift) & 255u) : 256u;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank = __popc(peers & lt);
-    if (valid && rank == 0) s_wc[warp][d] = __popc(peers);
-    __syncthreads();
-    uint32_t run = s_run[tid];
-#pragma unroll
-    for (int w = 0; w < RS_THREADS / 32; ++w) {
-      const uint32_t c = s_wc[w][tid];
-      s_wc[w][tid] = run;
-      run += c;
-    }
-    s_run[tid] = run;
-    __syncthreads();
-    if (valid) {
-      const uint32_t pos = s_base[d] + s_wc[warp][d] + rank;
-      kout[pos] = key;
-      vout[pos] = vin[idx];
-    }
-    __syncthreads();
-  }
-}
-
-// ---- exclusive scan (in place) --------------------------------------------
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 4;
-constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
-
-__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total) {
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v) {
   __shared__ uint32_t ws[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t x = v;
@@ -227,57 +187,87 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* total)
     if (lane < nw) ws[lane] = s;
   }
   __syncthreads();
-  const uint32_t before = (warp > 0 ? ws[warp - 1] : 0u) + x - v;
-  if (total) *total = ws[(blockDim.x >> 5) - 1];
+  return (warp > 0 ? ws[warp - 1] : 0u) + x - v;
+}
+
+// One pass over a tile of RS_THREADS x ROUNDS keys.  Tiles are numbered in
+// the order their blocks start (a ticket), so a block only waits for blocks
+// that run already.  look[tile][digit]: 0 = nothing yet, 1 << 30 | the tile's
+// count, 2 << 30 | the count of all tiles up to it.  With five launches for
+// the sort instead of twenty, its kernels take 42 us instead of 141 for
+// 30,001 keys and 143 instead of 160 for 1.31 M (cold).
+template <int ROUNDS>
+__global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                                       uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                       uint32_t n, int shift, const uint32_t* __restrict__ hist,
+                                                       uint32_t* look, uint32_t* ticket, uint32_t* failed) {
+  constexpr int WARPS = RS_THREADS / 32;
+  __shared__ uint32_t s_tile;
+  __shared__ uint32_t s_wc[WARPS][256];  // per warp: its count of each digit, then its first place in the tile
+  __shared__ uint32_t s_base[256];       // place of the tile's first key of each digit
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) s_wc[w][tid] = 0;
   __syncthreads();
-  return before;
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_blocks(uint32_t* data, uint64_t m, uint32_t* sums) {
-  const uint64_t base = (uint64_t)blockIdx.x * SCAN_CHUNK + (uint64_t)threadIdx.x * SCAN_ITEMS;
-  uint32_t v[SCAN_ITEMS], s = 0;
+  const uint32_t tile = s_tile;
+  const uint64_t base = (uint64_t)tile * (RS_THREADS * ROUNDS) + (uint32_t)(warp * 32 * ROUNDS + lane);
+  const uint32_t lt = (1u << lane) - 1u;
+  uint32_t key[ROUNDS], rank[ROUNDS];
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    v[k] = (base + k < m) ? data[base + k] : 0u;
-    s += v[k];
+  for (int r = 0; r < ROUNDS; ++r) key[r] = base + 32 * r < n ? kin[base + 32 * r] : 0u;
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    const bool valid = base + 32 * r < n;
+    const uint32_t d = valid ? ((key[r] >> shift) & 255u) : 256u;
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    const uint32_t before = valid ? s_wc[warp][d] : 0u;
+    __syncwarp();
+    if (valid && (peers & lt) == 0u) s_wc[warp][d] = before + __popc(peers);
+    __syncwarp();
+    rank[r] = before + __popc(peers & lt);
   }
-  uint32_t total;
-  uint32_t run = block_exclusive(s, &total);
+  __syncthreads();
+  uint32_t count = 0;
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k) {
-    if (base + k < m) data[base + k] = run;
-    run += v[k];
+  for (int w = 0; w < WARPS; ++w) {
+    const uint32_t c = s_wc[w][tid];
+    s_wc[w][tid] = count;
+    count += c;
   }
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_single(uint32_t* sums, uint32_t nb) {
-  uint32_t carry = 0;
-  for (uint32_t c0 = 0; c0 < nb; c0 += SCAN_CHUNK) {
-    const uint32_t base = c0 + threadIdx.x * SCAN_ITEMS;
-    uint32_t v[SCAN_ITEMS], s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-      v[k] = (base + k < nb) ? sums[base + k] : 0u;
-      s += v[k];
+  // the digit's keys in the tiles before this one
+  uint32_t prefix = 0;
+  volatile uint32_t* mine = look + (uint64_t)tile * 256 + tid;
+  if (tile == 0) {
+    *mine = (2u << 30) | count;
+  } else {
+    *mine = (1u << 30) | count;
+    uint32_t polls = 0;
+    for (int64_t t = (int64_t)tile - 1; t >= 0;) {
+      const uint32_t v = *(volatile uint32_t*)(look + (uint64_t)t * 256 + tid);
+      if ((v >> 30) == 0u) {
+        if (++polls < RS_POLLS) continue;
+        *failed = 1u;
+        break;
+      }
+      prefix += v & 0x3fffffffu;
+      if ((v >> 30) == 2u) break;
+      --t;
     }
-    uint32_t total;
-    uint32_t run = carry + block_exclusive(s, &total);
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-      if (base + k < nb) sums[base + k] = run;
-      run += v[k];
-    }
-    carry += total;
+    *mine = (2u << 30) | (prefix + count);
   }
-}
-
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint32_t* data, uint64_t m, const uint32_t* sums) {
-  const uint64_t base = (uint64_t)blockIdx.x * SCAN_CHUNK + (uint64_t)threadIdx.x * SCAN_ITEMS;
-  const uint32_t add = sums[blockIdx.x];
+  const uint32_t first = block_exclusive(hist[tid]);
+  s_base[tid] = first + prefix;
+  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; ++k)
-    if (base + k < m) data[base + k] += add;
+  for (int r = 0; r < ROUNDS; ++r) {
+    if (base + 32 * r >= n) continue;
+    const uint32_t d = (key[r] >> shift) & 255u;
+    const uint32_t pos = s_base[d] + s_wc[warp][d] + rank[r];
+    if (pos >= n) continue;  // (only after a failed wait)
+    kout[pos] = key[r];
+    vout[pos] = vin[base + 32 * r];
+  }
 }
 
 // ---- Karras radix tree ------------------------------------------------------
@@ -330,26 +320,6 @@ __device__ __forceinline__ void node_box(uint32_t c, const uint32_t* vals, const
   } else {
     lo = __ldcg(ilo + c);
     hi = __ldcg(ihi + c);
-  }
-}
-
-__global__ void k_bottom_up(uint32_t n, const uint32_t* __restrict__ vals, const float4* __restrict__ plo,
-                            const float4* __restrict__ phi, const uint32_t* __restrict__ parent_leaf,
-                            const uint32_t* __restrict__ parent_int, const uint32_t* __restrict__ left,
-                            const uint32_t* __restrict__ right, float4* ilo, float4* ihi, uint32_t* flags) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || n < 2) return;
-  uint32_t p = parent_leaf[i];
-  while (p != 0xffffffffu) {
-    __threadfence();
-    if (atomicAdd(&flags[p], 1u) == 0u) return;
-    __threadfence();
-    float4 a0, a1, b0, b1;
-    node_box(left[p], vals, plo, phi, ilo, ihi, a0, a1);
-    node_box(right[p], vals, plo, phi, ilo, ihi, b0, b1);
-    __stcg(ilo + p, make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.0f));
-    __stcg(ihi + p, make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.0f));
-    p = parent_int[p];
   }
 }
 
@@ -428,125 +398,229 @@ struct TreeletSmem {
   float opt[1 << TL];        // best SAH cost of each subset of the treelet's leaves
   uint8_t split[1 << TL];    // its best partition (one side)
   float4 llo[TL], lhi[TL];   // leaf boxes
-  float lcost[TL];
   uint32_t lcnt[TL];
-  uint32_t leaf[TL], inner[TL - 2];
-  int nl;
+  uint32_t leaf[TL], inner[TL];
+  uint32_t node[TL], set[TL];  // rebuilt nodes and the leaf subsets below them
+  uint32_t child[TL][2];
 };
 
+// Subsets of up to 7 leaves by size: 21 pairs, 35 triples, 35 of four, 21 of
+// five, 7 of six.
+__constant__ uint8_t c_subset[119] = {
+    3,   5,   6,   9,   10,  12,  17,  18,  20,  24,  33,  34,  36,  40,  48,  65,  66,  68,  72,  80,  96,
+    7,   11,  13,  14,  19,  21,  22,  25,  26,  28,  35,  37,  38,  41,  42,  44,  49,  50,  52,  56,  67,  69,
+    70,  73,  74,  76,  81,  82,  84,  88,  97,  98,  100, 104, 112,
+    15,  23,  27,  29,  30,  39,  43,  45,  46,  51,  53,  54,  57,  58,  60,  71,  75,  77,  78,  83,  85,  86,
+    89,  90,  92,  99,  101, 102, 105, 106, 108, 113, 114, 116, 120,
+    31,  47,  55,  59,  61,  62,  79,  87,  91,  93,  94,  103, 107, 109, 110, 115, 117, 118, 121, 122, 124,
+    63,  95,  111, 119, 123, 125, 126};
+
 // Treelet restructuring (Karras and Aila, HPG 2013) of the subtree at
-// `root`, by one warp: lane 0 grows the treelet (the largest-area leaf is
-// expanded until TL leaves), the lanes then share the dynamic programme over
-// the subsets of its leaves, one subset size per round (a subset's
-// partitions only use smaller subsets), and lane 0 rebuilds the subtree when
-// the best topology is cheaper.  Every subset's cost is computed by the same
-// operations in the same order as a serial loop would.  All 32 lanes call
-// it with the same root.
+// `root`, by one warp.  Lane k holds the treelet's leaf k while it grows (the
+// leaf of largest area is opened until there are TL), with its children's
+// indices loaded ahead, so a step costs one memory latency.  The lanes then
+// share the dynamic programme over the subsets of the leaves: all boxes
+// first, then the subsets by size, several lanes for the partitions of the
+// largest; and each rebuilds one node when the best topology is cheaper.
+// What bounds the kernel is the chain of treelets from a leaf to the root:
+// with the growth, the boxes and the rebuilding on one lane it took 351 us
+// for 30,001 triangles and 2.4 ms for 1.31 M, now 180 us and 0.51 ms.  All
+// 32 lanes call it with the same root.
 __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSmem& s) {
   const int lane = threadIdx.x & 31;
-  __syncwarp();  // the root's box, count and cost, just written by its lane, are visible to lane 0
-  if (lane == 0) {
-    int nl = 2, ni = 0;
-    s.leaf[0] = __ldcg(t.left + root);
-    s.leaf[1] = __ldcg(t.right + root);
-    sah_child(t, s.leaf[0], s.llo[0], s.lhi[0], s.lcnt[0], s.lcost[0]);
-    sah_child(t, s.leaf[1], s.llo[1], s.lhi[1], s.lcnt[1], s.lcost[1]);
-    while (nl < TL) {
-      int best = -1;
-      float ba = -1.0f;
-      for (int k = 0; k < nl; ++k) {
-        if (s.leaf[k] & LEAF_BIT) continue;
-        const float a = box_half_area(s.llo[k], s.lhi[k]);
-        if (a > ba) {
-          ba = a;
-          best = k;
-        }
-      }
-      if (best < 0) break;
-      const uint32_t c = s.leaf[best];
-      s.inner[ni++] = c;
-      s.leaf[best] = __ldcg(t.left + c);
-      s.leaf[nl] = __ldcg(t.right + c);
-      sah_child(t, s.leaf[best], s.llo[best], s.lhi[best], s.lcnt[best], s.lcost[best]);
-      sah_child(t, s.leaf[nl], s.llo[nl], s.lhi[nl], s.lcnt[nl], s.lcost[nl]);
-      ++nl;
+  __syncwarp();  // the root's box, count and cost, just written by its lane, are visible
+  uint32_t id = LEAF_BIT, cnt = 0, lc = 0, rc = 0, inner = 0;
+  float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+  float cost = 0.0f;
+  auto load = [&](uint32_t c) {
+    id = c;
+    if (!(c & LEAF_BIT)) {
+      lc = __ldcg(t.left + c);
+      rc = __ldcg(t.right + c);
     }
-    s.nl = nl;
+    sah_child(t, c, lo, hi, cnt, cost);
+  };
+  if (lane < 2) load(__ldcg((lane ? t.right : t.left) + root));
+  int nl = 2;
+  for (; nl < TL; ++nl) {
+    // (areas are not negative, so their bits order as the floats)
+    const bool open = lane < nl && !(id & LEAF_BIT);
+    const uint32_t a = open ? __float_as_uint(box_half_area(lo, hi)) + 1u : 0u;
+    const uint32_t best = __reduce_max_sync(0xffffffffu, a);
+    if (best == 0u) break;
+    const int owner = __ffs(__ballot_sync(0xffffffffu, a == best)) - 1;
+    const uint32_t c = __shfl_sync(0xffffffffu, id, owner);
+    const uint32_t l = __shfl_sync(0xffffffffu, lc, owner), r = __shfl_sync(0xffffffffu, rc, owner);
+    if (lane == nl - 2) inner = c;
+    if (lane == owner) load(l);
+    else if (lane == nl) load(r);
   }
-  __syncwarp();
-  const int nl = s.nl;
   if (nl < 3) return;  // two leaves have one topology
   const uint32_t full = (1u << nl) - 1u;
-  for (uint32_t sset = lane + 1; sset <= full; sset += 32)
-    if ((sset & (sset - 1u)) == 0u) {
-      s.opt[sset] = s.lcost[__ffs(sset) - 1];
-      s.split[sset] = 0;
-    }
+  if (lane < nl) {
+    s.llo[lane] = lo;
+    s.lhi[lane] = hi;
+    s.lcnt[lane] = cnt;
+    s.leaf[lane] = id;
+    s.inner[lane] = inner;
+    s.opt[1u << lane] = cost;
+  }
   __syncwarp();
-  for (int size = 2; size <= nl; ++size) {
-    for (uint32_t sset = lane + 1; sset <= full; sset += 32) {
-      if (__popc(sset) != size) continue;
-      float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
-      for (int k = 0; k < nl; ++k)
-        if (sset & (1u << k)) {
-          lo = box_min(lo, s.llo[k]);
-          hi = box_max(hi, s.lhi[k]);
-        }
-      const uint32_t low = sset & (0u - sset), rest = sset ^ low;
-      float best = s.opt[low] + s.opt[rest];
-      uint32_t bp = low;
-      // partitions (P, S \ P) with the lowest member in P, each once:
-      // P = low + a nonempty proper subset of the rest
-      for (uint32_t q = (rest - 1u) & rest; q; q = (q - 1u) & rest) {
-        const uint32_t pset = q | low;
+  // boxes of the subsets lane, lane + 32, + 64, + 96: the lane's bits choose
+  // among the first five leaves
+  {
+    const float4 elo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), ehi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
+    float4 blo = elo, bhi = ehi;
+    for (int k = 0; k < 5 && k < nl; ++k)
+      if (lane & (1 << k)) {
+        blo = box_min(blo, s.llo[k]);
+        bhi = box_max(bhi, s.lhi[k]);
+      }
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint32_t sset = (uint32_t)lane + 32u * j;
+      if (sset > full || (sset & (sset - 1u)) == 0u) continue;
+      float4 ulo = blo, uhi = bhi;
+      if (j & 1u) {
+        ulo = box_min(ulo, s.llo[5]);
+        uhi = box_max(uhi, s.lhi[5]);
+      }
+      if (j & 2u) {
+        ulo = box_min(ulo, s.llo[6]);
+        uhi = box_max(uhi, s.lhi[6]);
+      }
+      s.opt[sset] = SAH_CI * box_half_area(ulo, uhi);  // + the best partition's cost, below
+    }
+  }
+  __syncwarp();
+  // Best partition (P, S \ P) of a subset with its lowest member in P, each
+  // once: P = low + fixed + a subset of `rest`; P = S is skipped.
+  auto best_partition = [&](uint32_t sset, uint32_t fixed, uint32_t rest, float& best, uint32_t& bp) {
+    uint32_t q = rest;
+    best = 3.4e38f;
+    bp = 0;
+    while (true) {
+      const uint32_t pset = q | fixed;
+      if (pset != sset) {
         const float c = s.opt[pset] + s.opt[sset ^ pset];
         if (c < best) {
           best = c;
           bp = pset;
         }
       }
-      s.opt[sset] = SAH_CI * box_half_area(lo, hi) + best;
+      if (q == 0u) break;
+      q = (q - 1u) & rest;
+    }
+  };
+  constexpr int FIRST[6] = {0, 0, 0, 21, 56, 91};  // of c_subset, by size
+  constexpr int NUM[6] = {0, 0, 21, 35, 35, 21};
+  for (int size = 2; size <= 5 && size <= nl; ++size) {
+    for (int i = lane; i < NUM[size]; i += 32) {
+      const uint32_t sset = c_subset[FIRST[size] + i];
+      if (sset > full) continue;
+      const uint32_t low = sset & (0u - sset);
+      float best;
+      uint32_t bp;
+      best_partition(sset, low, sset ^ low, best, bp);
+      s.opt[sset] += best;
       s.split[sset] = (uint8_t)bp;
     }
     __syncwarp();
   }
-  if (lane == 0 && s.opt[full] < __ldcg(t.cost + root) * (1.0f - 1e-6f)) {
-    // rebuild: the root keeps its id, the other internal subsets reuse inner[]
-    uint32_t st_set[TL], st_node[TL];
-    int sp = 0, next = 0;
-    st_set[sp] = full;
-    st_node[sp++] = root;
-    while (sp) {
-      --sp;
-      const uint32_t sset = st_set[sp], node = st_node[sp];
+  if (nl >= 6) {
+    // subsets of six: four lanes each, which fix the membership of the two
+    // highest members
+    const int i = lane >> 2;
+    const uint32_t sset = i < 7 ? c_subset[112 + i] : 0xffu;
+    float best = 3.4e38f;
+    uint32_t bp = 0;
+    if (sset <= full) {
+      const uint32_t low = sset & (0u - sset);
+      uint32_t rest = sset ^ low;
+      const uint32_t h1 = 0x80000000u >> __clz(rest);
+      rest ^= h1;
+      const uint32_t h2 = 0x80000000u >> __clz(rest);
+      rest ^= h2;
+      best_partition(sset, low | ((lane & 1) ? h1 : 0u) | ((lane & 2) ? h2 : 0u), rest, best, bp);
+    }
+#pragma unroll
+    for (int m = 1; m <= 2; m <<= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, m);
+      const uint32_t op = __shfl_xor_sync(0xffffffffu, bp, m);
+      if (ob < best || (ob == best && op < bp)) {
+        best = ob;
+        bp = op;
+      }
+    }
+    if (sset <= full && (lane & 3) == 0) {
+      s.opt[sset] += best;
+      s.split[sset] = (uint8_t)bp;
+    }
+    __syncwarp();
+  }
+  if (nl == 7) {
+    // the full set: the lane's bits are the membership of leaves 1..5
+    float best;
+    uint32_t bp;
+    best_partition(full, 1u | ((uint32_t)lane << 1), 64u, best, bp);
+#pragma unroll
+    for (int m = 1; m <= 16; m <<= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, m);
+      const uint32_t op = __shfl_xor_sync(0xffffffffu, bp, m);
+      if (ob < best || (ob == best && op < bp)) {
+        best = ob;
+        bp = op;
+      }
+    }
+    if (lane == 0) {
+      s.opt[full] += best;
+      s.split[full] = (uint8_t)bp;
+    }
+    __syncwarp();
+  }
+  if (!(s.opt[full] < __ldcg(t.cost + root) * (1.0f - 1e-6f))) {
+    __syncwarp();
+    return;
+  }
+  // rebuild: the root keeps its id, the other internal subsets reuse inner[]
+  if (lane == 0) {
+    int built = 1, next = 0;
+    s.set[0] = full;
+    s.node[0] = root;
+    for (int i = 0; i < built; ++i) {
+      const uint32_t sset = s.set[i];
       const uint32_t part[2] = {s.split[sset], sset ^ (uint32_t)s.split[sset]};
-      uint32_t ch[2];
       for (int h = 0; h < 2; ++h) {
         if ((part[h] & (part[h] - 1u)) == 0u) {
-          ch[h] = s.leaf[__ffs(part[h]) - 1];
+          s.child[i][h] = s.leaf[__ffs(part[h]) - 1];
         } else {
-          ch[h] = s.inner[next++];
-          st_set[sp] = part[h];
-          st_node[sp++] = ch[h];
+          s.child[i][h] = s.node[built] = s.inner[next++];
+          s.set[built++] = part[h];
         }
-        if (ch[h] & LEAF_BIT) __stcg(t.parent_leaf + (ch[h] & ~LEAF_BIT), node);
-        else __stcg(t.parent_int + ch[h], node);
       }
-      __stcg(t.left + node, ch[0]);
-      __stcg(t.right + node, ch[1]);
-      float4 lo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), hi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
-      uint32_t cnt = 0;
-      for (int k = 0; k < nl; ++k)
-        if (sset & (1u << k)) {
-          lo = box_min(lo, s.llo[k]);
-          hi = box_max(hi, s.lhi[k]);
-          cnt += s.lcnt[k];
-        }
-      __stcg(t.ilo + node, lo);
-      __stcg(t.ihi + node, hi);
-      __stcg(t.count + node, cnt);
-      __stcg(t.cost + node, s.opt[sset]);
     }
+  }
+  __syncwarp();
+  if (lane < nl - 1) {  // a binary tree over nl leaves has nl - 1 nodes
+    const uint32_t node = s.node[lane], sset = s.set[lane];
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t c = s.child[lane][h];
+      if (c & LEAF_BIT) __stcg(t.parent_leaf + (c & ~LEAF_BIT), node);
+      else __stcg(t.parent_int + c, node);
+    }
+    __stcg(t.left + node, s.child[lane][0]);
+    __stcg(t.right + node, s.child[lane][1]);
+    float4 blo = make_float4(3.4e38f, 3.4e38f, 3.4e38f, 0.0f), bhi = make_float4(-3.4e38f, -3.4e38f, -3.4e38f, 0.0f);
+    uint32_t n = 0;
+    for (int k = 0; k < nl; ++k)
+      if (sset & (1u << k)) {
+        blo = box_min(blo, s.llo[k]);
+        bhi = box_max(bhi, s.lhi[k]);
+        n += s.lcnt[k];
+      }
+    __stcg(t.ilo + node, blo);
+    __stcg(t.ihi + node, bhi);
+    __stcg(t.count + node, n);
+    __stcg(t.cost + node, s.opt[sset]);
   }
   __syncwarp();
 }
@@ -599,6 +673,7 @@ __global__ void __launch_bounds__(SAH_THREADS) k_bottom_up_sah(SahTree t, int re
 }
 
 // ---- collapse to 8-wide compressed nodes -------------------------------------
+
 struct CollapseArgs {
   uint32_t n;
   const uint32_t* vals;
@@ -613,215 +688,232 @@ struct CollapseArgs {
   const int32_t* mats;  // material per triangle, or null
   uint4* nodes;
   float4* tris;
-  uint32_t* counters;  // [0] nodes, [1] tri slots
+  uint32_t* source;     // binary node of each 8-wide node, in node order
+  BvhDeviceInfo* info;
 };
 
-__device__ __forceinline__ uint32_t sub_count(const CollapseArgs& a, uint32_t c) {
-  return (c & LEAF_BIT) ? 1u : a.count[c];
-}
-__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
-  const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
-  return x * y + y * z + z * x;
-}
-
-// Smallest e with 255 * 2^e >= ext, clamped to the normal float range.
-__device__ int grid_exponent(double ext) {
-  if (!(ext > 0.0)) return -126;
-  int e;
-  frexp(ext / 255.0, &e);  // ext/255 = m * 2^e, m in [0.5, 1)
-  while (ldexp(255.0, e - 1) >= ext && e > -126) --e;
-  while (ldexp(255.0, e) < ext) ++e;
+// Smallest e (within [-126, 127]) with 255 * 2^e >= ext.
+__device__ __forceinline__ int grid_exponent(float ext) {
+  if (!(ext > 0.0f)) return -126;
+  const uint32_t q = __float_as_uint(__fdiv_ru(ext, 255.0f));  // 2^e >= q
+  const int e = (int)(q >> 23) - 127 + ((q & 0x7fffffu) ? 1 : 0);
   return max(-126, min(127, e));
 }
 
-// Collapse levels run as a fixed sequence of launches with no host round
-// trip: level l reads its work count from levels[l] (written by level l-1)
-// and appends the next level's work, counting it in levels[l+1]; a level
-// with no work returns at once.
-constexpr int COLLAPSE_LAUNCHES = 24;
+constexpr int COLLAPSE_THREADS = 128;
 
-__global__ void k_collapse_init(uint32_t* counters, uint32_t* levels, uint2* work0, uint2 root) {
-  counters[0] = 1u;  // node 0 is the root
-  counters[1] = 0u;
-  for (int l = 0; l <= COLLAPSE_LAUNCHES + 1; ++l) levels[l] = l == 0 ? 1u : 0u;
-  work0[0] = root;
-}
-
-__device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restrict__ next, uint32_t* next_count);
-
-__global__ void k_collapse(CollapseArgs a, const uint2* __restrict__ work, const uint32_t* __restrict__ nwork_p,
-                           uint2* __restrict__ next, uint32_t* next_count) {
-  const uint32_t nwork = *nwork_p;
-  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nwork; w += gridDim.x * blockDim.x)
-    collapse_one(a, work[w], next, next_count);
-}
-
-__device__ void collapse_one(const CollapseArgs& a, uint2 item, uint2* __restrict__ next, uint32_t* next_count) {
-  const uint32_t dst = item.x, src = item.y;
-  uint32_t cand[8];
-  int nc;
-  if (!(src & LEAF_BIT) && sub_count(a, src) > 3u) {
-    cand[0] = a.left[src];
-    cand[1] = a.right[src];
-    nc = 2;
-  } else {
-    cand[0] = src;
-    nc = 1;
-  }
-  float4 clo[8], chi[8];
-  for (int k = 0; k < nc; ++k) node_box(cand[k], a.vals, a.plo, a.phi, a.ilo, a.ihi, clo[k], chi[k]);
-  while (nc < 8) {
-    int best = -1;
-    float best_area = -1.0f;
-    for (int k = 0; k < nc; ++k) {
-      if ((cand[k] & LEAF_BIT) || sub_count(a, cand[k]) <= 3u) continue;
-      const float ar = half_area(clo[k], chi[k]);
-      if (ar > best_area) {
-        best_area = ar;
-        best = k;
+// All blocks of the cooperative grid meet; false once a wait (bounded) has
+// run out in some block.  Memory written before is visible after it to loads
+// that bypass L1.
+__device__ __forceinline__ bool collapse_barrier(BvhDeviceInfo* info, uint32_t k) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&info->barrier, 1u);
+    const uint32_t target = (k + 1) * gridDim.x;
+    bool ok = false;
+    for (uint32_t it = 0; it < (1u << 22); ++it) {
+      uint32_t v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&info->barrier) : "memory");
+      if (v >= target) {
+        ok = true;
+        break;
       }
+      __nanosleep(32);
     }
-    if (best < 0) break;
-    const uint32_t c = cand[best];
-    cand[best] = a.left[c];
-    cand[nc] = a.right[c];
-    node_box(cand[best], a.vals, a.plo, a.phi, a.ilo, a.ihi, clo[best], chi[best]);
-    node_box(cand[nc], a.vals, a.plo, a.phi, a.ilo, a.ihi, clo[nc], chi[nc]);
-    ++nc;
+    if (!ok) atomicExch(&info->failed, 1u);
+    s_ok = ok && *(volatile uint32_t*)&info->failed == 0u;
   }
-  // internal children take the first slots
-  uint32_t num_int = 0, num_tri = 0;
-  for (int k = 0; k < nc; ++k) {
-    const uint32_t cnt = sub_count(a, cand[k]);
-    if (cnt <= 3u) {
-      num_tri += cnt;
-      continue;
-    }
-    const int j = (int)num_int++;
-    if (j == k) continue;
-    const uint32_t c = cand[k];
-    const float4 lo = clo[k], hi = chi[k];
-    cand[k] = cand[j];
-    clo[k] = clo[j];
-    chi[k] = chi[j];
-    cand[j] = c;
-    clo[j] = lo;
-    chi[j] = hi;
-  }
-  const uint32_t child_base = num_int ? atomicAdd(&a.counters[0], num_int) : 0u;
-  const uint32_t tri_base = num_tri ? atomicAdd(&a.counters[1], num_tri) : 0u;
-  // node frame
-  float4 nlo = clo[0], nhi = chi[0];
-  for (int k = 1; k < nc; ++k) {
-    nlo.x = fminf(nlo.x, clo[k].x);
-    nlo.y = fminf(nlo.y, clo[k].y);
-    nlo.z = fminf(nlo.z, clo[k].z);
-    nhi.x = fmaxf(nhi.x, chi[k].x);
-    nhi.y = fmaxf(nhi.y, chi[k].y);
-    nhi.z = fmaxf(nhi.z, chi[k].z);
-  }
-  const float p[3] = {nlo.x, nlo.y, nlo.z};
-  const float ph[3] = {nhi.x, nhi.y, nhi.z};
-  int e[3];
-  for (int ax = 0; ax < 3; ++ax) e[ax] = grid_exponent((double)ph[ax] - (double)p[ax]);
-  uint8_t qlo[3][8], qhi[3][8];
-  uint32_t leaves = 0, toff = 0;
-  for (int k = 0; k < 8; ++k) {
-    for (int ax = 0; ax < 3; ++ax) {
-      qlo[ax][k] = 0;
-      qhi[ax][k] = 0;
-    }
-  }
-  for (int k = 0; k < nc; ++k) {
-    const float lo3[3] = {clo[k].x, clo[k].y, clo[k].z};
-    const float hi3[3] = {chi[k].x, chi[k].y, chi[k].z};
-    for (int ax = 0; ax < 3; ++ax) {
-      const double sc = ldexp(1.0, e[ax]);
-      double ql = floor(((double)lo3[ax] - (double)p[ax]) / sc);
-      double qh = ceil(((double)hi3[ax] - (double)p[ax]) / sc);
-      ql = fmin(fmax(ql, 0.0), 255.0);
-      qh = fmin(fmax(qh, 0.0), 255.0);
-      while (ql > 0.0 && (double)p[ax] + ql * sc > (double)lo3[ax]) ql -= 1.0;
-      while (qh < 255.0 && (double)p[ax] + qh * sc < (double)hi3[ax]) qh += 1.0;
-      qlo[ax][k] = (uint8_t)ql;
-      qhi[ax][k] = (uint8_t)qh;
-    }
-    const uint32_t cnt = sub_count(a, cand[k]);
-    if (cnt > 3u) {
-      const uint32_t slot = atomicAdd(next_count, 1u);
-      next[slot] = make_uint2(child_base + (uint32_t)k, cand[k]);
-    } else {
-      leaves |= ((1u << cnt) - 1u) << (3 * k);
-      // the (at most 3) primitives below, left to right
-      uint32_t leaves[3], st[4];
-      int nlv = 0, sp = 0;
-      st[sp++] = cand[k];
-      while (sp) {
-        const uint32_t c = st[--sp];
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// The node numbers are the work list: level l is the range of nodes that
+// level l - 1 took, and source[node] says which binary node each stands for.
+// Eight lanes collapse one node: lane k holds candidate k, its children's
+// indices loaded ahead (a step of the growth costs one memory latency), and
+// then quantises and writes child k.  Bound by those latencies, level after
+// level: 70 us for 30,001 triangles and 269 for 1.31 M, where 24 launches
+// with a thread per node and the grid in FP64 took 589 and 1,200 (cold).
+__global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, k = lane & 7, g0 = lane & 24;  // candidate, first lane of the group
+  const uint32_t gmask = 0xffu << g0, glt = ((1u << lane) - 1u) & gmask;
+  const uint32_t groups = gridDim.x * (COLLAPSE_THREADS / 8);
+  const uint32_t group = (blockIdx.x * COLLAPSE_THREADS + threadIdx.x) >> 3;
+  uint32_t begin = 0, end = 1;
+  for (uint32_t level = 0;; ++level) {
+    // (whole warps run each round: the groups of a warp are consecutive)
+    for (uint32_t w0 = begin + (group & ~3u); w0 < end; w0 += groups) {
+      const uint32_t dst = w0 + (group & 3u);
+      const bool active = dst < end;
+      // candidates
+      uint32_t id = LEAF_BIT, cnt = 0, lc = 0, rc = 0;
+      float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.0f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
+      auto load = [&](uint32_t c) {
+        id = c;
         if (c & LEAF_BIT) {
-          leaves[nlv++] = c & ~LEAF_BIT;
+          cnt = 1u;
         } else {
-          st[sp++] = a.right[c];
-          st[sp++] = a.left[c];
+          cnt = a.count[c];
+          lc = a.left[c];
+          rc = a.right[c];
+        }
+        node_box(c, a.vals, a.plo, a.phi, a.ilo, a.ihi, lo, hi);
+      };
+      int nc = 0;
+      if (active) {
+        const uint32_t src = __ldcg(a.source + dst);
+        nc = !(src & LEAF_BIT) && a.count[src] > 3u ? 2 : 1;
+        if (k < nc) load(nc == 1 ? src : (k ? a.right[src] : a.left[src]));
+      }
+      while (true) {
+        // the openable candidate of largest area (its bits order as the
+        // float), the first of equals
+        const bool open = k < nc && nc < 8 && !(id & LEAF_BIT) && cnt > 3u;
+        uint32_t best = open ? __float_as_uint(box_half_area(lo, hi)) + 1u : 0u;
+        const uint32_t mine = best;
+#pragma unroll
+        for (int m = 1; m <= 4; m <<= 1) best = max(best, __shfl_xor_sync(FULL, best, m));
+        const bool go = best != 0u;
+        if (!__any_sync(FULL, go)) break;
+        const uint32_t at = __ballot_sync(FULL, go && mine == best) & gmask;
+        const int owner = at ? __ffs((int)at) - 1 : lane;
+        const uint32_t l = __shfl_sync(FULL, lc, owner), r = __shfl_sync(FULL, rc, owner);
+        if (go) {
+          if (lane == owner) load(l);
+          else if (k == nc) load(r);
+          ++nc;
         }
       }
-      for (uint32_t q = 0; q < cnt; ++q) {
-        const uint32_t prim = a.vals[leaves[q]];
-        const float* t = a.verts + 9ull * prim;
-        float4* o = a.tris + (size_t)(TRI_BYTES / 16) * (tri_base + toff + q);
-        o[0] = make_float4(t[0], t[1], t[2], __int_as_float((int)prim));
-        o[1] = make_float4(t[3], t[4], t[5], __int_as_float(a.mats ? a.mats[prim] : 0));
-        o[2] = make_float4(t[6], t[7], t[8], 0.0f);
-        o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      // slots: internal children first, then leaves, in candidate order
+      const bool is_int = k < nc && cnt > 3u, is_leaf = k < nc && !is_int;
+      const uint32_t imask = __ballot_sync(FULL, is_int) & gmask, lmask = __ballot_sync(FULL, is_leaf) & gmask;
+      const uint32_t num_int = __popc(imask);
+      const uint32_t slot = is_int ? __popc(imask & glt) : is_leaf ? num_int + __popc(lmask & glt) : (uint32_t)k;
+      uint32_t toff = is_leaf ? cnt : 0u;
+#pragma unroll
+      for (int m = 1; m <= 4; m <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, toff, m, 8);
+        if (k >= m) toff += v;
       }
-      toff += cnt;
+      const uint32_t num_tri = __shfl_sync(FULL, toff, 7, 8);
+      toff -= is_leaf ? cnt : 0u;
+      // node and triangle numbers, one atomic each per warp
+      uint32_t child_base = num_int, tri_base = num_tri;
+#pragma unroll
+      for (int m = 8; m <= 16; m <<= 1) {
+        const uint32_t u = __shfl_up_sync(FULL, child_base, m), v = __shfl_up_sync(FULL, tri_base, m);
+        if (lane >= m) {
+          child_base += u;
+          tri_base += v;
+        }
+      }
+      uint32_t b0 = 0, b1 = 0;
+      if (lane == 31) {
+        if (child_base) b0 = atomicAdd(&a.info->level[level % 3u], child_base);
+        if (tri_base) b1 = atomicAdd(&a.info->tris, tri_base);
+      }
+      child_base += end + __shfl_sync(FULL, b0, 31) - num_int;
+      tri_base += __shfl_sync(FULL, b1, 31) - num_tri;
+      // node frame and grid
+      float p[3] = {lo.x, lo.y, lo.z}, q[3] = {hi.x, hi.y, hi.z};
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+        for (int m = 1; m <= 4; m <<= 1) {
+          p[ax] = fminf(p[ax], __shfl_xor_sync(FULL, p[ax], m));
+          q[ax] = fmaxf(q[ax], __shfl_xor_sync(FULL, q[ax], m));
+        }
+      uint32_t leaves = is_leaf ? ((1u << cnt) - 1u) << (3u * slot) : 0u;
+#pragma unroll
+      for (int m = 1; m <= 4; m <<= 1) leaves |= __shfl_xor_sync(FULL, leaves, m);
+      if (!active) continue;
+      int e[3];
+      uint8_t* bytes = (uint8_t*)a.nodes + (size_t)NODE_BYTES * dst + 32 + slot;
+      const float clo[3] = {lo.x, lo.y, lo.z}, chi[3] = {hi.x, hi.y, hi.z};
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax) {
+        e[ax] = grid_exponent(__fsub_ru(q[ax], p[ax]));
+        // rounded outward: p + 2^e * ql <= lo and p + 2^e * qh >= hi exactly
+        uint32_t ql = 0, qh = 0;
+        if (k < nc) {
+          ql = (uint32_t)fminf(fmaxf(floorf(ldexpf(__fsub_rd(clo[ax], p[ax]), -e[ax])), 0.0f), 255.0f);
+          qh = (uint32_t)fminf(fmaxf(ceilf(ldexpf(__fsub_ru(chi[ax], p[ax]), -e[ax])), 0.0f), 255.0f);
+        }
+        bytes[8 * ax] = (uint8_t)ql;
+        bytes[8 * (3 + ax)] = (uint8_t)qh;
+      }
+      uint4* np = a.nodes + (size_t)(NODE_BYTES / 16) * dst;
+      if (k == 0)
+        np[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), (uint32_t)(e[0] + 127) << 23);
+      if (k == 1)
+        np[1] = make_uint4((uint32_t)(e[1] + 127) << 23, (uint32_t)(e[2] + 127) << 23, child_base, tri_base);
+      if (k == 2) np[5] = make_uint4(leaves | (((1u << num_int) - 1u) << 24), 0u, 0u, 0u);
+      if (is_int) a.source[child_base + slot] = id;
+      if (is_leaf) {
+        // the (at most 3) primitives below, left to right
+        uint32_t leaf[3] = {id, 0u, 0u};
+        if (cnt == 2u) {
+          leaf[0] = lc;
+          leaf[1] = rc;
+        } else if (cnt == 3u) {
+          const bool in_left = !(lc & LEAF_BIT);
+          const uint32_t c = in_left ? lc : rc;
+          const uint32_t x = a.left[c], y = a.right[c];
+          leaf[0] = in_left ? x : lc;
+          leaf[1] = in_left ? y : x;
+          leaf[2] = in_left ? rc : y;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) {
+          if (j >= cnt) break;
+          const uint32_t prim = a.vals[leaf[j] & ~LEAF_BIT];
+          const float* t = a.verts + 9ull * prim;
+          float4* o = a.tris + (size_t)(TRI_BYTES / 16) * (tri_base + toff + j);
+          o[0] = make_float4(t[0], t[1], t[2], __int_as_float((int)prim));
+          o[1] = make_float4(t[3], t[4], t[5], __int_as_float(a.mats ? a.mats[prim] : 0));
+          o[2] = make_float4(t[6], t[7], t[8], 0.0f);
+          o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+      }
+    }
+    // The nodes a level took are counted in one of three words, so that the
+    // count stands still once the level is over: block 0 clears the next
+    // level's, which all blocks read two barriers ago.
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.info->level[(level + 1u) % 3u] = 0u;
+    if (!collapse_barrier(a.info, level)) return;
+    begin = end;
+    end += __ldcg(&a.info->level[level % 3u]);
+    if (begin == end) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.info->nodes = end;
+        a.info->depth = level + 1u;
+      }
+      return;
     }
   }
-  auto pack4 = [](const uint8_t* b) {
-    return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
-  };
-  auto scale = [&](int ax) { return (uint32_t)(e[ax] + 127) << 23; };  // 2^e
-  uint4* np = a.nodes + (size_t)(NODE_BYTES / 16) * dst;
-  np[0] = make_uint4(__float_as_uint(p[0]), __float_as_uint(p[1]), __float_as_uint(p[2]), scale(0));
-  np[1] = make_uint4(scale(1), scale(2), child_base, tri_base);
-  np[2] = make_uint4(pack4(qlo[0]), pack4(qlo[0] + 4), pack4(qlo[1]), pack4(qlo[1] + 4));
-  np[3] = make_uint4(pack4(qlo[2]), pack4(qlo[2] + 4), pack4(qhi[0]), pack4(qhi[0] + 4));
-  np[4] = make_uint4(pack4(qhi[1]), pack4(qhi[1] + 4), pack4(qhi[2]), pack4(qhi[2] + 4));
-  np[5] = make_uint4(leaves | (((1u << num_int) - 1u) << 24), 0u, 0u, 0u);
+}
+
+// Start values of a build: the tables that count up, the bounds, node 0 (the
+// root).
+__global__ void k_build_init(uint32_t* zero, uint64_t words, BvhDeviceInfo* info, uint32_t* source, uint32_t root) {
+  for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    BvhDeviceInfo b;
+    b.nodes = b.tris = b.depth = b.failed = b.barrier = 0u;
+    for (int k = 0; k < 3; ++k) b.level[k] = 0u;
+    for (int k = 0; k < 12; ++k) b.bounds[k] = (k / 3) & 1 ? (int)0x80000000 : 0x7fffffff;  // max, min
+    for (int k = 0; k < RS_PASSES; ++k) b.ticket[k] = 0u;
+    *info = b;
+    source[0] = root;
+  }
 }
 
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 }  // namespace
-
-Status device_exclusive_scan(uint32_t* d, uint64_t m, uint32_t* tmp, cudaStream_t s) {
-  const uint32_t nb = cdiv(m, SCAN_CHUNK);
-  k_scan_blocks<<<nb, SCAN_THREADS, 0, s>>>(d, m, tmp);
-  k_scan_single<<<1, SCAN_THREADS, 0, s>>>(tmp, nb);
-  k_scan_add<<<nb, SCAN_THREADS, 0, s>>>(d, m, tmp);
-  LISA_CUDA(cudaGetLastError());
-  return Status();
-}
-
-// Sorts (keys, vals) by the low 32 bits of keys; stable.  Result in keys/vals.
-Status device_radix_sort(uint32_t* keys, uint32_t* vals, uint32_t* keys2, uint32_t* vals2, uint32_t n,
-                         uint32_t* hist, uint32_t* scan_tmp, int bits, cudaStream_t s) {
-  const uint32_t tiles = cdiv(n, RS_TILE);
-  uint32_t *ki = keys, *vi = vals, *ko = keys2, *vo = vals2;
-  for (int shift = 0; shift < bits; shift += 8) {
-    k_rs_hist<<<tiles, RS_THREADS, 0, s>>>(ki, n, shift, hist, tiles);
-    LISA_TRY(device_exclusive_scan(hist, 256ull * tiles, scan_tmp, s));
-    k_rs_scatter<<<tiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, hist, tiles);
-    LISA_CUDA(cudaGetLastError());
-    std::swap(ki, ko);
-    std::swap(vi, vo);
-  }
-  if (ki != keys) {
-    LISA_CUDA(cudaMemcpyAsync(keys, ki, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-    LISA_CUDA(cudaMemcpyAsync(vals, vi, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-  }
-  return Status();
-}
 
 namespace {
 template <class T>
@@ -834,19 +926,6 @@ Status take(ScratchSource& src, T** p, uint64_t count, const char* what) {
 inline uint64_t al256(uint64_t b) { return (std::max<uint64_t>(b, 16) + 255) & ~255ull; }
 }  // namespace
 
-size_t bvh_temp_bytes(uint32_t n) {
-  const uint64_t tiles = cdiv(n, RS_TILE);
-  uint64_t b = 0;
-  b += 4 * al256(16ull * n);                                   // plo phi ilo ihi
-  b += 4 * al256(4ull * n);                                    // keys vals keys2 vals2
-  b += al256(4ull * 256 * tiles) + al256(4ull * (cdiv(256ull * tiles, SCAN_CHUNK) + 16));
-  b += 7 * al256(4ull * n);                                    // tree links and flags
-  b += al256(16) + al256(48);                                  // counters, bounds
-  b += al256(4ull * 32);                                       // collapse level counts
-  b += 2 * al256(8ull * (n + 1));                              // collapse work lists
-  return (size_t)b;
-}
-
 // Most 8-wide nodes that n triangles can give.  A node with an internal
 // child has eight children (the collapse opens candidates until there are
 // eight or none is left to open), the others (T, below F such nodes) hold at
@@ -854,28 +933,32 @@ size_t bvh_temp_bytes(uint32_t n) {
 // n >= 4 T + 7 F - T + 1 >= 3 (F + T) + 1.
 static uint32_t max_nodes(uint32_t n) { return n / 3 + 1; }
 
+static uint32_t sort_tiles(uint32_t n) { return cdiv(n, (uint64_t)RS_THREADS * rs_rounds(n)); }
+// Words of the tables that a build counts up in: look-back states and digit
+// histograms of the sort, arrival flags of the bottom-up pass.
+static uint64_t counted_words(uint32_t n) { return (uint64_t)RS_PASSES * 256 * (sort_tiles(n) + 1) + n; }
+
+size_t bvh_temp_bytes(uint32_t n) {
+  uint64_t b = 0;
+  b += 4 * al256(16ull * n);                // plo phi ilo ihi
+  b += 4 * al256(4ull * n);                 // keys vals keys2 vals2
+  b += 6 * al256(4ull * n);                 // tree links, counts and costs
+  b += al256(4ull * counted_words(n));
+  b += al256(4ull * max_nodes(n));          // collapse work list
+  b += al256(sizeof(BvhDeviceInfo));
+  return (size_t)b;
+}
+
 size_t bvh_output_bytes(uint32_t n) {
   return (size_t)(al256((uint64_t)NODE_BYTES * max_nodes(n)) + al256((uint64_t)TRI_BYTES * n));
 }
 
-Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
-                 uint4** d_nodes, float4** d_tris, BvhBuildResult* info, const int32_t* d_mat, bool refine) {
-  auto t0 = std::chrono::steady_clock::now();
-  if (n == 0) {
-    *d_nodes = nullptr;
-    *d_tris = nullptr;
-    info->num_nodes = 0;
-    info->num_tri_slots = 0;
-    info->depth = 0;
-    for (int k = 0; k < 3; ++k) info->bmin[k] = info->bmax[k] = 0.0f;
-    return Status();
-  }
+Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
+                   uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info, const int32_t* d_mat, bool refine) {
   float4 *plo, *phi, *ilo, *ihi;
-  uint32_t *keys, *vals, *keys2, *vals2, *hist, *scan_tmp;
-  uint32_t *left, *right, *first, *last, *par_int, *par_leaf, *flags, *counters;
-  int* bounds;
-  uint2 *work0, *work1;
-  const uint32_t tiles = cdiv(n, RS_TILE);
+  uint32_t *keys, *vals, *keys2, *vals2;
+  uint32_t *left, *right, *first, *last, *par_int, *par_leaf, *counted, *source;
+  BvhDeviceInfo* info;
   const char* w = "bvh build scratch";
   LISA_TRY(take(tmp, &plo, n, w));
   LISA_TRY(take(tmp, &phi, n, w));
@@ -885,97 +968,103 @@ Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource
   LISA_TRY(take(tmp, &vals, n, w));
   LISA_TRY(take(tmp, &keys2, n, w));
   LISA_TRY(take(tmp, &vals2, n, w));
-  LISA_TRY(take(tmp, &hist, 256ull * tiles, w));
-  LISA_TRY(take(tmp, &scan_tmp, cdiv(256ull * tiles, SCAN_CHUNK) + 16, w));
   LISA_TRY(take(tmp, &left, n, w));
   LISA_TRY(take(tmp, &right, n, w));
   LISA_TRY(take(tmp, &first, n, w));
   LISA_TRY(take(tmp, &last, n, w));
   LISA_TRY(take(tmp, &par_int, n, w));
   LISA_TRY(take(tmp, &par_leaf, n, w));
-  LISA_TRY(take(tmp, &flags, n, w));
-  LISA_TRY(take(tmp, &counters, 4, w));
-  uint32_t* levels = nullptr;
-  LISA_TRY(take(tmp, &levels, 32, w));
-  LISA_TRY(take(tmp, &bounds, 12, w));
-  LISA_TRY(take(tmp, &work0, n + 1, w));
-  LISA_TRY(take(tmp, &work1, n + 1, w));
+  LISA_TRY(take(tmp, &counted, counted_words(n), w));
+  LISA_TRY(take(tmp, &source, max_nodes(n), w));
+  LISA_TRY(take(tmp, &info, 1, w));
+  uint4* nodes = nullptr;
+  float4* tris = nullptr;
+  LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), "bvh nodes"));
+  LISA_TRY(take(out, &tris, (uint64_t)(TRI_BYTES / 16) * n, "bvh triangles"));
+  int dev = 0, sms = 0;
+  LISA_CUDA(cudaGetDevice(&dev));
+  LISA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 
-  int hb[12];
-  for (int k = 0; k < 3; ++k) {
-    hb[k] = 0x7fffffff;
-    hb[3 + k] = (int)0x80000000;
-    hb[6 + k] = 0x7fffffff;
-    hb[9 + k] = (int)0x80000000;
+  const uint32_t root = n > 1 ? 0u : LEAF_BIT;
+  k_build_init<<<std::min<uint32_t>(cdiv(counted_words(n), 1024), (uint32_t)sms * 8u), 256, 0, s>>>(
+      counted, counted_words(n), info, source, root);
+  k_prim_bounds<<<std::min<uint32_t>(cdiv(n, 256), (uint32_t)sms * 8u), 256, 0, s>>>(d_verts, n, plo, phi, info->bounds);
+  k_morton<<<cdiv(n, 256), 256, 0, s>>>(plo, phi, n, info->bounds, keys, vals);
+  const uint32_t tiles = sort_tiles(n);
+  uint32_t* hist = counted + (uint64_t)RS_PASSES * 256 * tiles;
+  uint32_t* flags = hist + RS_PASSES * 256;
+  k_rs_hist<<<std::min<uint32_t>(cdiv(n, RS_THREADS), (uint32_t)sms * 4u), RS_THREADS, 0, s>>>(keys, n, hist);
+  for (int p = 0; p < RS_PASSES; ++p) {
+    const uint32_t *ki = p & 1 ? keys2 : keys, *vi = p & 1 ? vals2 : vals;
+    uint32_t *ko = p & 1 ? keys : keys2, *vo = p & 1 ? vals : vals2;
+    uint32_t* look = counted + (uint64_t)p * 256 * tiles;
+    if (rs_rounds(n) == 4)
+      k_rs_pass<4><<<tiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, 8 * p, hist + 256 * p, look, &info->ticket[p],
+                                                &info->failed);
+    else
+      k_rs_pass<16><<<tiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, 8 * p, hist + 256 * p, look, &info->ticket[p],
+                                                 &info->failed);
   }
-  LISA_CUDA(cudaMemcpyAsync(bounds, hb, sizeof(hb), cudaMemcpyHostToDevice, s));
-  const int nblk = (int)std::min<uint32_t>(cdiv(n, 256), 4096);
-  k_prim_bounds<<<nblk, 256, 0, s>>>(d_verts, n, plo, phi, bounds);
-  k_morton<<<cdiv(n, 256), 256, 0, s>>>(plo, phi, n, bounds, keys, vals);
   LISA_CUDA(cudaGetLastError());
-  LISA_TRY(device_radix_sort(keys, vals, keys2, vals2, n, hist, scan_tmp, 32, s));
   if (n > 1) {
     k_karras<<<cdiv(n - 1, 256), 256, 0, s>>>(keys, n, left, right, first, last, par_int, par_leaf);
-    LISA_CUDA(cudaMemsetAsync(flags, 0, sizeof(uint32_t) * n, s));
     // boxes, counts and SAH costs bottom up, with treelet restructuring
     // unless refine is off; first/last become count/cost
     const SahTree st{n, vals, plo, phi, par_leaf, par_int, left, right, ilo, ihi, first, (float*)last, flags};
     k_bottom_up_sah<<<cdiv(n, SAH_THREADS), SAH_THREADS, 0, s>>>(st, refine ? 1 : 0);
     LISA_CUDA(cudaGetLastError());
   }
-  // outputs
+  int occ = 0;
+  LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_collapse, COLLAPSE_THREADS, 0));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min<uint32_t>(cdiv(n, 256), (uint32_t)(sms * std::max(occ, 1))));
+  cfg.blockDim = dim3(COLLAPSE_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const CollapseArgs a{n, vals, plo, phi, ilo, ihi, left, right, first, d_verts, d_mat, nodes, tris, source, info};
+  LISA_CUDA(cudaLaunchKernelEx(&cfg, k_collapse, a));
+  *d_nodes = nodes;
+  *d_tris = tris;
+  *d_info = info;
+  return Status();
+}
+
+Status bvh_result(const BvhDeviceInfo& h, uint32_t n, BvhBuildResult* info) {
+  if (h.failed) return Status(LISA_ERR_DEVICE, "bvh build: a device-side wait ran out");
+  if (h.tris != n) return Status(LISA_ERR_DEVICE, "bvh build: leaf triangle count mismatch");
+  info->num_nodes = h.nodes;
+  info->num_tri_slots = h.tris;
+  info->depth = h.depth;
+  for (int k = 0; k < 3; ++k) {
+    info->bmin[k] = ord2f(h.bounds[k]);
+    info->bmax[k] = ord2f(h.bounds[3 + k]);
+  }
+  return Status();
+}
+
+Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
+                 uint4** d_nodes, float4** d_tris, BvhBuildResult* info, const int32_t* d_mat, bool refine) {
+  auto t0 = std::chrono::steady_clock::now();
+  *d_nodes = nullptr;
+  *d_tris = nullptr;
+  if (n == 0) {
+    info->num_nodes = 0;
+    info->num_tri_slots = 0;
+    info->depth = 0;
+    for (int k = 0; k < 3; ++k) info->bmin[k] = info->bmax[k] = 0.0f;
+    return Status();
+  }
   uint4* nodes = nullptr;
   float4* tris = nullptr;
-  LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), "bvh nodes"));
-  LISA_TRY(take(out, &tris, (uint64_t)(TRI_BYTES / 16) * n, "bvh triangles"));
-  const uint2 root = make_uint2(0u, n > 1 ? 0u : LEAF_BIT);
-  k_collapse_init<<<1, 1, 0, s>>>(counters, levels, work0, root);
-  LISA_CUDA(cudaGetLastError());
-  CollapseArgs a{n, vals, plo, phi, ilo, ihi, left, right, first, d_verts, d_mat, nodes, tris, counters};
-  // a level holds at most one work item per 8-wide node, fewer than n/2
-  int dev = 0, sms = 0;
-  LISA_CUDA(cudaGetDevice(&dev));
-  LISA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const uint32_t cgrid = std::max<uint32_t>(1u, std::min<uint32_t>(cdiv(n / 2 + 1, 64), (uint32_t)sms * 16u));
-  for (int l = 0; l < COLLAPSE_LAUNCHES; ++l)
-    k_collapse<<<cgrid, 64, 0, s>>>(a, (l & 1) ? work1 : work0, levels + l, (l & 1) ? work0 : work1,
-                                    levels + l + 1);
-  LISA_CUDA(cudaGetLastError());
-  uint32_t hc[2];
-  uint32_t hl[COLLAPSE_LAUNCHES + 1];
-  LISA_CUDA(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, s));
-  LISA_CUDA(cudaMemcpyAsync(hl, levels, sizeof(hl), cudaMemcpyDeviceToHost, s));
-  LISA_CUDA(cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, s));
+  BvhDeviceInfo *d_info = nullptr, h;
+  LISA_TRY(enqueue_bvh(d_verts, n, s, tmp, out, &nodes, &tris, &d_info, d_mat, refine));
+  LISA_CUDA(cudaMemcpyAsync(&h, d_info, sizeof(h), cudaMemcpyDeviceToHost, s));
   LISA_CUDA(cudaStreamSynchronize(s));
-  uint32_t depth = 0;
-  while (depth < (uint32_t)COLLAPSE_LAUNCHES && hl[depth] > 0) ++depth;
-  if (depth == (uint32_t)COLLAPSE_LAUNCHES && hl[COLLAPSE_LAUNCHES] > 0) {
-    // a tree deeper than the fixed launches: the remaining levels, one host
-    // round trip each (slot C holds the level's count, slot C+1 the next's)
-    uint32_t* cur = levels + COLLAPSE_LAUNCHES;
-    uint32_t nwork = hl[COLLAPSE_LAUNCHES];
-    uint2 *wi = (COLLAPSE_LAUNCHES & 1) ? work1 : work0, *wo = (COLLAPSE_LAUNCHES & 1) ? work0 : work1;
-    while (nwork > 0) {
-      LISA_CUDA(cudaMemsetAsync(cur + 1, 0, sizeof(uint32_t), s));
-      k_collapse<<<cdiv(nwork, 64), 64, 0, s>>>(a, wi, cur, wo, cur + 1);
-      LISA_CUDA(cudaGetLastError());
-      LISA_CUDA(cudaMemcpyAsync(cur, cur + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-      LISA_CUDA(cudaMemcpyAsync(&nwork, cur + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      LISA_CUDA(cudaStreamSynchronize(s));
-      std::swap(wi, wo);
-      ++depth;
-    }
-    LISA_CUDA(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, s));
-    LISA_CUDA(cudaStreamSynchronize(s));
-  }
-  if (hc[1] != n) return Status(LISA_ERR_DEVICE, "bvh build: leaf triangle count mismatch");
-  info->num_nodes = hc[0];
-  info->num_tri_slots = hc[1];
-  info->depth = depth;
-  for (int k = 0; k < 3; ++k) {
-    info->bmin[k] = ord2f(hb[k]);
-    info->bmax[k] = ord2f(hb[3 + k]);
-  }
+  LISA_TRY(bvh_result(h, n, info));
   *d_nodes = nodes;
   *d_tris = tris;
   info->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -57,6 +57,7 @@ enum StatusBits : uint32_t {
   ST_GUIDE_NONFINITE = 8u,
   // 16: a bounded tensor-core wait ran out (LISA_STATUS_WAIT_TIMEOUT)
   ST_BOUNDS = 32u,  // bounds-checked builds: a BVH or triangle index out of range
+  ST_BVH_BUILD = 64u,  // a BVH built and traced without the host in between failed to build
 };
 
 // Bounds-checked builds (-DLISA_BOUNDS, a stand-in for a memory checker):

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <map>
 #include <memory>
 #include <string>
@@ -116,6 +117,27 @@ struct BvhBuildResult {
   float bmin[3], bmax[3];
 };
 
+// What a build leaves on the device, for the host and for kernels that
+// follow it on the stream.
+struct BvhDeviceInfo {
+  uint32_t nodes;      // 8-wide nodes
+  uint32_t tris;       // leaf triangles written
+  uint32_t depth;
+  uint32_t failed;     // a bounded wait ran out
+  int bounds[12];      // scene min, max and centroid min, max, as order-preserving ints
+  uint32_t level[3];   // nodes taken by the collapse's current level (in turn)
+  uint32_t barrier;    // arrivals of the collapse's blocks
+  uint32_t ticket[4];  // tiles started, per sort pass
+};
+
+// The float of an order-preserving int.
+__host__ __device__ inline float ord2f(int i) {
+  const int j = i >= 0 ? i : i ^ 0x7fffffff;
+  float f;
+  memcpy(&f, &j, 4);
+  return f;
+}
+
 // Builds the 8-wide compressed BVH of `num_prims` triangles whose vertices
 // are d_verts (3 float3 per triangle, device).  Temporaries come from `tmp`,
 // the node and leaf-triangle arrays from `out`.  With d_mat (one material
@@ -125,6 +147,12 @@ struct BvhBuildResult {
 Status build_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, ScratchSource& tmp,
                  ScratchSource& out, uint4** d_nodes, float4** d_tris, BvhBuildResult* info,
                  const int32_t* d_mat = nullptr, bool refine = true);
+// The same without waiting for it (num_prims > 0): bvh_result checks and
+// unpacks *d_info once the stream has run.
+Status enqueue_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, ScratchSource& tmp,
+                   ScratchSource& out, uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info,
+                   const int32_t* d_mat, bool refine);
+Status bvh_result(const BvhDeviceInfo& h, uint32_t num_prims, BvhBuildResult* info);
 // Device bytes build_bvh takes from `tmp` and from `out` for n triangles.
 size_t bvh_temp_bytes(uint32_t n);
 size_t bvh_output_bytes(uint32_t n);
@@ -235,9 +263,11 @@ Status trace_rays(Renderer& r, const float* d_rays, uint32_t n, int32_t* d_prim,
                   bool brute);
 Status trace_count(Renderer& r, const float* d_rays, uint32_t n, uint64_t* visits, uint64_t* tests);
 // Closest hit (or brute force) of n device rays against the scene d_scene;
-// d_ctrl receives the device status word.  Synchronises `s`.
+// d_ctrl receives the device status word (cleared: the stream has cleared it
+// already).  Synchronises `s`.
 Status launch_trace_closest(const SceneDev* d_scene, WaveCtrl* d_ctrl, const float* d_rays, uint32_t n,
-                            int32_t* d_prim, float* d_t, cudaStream_t s, int sm_count, bool brute);
+                            int32_t* d_prim, float* d_t, cudaStream_t s, int sm_count, bool brute,
+                            bool cleared = false);
 
 // error string per thread (api.cu)
 void set_last_error(const Status& s);

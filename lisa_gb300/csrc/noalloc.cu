@@ -57,6 +57,34 @@ std::mutex g_mu;
 ScratchEntry g_scratch[MAX_CONTEXTS] = {};
 int g_scratch_used = 0, g_scratch_next = 0;
 
+// The scene record of a soup whose BVH the stream has just built, and a
+// clear status word.  A build that failed sets its status bit and leaves an
+// empty scene, which every ray misses.
+__global__ void k_soup_scene(SceneDev* out, WaveCtrl* ctrl, const uint4* nodes, const float4* tris,
+                             uint32_t num_triangles, const BvhDeviceInfo* info) {
+  SceneDev h = {};
+  h.nodes = nodes;
+  h.tris = tris;
+  h.num_prims = num_triangles;
+  h.extent = 1.0f;
+  uint32_t status = 0;
+  if (info) {
+    if (info->failed != 0u || info->tris != num_triangles) {
+      status = ST_BVH_BUILD;
+    } else {
+      h.num_nodes = info->nodes;
+      double e2 = 0.0;
+      for (int k = 0; k < 3; ++k) {
+        const double d = (double)(ord2f(info->bounds[3 + k]) - ord2f(info->bounds[k]));
+        e2 += d * d;
+      }
+      if (e2 > 0.0 && e2 < 1e76) h.extent = (float)sqrt(e2);
+    }
+  }
+  *out = h;
+  ctrl->status = status;
+}
+
 // Device address of the scratch array in the current context (looked up
 // once per context).
 Status scratch_address(void** out) {
@@ -107,22 +135,16 @@ Status trace_soup_noalloc(const float* d_vertices, uint32_t num_triangles, const
   WaveCtrl* d_ctrl = nullptr;
   LISA_TRY(region.get((void**)&d_scene, sizeof(SceneDev), "scene record"));
   LISA_TRY(region.get((void**)&d_ctrl, sizeof(WaveCtrl), "status word"));
+  // build, scene record and rays follow one another on the stream; the host
+  // waits once, for the status word that tells of all three
   uint4* nodes = nullptr;
   float4* tris = nullptr;
-  BvhBuildResult info;
-  LISA_TRY(build_bvh(d_vertices, num_triangles, stream, region, region, &nodes, &tris, &info));
-  SceneDev h;
-  std::memset(&h, 0, sizeof(h));
-  h.nodes = nodes;
-  h.tris = tris;
-  h.num_prims = num_triangles;
-  h.num_nodes = info.num_nodes;
-  double e2 = 0.0;
-  for (int k = 0; k < 3; ++k) e2 += (double)(info.bmax[k] - info.bmin[k]) * (info.bmax[k] - info.bmin[k]);
-  h.extent = (e2 > 0.0 && e2 < 1e76) ? (float)std::sqrt(e2) : 1.0f;
-  LISA_CUDA(cudaMemcpyAsync(d_scene, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
-  // launch_trace_closest clears the status word before tracing
-  return launch_trace_closest(d_scene, d_ctrl, d_rays, num_rays, d_prim, d_t, stream, sm, false);
+  BvhDeviceInfo* d_info = nullptr;
+  if (num_triangles)
+    LISA_TRY(enqueue_bvh(d_vertices, num_triangles, stream, region, region, &nodes, &tris, &d_info, nullptr, true));
+  k_soup_scene<<<1, 1, 0, stream>>>(d_scene, d_ctrl, nodes, tris, num_triangles, d_info);
+  LISA_CUDA(cudaGetLastError());
+  return launch_trace_closest(d_scene, d_ctrl, d_rays, num_rays, d_prim, d_t, stream, sm, false, true);
 }
 
 }  // namespace

@@ -2147,9 +2147,9 @@ Status renderer_get_ppm(Renderer& r, int scene, uint8_t* rgb8) {
 }
 
 Status launch_trace_closest(const SceneDev* d_scene, WaveCtrl* d_ctrl, const float* d_rays, uint32_t n,
-                            int32_t* d_prim, float* d_t, cudaStream_t s, int sm_count, bool brute) {
+                            int32_t* d_prim, float* d_t, cudaStream_t s, int sm_count, bool brute, bool cleared) {
   if (n == 0) return Status();
-  LISA_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(WaveCtrl), s));
+  if (!cleared) LISA_CUDA(cudaMemsetAsync(d_ctrl, 0, sizeof(WaveCtrl), s));
   const uint32_t blocks = std::min<uint32_t>((n + 127) / 128, (uint32_t)sm_count * 16);
   if (brute) {
     k_brute_rays<<<blocks, 128, 0, s>>>(d_scene, d_rays, n, d_prim, d_t);
