@@ -134,7 +134,9 @@ typedef struct lisa_options {
                                 waves (0 = fill the wavefront)                */
   uint32_t refill_idle;      /* persistent traversal kernels take new work once
                                 this many of a warp's 32 lanes are idle
-                                (1..32; 0 = 12)                               */
+                                (1..32; 0 = 12; the closest-hit kernel four
+                                fewer, the emitter search four more, whole
+                                paths eight more)                             */
   uint32_t estimator;        /* LISA_ESTIMATOR_*                               */
   uint32_t bvh_lbvh_only;    /* 1 = keep the plain LBVH: skip its SAH treelet
                                 restructuring before the 8-wide collapse      */
@@ -158,7 +160,7 @@ typedef struct lisa_render_stats {
   uint64_t samples_total;      /* samples per pixel accumulated so far        */
   double ms_device;            /* CUDA-event time of the whole call            */
   double ms_trace;             /* stage sums (only with stage_timing)          */
-  double ms_shade;
+  double ms_shade;             /* 0: shading is part of the emitter search     */
   double ms_nee;
   double ms_guide;
   double ms_other;

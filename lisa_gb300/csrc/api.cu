@@ -389,8 +389,9 @@ __global__ void k_emit_of_prim(int32_t* m, uint32_t n, const int32_t* em, uint32
 // scene-wide indices).
 __global__ void k_emit_global_ids(float4* tris, uint32_t n, const int32_t* __restrict__ global) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    float4& v0 = tris[(TRI_BYTES / 16) * (size_t)k];
-    v0.w = __int_as_float(global[__float_as_int(v0.w)]);
+    float4* t = tris + (TRI_BYTES / 16) * (size_t)k;
+    const float id = __int_as_float(global[__float_as_int(t[0].w)]);
+    t[0].w = t[1].w = t[2].w = id;
   }
 }
 
@@ -661,9 +662,11 @@ Status renderer_create(const lisa_renderer_params* scenes, int n, const lisa_opt
   LISA_TRY(r->arena.alloc((void**)&r->ps_att, sizeof(float4) * W, "path state"));
   LISA_TRY(r->arena.alloc((void**)&r->ps_col, sizeof(float4) * W, "path state"));
   LISA_TRY(r->arena.alloc((void**)&r->ps_rng, sizeof(uint32_t) * W, "path state"));
-  LISA_TRY(r->arena.alloc((void**)&r->nee_a, sizeof(float4) * W, "emitter queue"));
-  LISA_TRY(r->arena.alloc((void**)&r->nee_b, sizeof(float4) * W, "emitter queue"));
-  LISA_TRY(r->arena.alloc((void**)&r->nee_c, sizeof(float4) * W, "emitter queue"));
+  if (r->opts.mode == LISA_MODE_GUIDED) {  // the vertices that the guide's inference reads
+    LISA_TRY(r->arena.alloc((void**)&r->nee_a, sizeof(float4) * W, "emitter queue"));
+    LISA_TRY(r->arena.alloc((void**)&r->nee_b, sizeof(float4) * W, "emitter queue"));
+    LISA_TRY(r->arena.alloc((void**)&r->nee_c, sizeof(float4) * W, "emitter queue"));
+  }
   LISA_TRY(r->arena.alloc((void**)&r->ctrl, sizeof(WaveCtrl), "control block"));
   LISA_CUDA(cudaMemsetAsync(r->ctrl, 0, sizeof(WaveCtrl), r->stream));
   if (r->opts.mode == LISA_MODE_GUIDED) LISA_TRY(guide_renderer_init(*r));

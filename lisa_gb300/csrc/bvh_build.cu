@@ -872,10 +872,11 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
           const uint32_t prim = a.vals[leaf[j] & ~LEAF_BIT];
           const float* t = a.verts + 9ull * prim;
           float4* o = a.tris + (size_t)(TRI_BYTES / 16) * (tri_base + toff + j);
-          o[0] = make_float4(t[0], t[1], t[2], __int_as_float((int)prim));
-          o[1] = make_float4(t[3], t[4], t[5], __int_as_float(a.mats ? a.mats[prim] : 0));
-          o[2] = make_float4(t[6], t[7], t[8], 0.0f);
-          o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float id = __int_as_float((int)prim);
+          o[0] = make_float4(t[0], t[3], t[6], id);
+          o[1] = make_float4(t[1], t[4], t[7], id);
+          o[2] = make_float4(t[2], t[5], t[8], id);
+          o[3] = make_float4(__int_as_float(a.mats ? a.mats[prim] : 0), 0.0f, 0.0f, 0.0f);
         }
       }
     }

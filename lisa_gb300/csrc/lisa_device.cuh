@@ -12,15 +12,17 @@
 //            triangles says that leaf child c has a q-th triangle (at most
 //            3); the node's triangles lie one after another from tri_base.
 //            An empty slot has none of these bits.
-//   tris   : 4 x float4 per leaf triangle slot, in leaf order:
-//            (v0.xyz, original triangle id as int bits),
-//            (v1, its material if that is an emitter, else -1), (v2, 0), 0
-//            -- 64 B, so a triangle is a 32- and a 16-byte load
+//   tris   : 4 x float4 per leaf triangle slot, in leaf order: the three
+//            vertices' x, y and z, each with the original triangle id as int
+//            bits, and (material if that is an emitter, else -1; 0 0 0).  One
+//            float4 per axis, so the triangle test loads the ray's shear axes
+//            by address and selects nothing
 //   prims  : 5 x float4 per original triangle (shading record):
 //            (v0, n0.x) (v1, n0.y) (v2, n0.z) (n1, n2.x) (n2.y, n2.z, mat, 0)
 //   mats   : DevMaterial, 48 B each
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -128,7 +130,7 @@ struct WaveDesc {
   WaveGroup groups[MAX_GROUPS];
 };
 
-enum { HEAD_TRACE = 0, HEAD_SHADE = 1, HEAD_NEE = 2, HEAD_GUIDE = 3 };
+enum { HEAD_TRACE = 0, HEAD_NEE = 2 };
 struct WaveCtrl {
   uint32_t qcount[2];
   uint32_t nee_count;
@@ -159,19 +161,22 @@ struct RayPre {
   float ix, iy, iz;  // 1/d per axis
   float slack;       // absolute slack on the best distance, in t units
 };
-// The shear of the triangle test, along the axis kz of the largest |d|.
+// The shear of the triangle test, along the axis kz of the largest |d|, and
+// the origin on the shear's axes kx = kz + 1, ky = kz + 2 (mod 3), kz.
 struct RayShear {
   float Sx, Sy, Sz;
   int kz;
+  V3 o;
 };
 
-// Components of a vector on the shear's axes: kx = kz + 1, ky = kz + 2
-// (mod 3).  The published test swaps kx and ky for a negative d[kz] to keep
-// the winding; that negates U, V, W, det and T exactly (each is a
-// difference or a sum of products) and leaves t as it is, so here they stay.
-__device__ __forceinline__ float on_kx(float x, float y, float z, int kz) { return kz == 0 ? y : (kz == 1 ? z : x); }
-__device__ __forceinline__ float on_ky(float x, float y, float z, int kz) { return kz == 0 ? z : (kz == 1 ? x : y); }
-__device__ __forceinline__ float on_kz(float x, float y, float z, int kz) { return kz == 0 ? x : (kz == 1 ? y : z); }
+// Components of a vector on the shear's axes.  The published test swaps kx
+// and ky for a negative d[kz] to keep the winding; that negates U, V, W, det
+// and T exactly (each is a difference or a sum of products) and leaves t as
+// it is, so here they stay.
+__device__ __forceinline__ V3 on_shear_axes(V3 v, int kz) {
+  return v3(kz == 0 ? v.y : (kz == 1 ? v.z : v.x), kz == 0 ? v.z : (kz == 1 ? v.x : v.y),
+            kz == 0 ? v.x : (kz == 1 ? v.y : v.z));
+}
 
 __device__ __forceinline__ void ray_prepare(V3 o, V3 d, float extent, RayPre& r, RayShear& h) {
   r.ox = o.x;
@@ -179,22 +184,24 @@ __device__ __forceinline__ void ray_prepare(V3 o, V3 d, float extent, RayPre& r,
   r.oz = o.z;
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   const int kz = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
-  const float dz = on_kz(d.x, d.y, d.z, kz);
+  const V3 dk = on_shear_axes(d, kz);
   h.kz = kz;
-  h.Sx = fdiv(on_kx(d.x, d.y, d.z, kz), dz);
-  h.Sy = fdiv(on_ky(d.x, d.y, d.z, kz), dz);
+  h.o = on_shear_axes(o, kz);
+  h.Sx = fdiv(dk.x, dk.z);
+  h.Sy = fdiv(dk.y, dk.z);
   // __frcp_rn is the correctly rounded 1/x, the same value as 1.0f/x: the
   // shear's 1/dz, and the node-culling reciprocal of that (dominant) axis
-  h.Sz = __frcp_rn(dz);
+  h.Sz = __frcp_rn(dk.z);
   // The other two axes' reciprocals serve node culling only; __fdividef is
   // within 2 ulp there, which the slab padding covers (see trav_node).  A
-  // zero or vanishing component takes a huge finite reciprocal of its sign
-  // instead of infinity: the node test then keeps that axis's slab (the
-  // ray's constant coordinate against the padded box) instead of turning it
-  // into NaN and dropping it, which made such rays visit most of the tree.
-  const float qx = ax > 1e-30f ? __fdividef(1.0f, d.x) : copysignf(1e30f, d.x);
-  const float qy = ay > 1e-30f ? __fdividef(1.0f, d.y) : copysignf(1e30f, d.y);
-  const float qz = az > 1e-30f ? __fdividef(1.0f, d.z) : copysignf(1e30f, d.z);
+  // zero or vanishing component's is limited to 1e20 of the dominant one's:
+  // the node test then keeps that axis's slab (the ray's constant coordinate
+  // against the padded box) instead of turning it into NaN and dropping it,
+  // which made such rays visit most of the tree.
+  const float most = 1e20f * fabsf(h.Sz);
+  const float qx = copysignf(fminf(fabsf(__fdividef(1.0f, d.x)), most), d.x);
+  const float qy = copysignf(fminf(fabsf(__fdividef(1.0f, d.y)), most), d.y);
+  const float qz = copysignf(fminf(fabsf(__fdividef(1.0f, d.z)), most), d.z);
   r.ix = kz == 0 ? h.Sz : qx;
   r.iy = kz == 1 ? h.Sz : qy;
   r.iz = kz == 2 ? h.Sz : qz;
@@ -202,18 +209,15 @@ __device__ __forceinline__ void ray_prepare(V3 o, V3 d, float extent, RayPre& r,
   r.slack = __fdividef(3.814697265625e-6f * extent, fmaxf(ax, fmaxf(ay, az)));
 }
 
-// Returns t of the hit (or +inf).  prim_t < tbest test is the caller's.
-__device__ __forceinline__ float intersect_tri(V3 o, const RayShear& h, V3 va, V3 vb, V3 vc, float tmin) {
+// Returns t of the hit (or +inf) of the triangle whose vertices are a, b, c
+// on the shear's axes.  prim_t < tbest test is the caller's.
+__device__ __forceinline__ float intersect_tri(const RayShear& h, V3 va, V3 vb, V3 vc, float tmin) {
   // translate to the ray origin
-  const V3 a = va - o, b = vb - o, c = vc - o;
-  const int kz = h.kz;
-  const float Akx = on_kx(a.x, a.y, a.z, kz), Aky = on_ky(a.x, a.y, a.z, kz), Akz = on_kz(a.x, a.y, a.z, kz);
-  const float Bkx = on_kx(b.x, b.y, b.z, kz), Bky = on_ky(b.x, b.y, b.z, kz), Bkz = on_kz(b.x, b.y, b.z, kz);
-  const float Ckx = on_kx(c.x, c.y, c.z, kz), Cky = on_ky(c.x, c.y, c.z, kz), Ckz = on_kz(c.x, c.y, c.z, kz);
+  const V3 a = va - h.o, b = vb - h.o, c = vc - h.o;
   // shear
-  const float Axs = fsub(Akx, fmul(h.Sx, Akz)), Ays = fsub(Aky, fmul(h.Sy, Akz));
-  const float Bxs = fsub(Bkx, fmul(h.Sx, Bkz)), Bys = fsub(Bky, fmul(h.Sy, Bkz));
-  const float Cxs = fsub(Ckx, fmul(h.Sx, Ckz)), Cys = fsub(Cky, fmul(h.Sy, Ckz));
+  const float Axs = fsub(a.x, fmul(h.Sx, a.z)), Ays = fsub(a.y, fmul(h.Sy, a.z));
+  const float Bxs = fsub(b.x, fmul(h.Sx, b.z)), Bys = fsub(b.y, fmul(h.Sy, b.z));
+  const float Cxs = fsub(c.x, fmul(h.Sx, c.z)), Cys = fsub(c.y, fmul(h.Sy, c.z));
   // scaled barycentrics (edge functions)
   const float U = fsub(fmul(Cxs, Bys), fmul(Cys, Bxs));
   const float V = fsub(fmul(Axs, Cys), fmul(Ays, Cxs));
@@ -221,7 +225,7 @@ __device__ __forceinline__ float intersect_tri(V3 o, const RayShear& h, V3 va, V
   if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return __int_as_float(0x7f800000);
   const float det = fadd(fadd(U, V), W);
   if (det == 0.0f) return __int_as_float(0x7f800000);
-  const float Az = fmul(h.Sz, Akz), Bz = fmul(h.Sz, Bkz), Cz = fmul(h.Sz, Ckz);
+  const float Az = fmul(h.Sz, a.z), Bz = fmul(h.Sz, b.z), Cz = fmul(h.Sz, c.z);
   const float T = fadd(fadd(fmul(U, Az), fmul(V, Bz)), fmul(W, Cz));
   const float t = fdiv(T, det);
   if (!(t > tmin)) return __int_as_float(0x7f800000);
@@ -232,11 +236,15 @@ __device__ __forceinline__ float intersect_tri(V3 o, const RayShear& h, V3 va, V
 // Closest-hit traversal of the 8-wide compressed BVH, one node per step.
 //
 // Box tests are made conservative by padding each slab distance by
-// 2^-20 (|c| + 255 |s|), which bounds the rounding of q*s + c with
-// s = 2^e/d and c = (p-o)/d -- 1/d within 2 ulp, p-o, the product, the fma
-// and the padding's own subtraction: about 9 * 2^-24 (|c| + 255 |s|) in all,
-// against 16 * 2^-24 -- so the traversal never culls a box the exact ray
-// enters.  Candidates are culled against best_t*(1+2^-16) + slack.
+// 2^-20 (|c| + 512 |s|) with s = 2^e/d and c = (p-o)/d.  A slab is
+// f s + (c - 1024 s -+ pad), f = 1024 + q, the half-precision number whose
+// bits are 0x6400 | q: two roundings of 2^-24 (|c| + 1024 |s|) in the
+// constant; 1/d within 2 ulp, p-o, the products and the padding's own
+// subtraction are about 9 * 2^-24 (|c| + 255 |s|).  Together that is
+// 2^-24 (11 |c| + 4343 |s|) against 2^-24 (16 |c| + 8192 |s|) -- so the
+// traversal never culls a box the exact ray enters.  (An overflow makes the
+// axis NaN, which the minima and maxima drop: the box is kept.)  Candidates
+// are culled against best_t*(1+2^-16) + slack.
 // Together with the lowest-index tie rule the result equals a brute-force
 // scan with the same triangle test.
 //
@@ -251,8 +259,8 @@ __device__ __forceinline__ float intersect_tri(V3 o, const RayShear& h, V3 va, V
 // So a node is three 32-byte loads instead of five of 16, the boxes are
 // tested two at a time with packed FP32 operations, the hit children are
 // ordered in registers by their distance bits (the nearest never goes
-// through the stack), and the leaf triangles follow from the hit mask by a
-// bit spread.
+// through the stack), the leaf triangles follow from the hit mask by a bit
+// spread, and their test reads the vertices' axes in the ray's order.
 
 struct TraceScene {
   const uint4* nodes;
@@ -308,8 +316,8 @@ __device__ __forceinline__ Words8 load32(const void* p) {
 // Per-warp scratch of the traversal (shared memory): what a lane needs to
 // test another lane's triangle, and the exchange of the triangle passes.
 struct TriPass {
-  float4 ray0[32];             // origin xyz, tmin
-  float4 ray1[32];             // shear Sx, Sy, Sz, kz (int bits)
+  float4 ray0[32];             // origin on the shear's axes, tmin
+  float4 ray1[32];             // shear Sx, Sy, Sz; byte offsets of the axes in a triangle (kx, ky << 8, kz << 16)
   unsigned long long key[32];  // (t bits << 32 | triangle id) of each lane's best hit
   unsigned long long list[32]; // address of the pass's j-th triangle | lane that asks for it
   int mat[32];
@@ -329,11 +337,6 @@ struct TravState {
   bool any;  // stop at the first non-emitter hit found (see trav_pop)
 };
 
-// Byte k of w as the float 2^23 + byte (exact; subtract 2^23 for the value).
-__device__ __forceinline__ float byte_biased(uint32_t w, int k) {
-  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7650u | (uint32_t)k));
-}
-
 // Starts a ray; returns false when there is nothing to traverse (empty
 // scene or zero direction), in which case the ray is a miss.  With `any`
 // the traversal ends at the first hit it finds: best_prim then says only
@@ -351,8 +354,9 @@ __device__ __forceinline__ bool trav_begin(TravState& s, const TraceScene& sc, V
   RayShear h;
   ray_prepare(o, d, sc.extent, s.r, h);
   const int lane = threadIdx.x & 31;
-  tp.ray0[lane] = make_float4(o.x, o.y, o.z, tmin);
-  tp.ray1[lane] = make_float4(h.Sx, h.Sy, h.Sz, __int_as_float(h.kz));
+  tp.ray0[lane] = make_float4(h.o.x, h.o.y, h.o.z, tmin);
+  tp.ray1[lane] = make_float4(h.Sx, h.Sy, h.Sz,
+                              __int_as_float(h.kz == 0 ? 0x002010 : (h.kz == 1 ? 0x100020 : 0x201000)));
   return true;
 }
 
@@ -369,10 +373,21 @@ struct NodeWork {
   float next_t;       // its entry distance (rounded down; NaN when there is none)
 };
 
-// Near and far distances of children c and c + 1 on one axis, packed.
-__device__ __forceinline__ float2 slab2(uint32_t w, int k, float s, float c) {
-  const float2 q = __fadd2_rn(make_float2(byte_biased(w, k), byte_biased(w, k + 1)), make_float2(-8388608.0f, -8388608.0f));
-  return __ffma2_rn(q, make_float2(s, s), make_float2(c, c));
+// Distances of two children's planes on one axis: bytes k and k + 1 of w as
+// halves (one permute), widened and multiplied on the FMA pipe (C is the
+// constant of the slab, see above).
+__device__ __forceinline__ float2 slab2(uint32_t w, int k, float s, float C) {
+  const uint32_t h = __byte_perm(w, 0x64646464u, 0x4040u | (uint32_t)k | ((uint32_t)(k + 1) << 8));
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+  return __ffma2_rn(f, make_float2(s, s), make_float2(C, C));
+}
+
+// a - b on the FMA pipe (an integer multiply-add; `one` is 1, which the
+// compiler does not know), to spare the ALU pipe.
+__device__ __forceinline__ uint32_t sub_fma_pipe(uint32_t a, uint32_t one, uint32_t neg_b) {
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(one), "r"(neg_b));
+  return d;
 }
 
 template <bool COUNT>
@@ -394,13 +409,14 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
   const float cx = (__uint_as_float(A.v[0]) - r.ox) * r.ix;
   const float cy = (__uint_as_float(A.v[1]) - r.oy) * r.iy;
   const float cz = (__uint_as_float(A.v[2]) - r.oz) * r.iz;
-  const float gx = fmaf(255.0f, fabsf(sx), fabsf(cx));
-  const float gy = fmaf(255.0f, fabsf(sy), fabsf(cy));
-  const float gz = fmaf(255.0f, fabsf(sz), fabsf(cz));
+  const float gx = fmaf(512.0f, fabsf(sx), fabsf(cx));
+  const float gy = fmaf(512.0f, fabsf(sy), fabsf(cy));
+  const float gz = fmaf(512.0f, fabsf(sz), fabsf(cz));
   constexpr float PAD = 9.5367431640625e-7f;
-  const float cnx = fmaf(-PAD, gx, cx), cfx = fmaf(PAD, gx, cx);
-  const float cny = fmaf(-PAD, gy, cy), cfy = fmaf(PAD, gy, cy);
-  const float cnz = fmaf(-PAD, gz, cz), cfz = fmaf(PAD, gz, cz);
+  const float mx = fmaf(-1024.0f, sx, cx), my = fmaf(-1024.0f, sy, cy), mz = fmaf(-1024.0f, sz, cz);
+  const float cnx = fmaf(-PAD, gx, mx), cfx = fmaf(PAD, gx, mx);
+  const float cny = fmaf(-PAD, gy, my), cfy = fmaf(PAD, gy, my);
+  const float cnz = fmaf(-PAD, gz, mz), cfz = fmaf(PAD, gz, mz);
   const bool negx = r.ix < 0.0f, negy = r.iy < 0.0f, negz = r.iz < 0.0f;
   const uint32_t nx[2] = {negx ? B.v[6] : B.v[0], negx ? B.v[7] : B.v[1]};
   const uint32_t fx[2] = {negx ? B.v[0] : B.v[6], negx ? B.v[1] : B.v[7]};
@@ -438,6 +454,8 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
     // the others, farthest first: the next larger key is the smallest of
     // key - (k + 1) in unsigned arithmetic
     const int sp0 = s.sp;
+    uint32_t one = 1;
+    asm volatile("" : "+r"(one));
     int at = sp0 + n - 2;
     s.sp = at + 1;
     if (s.sp > TRAV_STACK) {
@@ -446,9 +464,11 @@ __device__ __forceinline__ NodeWork trav_node(TravState& s, const TraceScene& sc
     }
 #pragma unroll 1
     for (; at >= sp0; --at) {
-      const uint32_t o = k + 1u;
-      k = o + min(min(min(key[0] - o, key[1] - o), min(key[2] - o, key[3] - o)),
-                  min(min(key[4] - o, key[5] - o), min(key[6] - o, key[7] - o)));
+      const uint32_t o = ~k;  // -(k + 1)
+      uint32_t m[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) m[c] = sub_fma_pipe(key[c], one, o);
+      k = min(min(min(m[0], m[1]), min(m[2], m[3])), min(min(m[4], m[5]), min(m[6], m[7]))) - o;
       if (at < TRAV_STACK) stack[at] = make_uint2(child_base + (k & 7u), k & ~7u);
     }
   }
@@ -475,14 +495,13 @@ __device__ __forceinline__ const char* first_tri(const TraceScene& sc, const Nod
 }
 
 // Tests the triangle at p with the ray (r0, r1) of TriPass.
-__device__ __forceinline__ float test_tri(const char* p, float4 r0, float4 r1, int& prim, int& mat) {
-  const Words8 t = load32(p);
-  const float4 c = __ldg((const float4*)(p + 32));
-  prim = (int)t.v[3];
-  mat = (int)t.v[7];
-  const RayShear h{r1.x, r1.y, r1.z, __float_as_int(r1.w)};
-  return intersect_tri(ld3(r0), h, v3(__uint_as_float(t.v[0]), __uint_as_float(t.v[1]), __uint_as_float(t.v[2])),
-                       v3(__uint_as_float(t.v[4]), __uint_as_float(t.v[5]), __uint_as_float(t.v[6])), ld3(c), r0.w);
+__device__ __forceinline__ float test_tri(const char* p, float4 r0, float4 r1, int& prim) {
+  const uint32_t at = __float_as_uint(r1.w);
+  const float4 x = __ldg((const float4*)(p + (at & 0xffu))), y = __ldg((const float4*)(p + ((at >> 8) & 0xffu))),
+               z = __ldg((const float4*)(p + (at >> 16)));
+  prim = __float_as_int(x.w);
+  const RayShear h{r1.x, r1.y, r1.z, 0, ld3(r0)};
+  return intersect_tri(h, v3(x.x, y.x, z.x), v3(x.y, y.y, z.y), v3(x.z, y.z, z.z), r0.w);
 }
 
 // Tests the triangles of all lanes of the warp, up to 32 at a time.  Either
@@ -537,11 +556,10 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
     }
     bool better = false;
     unsigned long long key = 0;
-    int mat = 0;
     const int o = (int)(e & 31u);
     if (test) {
       int prim;
-      const float t = test_tri((const char*)(e & ~31ull), tp.ray0[o], tp.ray1[o], prim, mat);
+      const float t = test_tri((const char*)(e & ~31ull), tp.ray0[o], tp.ray1[o], prim);
       if (COUNT) ++tests;
       const unsigned long long okey = *(volatile unsigned long long*)&tp.key[o];
       const float bt = __uint_as_float((uint32_t)(okey >> 32));
@@ -553,7 +571,7 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
     }
     __syncwarp();
     if (MAT) {
-      if (better && tp.key[o] == key) tp.mat[o] = mat;
+      if (better && tp.key[o] == key) tp.mat[o] = __ldg((const int*)((e & ~31ull) + 48));
       __syncwarp();
     }
   }
@@ -732,7 +750,8 @@ __device__ __forceinline__ void brute_hit(const SceneDev& sc, V3 o, V3 d, float 
   for (uint32_t p = 0; p < sc.num_prims; ++p) {
     const float4* pr = sc.prims + 5ull * p;
     const float4 a = __ldg(pr + 0), b = __ldg(pr + 1), c = __ldg(pr + 2);
-    const float t = intersect_tri(o, h, ld3(a), ld3(b), ld3(c), tmin);
+    const float t = intersect_tri(h, on_shear_axes(ld3(a), h.kz), on_shear_axes(ld3(b), h.kz),
+                                  on_shear_axes(ld3(c), h.kz), tmin);
     if (t < best_t) {
       best_t = t;
       best = (int)p;

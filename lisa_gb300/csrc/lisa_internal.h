@@ -229,7 +229,6 @@ struct Renderer {
   int nee_blocks = 0, nee_threads = 128;
   int nee_pb_blocks = 0;  // physically based emitter kernel
   int path_blocks = 0;    // whole-path kernel
-  int shade_blocks = 0, shade_threads = 256;
   // events for stage timing
   std::vector<cudaEvent_t> ev_pool;
   // CUDA graph of the last launch sequence, reused while its shape (waves
@@ -237,7 +236,7 @@ struct Renderer {
   cudaGraphExec_t graph_exec = nullptr;
   std::vector<uint64_t> graph_key;
   std::vector<std::pair<int, std::pair<size_t, size_t>>> graph_marks;
-  uint32_t graph_launches[5] = {0, 0, 0, 0, 0};  // trace, shade, nee, total, guide
+  uint32_t graph_launches[5] = {0, 0, 0, 0, 0};  // trace, -, nee, total, guide
   // guided mode
   std::vector<std::unique_ptr<GuideNet>> guides;
   float4* rec_list = nullptr;    // rec_cap kept training records (4 float4 each, then rec_cap float4: rec_col)

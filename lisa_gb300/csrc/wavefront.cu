@@ -4,13 +4,15 @@
 //
 //   raygen      one path per (scene, pixel, sample) slot          shader.cu:126-155
 //   trace       closest hit of every queued ray (persistent warps) shader.cu:77-98
-//   shade       per hit, by material class:                       shader.cu:211-255
+//   nee         shades 32 hits at a time, by material class:      shader.cu:211-255
 //                 miss / emitter -> path ends (emitter adds Le*att)
 //                 dielectric     -> Fresnel reflect / refract, next ray
-//                 opaque         -> att *= albedo, enqueue emitter search
-//   nee         up to 30 hemisphere rays per opaque vertex until one
-//               returns the (stale) emitter, then the bounce          shader.cu:196-209,248-253
+//                 opaque         -> up to 30 hemisphere rays until one
+//                   returns the (stale) emitter, att *= albedo, then
+//                   the bounce                                      shader.cu:196-209,248-253
 //   accumulate  per pixel, Kahan FP32 sum + FP64 sum of squares     shader.cu:156-166
+//
+// Small plain waves run whole paths in one kernel instead (k_paths).
 //
 // The persistent kernels take work with warp-aggregated atomics (one atomic
 // per warp per refill); queue appends are warp-aggregated the same way.
@@ -37,41 +39,30 @@ namespace lisa {
 
 constexpr uint32_t FULL = 0xffffffffu;
 
-#ifndef LISA_NEE_MIN_BLOCKS
-#define LISA_NEE_MIN_BLOCKS 6  // 6 x 128 threads per SM (80 registers; measured best of 6..8)
-#endif
-// Residency of the closest-hit and shade kernels: blocks per SM the
-// compiler must fit (0 = its own register choice).  Measured: the closest-hit
-// kernel at 8 (64 registers, no spills) is 4 % faster than at 7 (72); the
-// shade kernel is fastest with its own choice (56 registers).
+// Residency: blocks of 128 threads per SM that the compiler must fit.
+// Measured: the closest-hit kernel at 8 (64 registers, no spills) is 4 %
+// faster than at 7; the emitter-search kernels at 6 (80 registers) are best of
+// 5..8 -- more blocks leave less L1 for the BVH beside their shared memory
+// (soup frame: 105, 103, 109, 110 ms).
 #ifndef LISA_TRACE_MIN_BLOCKS
 #define LISA_TRACE_MIN_BLOCKS 8
 #endif
-#ifndef LISA_SHADE_MIN_BLOCKS
-#define LISA_SHADE_MIN_BLOCKS 0
-#endif
-#if LISA_TRACE_MIN_BLOCKS > 0
-#define LISA_TRACE_BOUNDS __launch_bounds__(128, LISA_TRACE_MIN_BLOCKS)
-#else
-#define LISA_TRACE_BOUNDS __launch_bounds__(128)
-#endif
-#if LISA_SHADE_MIN_BLOCKS > 0
-#define LISA_SHADE_BOUNDS __launch_bounds__(256, LISA_SHADE_MIN_BLOCKS)
-#else
-#define LISA_SHADE_BOUNDS __launch_bounds__(256)
+#ifndef LISA_NEE_MIN_BLOCKS
+#define LISA_NEE_MIN_BLOCKS 6
 #endif
 #ifndef LISA_NEE_PB_MIN_BLOCKS
-#define LISA_NEE_PB_MIN_BLOCKS 7  // physically based emitter kernel: 7 x 128 threads per SM
+#define LISA_NEE_PB_MIN_BLOCKS 6
 #endif
 #ifndef LISA_PATHS_MIN_BLOCKS
-#define LISA_PATHS_MIN_BLOCKS 5  // whole-path kernel: 5 x 128 threads per SM (96 registers; best of 4..6)
+#define LISA_PATHS_MIN_BLOCKS 5  // whole paths: 96 registers, best of 4..6
 #endif
-#ifndef LISA_PATHS_REFILL_IDLE
-#define LISA_PATHS_REFILL_IDLE 20  // idle lanes that trigger a round of k_paths (best of 8, 12, .. 28: its rounds are long)
-#endif
-#ifndef LISA_REFILL_IDLE
-#define LISA_REFILL_IDLE 12  // default: idle lanes (of 32) that trigger a refill round
-#endif
+// Idle lanes (of 32) that trigger a refill round: the option (default 12)
+// plus this much for each kind of kernel, whose rounds differ in length.
+// Measured by default: closest hit 8 (4, 8, 10, 12, 16 tried: 14.05 ms a step
+// of the 1.31 M-triangle icosphere box at 8, 14.19 at 12), emitter search 16
+// (12.1 ms against 12.4 at 12 and 12.7 at 8), whole paths 20 (5.15 ms of 4 Mi
+// Cornell box paths against 5.26 at 16 and 5.61 at 12).
+constexpr int REFILL_DEFAULT = 12, REFILL_TRACE = -4, REFILL_NEE = 4, REFILL_PATHS = 8;
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
@@ -210,7 +201,6 @@ __global__ void k_raygen(WaveBufs b, const WaveDesc* __restrict__ wave) {
     b.ctrl->qcount[1] = 0;
     b.ctrl->nee_count = 0;
     b.ctrl->head[HEAD_TRACE] = 0;
-    b.ctrl->head[HEAD_SHADE] = 0;
     b.ctrl->head[HEAD_NEE] = 0;
     b.ctrl->guided_count = 0;
     b.ctrl->rec_count = 0;
@@ -236,15 +226,14 @@ __global__ void k_raygen(WaveBufs b, const WaveDesc* __restrict__ wave) {
 // and takes the next ray as soon as its own is done (warp-aggregated fetch).
 
 template <bool COUNT>
-__global__ void LISA_TRACE_BOUNDS k_trace(WaveBufs b, int depth) {
+__global__ void __launch_bounds__(128, LISA_TRACE_MIN_BLOCKS) k_trace(WaveBufs b, int depth) {
   const int q = depth & 1;
   const uint32_t count = *(volatile uint32_t*)&b.ctrl->qcount[q];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    // shade/nee of this depth have not started; the previous depth's
+    // the emitter search of this depth has not started; the previous depth's
     // consumers of these counters have finished
     b.ctrl->qcount[q ^ 1] = 0;
     b.ctrl->nee_count = 0;
-    b.ctrl->head[HEAD_SHADE] = 0;
     b.ctrl->head[HEAD_NEE] = 0;
     if (depth > 0) b.ctrl->rays_bounce += count;
   }
@@ -350,75 +339,86 @@ __device__ __forceinline__ V3 dielectric_bounce(const DevMaterial& m, V3 d, V3 N
   return bsdf::refract(cosI, d, nrm, eta);
 }
 
+// An opaque hit: a vertex for the emitter search.  The path's throughput is
+// still the one before the vertex (its albedo is applied when the vertex is
+// left).
+struct Vertex {
+  V3 p, N;
+  uint32_t slot, scene;
+  int mat;
+  float4 att;
+};
+
+// Shades entry i of the depth's ray queue (valid: there is one): misses and
+// emitters end their path, a dielectric's ray goes to the next queue, an
+// opaque hit is returned as a vertex.  Called by all 32 lanes, on consecutive
+// entries, so that the queue reads coalesce.
 template <bool PHYS>
-__global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
+__device__ __forceinline__ bool shade_ray(const WaveBufs& b, int depth, uint32_t i, bool valid, Vertex& v) {
   const int q = depth & 1;
-  const uint32_t count = *(volatile uint32_t*)&b.ctrl->qcount[q];
-  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->head[HEAD_TRACE] = 0;  // trace of this depth is done
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  for (uint32_t base = gw * 32; base < count; base += warps * 32) {
-    const uint32_t i = base + lane;
-    bool want_ray = false, want_nee = false;
-    V3 p = v3(0.0f), nd = v3(0.0f), N = v3(0.0f), d = v3(0.0f);
-    uint32_t slot = 0;
-    int mat_idx = 0;
-    uint32_t scene = 0;
-    if (i < count) {
-      const int2 h = b.hit[i];
-      const float4 o4 = b.ro[q][i];
-      const float4 d4 = b.rd[q][i];
-      slot = __float_as_uint(o4.w);
-      scene = __float_as_uint(d4.w);
-      if (h.x >= 0) {  // a miss adds the background, 0 (optix_wrapper.cc:354-356), and ends the path
-        const SceneDev& sc = b.scenes[scene];
-        mat_idx = prim_material(sc, h.x);
-        const DevMaterial& m = sc.mats[mat_idx];
-        float4 att = b.ps_att[slot];
-        if (m.cls == MAT_EMIT) {
-          const float4 col = b.ps_col[slot];
-          const V3 le = emitter_hit<PHYS>(sc, m, h.x, __int_as_float(h.y), ld3(d4), att);
-          const V3 c = ld3(col) + le;
-          b.ps_col[slot] = make_float4(c.x, c.y, c.z, col.w);
-        } else if (!PHYS || depth < (int)sc.num_bounces) {
-          // (physically based: the ray leaving the last vertex only gathers
-          // the emission it reaches, so any other hit ends the path)
-          d = ld3(d4);
-          const float t = __int_as_float(h.y);
-          p = ld3(o4) + t * d;
-          N = barycentric_normal(p, sc.prims + 5ull * h.x);
+  bool want_ray = false, vertex = false;
+  V3 nd = v3(0.0f);
+  if (valid) {
+    const int2 h = b.hit[i];
+    const float4 o4 = b.ro[q][i];
+    const float4 d4 = b.rd[q][i];
+    v.slot = __float_as_uint(o4.w);
+    v.scene = __float_as_uint(d4.w);
+    if (h.x >= 0) {  // a miss adds the background, 0 (optix_wrapper.cc:354-356), and ends the path
+      const SceneDev& sc = b.scenes[v.scene];
+      v.mat = prim_material(sc, h.x);
+      v.att = b.ps_att[v.slot];
+      const DevMaterial& m = sc.mats[v.mat];
+      const float t = __int_as_float(h.y);
+      if (m.cls == MAT_EMIT) {
+        const float4 col = b.ps_col[v.slot];
+        const V3 c = ld3(col) + emitter_hit<PHYS>(sc, m, h.x, t, ld3(d4), v.att);
+        b.ps_col[v.slot] = make_float4(c.x, c.y, c.z, col.w);
+      } else if (!PHYS || depth < (int)sc.num_bounces) {
+        // (physically based: the ray leaving the last vertex only gathers
+        // the emission it reaches, so any other hit ends the path)
+        const V3 d = ld3(d4);
+        v.p = ld3(o4) + t * d;
+        v.N = barycentric_normal(v.p, sc.prims + 5ull * h.x);
+        if (m.cls == MAT_DIELECTRIC) {
           // the reference estimator traces num_bounces rays; the physically
           // based one also the ray leaving its last vertex
-          const bool last = !PHYS && depth + 1 >= (int)sc.num_bounces;
-          if (m.cls == MAT_DIELECTRIC) {
-            V3 a = ld3(att);
-            uint32_t seed = b.ps_rng[slot];
-            nd = dielectric_bounce<PHYS>(m, d, N, a, seed);
-            b.ps_rng[slot] = seed;
-            b.ps_att[slot] = make_float4(a.x, a.y, a.z, PHYS ? 0.0f : att.w);
-            want_ray = !last && !is_zero(nd);
-            if (PHYS && want_ray && depth + 1 == (int)sc.num_bounces) want_ray = final_ray_wanted(sc, p, nd);
-          } else {
-            const V3 a = ld3(att) * v3(m.albedo[0], m.albedo[1], m.albedo[2]);
-            b.ps_att[slot] = make_float4(a.x, a.y, a.z, att.w);
-            want_nee = true;
-          }
+          V3 a = ld3(v.att);
+          uint32_t seed = b.ps_rng[v.slot];
+          nd = dielectric_bounce<PHYS>(m, d, v.N, a, seed);
+          b.ps_rng[v.slot] = seed;
+          b.ps_att[v.slot] = make_float4(a.x, a.y, a.z, PHYS ? 0.0f : v.att.w);
+          want_ray = (PHYS || depth + 1 < (int)sc.num_bounces) && !is_zero(nd);
+          if (PHYS && want_ray && depth + 1 == (int)sc.num_bounces) want_ray = final_ray_wanted(sc, v.p, nd);
+        } else {
+          vertex = true;
         }
       }
     }
-    const uint32_t ri = warp_reserve(&b.ctrl->qcount[q ^ 1], want_ray);
-    if (want_ray && queue_fits(b, ri)) {
-      b.ro[q ^ 1][ri] = make_float4(p.x, p.y, p.z, __uint_as_float(slot));
-      b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(scene));
-    }
-    const uint32_t ni = warp_reserve(&b.ctrl->nee_count, want_nee);
-    if (want_nee && queue_fits(b, ni)) {
-      b.nee_a[ni] = make_float4(p.x, p.y, p.z, __uint_as_float(slot));
-      b.nee_b[ni] = make_float4(N.x, N.y, N.z, __int_as_float(mat_idx));
-      b.nee_c[ni] = make_float4(d.x, d.y, d.z, __uint_as_float(scene));
-    }
   }
+  const uint32_t ri = warp_reserve(&b.ctrl->qcount[q ^ 1], want_ray);
+  if (want_ray && queue_fits(b, ri)) {
+    b.ro[q ^ 1][ri] = make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(v.slot));
+    b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(v.scene));
+  }
+  return vertex;
+}
+
+// Throughput after the vertex's material (shader.cu:248).
+__device__ __forceinline__ V3 vertex_throughput(float4 att, const DevMaterial& m) {
+  return ld3(att) * v3(m.albedo[0], m.albedo[1], m.albedo[2]);
+}
+
+// Guided mode: the vertex's entry of the queue that the guide's inference
+// reads.  Called by all 32 lanes; returns the entry.
+__device__ __forceinline__ uint32_t queue_vertex(const WaveBufs& b, bool vertex, const Vertex& v, V3 d) {
+  const uint32_t ni = warp_reserve(&b.ctrl->nee_count, vertex);
+  if (vertex && queue_fits(b, ni)) {
+    b.nee_a[ni] = make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(v.slot));
+    b.nee_b[ni] = make_float4(v.N.x, v.N.y, v.N.z, __int_as_float(v.mat));
+    b.nee_c[ni] = make_float4(d.x, d.y, d.z, __uint_as_float(v.scene));
+  }
+  return ni;
 }
 
 // ---------------------------------------------------------------------------
@@ -433,12 +433,14 @@ __global__ void LISA_SHADE_BOUNDS k_shade(WaveBufs b, int depth) {
 // 30 rays of different lengths.
 //
 // Bound by issue: most tries are decided without a traversal, so the kernel
-// is the arithmetic around the queue.  A warp therefore prepares 32 vertices
-// at a time, each lane testing all tries of its own vertex, and keeps the
-// answers as a bit mask.  (One warp-wide search per vertex and per
-// traversal, 32 lanes on the tries of one vertex, took 13.3 ms of the
-// 1.31 M-triangle icosphere step's 59 M vertices; this takes 10.3 ms, and
-// 2.5 instead of 3.3 ms on the Cornell box frame.)
+// is the arithmetic around the queue.  A warp therefore shades 32 rays at a
+// time, each lane then testing all tries of its own vertex, and keeps the
+// answers as a bit mask; shading, bound by memory latency in a kernel of its
+// own, overlaps the other warps' traversals here, and its vertices never go
+// through memory.  On the 1.31 M-triangle icosphere step (86 M rays, 59 M
+// vertices) shading and search take 12.1 ms: 5.8 + 13.3 with a shading
+// kernel and one warp-wide search per vertex and traversal, 5.7 + 8.9 with a
+// shading kernel and prepared vertices.
 
 // Guided bounce at an opaque vertex with roughness 1, where the reference
 // draws hemi(N) (lambertian.cu:7-13): one-sample MIS between that sampler
@@ -461,35 +463,62 @@ __device__ __forceinline__ V3 guided_bounce(const float* o, V3 N, uint32_t& seed
   return w;
 }
 
-// Queue entries a warp of k_nee has prepared (shared memory).
+// A warp of k_nee's vertices in shared memory: those it has prepared and not
+// yet started, and each lane's own, which only the bookkeeping rounds touch
+// (in registers it would cost the traversal a quarter of its occupancy).
 struct NeeVertices {
-  float4 p[32];         // position, slot
-  float4 n[32];         // normal, material
-  uint4 s[32];          // stream state, emitter flag, candidate tries, scene
-  uint32_t entry[32];
+  float4 p[32];      // position, slot
+  float4 n[32];      // normal, material
+  uint4 s[32];       // stream state, emitter flag, candidate tries, scene
+  uint32_t ray[32];  // ray queue entry (its direction is the incoming one)
+};
+struct NeeLanes {
+  float4 n[32];      // normal, material
+  float4 d[32];      // shadow ray's direction, slot
+  uint4 s[32];       // stream state, emitter flag, candidate tries, tries made
+  uint2 r[32];       // ray queue entry, scene
 };
 
+// The whole warp shades 32 consecutive rays and prepares the opaque hits'
+// emitter searches, whose tries are tested (emit_candidates) on all lanes.
+// Returns the number of vertices.  A function of its own: inlined, its
+// registers would be spilled inside the traversal.
+template <bool GUIDED>
+__device__ __noinline__ uint32_t fill_vertices(const WaveBufs& b, int depth, uint32_t base, uint32_t count,
+                                               NeeVertices& vb) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t i = base + (uint32_t)lane;
+  Vertex v;
+  const bool vertex = shade_ray<false>(b, depth, i, i < count, v);
+  if (GUIDED) queue_vertex(b, vertex, v, vertex ? ld3(b.rd[depth & 1][i]) : v3(0.0f));
+  const uint32_t vmask = __ballot_sync(FULL, vertex);
+  if (vertex) {
+    const uint32_t k = __popc(vmask & lanemask_lt()), vseed = b.ps_rng[v.slot];
+    vb.p[k] = make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(v.slot));
+    vb.n[k] = make_float4(v.N.x, v.N.y, v.N.z, __int_as_float(v.mat));
+    vb.s[k] = make_uint4(vseed, __float_as_uint(v.att.w), emit_candidates(b.scenes[v.scene], v.p, v.N, vseed), v.scene);
+    vb.ray[k] = i;
+  }
+  return __popc(vmask);
+}
+
 template <bool COUNT, bool GUIDED = false>
-__global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, int depth) {
+__global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(const __grid_constant__ WaveBufs b, int depth) {
   const int q = depth & 1;
-  const uint32_t count = *(volatile uint32_t*)&b.ctrl->nee_count;
+  const uint32_t count = *(volatile uint32_t*)&b.ctrl->qcount[q];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = lanemask_lt();
   uint2 stack[TRAV_STACK];
   TravState s;
   TraceScene ts;
-  const SceneDev* sc = nullptr;
   bool have = false, exhausted = false, ray_active = false;
-  uint32_t entry = 0, slot = 0, tries = 0, seed = 0;
-  int stale = -1, mat_idx = 0;
   // the vertex position lives in the shadow ray's origin (s.r.o*)
-  V3 N = v3(0.0f), dir = v3(0.0f);
   s.r.ox = s.r.oy = s.r.oz = 0.0f;
-  uint32_t shadow = 0, walked = 0, visits = 0, tests = 0;
+  uint32_t shadow = 0, walked = 0, visits = 0, tests = 0, vertices = 0;
   bool pending = false;  // a finished shadow ray not yet evaluated
-  bool emit_pass = false;  // the finished traversal was of the emitters' own BVH
-  uint32_t cand = 0;       // the vertex's tries that may reach an emitter (emit_candidates)
-  // vertices the warp has taken from the queue and prepared, not yet started
+  bool emit_pass = false;  // the traversal is of the emitters' own BVH
+  __shared__ NeeLanes lane_buf[4];
+  NeeLanes& vl = lane_buf[threadIdx.x >> 5];
   __shared__ NeeVertices vertex_buf[4];
   NeeVertices& vb = vertex_buf[threadIdx.x >> 5];
   uint32_t vb_next = 0, vb_count = 0;  // (the same in every lane)
@@ -509,9 +538,9 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
     // shared by many lanes; otherwise the warp keeps traversing.
     const uint32_t busy = __ballot_sync(FULL, ray_active);
     if (__popc(busy) <= (int)b.refill_busy_max) {
-      bool want_ray = false;
+      bool want_ray = false, start = false, nearer = false;
       V3 nd = v3(0.0f);
-      if (pending && emit_pass) {
+      if (pending && emit_pass && s.best_prim >= 0) {
         // A try with the flag unset matters only if its closest hit is an
         // emitter.  The emitters' BVH gave the nearest emitter on the ray
         // (if none, the try is inconsequential: evaluated as a miss); the
@@ -519,23 +548,14 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
         // unless a triangle is nearer (or as near with a lower index) --
         // the same closest hit as one traversal of the whole scene.  Such a
         // triangle is not an emitter's, so that pass ends at the first one.
-        emit_pass = false;
-        if (s.best_prim >= 0) {
-          const float te = s.best_t;
-          const int pe = s.best_prim, me = s.best_mat;
-          ts = trace_scene(*sc);
-          ray_active = trav_begin(s, ts, v3(s.r.ox, s.r.oy, s.r.oz), dir, RAY_TMIN, RAY_TMAX, tp);
-          s.best_t = te;
-          s.best_prim = pe;
-          s.best_mat = me;
-          s.cull = fmaf(te, 1.52587890625e-5f, te) + s.r.slack;
-          s.any = true;
-          ++walked;
-          pending = !ray_active;
-        }
+        nearer = start = true;
+        pending = false;
       }
+      emit_pass = emit_pass && !pending && !nearer;
       if (pending) {
         pending = false;
+        uint4 s4 = vl.s[lane];
+        int stale = (int)s4.y;
         if (s.best_prim >= 0) {
           // the occlusion hit program marks a hit only on an emitter and
           // otherwise leaves the flag as it was (shader.cu:177-184)
@@ -544,41 +564,47 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
           stale = -1;  // miss (shader.cu:172-175)
         }
         const bool lit = stale >= 0;
-        if (lit || ++tries == (uint32_t)NEE_TRIES) {
-          const float4 at = b.ps_att[slot];
-          const V3 att = ld3(at);
+        if (lit || ++s4.w == (uint32_t)NEE_TRIES) {
+          const float4 n4 = vl.n[lane], d4 = vl.d[lane];
+          const uint2 r2 = vl.r[lane];
+          const V3 N = ld3(n4);
+          const uint32_t slot = __float_as_uint(d4.w);
+          uint32_t seed = s4.x;
+          const SceneDev& sc = b.scenes[r2.y];
+          const DevMaterial& m = sc.mats[__float_as_int(n4.w)];
+          const V3 att = vertex_throughput(b.ps_att[slot], m);
           if (lit) {
-            const DevMaterial& em = sc->mats[stale];
-            const float brdf = bsdf::BRDF(N, dir, sc->mats[mat_idx]);
+            const DevMaterial& em = sc.mats[stale];
+            const float brdf = bsdf::BRDF(N, ld3(d4), m);
             const float4 c = b.ps_col[slot];
             const V3 col = ld3(c) + (v3(em.emission[0], em.emission[1], em.emission[2]) * brdf) * att;
             b.ps_col[slot] = make_float4(col.x, col.y, col.z, c.w);
           }
-          if (GUIDED && sc->mats[mat_idx].roughness == 1.0f) {
+          if (GUIDED && m.roughness == 1.0f) {
             // the bounce of a guided vertex is drawn by k_guided_infer,
             // after the guide has seen the emitter flag this search left
             want_ray = false;
           } else {
-            const V3 D = ld3(b.nee_c[entry]);
+            const V3 D = ld3(b.rd[q][r2.x]);
             // the bounce is drawn at every vertex, the last one included, so
             // the per-pixel stream advances exactly as in the reference
-            nd = bsdf::bounce(D, N, seed, sc->mats[mat_idx]);
-            want_ray = depth + 1 < (int)sc->num_bounces && !is_zero(nd);
+            nd = bsdf::bounce(D, N, seed, m);
+            want_ray = depth + 1 < (int)sc.num_bounces && !is_zero(nd);
           }
           b.ps_rng[slot] = seed;
           b.ps_att[slot] = make_float4(att.x, att.y, att.z, __int_as_float(stale));
           have = false;
         }
+        vl.s[lane] = make_uint4(s4.x, (uint32_t)stale, s4.z, s4.w);
       }
       const uint32_t ri = warp_reserve(&b.ctrl->qcount[q ^ 1], want_ray);
       if (want_ray && queue_fits(b, ri)) {
-        b.ro[q ^ 1][ri] = make_float4(s.r.ox, s.r.oy, s.r.oz, __uint_as_float(slot));
-        b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float((uint32_t)(sc - b.scenes)));
+        b.ro[q ^ 1][ri] = make_float4(s.r.ox, s.r.oy, s.r.oz, vl.d[lane].w);
+        b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(vl.r[lane].y));
       }
       // Idle lanes take their next vertices from the warp's buffer.  An empty
-      // buffer is filled by the whole warp: 32 consecutive queue entries at
-      // once, so that their loads coalesce and the test of their tries
-      // (emit_candidates) runs on 32 lanes.
+      // buffer is filled by the whole warp: it shades 32 consecutive rays, and
+      // the opaque hits' tries are tested (emit_candidates) on all lanes.
       while (__any_sync(FULL, !have && !exhausted)) {
         if (vb_next == vb_count) {
           uint32_t base = 0;
@@ -592,17 +618,8 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
             break;
           }
           vb_next = 0;
-          vb_count = min(32u, count - base);
-          if (lane < (int)vb_count) {
-            const float4 a4 = b.nee_a[base + lane], b4 = b.nee_b[base + lane];
-            const uint32_t vslot = __float_as_uint(a4.w);
-            const uint32_t scene = __float_as_uint(__ldg(&b.nee_c[base + lane].w));
-            const uint32_t flag = __float_as_uint(b.ps_att[vslot].w), vseed = b.ps_rng[vslot];
-            vb.p[lane] = a4;
-            vb.n[lane] = b4;
-            vb.s[lane] = make_uint4(vseed, flag, emit_candidates(b.scenes[scene], ld3(a4), ld3(b4), vseed), scene);
-            vb.entry[lane] = base + lane;
-          }
+          vb_count = fill_vertices<GUIDED>(b, depth, base, count, vb);
+          vertices += vb_count;
           __syncwarp();
         }
         const bool need = !have && !exhausted;
@@ -610,20 +627,15 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
         const uint32_t k = vb_next + __popc(nmask & lt);
         vb_next = min(vb_next + (uint32_t)__popc(nmask), vb_count);
         if (need && k < vb_count) {
-          const float4 a4 = vb.p[k], b4 = vb.n[k];
-          const uint4 s4 = vb.s[k];
-          entry = vb.entry[k];
+          const float4 a4 = vb.p[k];
+          const uint4 v4 = vb.s[k];
           s.r.ox = a4.x;
           s.r.oy = a4.y;
           s.r.oz = a4.z;
-          slot = __float_as_uint(a4.w);
-          N = ld3(b4);
-          mat_idx = __float_as_int(b4.w);
-          seed = s4.x;
-          stale = (int)s4.y;
-          cand = s4.z;
-          sc = b.scenes + s4.w;
-          tries = 0;
+          vl.n[lane] = vb.n[k];
+          vl.d[lane] = make_float4(0.0f, 0.0f, 0.0f, a4.w);
+          vl.s[lane] = make_uint4(v4.x, v4.y, v4.z, 0u);
+          vl.r[lane] = make_uint2(vb.ray[k], v4.w);
           have = true;
         }
         __syncwarp();
@@ -641,40 +653,58 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
       //
       // The next try of a vertex whose flag is unset is its next candidate:
       // the LCG jumps over the tries before it.
-      uint32_t skipped = 0;
-      if (have && !ray_active && !pending && stale < 0) {
-        skipped = (uint32_t)__ffs((int)(cand >> tries)) - 1u;  // (the last try is always a candidate)
-        const uint2 j = s_jump[skipped];
-        seed = j.x * seed + j.y;
-        tries += skipped;
-      }
-      if (have && !ray_active && !pending) {
-        const V3 p = v3(s.r.ox, s.r.oy, s.r.oz);
-        shadow += skipped + 1;
-        const float hx = rng11(seed);
-        const float hy = rng11(seed);
-        const float hz = rng11(seed);
-        dir = bsdf::hemisphere_direction(N, hx, hy, hz);
-        const bool capable = emit_may_hit(*sc, p, dir);
-        if (!capable && stale < 0) {
+      const V3 p = v3(s.r.ox, s.r.oy, s.r.oz);
+      const float4 d4 = vl.d[lane];
+      const SceneDev& sc = b.scenes[have ? vl.r[lane].y : 0u];
+      V3 dir = ld3(d4);
+      bool any = nearer;
+      if (have && !ray_active && !start) {
+        uint4 s4 = vl.s[lane];
+        if ((int)s4.y < 0) {
+          const uint32_t skipped = (uint32_t)__ffs((int)(s4.z >> s4.w)) - 1u;  // (the last try is always a candidate)
+          const uint2 j = s_jump[skipped];
+          s4.x = j.x * s4.x + j.y;
+          s4.w += skipped;
+          shadow += skipped;
+        }
+        ++shadow;
+        const float hx = rng11(s4.x);
+        const float hy = rng11(s4.x);
+        const float hz = rng11(s4.x);
+        dir = bsdf::hemisphere_direction(ld3(vl.n[lane]), hx, hy, hz);
+        vl.s[lane] = s4;
+        vl.d[lane] = make_float4(dir.x, dir.y, dir.z, d4.w);
+        const bool capable = emit_may_hit(sc, p, dir);
+        if (!capable && (int)s4.y < 0) {
           s.best_prim = -1;  // an inconsequential try: evaluated as a miss
           pending = true;
         } else {
           // with the flag unset, a ray that may reach an emitter first asks
           // the emitters' own BVH (scenes with more than a few emitter
           // triangles; with a few, the bounds test above is as selective)
-          emit_pass = stale < 0 && sc->num_etris >= EMIT_BVH_MIN_TRIS;
-          ts = emit_pass ? trace_scene_emit(*sc) : trace_scene(*sc);
-          ray_active = trav_begin(s, ts, p, dir, RAY_TMIN, RAY_TMAX, tp);
-          if (ray_active) {
-            s.any = !capable;
-            ++walked;
-          } else {
-            emit_pass = false;
-          }
-          pending = !ray_active;  // nothing to traverse: a miss
+          emit_pass = (int)s4.y < 0 && sc.num_etris >= EMIT_BVH_MIN_TRIS;
+          any = !capable;
+          start = true;
         }
       }
+      if (start) {
+        const float te = s.best_t;
+        const int pe = s.best_prim, me = s.best_mat;
+        ts = emit_pass ? trace_scene_emit(sc) : trace_scene(sc);
+        ray_active = trav_begin(s, ts, p, dir, RAY_TMIN, RAY_TMAX, tp, any);
+        if (nearer) {
+          s.best_t = te;
+          s.best_prim = pe;
+          s.best_mat = me;
+          s.cull = fmaf(te, 1.52587890625e-5f, te) + s.r.slack;
+        }
+        if (ray_active) ++walked;
+        else emit_pass = false;
+        pending = !ray_active;  // nothing to traverse: a miss
+      }
+      // while few lanes have a ray and some have a try to evaluate, the
+      // bookkeeping goes on: most vertices need no traversal at all
+      if (__popc(__ballot_sync(FULL, ray_active)) <= (int)b.refill_busy_max && __any_sync(FULL, pending)) continue;
     }
     if (trav_step_warp<COUNT, true>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
       ray_active = false;
@@ -683,14 +713,12 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(WaveBufs b, in
   }
   warp_add64(&b.ctrl->rays_shadow, shadow);
   warp_add64(&b.ctrl->shadow_walked, walked);
+  if (lane == 0 && vertices) atomicAdd(&b.ctrl->nee_total, (unsigned long long)vertices);
   if (COUNT) {
     warp_add64(&b.ctrl->node_visits[1], visits);
     warp_add64(&b.ctrl->tri_tests[1], tests);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    b.ctrl->head[HEAD_TRACE] = 0;
-    b.ctrl->nee_total += count;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->head[HEAD_TRACE] = 0;  // trace of this depth is done
 }
 
 // Training records of guided vertices, in two halves so that the slot's
@@ -772,53 +800,118 @@ __device__ __forceinline__ bool guided_compat_vertex(const WaveBufs& b, int dept
 // emitter picked by area x luminance (two-sided emitters), weighted against
 // the bounce's density by the power heuristic.  Bounce: the diffuse lobe
 // with probability = roughness (cosine-weighted), else a mirror; the
-// throughput keeps the albedo applied by k_shade.  ps_att.w carries the
+// throughput takes the albedo when the vertex is left.  ps_att.w carries the
 // solid-angle density of the last diffuse bounce (0 after a camera ray or a
-// specular event) for the weight at an emitter hit (k_shade<true>).
+// specular event) for the weight at an emitter hit (emitter_hit).
 //
 // Plain mode finishes each vertex here.  Guided mode (SPLIT) only traces the
 // shadow ray and leaves (direction, density, cosine, emitter material,
 // visibility) in nee_light; k_guided_infer weighs it with the guide's density
 // and draws the bounce once the guide's inference has run.
 
+// A warp of k_nee_pb's vertices in shared memory: prepared ones, and each
+// lane's own (see NeeLanes).
+struct PbVertices {
+  float4 p[32];      // position, slot
+  float4 n[32];      // normal that faces the incoming ray, material
+  float4 w[32];      // direction to the emitter sample, its distance (0: no shadow ray)
+  float4 l[32];      // density and cosine of the sample, its emitter's material, scene
+  uint4 s[32];       // stream state, ray queue entry, emitter queue entry (SPLIT), -
+};
+
+// The whole warp shades 32 consecutive rays and draws the opaque hits'
+// emitter samples; returns the number of vertices (see fill_vertices).
+template <bool SPLIT>
+__device__ __noinline__ uint32_t fill_pb_vertices(const WaveBufs& b, int depth, uint32_t base, uint32_t count,
+                                                  PbVertices& vb) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t i = base + (uint32_t)lane;
+  Vertex v;
+  const bool vertex = shade_ray<true>(b, depth, i, i < count, v);
+  const V3 d = vertex ? ld3(b.rd[depth & 1][i]) : v3(0.0f);
+  const uint32_t ventry = SPLIT ? queue_vertex(b, vertex, v, d) : 0u;
+  const uint32_t vmask = __ballot_sync(FULL, vertex);
+  if (vertex) {
+    const uint32_t k = __popc(vmask & lanemask_lt());
+    const SceneDev& vs = b.scenes[v.scene];
+    uint32_t vseed = b.ps_rng[v.slot];
+    const V3 n = dot(v.N, d) < 0.0f ? v.N : -v.N;
+    V3 w = v3(0.0f);
+    float vpl = 0.0f, vcos = 0.0f, far = 0.0f;
+    int vem = 0;
+    if (vs.mats[v.mat].roughness > 0.0f && vs.num_emit > 0) {
+      V3 y;
+      const uint32_t e = sample_emitter(vs, vseed, y);
+      const V3 to = y - v.p;
+      const float d2 = dot(to, to);
+      const float dist = fsqrt(d2);
+      w = to * fdiv(1.0f, dist);
+      vcos = dot(n, w);
+      const float cos_y = fabsf(dot(ld3(__ldg(vs.emit + 4ull * e + 3)), w));
+      if (vcos > 0.0f && cos_y > 0.0f && dist > 0.0f) {
+        vpl = fdiv(fmul(__ldg(vs.emit + 4ull * e).w, d2), cos_y);
+        vem = __float_as_int(__ldg(vs.emit + 4ull * e + 1).w);
+        far = dist;
+      }
+    }
+    vb.p[k] = make_float4(v.p.x, v.p.y, v.p.z, __uint_as_float(v.slot));
+    vb.n[k] = make_float4(n.x, n.y, n.z, __int_as_float(v.mat));
+    vb.w[k] = make_float4(w.x, w.y, w.z, far);
+    vb.l[k] = make_float4(vpl, vcos, __int_as_float(vem), __uint_as_float(v.scene));
+    vb.s[k] = make_uint4(vseed, i, ventry, 0u);
+  }
+  return __popc(vmask);
+}
+
 template <bool COUNT, bool SPLIT>
-__global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs b, int depth) {
+__global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(const __grid_constant__ WaveBufs b, int depth) {
   const int q = depth & 1;
-  const uint32_t count = *(volatile uint32_t*)&b.ctrl->nee_count;
+  const uint32_t count = *(volatile uint32_t*)&b.ctrl->qcount[q];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = lanemask_lt();
   uint2 stack[TRAV_STACK];
   TravState s;
   TraceScene ts;
-  const SceneDev* sc = nullptr;
-  bool have = false, exhausted = false, ray_active = false, pending = false, shadow = false;
-  uint32_t entry = 0, slot = 0, seed = 0;
-  int mat_idx = 0, em_m = 0;
-  V3 Ns = v3(0.0f), wi = v3(0.0f);  // the vertex position lives in s.r.o*
-  float pl = 0.0f, cos_x = 0.0f;
-  s.r.ox = s.r.oy = s.r.oz = 0.0f;
-  uint32_t nshadow = 0, visits = 0, tests = 0;
+  bool have = false, exhausted = false, ray_active = false, pending = false;
+  uint32_t nshadow = 0, visits = 0, tests = 0, vertices = 0;
   __shared__ TriPass tri_pass[4];
   TriPass& tp = tri_pass[threadIdx.x >> 5];
+  __shared__ PbVertices vertex_buf[4], lane_buf[4];
+  PbVertices& vb = vertex_buf[threadIdx.x >> 5];
+  PbVertices& vl = lane_buf[threadIdx.x >> 5];
+  uint32_t vb_next = 0, vb_count = 0;  // (the same in every lane)
+  bool queue_empty = false;
   while (true) {
     const uint32_t busy = __ballot_sync(FULL, ray_active);
     if (__popc(busy) <= (int)b.refill_busy_max) {
       bool want_ray = false;
       V3 nd = v3(0.0f);
+      // the lane's vertex (undefined without one)
+      const float4 p4 = vl.p[lane];
+      const uint32_t slot = __float_as_uint(p4.w), scene = __float_as_uint(vl.l[lane].w);
       if (pending) {
         pending = false;
-        const bool lit = shadow && s.best_prim < 0;
+        const float4 n4 = vl.n[lane], w4 = vl.w[lane], l4 = vl.l[lane];
+        const uint4 s4 = vl.s[lane];
+        const SceneDev& sc = b.scenes[scene];
+        const DevMaterial& m = sc.mats[__float_as_int(n4.w)];
+        const V3 Ns = ld3(n4), wi = ld3(w4);
+        const float pl = l4.x, cos_x = l4.y;
+        const int em_m = __float_as_int(l4.z);
+        const uint32_t ray = s4.y, entry = s4.z;
+        uint32_t seed = s4.x;
+        const bool lit = w4.w > 0.0f && s.best_prim < 0;
+        const float4 at = b.ps_att[slot];
+        const V3 att = vertex_throughput(at, m);
         if (SPLIT) {
           b.nee_light[2ull * entry] = make_float4(wi.x, wi.y, wi.z, pl);
           b.nee_light[2ull * entry + 1] = make_float4(cos_x, __int_as_float(em_m), lit ? 1.0f : 0.0f, 0.0f);
           b.ps_rng[slot] = seed;
+          b.ps_att[slot] = make_float4(att.x, att.y, att.z, at.w);
         } else {
-          const DevMaterial& m = sc->mats[mat_idx];
           const float r = m.roughness;
-          const float4 at = b.ps_att[slot];
-          const V3 att = ld3(at);
           if (lit) {
-            const DevMaterial& em = sc->mats[em_m];
+            const DevMaterial& em = sc.mats[em_m];
             const float fcos = fmul(r, fdiv(cos_x, PI_F));
             // power heuristic against the bounce (traced at every vertex, the
             // last one's for the emission it reaches only)
@@ -833,11 +926,10 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs
             nd = cosine_dir(Ns, seed);
             prev = fmul(r, fdiv(dot(Ns, nd), PI_F));
           } else {
-            nd = reflect(ld3(b.nee_c[entry]), Ns);
+            nd = reflect(ld3(b.rd[q][ray]), Ns);
           }
           want_ray = !is_zero(nd);
-          if (want_ray && depth + 1 == (int)sc->num_bounces)
-            want_ray = final_ray_wanted(*sc, v3(s.r.ox, s.r.oy, s.r.oz), nd);
+          if (want_ray && depth + 1 == (int)sc.num_bounces) want_ray = final_ray_wanted(sc, ld3(p4), nd);
           b.ps_rng[slot] = seed;
           b.ps_att[slot] = make_float4(att.x, att.y, att.z, prev);
         }
@@ -845,62 +937,54 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs
       }
       const uint32_t ri = warp_reserve(&b.ctrl->qcount[q ^ 1], want_ray);
       if (want_ray && queue_fits(b, ri)) {
-        b.ro[q ^ 1][ri] = make_float4(s.r.ox, s.r.oy, s.r.oz, __uint_as_float(slot));
-        b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float((uint32_t)(sc - b.scenes)));
+        b.ro[q ^ 1][ri] = p4;
+        b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(scene));
       }
-      const bool need = !have && !exhausted;
-      const uint32_t nmask = __ballot_sync(FULL, need);
-      if (nmask) {
-        const int leader = __ffs(nmask) - 1;
-        uint32_t base = 0;
-        if (lane == leader) base = atomicAdd(&b.ctrl->head[HEAD_NEE], (uint32_t)__popc(nmask));
-        base = __shfl_sync(FULL, base, leader);
-        if (need) {
-          entry = base + __popc(nmask & lt);
-          if (entry < count) {
-            const float4 a4 = b.nee_a[entry], b4 = b.nee_b[entry];
-            const V3 p = ld3(a4);
-            s.r.ox = p.x;
-            s.r.oy = p.y;
-            s.r.oz = p.z;
-            slot = __float_as_uint(a4.w);
-            const V3 N = ld3(b4);
-            mat_idx = __float_as_int(b4.w);
-            seed = b.ps_rng[slot];
-            const float4 c4 = b.nee_c[entry];
-            sc = b.scenes + __float_as_uint(c4.w);
-            ts = trace_scene(*sc);
-            Ns = dot(N, ld3(c4)) < 0.0f ? N : -N;  // faces the incoming ray
-            have = true;
-            shadow = false;
-            wi = v3(0.0f);
-            pl = cos_x = 0.0f;
-            em_m = 0;
-            if (sc->mats[mat_idx].roughness > 0.0f && sc->num_emit > 0) {
-              V3 y;
-              const uint32_t k = sample_emitter(*sc, seed, y);
-              const V3 w = y - p;
-              const float d2 = dot(w, w);
-              const float dist = fsqrt(d2);
-              wi = w * fdiv(1.0f, dist);
-              cos_x = dot(Ns, wi);
-              const float cos_y = fabsf(dot(ld3(__ldg(sc->emit + 4ull * k + 3)), wi));
-              if (cos_x > 0.0f && cos_y > 0.0f && dist > 0.0f) {
-                pl = fdiv(fmul(__ldg(sc->emit + 4ull * k).w, d2), cos_y);
-                em_m = __float_as_int(__ldg(sc->emit + 4ull * k + 1).w);
-                shadow = true;
-                ++nshadow;
-                // stop short of the emitter itself; any blocker will do
-                ray_active = trav_begin(s, ts, p, wi, RAY_TMIN, fmul(dist, 0.9990234375f), tp, true);
-              }
-            }
-            pending = !ray_active;  // no shadow ray, or nothing to traverse
-          } else {
-            exhausted = true;
+      // Idle lanes take their next vertices from the warp's buffer; an empty
+      // one is filled by the whole warp, which shades 32 consecutive rays and
+      // draws the opaque hits' emitter samples.
+      while (__any_sync(FULL, !have && !exhausted)) {
+        if (vb_next == vb_count) {
+          uint32_t base = 0;
+          if (!queue_empty) {
+            if (lane == 0) base = atomicAdd(&b.ctrl->head[HEAD_NEE], 32u);
+            base = __shfl_sync(FULL, base, 0);
           }
+          if (queue_empty || base >= count) {
+            queue_empty = true;
+            if (!have) exhausted = true;
+            break;
+          }
+          vb_next = 0;
+          vb_count = fill_pb_vertices<SPLIT>(b, depth, base, count, vb);
+          vertices += vb_count;
+          __syncwarp();
         }
+        const bool need = !have && !exhausted;
+        const uint32_t nmask = __ballot_sync(FULL, need);
+        const uint32_t k = vb_next + __popc(nmask & lt);
+        vb_next = min(vb_next + (uint32_t)__popc(nmask), vb_count);
+        if (need && k < vb_count) {
+          const float4 a4 = vb.p[k], w4 = vb.w[k], l4 = vb.l[k];
+          vl.p[lane] = a4;
+          vl.n[lane] = vb.n[k];
+          vl.w[lane] = w4;
+          vl.l[lane] = l4;
+          vl.s[lane] = vb.s[k];
+          have = true;
+          s.best_prim = -1;
+          if (w4.w > 0.0f) {
+            ++nshadow;
+            ts = trace_scene(b.scenes[__float_as_uint(l4.w)]);
+            // stop short of the emitter itself; any blocker will do
+            ray_active = trav_begin(s, ts, ld3(a4), ld3(w4), RAY_TMIN, fmul(w4.w, 0.9990234375f), tp, true);
+          }
+          pending = !ray_active;  // no shadow ray, or nothing to traverse
+        }
+        __syncwarp();
       }
       if (!__any_sync(FULL, have)) break;
+      if (__popc(__ballot_sync(FULL, ray_active)) <= (int)b.refill_busy_max && __any_sync(FULL, pending)) continue;
     }
     if (trav_step_warp<COUNT, true>(ray_active, s, ts, stack, visits, tests, &b.ctrl->status, tp)) {
       ray_active = false;
@@ -909,14 +993,12 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(WaveBufs
   }
   warp_add64(&b.ctrl->rays_shadow, nshadow);
   warp_add64(&b.ctrl->shadow_walked, nshadow);  // every shadow ray of this estimator is traced
+  if (lane == 0 && vertices) atomicAdd(&b.ctrl->nee_total, (unsigned long long)vertices);
   if (COUNT) {
     warp_add64(&b.ctrl->node_visits[1], visits);
     warp_add64(&b.ctrl->tri_tests[1], tests);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    b.ctrl->head[HEAD_TRACE] = 0;
-    b.ctrl->nee_total += count;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->head[HEAD_TRACE] = 0;  // trace of this depth is done
 }
 
 // Physically based estimator: the emitter sample of k_nee_pb weighed
@@ -1645,7 +1727,8 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
   }
 }
 
-WaveBufs make_bufs(Renderer& r) {
+// kind: REFILL_*, of the kernel the buffers go to
+WaveBufs make_bufs(Renderer& r, int kind = 0) {
   WaveBufs b;
   std::memset(&b, 0, sizeof(b));
   b.ro[0] = r.ro[0];
@@ -1662,7 +1745,8 @@ WaveBufs make_bufs(Renderer& r) {
   b.ctrl = r.ctrl;
   b.scenes = r.d_scenes;
   b.capacity = r.capacity;
-  b.refill_busy_max = 32u - (r.opts.refill_idle ? std::min<uint32_t>(r.opts.refill_idle, 32u) : LISA_REFILL_IDLE);
+  const int idle = (r.opts.refill_idle ? (int)std::min<uint32_t>(r.opts.refill_idle, 32u) : REFILL_DEFAULT) + kind;
+  b.refill_busy_max = (uint32_t)(32 - std::min(std::max(idle, 1), 32));
   b.physical = r.opts.estimator == LISA_ESTIMATOR_PHYSICAL;
   b.rec_list = r.rec_list;
   b.rec_col = r.rec_list ? r.rec_list + 4ull * r.rec_cap : nullptr;
@@ -1710,12 +1794,12 @@ Status guide_collect(Renderer& r, int, uint32_t cap, cudaStream_t s) {
   return Status();
 }
 
-// Stage indices of the timer: 0 trace, 1 shade, 2 emitter search, 3 other,
+// Stage indices of the timer: 0 trace, 2 shading and emitter search, 3 other,
 // 4 guide inference, 5 guide training (sample collection, training, Adam).
 Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, lisa_render_stats* st,
                             StageTimer* tm) {
   WaveBufs b = make_bufs(r);
-  uint32_t launches[5] = {0, 0, 0, 0, 0};  // trace, shade, nee, guide, total
+  uint32_t launches[5] = {0, 0, 0, 0, 0};  // trace, -, nee, guide, total
   auto stage = [&](int which, auto&& fn) -> Status {
     size_t e0 = 0, e1 = 0;
     if (tm && tm->on) LISA_TRY(tm->ev(&e0));
@@ -1768,8 +1852,7 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
       const uint32_t grid = std::min<uint32_t>((uint32_t)r.path_blocks, std::max<uint32_t>(few, (paths + 32u * wpb - 1u) / (32u * wpb)));
       const uint32_t lanes = std::min<uint32_t>(32u, (paths + grid * wpb - 1u) / (grid * wpb));
       LISA_TRY(stage(0, [&] {
-        WaveBufs bp = b;
-        if (r.opts.refill_idle == 0) bp.refill_busy_max = 32u - LISA_PATHS_REFILL_IDLE;
+        const WaveBufs bp = make_bufs(r, REFILL_PATHS);
         if (physical) k_paths<true><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
         else k_paths<false><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
         return Status();
@@ -1789,23 +1872,19 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
     const uint32_t depths = waves[wv].bounces + (physical ? 1u : 0u);
     for (uint32_t d = 0; d < depths; ++d) {
       LISA_TRY(stage(0, [&] {
+        const WaveBufs b = make_bufs(r, REFILL_TRACE);
         if (counting) k_trace<true><<<r.trace_blocks, r.trace_threads, 0, r.stream>>>(b, (int)d);
         else k_trace<false><<<r.trace_blocks, r.trace_threads, 0, r.stream>>>(b, (int)d);
         return Status();
       }));
-      LISA_TRY(stage(1, [&] {
-        if (physical) k_shade<true><<<r.shade_blocks, r.shade_threads, 0, r.stream>>>(b, (int)d);
-        else k_shade<false><<<r.shade_blocks, r.shade_threads, 0, r.stream>>>(b, (int)d);
-        return Status();
-      }));
-      if (d == waves[wv].bounces) break;  // the emission-only depth has no vertices
       // the guide draws the bounces of the first guide_max_depth vertices
       // of a path (0 = all); deeper ones sample the BSDF (and, with the
       // reference estimator, never the last one, whose bounce is not traced)
-      const bool guided_d = guided && (physical || d + 1 < waves[wv].bounces) &&
+      const bool guided_d = guided && (physical ? d < waves[wv].bounces : d + 1 < waves[wv].bounces) &&
                             (r.opts.guide_max_depth == 0 || d < r.opts.guide_max_depth);
       LISA_TRY(stage(2, [&] {
         const dim3 g(physical ? r.nee_pb_blocks : r.nee_blocks), t(r.nee_threads);
+        const WaveBufs b = make_bufs(r, REFILL_NEE);
         if (physical) {
           if (guided_d) {
             if (counting) k_nee_pb<true, true><<<g, t, 0, r.stream>>>(b, (int)d);
@@ -1857,7 +1936,6 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
   }
   if (st) {
     st->launches_trace += launches[0];
-    st->launches_shade += launches[1];
     st->launches_nee += launches[2];
     st->launches_guide += launches[3];
     st->launches_total += launches[4];
@@ -1963,7 +2041,6 @@ Status renderer_render(Renderer& r, uint32_t spp_req, bool progressive, lisa_ren
         r.graph_key = key;
         r.graph_marks = tm.marks;
         r.graph_launches[0] = counts.launches_trace;
-        r.graph_launches[1] = counts.launches_shade;
         r.graph_launches[2] = counts.launches_nee;
         r.graph_launches[3] = counts.launches_total;
         r.graph_launches[4] = counts.launches_guide;
@@ -1972,7 +2049,6 @@ Status renderer_render(Renderer& r, uint32_t spp_req, bool progressive, lisa_ren
     if (s.ok()) {
       tm.marks = r.graph_marks;
       local.launches_trace = r.graph_launches[0];
-      local.launches_shade = r.graph_launches[1];
       local.launches_nee = r.graph_launches[2];
       local.launches_total = r.graph_launches[3];
       local.launches_guide = r.graph_launches[4];
@@ -2001,7 +2077,6 @@ Status renderer_render(Renderer& r, uint32_t spp_req, bool progressive, lisa_ren
       float t = 0.0f;
       LISA_CUDA(cudaEventElapsedTime(&t, r.ev_pool[m.second.first], r.ev_pool[m.second.second]));
       if (m.first == 0) local.ms_trace += t;
-      else if (m.first == 1) local.ms_shade += t;
       else if (m.first == 2) local.ms_nee += t;
       else if (m.first == 4) {
         local.ms_guide += t;
@@ -2205,9 +2280,6 @@ Status configure_launch(Renderer& r) {
   LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_paths<false>, tthreads, 0));
   bps = r.opts.blocks_per_sm ? (int)r.opts.blocks_per_sm : std::max(occ, 1);
   r.path_blocks = r.sm_count * std::min(bps, std::max(occ, 1));
-  LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_shade<false>, 256, 0));
-  r.shade_threads = 256;
-  r.shade_blocks = r.sm_count * std::max(occ, 1);
   return Status();
 }
 

@@ -15,9 +15,10 @@ struct WaveBufs {
   float4* ps_att;   // per slot: throughput xyz, w = stale emitter material (int, -1 none)
   float4* ps_col;   // per slot: radiance xyz,  w = scene<<24 | pixel
   uint32_t* ps_rng; // per slot: LCG state
-  float4* nee_a;    // emitter-search queue: hit point xyz, w = slot
-  float4* nee_b;    //                       shading normal xyz, w = material
-  float4* nee_c;    //                       incoming direction xyz, w = scene index (bits)
+  // the depth's vertices, for the guide's inference (guided mode; null otherwise)
+  float4* nee_a;    // hit point xyz, w = slot
+  float4* nee_b;    // shading normal xyz, w = material
+  float4* nee_c;    // incoming direction xyz, w = scene index (bits)
   WaveCtrl* ctrl;
   const SceneDev* scenes;
   uint32_t capacity;
