@@ -7,11 +7,12 @@
 // Network: 64 encoded inputs -> 4 x (64, ReLU) -> 40 outputs = 8 vMF lobes
 // (guide_mix.cuh).  FP32 master weights; BF16 copies, pre-swizzled into the
 // K-major 128-byte-swizzle layout the UMMA descriptors expect, are copied
-// into each CTA's shared memory.  A training CTA of 128 threads processes
-// tiles of 128 samples: thread t owns row t of every activation tile, and
-// TMEM lane t of every accumulator.  One elected thread issues tcgen05.mma (M = 128,
-// K = 16 per instruction) and commits to an mbarrier; waits are bounded and
-// a time-out sets a status bit instead of hanging.
+// into each CTA's shared memory.  A training CTA of 256 threads processes
+// tiles of 128 samples: threads t and t + 128 own the halves (columns 0..31
+// and 32..63) of row t of every activation tile and of TMEM lane t of every
+// accumulator.  One elected thread issues tcgen05.mma (M = 128, K = 16 per
+// instruction) and commits to an mbarrier, on which every thread waits;
+// waits are bounded and a time-out sets a status bit instead of hanging.
 //
 // Backward of layer l (weights W_l: out x in; its input H_{l-1} is
 // activation tile l, rows = samples):
@@ -186,23 +187,21 @@ __device__ __forceinline__ void reduce_scatter_round(const float* in, float* out
   }
 }
 
-// Column sums of the warp's 32 rows of v[64] added to the warp's own
-// s_db[0 .. count): a reduce-scatter by recursive halving leaves each lane
-// two of the 64 column sums (different columns in different lanes), which
-// it adds with plain stores -- no atomics, so the sums are the same in
-// every run.
+// Column sums of the warp's 32 rows of v[32] added to s_db[0 .. count): a
+// reduce-scatter by recursive halving leaves each lane one of the 32 column
+// sums, which it adds with a plain store -- no atomics, so the sums are the
+// same in every run.
 __device__ __forceinline__ void add_bias_grad(float* s_db, const float* v, int count) {
-  float a[32], b[16], c[8], d[4], e[2];
-  reduce_scatter_round<64>(v, a, 16);
-  reduce_scatter_round<32>(a, b, 8);
-  reduce_scatter_round<16>(b, c, 4);
-  reduce_scatter_round<8>(c, d, 2);
-  reduce_scatter_round<4>(d, e, 1);
+  float a[16], b[8], c[4], d[2], e[1];
+  reduce_scatter_round<32>(v, a, 16);
+  reduce_scatter_round<16>(a, b, 8);
+  reduce_scatter_round<8>(b, c, 4);
+  reduce_scatter_round<4>(c, d, 2);
+  reduce_scatter_round<2>(d, e, 1);
   const int lane = threadIdx.x & 31;
-  const int col = ((lane & 16) ? 32 : 0) + ((lane & 8) ? 16 : 0) + ((lane & 4) ? 8 : 0) + ((lane & 2) ? 4 : 0) +
-                  ((lane & 1) ? 2 : 0);
+  const int col = ((lane & 16) ? 16 : 0) + ((lane & 8) ? 8 : 0) + ((lane & 4) ? 4 : 0) + ((lane & 2) ? 2 : 0) +
+                  ((lane & 1) ? 1 : 0);
   if (col < count) s_db[col] += e[0];
-  if (col + 1 < count) s_db[col + 1] += e[1];
 }
 
 constexpr int DB_WORDS = 4 * 64 + 40;  // bias gradients of the five layers
@@ -214,24 +213,62 @@ __device__ __forceinline__ float bias_grad_total(const float* s_db, const float*
   return ((s_db[k] + s_db[DB_WORDS + k]) + s_db[2 * DB_WORDS + k]) + s_db[3 * DB_WORDS + k];
 }
 
-// Forward, loss gradient and backward of one 128-sample tile (thread t owns
-// sample i = row t): dW accumulates in TMEM (initialised by the first tile
-// of a batch), db and the loss in per-warp shared-memory sums (s_db: 4 x
-// DB_WORDS, s_loss: 4), added up in warp order by bias_grad_total.  The caller has the weights
-// (w) and biases (s_b) in shared memory and has met at a barrier since.
+constexpr int TRAIN_THREADS = 256;
+
+// 32 of a row's 64 columns (half h) as BF16 into a swizzled tile.
+__device__ __forceinline__ void store_half_row_bf16(uint8_t* tile, int row, int h, const float* v) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint4 q;
+    q.x = pack_bf16x2(v[8 * c + 0], v[8 * c + 1]);
+    q.y = pack_bf16x2(v[8 * c + 2], v[8 * c + 3]);
+    q.z = pack_bf16x2(v[8 * c + 4], v[8 * c + 5]);
+    q.w = pack_bf16x2(v[8 * c + 6], v[8 * c + 7]);
+    *(uint4*)(tile + row * 128 + (((4 * h + c) ^ (row & 7)) << 4)) = q;
+  }
+}
+
+// Features of sample i (zeros beyond n) into this thread's half of its row
+// of tile 0.
 template <int SRC>
-__device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint32_t n, float inv_n, uint8_t* w,
+__device__ __forceinline__ void train_features(const GuideSrc& src, uint32_t i, uint32_t n, uint8_t* act) {
+  const int row = threadIdx.x & 127, h = threadIdx.x >> 7;
+  float v[64];
+  if (i < n) {
+    load_features<SRC>(src, i, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 64; ++k) v[k] = 0.0f;
+  }
+  if (h == 0) store_half_row_bf16(act, row, 0, v);
+  else store_half_row_bf16(act, row, 1, v + 32);
+}
+
+// Forward, loss gradient and backward of one 128-sample tile (threads t and
+// t + 128 own sample i = row t) whose features are in tile 0
+// (train_features): dW accumulates in TMEM (initialised by the first tile of
+// a batch), db and the loss in shared-memory sums per 32 rows (s_db: 4 x
+// DB_WORDS, s_loss: 4), added up in order by bias_grad_total.  The caller has
+// the weights (w) and biases (s_b) in shared memory and has met at a barrier
+// since.  done(l) runs once layer l's dW is complete, while the next layer's
+// products are on the tensor core.  False after a time-out (the same in every
+// thread).
+//
+// A chain of eleven dependent products, each with its epilogue, bounds it:
+// what the next product does not need -- bias gradients, the accumulators of
+// the layer before -- is done while it runs.
+template <int SRC, class Done>
+__device__ __forceinline__ bool train_tile(const GuideSrc& src, uint32_t i, uint32_t n, float inv_n, uint8_t* w,
                                            uint8_t* act, uint32_t tmem, uint32_t lane_off, uint64_t* mbar,
                                            uint32_t& phase, bool first, volatile int* failed, uint32_t* status,
-                                           const float* s_b, float* s_db, float* s_loss) {
-  const int tid = threadIdx.x;
+                                           const float* s_b, float* s_db, float* s_loss, Done&& done) {
+  const int tid = threadIdx.x, row = tid & 127, h = tid >> 7, rows32 = row >> 5;
   auto wait_mma = [&]() {
-    if (tid == 0 && !tc::mbar_wait(mbar, phase)) {
+    if (!tc::mbar_wait(mbar, phase)) {
       atomicOr(status, ST_GUIDE_NONFINITE << 1);
-      *failed = 1;
+      *failed = 1;  // (read by all after the next block barrier)
     }
     phase ^= 1;
-    __syncthreads();
     tc::fence_after_sync();
   };
   auto sync_for_mma = [&]() {
@@ -239,12 +276,11 @@ __device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    return *failed == 0;
   };
   const bool valid = i < n;
-  float v[64];
   float wx = 0.0f, wy = 0.0f, wz = 1.0f, wt = 0.0f;
-  if (valid) {
-    load_features<SRC>(src, i, v);
+  if (valid && h == 0) {
     if (SRC == SRC_RAW) {
       wx = __ldg(src.dirs + 3ull * i);
       wy = __ldg(src.dirs + 3ull * i + 1);
@@ -257,33 +293,40 @@ __device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint
       wz = c.w;
       wt = d.x;
     }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 64; ++k) v[k] = 0.0f;
   }
-  store_row_bf16(act, tid, v);
   // forward
+  float g[64];
+#pragma unroll 1
   for (int l = 0; l < 5; ++l) {
-    sync_for_mma();
+    if (!sync_for_mma()) return false;
     const uint32_t N = l < 4 ? 64u : 48u;
     if (tid == 0) issue_layer(tmem + TM_FWD, act + l * TILE, w + (l < 4 ? (R_FWD + 64 * l) : R_W5) * 128, N, mbar);
     wait_mma();
-    if (*failed) return;
     if (l < 4) {
-      tc::tmem_ld16x<4>(tmem + TM_FWD + lane_off, v);
-      store_row_bias_relu(act + (l + 1) * TILE, tid, v, s_b + 64 * l);
-    } else {
-      tc::tmem_ld16x<3>(tmem + TM_FWD + lane_off, v);
+      float v[32];
+      tc::tmem_ld16x<2>(tmem + TM_FWD + 32 * h + lane_off, v);
+      const float4* b4 = reinterpret_cast<const float4*>(s_b + 64 * l + 32 * h);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 u = b4[2 * c], x = b4[2 * c + 1];
+        uint4 q;
+        q.x = bias_relu_bf16x2(v[8 * c + 0], v[8 * c + 1], u.x, u.y);
+        q.y = bias_relu_bf16x2(v[8 * c + 2], v[8 * c + 3], u.z, u.w);
+        q.z = bias_relu_bf16x2(v[8 * c + 4], v[8 * c + 5], x.x, x.y);
+        q.w = bias_relu_bf16x2(v[8 * c + 6], v[8 * c + 7], x.z, x.w);
+        *(uint4*)(act + (l + 1) * TILE + row * 128 + (((4 * h + c) ^ (row & 7)) << 4)) = q;
+      }
+    } else if (h == 0) {
+      tc::tmem_ld16x<3>(tmem + TM_FWD + lane_off, g);
     }
-    tc::fence_before_sync();
   }
-  // loss gradient at the output (40 values, padded with zeros to 64)
-  float g[64];
-  {
+  // loss gradient at the output (40 values, padded with zeros to 64): one
+  // thread per sample; the other half writes the padding
+  float lsum = 0.0f;
+  if (h == 0) {
     float o[40];
 #pragma unroll
-    for (int k = 0; k < 40; ++k) o[k] = v[k] + s_b[4 * 64 + k];
-    float lsum = 0.0f;
+    for (int k = 0; k < 40; ++k) o[k] = g[k] + s_b[4 * 64 + k];
     if (valid && wt != 0.0f) {
       const float il = rsqrtf(fmaxf(wx * wx + wy * wy + wz * wz, 1e-30f));
       lsum = guide::loss_grad(o, wx * il, wy * il, wz * il, wt * inv_n, g);
@@ -291,32 +334,30 @@ __device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint
 #pragma unroll
       for (int k = 0; k < 40; ++k) g[k] = 0.0f;
     }
+    store_half_row_bf16(act + 5 * TILE, row, 0, g);
+    uint4 q;
+    q.x = pack_bf16x2(g[32], g[33]);
+    q.y = pack_bf16x2(g[34], g[35]);
+    q.z = pack_bf16x2(g[36], g[37]);
+    q.w = pack_bf16x2(g[38], g[39]);
+    *(uint4*)(act + 5 * TILE + row * 128 + ((4 ^ (row & 7)) << 4)) = q;
+  } else {
 #pragma unroll
-    for (int k = 40; k < 64; ++k) g[k] = 0.0f;
-#pragma unroll
-    for (int o2 = 16; o2 > 0; o2 >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o2);
-    if ((tid & 31) == 0) s_loss[tid >> 5] += lsum;
+    for (int c = 5; c < 8; ++c) *(uint4*)(act + 5 * TILE + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
   }
-  float* const s_dbw = s_db + (tid >> 5) * DB_WORDS;  // this warp's sums
-  add_bias_grad(s_dbw + 4 * 64, g, 40);
-  // backward, layer 5 (index 4) down to layer 1 (index 0)
+  float* const s_dbw = s_db + rows32 * DB_WORDS;  // the sums of these 32 rows
+  // backward, layer 5 (index 4) down to layer 1 (index 0): dZ_l is in tile
+  // l + 1, the A operand of dH (K-major) and the upper 64-row block of A of
+  // dW (MN-major)
+#pragma unroll 1
   for (int l = 4; l >= 0; --l) {
-    // dZ_l (registers g) -> tile l + 1: A of dH (K-major) and the upper
-    // 64-row block of A of dW (MN-major)
     uint8_t* tl = act + l * TILE;
-    store_row_bf16(tl + TILE, tid, g);
-    sync_for_mma();
+    if (!sync_for_mma()) return false;
     if (tid == 0) {
       // dW_l += [H^T ; dZ^T] x (H^T)^T over the 128 samples (K = 128):
       // both operands MN-major, 16 samples (two 8-row atoms) per step
       const uint32_t idesc_mn = tc::idesc_bf16_f32_mn(128, 64);
       const uint32_t sh = tc::smem_u32(tl);
-#pragma unroll
-      for (uint32_t ks = 0; ks < 8; ++ks) {
-        const uint32_t base = sh + ks * 2048;
-        tc::mma_bf16(tmem + TM_DW + 64 * l, tc::sw128_mn_desc(base, TILE), tc::sw128_mn_desc(base, TILE), idesc_mn,
-                     (first && ks == 0) ? 0u : 1u);
-      }
       if (l > 0) {
         // dH_{l-1} = dZ_l W_l  (B = W_l^T rows)
         const uint32_t idesc = tc::idesc_bf16_f32(128, 64);
@@ -325,17 +366,37 @@ __device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint
         for (uint32_t k = 0; k < 4; ++k)
           tc::mma_bf16(tmem + TM_DH, tc::sw128_desc(sdz + 32 * k), tc::sw128_desc(swt + 32 * k), idesc, k);
       }
+#pragma unroll
+      for (uint32_t ks = 0; ks < 8; ++ks) {
+        const uint32_t base = sh + ks * 2048;
+        tc::mma_bf16(tmem + TM_DW + 64 * l, tc::sw128_mn_desc(base, TILE), tc::sw128_mn_desc(base, TILE), idesc_mn,
+                     (first && ks == 0) ? 0u : 1u);
+      }
       tc::mma_commit(mbar);
     }
+    // meanwhile: the bias gradients of layer l and dW of the layer above
+    if (l == 4) {
+      if (h == 0) {
+        add_bias_grad(s_dbw + 4 * 64, g, 32);
+#pragma unroll
+        for (int k = 40; k < 64; ++k) g[k] = 0.0f;
+        add_bias_grad(s_dbw + 4 * 64 + 32, g + 32, 8);
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o2);
+        if ((tid & 31) == 0) s_loss[rows32] += lsum;
+      }
+    } else {
+      add_bias_grad(s_dbw + 64 * l + 32 * h, g, 32);
+      done(l + 1);
+    }
     wait_mma();
-    if (*failed) return;
     if (l > 0) {
       // dZ_{l-1} = dH_{l-1} where H_{l-1} > 0: the BF16 bits of this
       // sample's row of tile l, +-0 masked out
-      tc::tmem_ld16x<4>(tmem + TM_DH + lane_off, g);
+      tc::tmem_ld16x<2>(tmem + TM_DH + 32 * h + lane_off, g);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const uint4 q = *(const uint4*)(tl + tid * 128 + ((c ^ (tid & 7)) << 4));
+      for (int c = 0; c < 4; ++c) {
+        const uint4 q = *(const uint4*)(tl + row * 128 + (((4 * h + c) ^ (row & 7)) << 4));
         const uint32_t hw[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -343,39 +404,36 @@ __device__ __forceinline__ void train_tile(const GuideSrc& src, uint32_t i, uint
           if ((hw[j] & 0x7fff0000u) == 0u) g[8 * c + 2 * j + 1] = 0.0f;
         }
       }
-      add_bias_grad(s_dbw + 64 * (l - 1), g, 64);
+      store_half_row_bf16(tl, row, h, g);
     }
-    tc::fence_before_sync();
   }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (*failed) return false;
+  done(0);
+  return true;
 }
 
-// Reads this thread's row o (< 64) of dW_l, l = 0..4 (rows 64..127 of the
-// accumulators: the TMEM lanes of warps 2 and 3), and hands each layer's
-// row to put(l, o, d) when the layer has that row (W5 has 40).
-template <class Put>
-__device__ __forceinline__ void flush_dw(uint32_t tmem, uint32_t lane_off, bool ok, Put&& put) {
-  const int warp = threadIdx.x >> 5;
-  if (warp < 2) return;
-  const int o = (warp - 2) * 32 + (threadIdx.x & 31);
-  for (int l = 0; l < 5; ++l) {
-    const int rows = l < 4 ? 64 : 40;
-    float d[64];
-    if (ok) {
+// Half of row o (< 64) of dW_l (rows 64..127 of the accumulator: the TMEM
+// lanes of warps 2, 3, 6 and 7) to the CTA's slot; W5 has 40 rows.
+__device__ __forceinline__ void flush_dw(uint32_t tmem, uint32_t lane_off, int l, float* slot) {
+  const int row = threadIdx.x & 127, h = threadIdx.x >> 7;
+  if (row < 64) return;  // (whole warps)
+  const int o = row - 64;
+  float d[32];
+  tc::tmem_ld16x<2>(tmem + TM_DW + 64 * l + 32 * h + lane_off, d);
+  if (o >= (l < 4 ? 64 : 40)) return;
+  float4* gw = reinterpret_cast<float4*>(slot + (l < 4 ? P_W + l * 4096 : P_W5) + o * 64 + 32 * h);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tc::tmem_ld16(tmem + TM_DW + 64 * l + lane_off + c * 16, d + c * 16);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 64; ++c) d[c] = 0.0f;
-    }
-    if (o < rows) put(l, o, d);
-  }
+  for (int k = 0; k < 8; ++k) gw[k] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
 }
 
 template <int SRC>
-__global__ void __launch_bounds__(128, 1) k_guide_train(const uint16_t* __restrict__ pack, const float* __restrict__ master,
-                                                        GuideSrc src, float inv_n, float* __restrict__ part,
-                                                        float* __restrict__ loss_part, uint32_t* status,
-                                                        uint32_t* __restrict__ step_bump) {
+__global__ void __launch_bounds__(TRAIN_THREADS, 1)
+    k_guide_train(const uint16_t* __restrict__ pack, const float* __restrict__ master, GuideSrc src, float inv_n,
+                  float* __restrict__ part, float* __restrict__ loss_part, uint32_t* status,
+                  uint32_t* __restrict__ step_bump) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* w = smem;
@@ -384,7 +442,7 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(const uint16_t* __restri
   __shared__ uint64_t mbar_w;  // the packed weights' bulk copy
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
-  __shared__ float s_db[4 * DB_WORDS];  // per warp
+  __shared__ float s_db[4 * DB_WORDS];  // per 32 rows
   __shared__ __align__(16) float s_b[4 * 64 + 48];  // biases
   __shared__ float s_loss[4];
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -407,9 +465,9 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(const uint16_t* __restri
     failed = 0;
   }
   if (tid < 4) s_loss[tid] = 0.0f;
-  for (int k = tid; k < 4 * DB_WORDS; k += 128) s_db[k] = 0.0f;
+  for (int k = tid; k < 4 * DB_WORDS; k += TRAIN_THREADS) s_db[k] = 0.0f;
   if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
-  for (int k = tid; k < 4 * 64 + 48; k += 128) s_b[k] = k < 4 * 64 + 40 ? __ldg(master + P_B + k) : 0.0f;
+  for (int k = tid; k < 4 * 64 + 48; k += TRAIN_THREADS) s_b[k] = k < 4 * 64 + 40 ? __ldg(master + P_B + k) : 0.0f;
   if (tid == 0 && !tc::mbar_wait(&mbar_w, 0)) {
     atomicOr(status, ST_GUIDE_NONFINITE << 1);
     failed = 1;
@@ -419,27 +477,25 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(const uint16_t* __restri
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_base;
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+  const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
   uint32_t phase = 0;
-  bool first = true;
-  for (uint32_t t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
-    train_tile<SRC>(src, src.first + t * 128 + tid, n, inv_n, w, act, tmem, lane_off, &mbar, phase, first, &failed,
-                    status, s_b, s_db, s_loss);
+  bool first = true, ok = failed == 0;
+  for (uint32_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+    const uint32_t i = src.first + t * 128 + (tid & 127);
+    const bool last = t + gridDim.x >= ntiles;
+    train_features<SRC>(src, i, n, act);
+    ok = train_tile<SRC>(src, i, n, inv_n, w, act, tmem, lane_off, &mbar, phase, first, &failed, status, s_b, s_db,
+                         s_loss, [&](int l) {
+                           if (last) flush_dw(tmem, lane_off, l, slot);
+                         });
     first = false;
   }
-  tc::fence_before_sync();
   __syncthreads();
-  tc::fence_after_sync();
-  const bool ok = !failed && !first;
-  flush_dw(tmem, lane_off, ok, [&](int l, int o, const float* d) {
-    float4* gw = reinterpret_cast<float4*>(slot + (l < 4 ? P_W + l * 4096 : P_W5) + o * 64);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) gw[k] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
-  });
-  __syncthreads();
-  for (int k = tid; k < DB_WORDS; k += 128) slot[P_B + k] = ok ? bias_grad_total(s_db, s_loss, k) : 0.0f;
+  if (!ok)
+    for (int k = tid; k < NPARAM; k += TRAIN_THREADS) slot[k] = 0.0f;
+  for (int k = tid; k < DB_WORDS; k += TRAIN_THREADS) slot[P_B + k] = ok ? bias_grad_total(s_db, s_loss, k) : 0.0f;
   if (tid == 0) loss_part[blockIdx.x] = ok ? bias_grad_total(s_db, s_loss, DB_WORDS) : 0.0f;
-  if (tid == 0 && failed) {
+  if (tid == 0 && !ok) {
     tc::mbar_wait(&mbar_w, 0, 1u << 20);       // a late weight copy: bounded second chance
     tc::mbar_wait(&mbar, phase ^ 1u, 1u << 20);  // and an MMA still in flight
   }
@@ -454,12 +510,17 @@ __global__ void __launch_bounds__(128, 1) k_guide_train(const uint16_t* __restri
 // (k + 1) x gridDim.x.  Memory written before the barrier (with a device
 // fence) is visible after it to loads that bypass L1.  The wait has an
 // iteration limit; false (the same in every thread of the CTA) when it
-// ran out, with the status bit set.
-__device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t k, uint32_t* status, volatile int* s_ok) {
+// ran out, with the status bit set.  Between arriving and waiting a CTA may
+// do work that needs nothing of the others.
+__device__ __forceinline__ void grid_arrive(uint32_t* counter) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(counter, 1u);
+  }
+}
+__device__ __forceinline__ bool grid_wait(uint32_t* counter, uint32_t k, uint32_t* status, volatile int* s_ok) {
+  if (threadIdx.x == 0) {
     const uint32_t target = (k + 1) * gridDim.x;
     bool ok = false;
     for (uint32_t it = 0; it < (1u << 22); ++it) {
@@ -469,7 +530,7 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t k, uint
         ok = true;
         break;
       }
-      __nanosleep(64);
+      if (it >= 64) __nanosleep(64);
     }
     if (!ok) atomicOr(status, ST_GUIDE_NONFINITE << 1);
     *s_ok = ok ? 1 : 0;
@@ -480,28 +541,33 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* counter, uint32_t k, uint
 
 // One wave's training rounds in one cooperative launch (one CTA per SM, all
 // resident): for each slice of `chunk` samples [s * chunk, (s + 1) * chunk)
-// of the batch (while the batch has samples), every CTA
+// of the batch (while the batch has samples), every CTA that has a tile of
+// the slice
 //   1. reads the current weights (a bulk copy behind a proxy fence) and
 //      biases (loads that bypass L1): other CTAs wrote them last round,
 //   2. runs its tiles of the slice (forward, loss gradient, backward),
 //   3. writes its dW, db and loss to its own slot of part / loss_part,
-// the grid meets, CTA c sums the slots over its share of 128 parameters
-// (the same order as k_guide_adam: deterministic) and applies Adam to
-// them, refreshing their FP32 master and BF16 forward / transposed copies,
-// and the grid meets again.  The same steps as a training launch followed
-// by an Adam launch per slice, without their launches and per-launch
-// set-up.  grid_bar: the grid barrier's arrival counter, zero at launch.
+// the grid meets, CTA c sums those slots over its share of 128 parameters
+// (the same order as k_guide_adam: deterministic) and applies Adam to them,
+// refreshing their FP32 master and BF16 forward / transposed copies, and the
+// grid meets again.  The next slice's features are encoded, and the share's
+// parameters and moments loaded, before the first meeting.  The same steps as
+// a training launch followed by an Adam launch per slice, without their
+// launches and per-launch set-up.  grid_bar: the grid barrier's arrival
+// counter, zero at launch.
+//
+// A round is a serial chain: with 256 threads a tile, the work that the next
+// product does not need behind it, and only the CTAs and slots that have a
+// tile, it takes 16.9 us for one tile (24 before), 20.2 us for 152 (27).
 constexpr uint32_t ADAM_SHARE = 128;  // parameters per CTA in the Adam phase (a multiple of 4)
 
 template <int SRC>
-__global__ void __launch_bounds__(128, 1) k_guide_train_rounds(uint16_t* __restrict__ pack, float* __restrict__ master,
-                                                               float* __restrict__ adam_m, float* __restrict__ adam_v,
-                                                               GuideSrc src, uint32_t chunk, uint32_t rounds,
-                                                               float lr, float* __restrict__ part,
-                                                               float* __restrict__ loss_part, uint32_t* grid_bar,
-                                                               float* __restrict__ loss_last, uint32_t* step_count,
-                                                               uint32_t* status,
-                                                               unsigned long long* __restrict__ sample_count) {
+__global__ void __launch_bounds__(TRAIN_THREADS, 1)
+    k_guide_train_rounds(uint16_t* __restrict__ pack, float* __restrict__ master, float* __restrict__ adam_m,
+                         float* __restrict__ adam_v, GuideSrc src, uint32_t chunk, uint32_t rounds, float lr,
+                         float* __restrict__ part, float* __restrict__ loss_part, uint32_t* grid_bar,
+                         float* __restrict__ loss_last, uint32_t* step_count, uint32_t* status,
+                         unsigned long long* __restrict__ sample_count) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* w = smem;
@@ -511,7 +577,7 @@ __global__ void __launch_bounds__(128, 1) k_guide_train_rounds(uint16_t* __restr
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
   __shared__ int bar_ok;
-  __shared__ float s_db[4 * DB_WORDS];  // per warp
+  __shared__ float s_db[4 * DB_WORDS];  // per 32 rows
   __shared__ __align__(16) float s_b[4 * 64 + 48];
   __shared__ float s_loss[4];
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -528,87 +594,111 @@ __global__ void __launch_bounds__(128, 1) k_guide_train_rounds(uint16_t* __restr
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_base;
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
+  const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
   const float inv_n = 1.0f / (float)chunk;
   // the Adam phase: for each share of 128 parameters p0.. of this CTA,
-  // thread (g, q) = (tid / 4, tid % 4) sums the slots j = q (mod 4) of
-  // parameters p0 + 4 g .. + 3 (one float4 a slot); the quad's sums meet by
-  // shuffles and thread (g, q) updates parameter p0 + 4 g + q
+  // thread (g, q) = (tid / 4, tid % 4) of the first 128 sums the slots
+  // j = q (mod 4) of parameters p0 + 4 g .. + 3 (one float4 a slot); the
+  // quad's sums meet by shuffles and thread (g, q) updates parameter
+  // p0 + 4 g + q
   const uint32_t qq = tid & 3;
   float* slot = part + (size_t)blockIdx.x * NPARAM;
   uint32_t phase = 0, wphase = 0, bars = 0, done = 0;
   bool w_busy = false;  // thread 0: a weight copy not waited for
+  // this CTA's first tile of round r: its features into tile 0
+  auto features = [&](uint32_t r) {
+    const uint32_t first = r * chunk;
+    if (r >= rounds || first >= n) return;
+    const uint32_t last = min(first + chunk, n), i = first + blockIdx.x * 128u + (uint32_t)(tid & 127);
+    if (blockIdx.x * 128u < last - first) train_features<SRC>(src, i, last, act);
+  };
+  features(0);
   for (uint32_t r = 0; r < rounds; ++r) {
     const uint32_t first = r * chunk;
     if (first >= n) break;  // the same in every CTA
     const uint32_t last = min(first + chunk, n);
-    // 1. weights (bulk copy; the other CTAs' generic-proxy writes of the
-    // last round are ordered before it by the grid barrier and the proxy
-    // fence) and biases (loads that bypass L1)
-    if (tid == 0) {
-      asm volatile("fence.proxy.async.global;" ::: "memory");
-      tc::bulk_load(w, pack, PACK_BYTES, &mbar_w);
-      w_busy = true;
-    }
-    for (int k = tid; k < 4 * 64 + 48; k += 128) s_b[k] = k < 4 * 64 + 40 ? __ldcg(master + P_B + k) : 0.0f;
-    for (int k = tid; k < 4 * DB_WORDS; k += 128) s_db[k] = 0.0f;
-    if (tid < 4) s_loss[tid] = 0.0f;
-    if (tid == 0) {
-      if (tc::mbar_wait(&mbar_w, wphase)) {
-        w_busy = false;
-      } else {
-        atomicOr(status, ST_GUIDE_NONFINITE << 1);
-        failed = 1;
-      }
-      wphase ^= 1u;
-    }
-    tc::fence_smem_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    // 2. this CTA's tiles of the slice
     const uint32_t ntiles = (last - first + 127) / 128;
-    bool any = false;
-    for (uint32_t t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
-      train_tile<SRC>(src, first + t * 128 + tid, last, inv_n, w, act, tmem, lane_off, &mbar, phase, !any, &failed,
-                      status, s_b, s_db, s_loss);
-      any = true;
+    const uint32_t nslots = min(ntiles, gridDim.x);  // CTAs with a tile
+    if (blockIdx.x < ntiles) {
+      // 1. weights (bulk copy; the other CTAs' generic-proxy writes of the
+      // last round are ordered before it by the grid barrier and the proxy
+      // fence) and biases (loads that bypass L1)
+      if (tid == 0) {
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        tc::bulk_load(w, pack, PACK_BYTES, &mbar_w);
+        w_busy = true;
+      }
+      for (int k = tid; k < 4 * 64 + 48; k += TRAIN_THREADS) s_b[k] = k < 4 * 64 + 40 ? __ldcg(master + P_B + k) : 0.0f;
+      for (int k = tid; k < 4 * DB_WORDS; k += TRAIN_THREADS) s_db[k] = 0.0f;
+      if (tid < 4) s_loss[tid] = 0.0f;
+      if (tid == 0) {
+        if (tc::mbar_wait(&mbar_w, wphase)) {
+          w_busy = false;
+        } else {
+          atomicOr(status, ST_GUIDE_NONFINITE << 1);
+          failed = 1;
+        }
+        wphase ^= 1u;
+      }
+      // 2. this CTA's tiles of the slice (train_tile begins with a block
+      // barrier)
+      bool ok = true;
+      for (uint32_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+        const uint32_t i = first + t * 128 + (tid & 127);
+        const bool last_tile = t + gridDim.x >= ntiles;
+        if (t != blockIdx.x) train_features<SRC>(src, i, last, act);
+        // 3. its slot
+        ok = train_tile<SRC>(src, i, last, inv_n, w, act, tmem, lane_off, &mbar, phase, t == blockIdx.x, &failed,
+                             status, s_b, s_db, s_loss, [&](int l) {
+                               if (last_tile) flush_dw(tmem, lane_off, l, slot);
+                             });
+      }
+      if (!ok)
+        for (int k = tid; k < NPARAM; k += TRAIN_THREADS) slot[k] = 0.0f;
+      for (int k = tid; k < DB_WORDS; k += TRAIN_THREADS) slot[P_B + k] = ok ? bias_grad_total(s_db, s_loss, k) : 0.0f;
+      if (tid == 0) loss_part[blockIdx.x] = ok ? bias_grad_total(s_db, s_loss, DB_WORDS) : 0.0f;
     }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    // 3. this CTA's slot (zeros when it had no tile this round)
-    const bool ok = any && !failed;
-    flush_dw(tmem, lane_off, ok, [&](int l, int o, const float* d) {
-      float4* gw = reinterpret_cast<float4*>(slot + (l < 4 ? P_W + l * 4096 : P_W5) + o * 64);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) gw[k] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
-    });
-    for (int k = tid; k < DB_WORDS; k += 128) slot[P_B + k] = ok ? bias_grad_total(s_db, s_loss, k) : 0.0f;
-    if (tid == 0) loss_part[blockIdx.x] = ok ? bias_grad_total(s_db, s_loss, DB_WORDS) : 0.0f;
-    if (!grid_barrier(grid_bar, bars++, status, &bar_ok) || failed) break;
-    // Adam on this CTA's share (the step of k_guide_adam)
+    grid_arrive(grid_bar);
+    // what needs nothing of the others: the next slice's features, this
+    // share's parameters and moments
+    features(r + 1);
+    const uint32_t i0 = blockIdx.x * ADAM_SHARE + 4u * (tid >> 2) + qq;
+    float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f;
+    if (tid < (int)ADAM_SHARE && i0 < (uint32_t)NPARAM) {
+      m0 = __ldcg(adam_m + i0);
+      v0 = __ldcg(adam_v + i0);
+      w0 = __ldcg(master + i0);
+    }
     const float t = (float)(t0 + done + 1);
     const float b1c = 1.0f - powf(0.9f, t), b2c = 1.0f - powf(0.999f, t);
-    if (blockIdx.x == 0 && warp == 0) {
+    if (!grid_wait(grid_bar, bars++, status, &bar_ok) || failed) break;
+    // Adam on this CTA's share (the step of k_guide_adam)
+    if (blockIdx.x == 0 && warp == 4) {
       float l = 0.0f;
-      for (uint32_t j = tid; j < gridDim.x; j += 32) l += __ldcg(loss_part + j);
+      for (uint32_t j = tid & 31; j < nslots; j += 32) l += __ldcg(loss_part + j);
 #pragma unroll
       for (int m = 16; m > 0; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
-      if (tid == 0) *loss_last = l;
+      if ((tid & 31) == 0) *loss_last = l;
     }
-    for (uint32_t p0 = blockIdx.x * ADAM_SHARE; p0 < (uint32_t)NPARAM; p0 += gridDim.x * ADAM_SHARE) {
+    for (uint32_t p0 = blockIdx.x * ADAM_SHARE; p0 < (uint32_t)NPARAM && tid < (int)ADAM_SHARE;
+         p0 += gridDim.x * ADAM_SHARE) {
       const uint32_t pq = p0 + 4u * (tid >> 2);
       float4 g4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (pq < (uint32_t)NPARAM) {
-        // (sixteen slots in flight per thread: the sum is latency-bound)
-#pragma unroll 16
-        for (uint32_t j = qq; j < gridDim.x; j += 4) {
-          const float4 x = __ldcg(reinterpret_cast<const float4*>(part + (size_t)j * NPARAM + pq));
-          g4.x += x.x;
-          g4.y += x.y;
-          g4.z += x.z;
-          g4.w += x.w;
+        // (up to 19 slots in flight per thread: the sum is latency-bound)
+        for (uint32_t j0 = qq; j0 < nslots; j0 += 76) {
+          float4 x[19];
+#pragma unroll
+          for (uint32_t k = 0; k < 19; ++k)
+            if (j0 + 4 * k < nslots) x[k] = __ldcg(reinterpret_cast<const float4*>(part + (size_t)(j0 + 4 * k) * NPARAM + pq));
+#pragma unroll
+          for (uint32_t k = 0; k < 19; ++k)
+            if (j0 + 4 * k < nslots) {
+              g4.x += x[k].x;
+              g4.y += x[k].y;
+              g4.z += x[k].z;
+              g4.w += x[k].w;
+            }
         }
       }
 #pragma unroll
@@ -623,8 +713,9 @@ __global__ void __launch_bounds__(128, 1) k_guide_train_rounds(uint16_t* __restr
       if (i < (uint32_t)NPARAM) {
         if (!isfinite(gi)) atomicOr(status, ST_GUIDE_NONFINITE);
         else {
-          float mi = __ldcg(adam_m + i), vi = __ldcg(adam_v + i);
-          const float wv = adam_update(__ldcg(master + i), gi, mi, vi, lr, b1c, b2c);
+          const bool own = i == i0;  // loaded before the grid met
+          float mi = own ? m0 : __ldcg(adam_m + i), vi = own ? v0 : __ldcg(adam_v + i);
+          const float wv = adam_update(own ? w0 : __ldcg(master + i), gi, mi, vi, lr, b1c, b2c);
           adam_m[i] = mi;
           adam_v[i] = vi;
           master[i] = wv;
@@ -642,7 +733,8 @@ __global__ void __launch_bounds__(128, 1) k_guide_train_rounds(uint16_t* __restr
     }
     asm volatile("fence.proxy.async.global;" ::: "memory");  // the pack, read next round by bulk copies
     ++done;
-    if (!grid_barrier(grid_bar, bars++, status, &bar_ok)) break;
+    grid_arrive(grid_bar);
+    if (!grid_wait(grid_bar, bars++, status, &bar_ok)) break;
   }
   if (blockIdx.x == 0 && tid == 0) {
     *step_count = t0 + done;
@@ -779,7 +871,7 @@ Status guide_launch_train(GuideNet& g, const GuideSrc& src, float inv_n, uint32_
   const uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)sm_count_current());
   g.nparts = grid;
   uint32_t* bump = adam_follows ? g.d_step : nullptr;
-  k_guide_train<SRC_RAW><<<grid, 128, TRAIN_SMEM, s>>>(g.w_bf16, g.master, src, inv_n, g.grad_part, g.loss_part,
+  k_guide_train<SRC_RAW><<<grid, TRAIN_THREADS, TRAIN_SMEM, s>>>(g.w_bf16, g.master, src, inv_n, g.grad_part, g.loss_part,
                                                        g.status, bump);
   LISA_CUDA(cudaGetLastError());
   return Status();
@@ -800,7 +892,7 @@ Status guide_launch_train_rounds(GuideNet& g, const GuideSrc& src, int src_kind,
   LISA_CUDA(cudaMemsetAsync(grid_bar, 0, sizeof(uint32_t), s));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)sm_count_current());
-  cfg.blockDim = dim3(128);
+  cfg.blockDim = dim3(TRAIN_THREADS);
   cfg.dynamicSmemBytes = TRAIN_SMEM;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
