@@ -8,6 +8,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -308,11 +309,78 @@ Status validate(const lisa_renderer_params& p) {
   if (p.num_materials < 0 || (p.num_materials > 0 && !p.materials)) return Status::invalid("bad material table");
   if (p.width == 0 || p.height == 0) return Status::invalid("width and height must be positive");
   if ((uint64_t)p.width * p.height >= (1ull << 24)) return Status::invalid("at most 2^24 - 1 pixels per scene");
-  const uint32_t T = (uint32_t)(p.num_vertices / 3);
-  for (uint32_t i = 0; i < T; ++i)
-    if (p.mat_indices[i] < 0 || p.mat_indices[i] >= p.num_materials)
-      return Status::invalid("material index out of range at triangle " + std::to_string(i));
   return Status();
+}
+
+// What creating a scene has to know about its triangles, found by
+// k_scan_prims: the first triangle whose material index is out of range (~0:
+// none), the number of emissive triangles and their bounds (order-preserving
+// ints).
+struct PrimScan {
+  uint32_t bad, emissive;
+  int lo[3], hi[3];
+};
+
+// One pass over the uploaded triangles: material check, what the BVH leaves
+// carry (leaf[p] = the material if it emits, else -1, so that the emitter
+// search reads the class of a hit without a material look-up), the emissive
+// triangles as a bit mask, their number and bounds.  em[m] = m for the nm
+// materials that emit, else -1.
+//
+// Bound by the 4 + 4 bytes a triangle that it streams (vertices are read for
+// emissive triangles only): 7 us for 1.31 M triangles, where three loops
+// over them on the host took 2.6 ms of a renderer's creation.  Bounds and
+// count stay in registers until a warp's last triangle, so a soup of
+// emitters costs a warp seven atomics, not each 32 triangles.
+__global__ void k_scan_prims(const float* __restrict__ v, const int32_t* __restrict__ m, uint32_t n,
+                             const int32_t* __restrict__ em, uint32_t nm, int32_t* __restrict__ leaf,
+                             uint32_t* __restrict__ mask, PrimScan* scan) {
+  const uint32_t lane = threadIdx.x & 31;
+  float lo[3], hi[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = INFINITY;
+    hi[k] = -INFINITY;
+  }
+  uint32_t bad = 0xffffffffu, emissive = 0;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < n; base += stride) {
+    const uint32_t i = base + lane;
+    bool emits = false;
+    if (i < n) {
+      const uint32_t k = (uint32_t)m[i];
+      if (k >= nm) bad = min(bad, i);
+      const int32_t e = k < nm ? __ldg(em + k) : -1;
+      leaf[i] = e;
+      emits = e >= 0;
+    }
+    const uint32_t bits = __ballot_sync(0xffffffffu, emits);
+    if (lane == 0) mask[base >> 5] = bits;
+    emissive += __popc(bits);
+    if (emits)
+      for (int j = 0; j < 9; ++j) {
+        const float c = v[9ull * i + j];
+        lo[j % 3] = fminf(lo[j % 3], c);  // (a coordinate that is not a number is passed over)
+        hi[j % 3] = fmaxf(hi[j % 3], c);
+      }
+  }
+  bad = __reduce_min_sync(0xffffffffu, bad);
+  if (lane == 0 && bad != 0xffffffffu) atomicMin(&scan->bad, bad);
+  if (emissive == 0) return;  // the same in all lanes
+  if (lane == 0) atomicAdd(&scan->emissive, emissive);
+  for (int k = 0; k < 3; ++k) {
+    const int a = __reduce_min_sync(0xffffffffu, f2ord(lo[k])), b = __reduce_max_sync(0xffffffffu, f2ord(hi[k]));
+    if (lane == 0) {
+      atomicMin(&scan->lo[k], a);
+      atomicMax(&scan->hi[k], b);
+    }
+  }
+}
+
+// Calls f(triangle) for each set bit, in triangle order.
+template <class F>
+void for_each_bit(const std::vector<uint32_t>& mask, F&& f) {
+  for (size_t k = 0; k < mask.size(); ++k)
+    for (uint32_t bits = mask[k]; bits; bits &= bits - 1) f((uint32_t)(32 * k) + (uint32_t)__builtin_ctz(bits));
 }
 }  // namespace
 
@@ -321,25 +389,25 @@ Status validate(const lisa_renderer_params& p) {
 // (v0, area pdf) (e1 = v1 - v0, material) (e2 = v2 - v0) (unit normal) and a
 // CDF entry over area x luminance; each material gets its area pdf
 // luminance / total.  Float steps as written (no contraction), sums in double.
-Status build_emitters(Renderer& r, const lisa_renderer_params& p, SceneGpu& s, std::vector<DevMaterial>& dm) {
+Status build_emitters(Renderer& r, const lisa_renderer_params& p, const std::vector<uint32_t>& emissive, SceneGpu& s,
+                      std::vector<DevMaterial>& dm) {
   const int M = p.num_materials;
-  const uint32_t T = (uint32_t)(p.num_vertices / 3);
   std::vector<float> lum(std::max(M, 1), 0.0f);
   for (int m = 0; m < M; ++m)
     if (dm[m].cls == MAT_EMIT)
       lum[m] = (0.2126f * dm[m].emission[0] + 0.7152f * dm[m].emission[1]) + 0.0722f * dm[m].emission[2];
   std::vector<float4> rec;
   std::vector<double> w;
-  for (uint32_t t = 0; t < T; ++t) {
+  for_each_bit(emissive, [&](uint32_t t) {
     const int m = p.mat_indices[t];
-    if (dm[m].cls != MAT_EMIT || !(lum[m] > 0.0f)) continue;
+    if (!(lum[m] > 0.0f)) return;
     const lisa_float3* v = p.vertices + 3ull * t;
     const float e1x = v[1].x - v[0].x, e1y = v[1].y - v[0].y, e1z = v[1].z - v[0].z;
     const float e2x = v[2].x - v[0].x, e2y = v[2].y - v[0].y, e2z = v[2].z - v[0].z;
     const float cx = e1y * e2z - e1z * e2y, cy = e1z * e2x - e1x * e2z, cz = e1x * e2y - e1y * e2x;
     const float len = std::sqrt(cx * cx + cy * cy + cz * cz);
     const float area = 0.5f * len;
-    if (!(area > 0.0f)) continue;
+    if (!(area > 0.0f)) return;
     const float inv = 1.0f / len;
     int32_t mb = m;
     float mf;
@@ -349,7 +417,7 @@ Status build_emitters(Renderer& r, const lisa_renderer_params& p, SceneGpu& s, s
     rec.push_back(make_float4(e2x, e2y, e2z, 0.0f));
     rec.push_back(make_float4(cx * inv, cy * inv, cz * inv, 0.0f));
     w.push_back((double)area * (double)lum[m]);
-  }
+  });
   s.num_emit = (uint32_t)w.size();
   if (!s.num_emit) return Status();
   double total = 0.0;
@@ -374,16 +442,6 @@ Status build_emitters(Renderer& r, const lisa_renderer_params& p, SceneGpu& s, s
   return Status();
 }
 
-// Per triangle: its material if that is an emitter, else -1 (what the BVH
-// leaves carry, so the emitter search reads the class of a hit without a
-// material look-up).
-__global__ void k_emit_of_prim(int32_t* m, uint32_t n, const int32_t* em, uint32_t nm) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t k = (uint32_t)m[i];
-    m[i] = k < nm ? em[k] : -1;
-  }
-}
-
 // Leaf triangles of the emitters' own BVH carry their index among the
 // emitters; make it the scene-wide triangle index (the tie rule compares
 // scene-wide indices).
@@ -398,13 +456,11 @@ __global__ void k_emit_global_ids(float4* tris, uint32_t n, const int32_t* __res
 // BVH over the scene's emissive triangles, built like the scene's (same
 // builder, so the same exact traversal); leaves carry scene-wide triangle
 // indices and emitter materials.
-Status build_emitter_bvh(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
+Status build_emitter_bvh(Renderer& r, const lisa_renderer_params& p, const std::vector<uint32_t>& emissive,
+                         SceneGpu& s) {
   std::vector<float> ev;
   std::vector<int32_t> gid, emat;
-  const uint32_t T = (uint32_t)(p.num_vertices / 3);
-  for (uint32_t t = 0; t < T; ++t) {
-    const int32_t m = p.mat_indices[t];
-    if (m < 0 || m >= p.num_materials || !p.materials[m].emit) continue;
+  for_each_bit(emissive, [&](uint32_t t) {
     for (int j = 0; j < 3; ++j) {
       const lisa_float3& v = p.vertices[3ull * t + j];
       ev.push_back(v.x);
@@ -412,10 +468,9 @@ Status build_emitter_bvh(Renderer& r, const lisa_renderer_params& p, SceneGpu& s
       ev.push_back(v.z);
     }
     gid.push_back((int32_t)t);
-    emat.push_back(m);
-  }
+    emat.push_back(p.mat_indices[t]);
+  });
   const uint32_t ne = (uint32_t)gid.size();
-  if (ne < EMIT_BVH_MIN_TRIS) return Status();  // the emitter search would not use it
   float* d_ev = nullptr;
   int32_t *d_gid = nullptr, *d_emat = nullptr;
   cudaError_t e = dev_alloc((void**)&d_ev, sizeof(float) * ev.size());
@@ -444,6 +499,26 @@ Status build_emitter_bvh(Renderer& r, const lisa_renderer_params& p, SceneGpu& s
   return st;
 }
 
+namespace {
+// Device copies of a scene's soup while it is created, and the builder's
+// scratch.  Its blocks go back to the cache once both streams are done.
+struct SceneUpload : TempDeviceBufs {
+  float *v = nullptr, *n = nullptr;
+  int32_t *m = nullptr, *leaf = nullptr, *em = nullptr;
+  uint32_t* mask = nullptr;
+  PrimScan* scan = nullptr;
+  cudaStream_t side = nullptr;
+  cudaEvent_t ready = nullptr;
+  ~SceneUpload() {
+    if (side) {
+      cudaStreamSynchronize(side);
+      cudaStreamDestroy(side);
+    }
+    if (ready) cudaEventDestroy(ready);
+  }
+};
+}  // namespace
+
 Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
   LISA_TRY(validate(p));
   s.params = p;
@@ -456,52 +531,63 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
   s.num_prims = (uint32_t)(p.num_vertices / 3);
   s.npix = p.width * p.height;
   const uint32_t T = s.num_prims;
-  // upload the soup (72 B + 4 B per triangle) and pack the shading records
-  float *d_v = nullptr, *d_n = nullptr;
-  int32_t* d_m = nullptr;
+  // upload the soup (72 B + 4 B per triangle); the BVH is built from
+  // positions and materials while the normals are copied and the shading
+  // records packed on a stream of their own (below 64 Ki triangles, 5 MB,
+  // the copies take less than the stream's creation)
+  PrimScan scan = {0xffffffffu, 0u, {INT32_MAX, INT32_MAX, INT32_MAX}, {INT32_MIN, INT32_MIN, INT32_MIN}};
+  std::vector<uint32_t> emissive;  // bit per triangle, when the host needs them
   if (T) {
-    LISA_CUDA(dev_alloc((void**)&d_v, sizeof(float) * 9ull * T));
-    LISA_CUDA(dev_alloc((void**)&d_n, sizeof(float) * 9ull * T));
-    LISA_CUDA(dev_alloc((void**)&d_m, sizeof(int32_t) * T));
-    LISA_CUDA(cudaMemcpyAsync(d_v, p.vertices, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, r.stream));
-    LISA_CUDA(cudaMemcpyAsync(d_n, p.normals, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, r.stream));
-    LISA_CUDA(cudaMemcpyAsync(d_m, p.mat_indices, sizeof(int32_t) * T, cudaMemcpyHostToDevice, r.stream));
-    LISA_TRY(r.arena.alloc((void**)&s.prims, sizeof(float4) * 5ull * T, "triangle records"));
-    k_pack_prims<<<r.sm_count * 8, 256, 0, r.stream>>>(d_v, d_n, d_m, T, s.prims);
-    cudaError_t e = cudaGetLastError();
-    // then d_m becomes what the BVH leaves carry: the emitter material or -1
     std::vector<int32_t> em(std::max(p.num_materials, 1), -1);
     for (int i = 0; i < p.num_materials; ++i) em[i] = p.materials[i].emit ? i : -1;
-    int32_t* d_em = nullptr;
-    if (e == cudaSuccess) e = dev_alloc((void**)&d_em, sizeof(int32_t) * em.size());
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(d_em, em.data(), sizeof(int32_t) * em.size(), cudaMemcpyHostToDevice, r.stream);
-    if (e == cudaSuccess) {
-      k_emit_of_prim<<<r.sm_count * 8, 256, 0, r.stream>>>(d_m, T, d_em, (uint32_t)em.size());
-      e = cudaGetLastError();
+    SceneUpload up;
+    up.stream = r.stream;
+    LISA_TRY(r.arena.alloc((void**)&s.prims, sizeof(float4) * 5ull * T, "triangle records"));
+    LISA_TRY(up.get((void**)&up.v, sizeof(float) * 9ull * T, "triangle upload"));
+    LISA_TRY(up.get((void**)&up.n, sizeof(float) * 9ull * T, "triangle upload"));
+    LISA_TRY(up.get((void**)&up.m, sizeof(int32_t) * T, "triangle upload"));
+    LISA_TRY(up.get((void**)&up.leaf, sizeof(int32_t) * T, "triangle upload"));
+    LISA_TRY(up.get((void**)&up.mask, sizeof(uint32_t) * ((T + 31u) / 32u), "triangle upload"));
+    LISA_TRY(up.get((void**)&up.em, sizeof(int32_t) * em.size(), "triangle upload"));
+    LISA_TRY(up.get((void**)&up.scan, sizeof(PrimScan), "triangle upload"));
+    if (T >= 65536u) LISA_CUDA(cudaStreamCreateWithFlags(&up.side, cudaStreamNonBlocking));
+    const cudaStream_t side = up.side ? up.side : r.stream;
+    LISA_CUDA(cudaMemcpyAsync(up.scan, &scan, sizeof(scan), cudaMemcpyHostToDevice, r.stream));
+    LISA_CUDA(cudaMemcpyAsync(up.em, em.data(), sizeof(int32_t) * em.size(), cudaMemcpyHostToDevice, r.stream));
+    LISA_CUDA(cudaMemcpyAsync(up.m, p.mat_indices, sizeof(int32_t) * T, cudaMemcpyHostToDevice, r.stream));
+    LISA_CUDA(cudaMemcpyAsync(up.v, p.vertices, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, r.stream));
+    k_scan_prims<<<std::min<uint32_t>((T + 255u) / 256u, (uint32_t)r.sm_count * 8u), 256, 0, r.stream>>>(
+        up.v, up.m, T, up.em, (uint32_t)p.num_materials, up.leaf, up.mask, up.scan);
+    LISA_CUDA(cudaGetLastError());
+    if (up.side) {  // the records' kernel reads positions and materials as well
+      LISA_CUDA(cudaEventCreateWithFlags(&up.ready, cudaEventDisableTiming));
+      LISA_CUDA(cudaEventRecord(up.ready, r.stream));
+      LISA_CUDA(cudaStreamWaitEvent(side, up.ready, 0));
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(r.stream);
-    if (e != cudaSuccess) {
-      cudaDeviceSynchronize();  // before the blocks are reused
-      dev_free(d_em);
-      dev_free(d_v);
-      dev_free(d_n);
-      dev_free(d_m);
-      return Status::cuda(e, "pack triangles");
+    const auto t0 = std::chrono::steady_clock::now();
+    BvhDeviceInfo *d_info = nullptr, info;
+    LISA_TRY(enqueue_bvh(up.v, T, r.stream, up, r.arena, &s.nodes, &s.tris, &d_info, up.leaf,
+                         r.opts.bvh_lbvh_only == 0));
+    LISA_CUDA(cudaMemcpyAsync(up.n, p.normals, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, side));
+    k_pack_prims<<<r.sm_count * 8, 256, 0, side>>>(up.v, up.n, up.m, T, s.prims);
+    LISA_CUDA(cudaGetLastError());
+    LISA_CUDA(cudaMemcpyAsync(&info, d_info, sizeof(info), cudaMemcpyDeviceToHost, r.stream));
+    LISA_CUDA(cudaMemcpyAsync(&scan, up.scan, sizeof(scan), cudaMemcpyDeviceToHost, r.stream));
+    LISA_CUDA(cudaStreamSynchronize(r.stream));
+    LISA_TRY(bvh_result(info, T, &s.bvh));
+    s.bvh.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (scan.bad != 0xffffffffu)
+      return Status::invalid("material index out of range at triangle " + std::to_string(scan.bad));
+    // the host's own work on emitters: their list for the physically based
+    // estimator, their BVH for the other (its search would not use a small one)
+    if (r.opts.estimator == LISA_ESTIMATOR_PHYSICAL ? scan.emissive > 0 : scan.emissive >= EMIT_BVH_MIN_TRIS) {
+      emissive.resize((T + 31u) / 32u);
+      LISA_CUDA(cudaMemcpyAsync(emissive.data(), up.mask, sizeof(uint32_t) * emissive.size(), cudaMemcpyDeviceToHost,
+                                r.stream));
+      LISA_CUDA(cudaStreamSynchronize(r.stream));
     }
-    dev_free(d_em);
+    if (up.side) LISA_CUDA(cudaStreamSynchronize(up.side));
   }
-  Status st;
-  {
-    TempDeviceBufs tmp;
-    tmp.stream = r.stream;
-    st = build_bvh(d_v, T, r.stream, tmp, r.arena, &s.nodes, &s.tris, &s.bvh, d_m, r.opts.bvh_lbvh_only == 0);
-    cudaStreamSynchronize(r.stream);
-  }
-  dev_free(d_v);
-  dev_free(d_n);
-  dev_free(d_m);
-  LISA_TRY(st);
   const float dx = s.bvh.bmax[0] - s.bvh.bmin[0], dy = s.bvh.bmax[1] - s.bvh.bmin[1],
               dz = s.bvh.bmax[2] - s.bvh.bmin[2];
   s.extent = std::sqrt(dx * dx + dy * dy + dz * dz);
@@ -510,34 +596,20 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
   // (far more than the triangle test's rounding outside an edge): an
   // emitter-search ray that misses them cannot end on an emitter
   {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool any = false;
-    for (uint32_t t = 0; t < T; ++t) {
-      const int32_t m = p.mat_indices[t];
-      if (m < 0 || m >= p.num_materials || !p.materials[m].emit) continue;
-      any = true;
-      for (int j = 0; j < 3; ++j) {
-        const lisa_float3& v = p.vertices[3ull * t + j];
-        const float c[3] = {v.x, v.y, v.z};
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = std::min(lo[k], c[k]);
-          hi[k] = std::max(hi[k], c[k]);
-        }
-      }
-    }
+    const bool any = scan.emissive > 0;
     s.has_emit_box = any;
     const float pad = 1e-4f * s.extent;
     for (int k = 0; k < 3; ++k) {
-      s.emit_lo[k] = any ? lo[k] - pad : 0.0f;
-      s.emit_hi[k] = any ? hi[k] + pad : 0.0f;
+      s.emit_lo[k] = any ? ord2f(scan.lo[k]) - pad : 0.0f;
+      s.emit_hi[k] = any ? ord2f(scan.hi[k]) + pad : 0.0f;
     }
   }
   // the emitters' own BVH (reference estimator's emitter search)
-  if (r.opts.estimator != LISA_ESTIMATOR_PHYSICAL && s.has_emit_box) LISA_TRY(build_emitter_bvh(r, p, s));
+  if (r.opts.estimator != LISA_ESTIMATOR_PHYSICAL && !emissive.empty()) LISA_TRY(build_emitter_bvh(r, p, emissive, s));
   // materials
   std::vector<DevMaterial> dm(std::max(p.num_materials, 1));
   for (int i = 0; i < p.num_materials; ++i) dm[i] = to_dev(p.materials[i]);
-  if (r.opts.estimator == LISA_ESTIMATOR_PHYSICAL) LISA_TRY(build_emitters(r, p, s, dm));
+  if (r.opts.estimator == LISA_ESTIMATOR_PHYSICAL) LISA_TRY(build_emitters(r, p, emissive, s, dm));
   LISA_TRY(r.arena.alloc((void**)&s.mats, sizeof(DevMaterial) * dm.size(), "materials"));
   LISA_CUDA(cudaMemcpyAsync(s.mats, dm.data(), sizeof(DevMaterial) * dm.size(), cudaMemcpyHostToDevice, r.stream));
   // accumulation

@@ -35,11 +35,6 @@ namespace {
 
 constexpr uint32_t LEAF_BIT = 0x80000000u;
 
-__device__ __forceinline__ int f2ord(float f) {
-  const int i = __float_as_int(f);
-  return i >= 0 ? i : i ^ 0x7fffffff;
-}
-
 // bounds[0..2] = min scene xyz, [3..5] = max scene xyz, [6..8] min centroid,
 // [9..11] max centroid, as order-preserving ints.  Blocks of 256.
 __global__ void k_prim_bounds(const float* __restrict__ v, uint32_t n, float4* __restrict__ lo,

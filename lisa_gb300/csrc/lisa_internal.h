@@ -113,8 +113,8 @@ struct BvhBuildResult {
   uint32_t num_nodes = 0;
   uint32_t num_tri_slots = 0;
   uint32_t depth = 0;
-  double build_ms = 0.0;
-  float bmin[3], bmax[3];
+  double build_ms = 0.0;  // host time from the first launch to the result
+  float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};
 };
 
 // What a build leaves on the device, for the host and for kernels that
@@ -130,7 +130,12 @@ struct BvhDeviceInfo {
   uint32_t ticket[4];  // tiles started, per sort pass
 };
 
-// The float of an order-preserving int.
+// Order-preserving ints of floats.
+__host__ __device__ inline int f2ord(float f) {
+  int i;
+  memcpy(&i, &f, 4);
+  return i >= 0 ? i : i ^ 0x7fffffff;
+}
 __host__ __device__ inline float ord2f(int i) {
   const int j = i >= 0 ? i : i ^ 0x7fffffff;
   float f;
