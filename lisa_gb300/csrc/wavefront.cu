@@ -149,7 +149,8 @@ __device__ __forceinline__ int find_group(const WaveDesc& w, uint32_t key, bool 
 // raygen (shader.cu:126-152)
 
 // Scene, pixel, stream state and camera ray of the wave's path `slot`
-// (shader.cu:126-152).
+// (shader.cu:126-152).  With one stream per pixel, a path that is not of its
+// group's first plane goes on with the state in `seed`, its predecessor's.
 __device__ __forceinline__ void camera_ray(const WaveBufs& b, const WaveDesc& w, uint32_t slot, uint32_t& scene,
                                            uint32_t& pix, uint32_t& seed, V3& org, V3& dir) {
   const WaveGroup& g = w.groups[find_group(w, slot, false)];
@@ -161,7 +162,7 @@ __device__ __forceinline__ void camera_ray(const WaveBufs& b, const WaveDesc& w,
   const uint32_t sample = g.sample0 + m;
   const uint32_t x = pix % sc.width, y = pix / sc.width;
   if (w.rng_mode == LISA_RNG_PER_PIXEL) {
-    seed = sc.pix_rng[pix];
+    if (m == 0) seed = sc.pix_rng[pix];
   } else {
     seed = tea<16>(pix, tea<4>(sample, w.seed));
   }
@@ -1111,6 +1112,17 @@ __global__ void __launch_bounds__(INFER_THREADS, INFER_BLOCKS_PER_SM) k_guided_i
   if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->infer_rows += *(volatile uint32_t*)&b.ctrl->nee_count;
 }
 
+// With one stream per pixel: the first path of the wave's pixel `item`, and
+// the distance from path `slot` to its pixel's next (0: the last one).
+__device__ __forceinline__ uint32_t first_of_pixel(const WaveDesc& w, uint32_t item) {
+  const WaveGroup& g = w.groups[find_group(w, item, true)];
+  return g.slot0 + (item - g.acc0);
+}
+__device__ __forceinline__ uint32_t next_of_pixel(const WaveDesc& w, uint32_t slot) {
+  const WaveGroup& g = w.groups[find_group(w, slot, false)];
+  return slot - g.slot0 + g.npix < g.nplanes * g.npix ? g.npix : 0u;
+}
+
 // ---------------------------------------------------------------------------
 // whole paths in one kernel (plain sampling, small waves)
 //
@@ -1118,22 +1130,23 @@ __global__ void __launch_bounds__(INFER_THREADS, INFER_BLOCKS_PER_SM) k_guided_i
 // search and bounce, depth after depth, advancing one BVH node per loop trip
 // like the stage kernels, whose routines it calls in the same order -- the
 // paths are the same bit for bit.  Nothing passes through memory but the
-// path's final radiance.
+// path's final radiance.  With CHAIN (one stream per pixel) a lane takes a
+// pixel's paths in turn, each going on with the stream of the one before.
 //
 // For small waves, whose time is the latency of the stages and not their
 // throughput: each stage launch ends with the wave's longest ray (up to a
 // hundred node visits of about a microsecond), and a frame is a chain of
 // three such launches per depth.  Here a path waits only for itself: a
 // 160 x 90 preview of the Cornell box takes 182 us instead of 397, a
-// 333 x 217 frame in eight one-sample waves 3.4 ms instead of 8.0.  It is
+// 333 x 217 frame of eight samples with one stream per pixel 1.9 instead of 8.3.  It is
 // bound by issue (58 % of the slots) and by instruction fetch: the loop is
 // 42 KB of code, so a routine is written once and shared by the ray kinds
 // (two more copies of trav_begin and of the triangle test cost 10 %).
-template <bool PHYS>
+template <bool PHYS, bool CHAIN>
 __global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b, const WaveDesc* __restrict__ wave,
                                                                       uint32_t lanes) {
   const WaveDesc& w = *wave;
-  const uint32_t count = w.paths;
+  const uint32_t count = CHAIN ? w.acc_items : w.paths;
   const int lane = threadIdx.x & 31;
   const uint32_t lt = lanemask_lt();
   uint2 stack[TRAV_STACK];
@@ -1170,6 +1183,7 @@ __global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b
       bool search = false;   // a vertex that needs its next try (reference estimator)
       bool leave = false;    // a vertex whose emitter search is over: draw the bounce
       bool lit = false, start = false, over = false;
+      bool fresh = false;    // a new path
       bool nearer = false;   // look for a triangle nearer than the emitter hit
       float tmax = RAY_TMAX;
       V3 p = v3(s.r.ox, s.r.oy, s.r.oz);
@@ -1334,8 +1348,16 @@ __global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b
       }
       if (over) {
         b.ps_col[slot] = make_float4(col.x, col.y, col.z, 0.0f);
-        if (w.rng_mode == LISA_RNG_PER_PIXEL) b.ps_rng[slot] = seed;
         have = false;
+        if (CHAIN) {
+          const uint32_t next = next_of_pixel(w, slot);
+          if (next) {
+            slot += next;
+            have = fresh = true;
+          } else {
+            b.ps_rng[slot] = seed;
+          }
+        }
       } else if (start && !shadow) {
         ++depth;
         ++nbounce;
@@ -1349,22 +1371,22 @@ __global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b
         base = __shfl_sync(FULL, base, leader);
         if (need) {
           slot = base + __popc(nmask & lt);
-          if (slot < count) {
-            uint32_t scene, pix;
-            camera_ray(b, w, slot, scene, pix, seed, p, D);
-            sc = b.scenes + scene;
-            att = v3(1.0f);
-            col = v3(0.0f);
-            stale = -1;
-            pdf = 0.0f;
-            depth = 0;
-            shadow = false;
-            have = true;
-            start = true;
-          } else {
-            exhausted = true;
-          }
+          have = fresh = slot < count;
+          exhausted = !have;
+          if (CHAIN && have) slot = first_of_pixel(w, slot);
         }
+      }
+      if (fresh) {
+        uint32_t scene, pix;
+        camera_ray(b, w, slot, scene, pix, seed, p, D);
+        sc = b.scenes + scene;
+        att = v3(1.0f);
+        col = v3(0.0f);
+        stale = -1;
+        pdf = 0.0f;
+        depth = 0;
+        shadow = false;
+        start = true;
       }
       if (!__any_sync(FULL, have)) break;
       if (start) {
@@ -1397,7 +1419,7 @@ __global__ void __launch_bounds__(128, LISA_PATHS_MIN_BLOCKS) k_paths(WaveBufs b
   warp_add64(&b.ctrl->rays_shadow, nshadow);
   warp_add64(&b.ctrl->shadow_walked, nwalked);
   warp_add64(&b.ctrl->nee_total, nvertex);
-  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->rays_primary += count;
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->rays_primary += w.paths;
 }
 
 // ---------------------------------------------------------------------------
@@ -1646,7 +1668,7 @@ struct WaveLaunch {
   bool train;        // guided wave: train the guide after it
   bool warm;         // guided wave: warm-up, sample the BSDF only
   uint32_t steps;    // guided wave: Adam steps after it, in proportion to its paths
-  uint32_t paths;
+  uint32_t items;    // paths, or with one stream per pixel the pixels they run through
   bool whole;        // rendered by k_paths, not stage by stage
 };
 
@@ -1665,6 +1687,7 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
                 std::vector<WaveDesc>& waves, std::vector<WaveLaunch>& wave_launch) {
   const uint32_t W = r.capacity;
   const bool per_pixel = r.opts.rng == LISA_RNG_PER_PIXEL;
+  const bool may_whole = !r.opts.stage_timing && !r.opts.count_traversal;
   const uint32_t max_whole = r.opts.estimator == LISA_ESTIMATOR_PHYSICAL ? PATHS_MAX_WAVE_PB : PATHS_MAX_WAVE;
   waves.clear();
   wave_launch.clear();
@@ -1682,8 +1705,9 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
                                             1u, (uint32_t)(((uint64_t)cur.paths * r.opts.guide_steps_per_wave +
                                                             (1ull << 21)) >> 22)))
                                       : 0u;
-    const bool whole = !cur_guided && cur.paths <= max_whole && !r.opts.stage_timing && !r.opts.count_traversal;
-    wave_launch.push_back(WaveLaunch{cur_b, (int)cur.groups[0].scene, cur_guided, false, false, steps, cur.paths, whole});
+    const uint32_t items = per_pixel ? cur.acc_items : cur.paths;
+    const bool whole = may_whole && !cur_guided && items <= max_whole;
+    wave_launch.push_back(WaveLaunch{cur_b, (int)cur.groups[0].scene, cur_guided, false, false, steps, items, whole});
     std::memset(&cur, 0, sizeof(cur));
     cur_b = 0;
   };
@@ -1715,7 +1739,17 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
       if (npix == 0 || r.scenes[s].params.num_bounces == 0) continue;
       if (one_scene) close();
       bool scene_in_cur = false;
+      // With one stream per pixel a pixel's samples are a chain.  k_paths
+      // runs it in one launch, each path of a pixel by the lane that ran the
+      // one before; stage by stage each sample is a wave.  (333 x 217 pixels,
+      // 8 samples: 1.77 ms, bound by the longest chain -- 640 x 360 pixels
+      // take 2.24 -- against 2.10 ms in waves of one sample.)
+      const bool chain = per_pixel && may_whole && !one_scene && npix <= max_whole;
       while (planes > 0) {
+        if (per_pixel && cur.acc_items && (cur.acc_items > max_whole || npix > max_whole - cur.acc_items)) {
+          close();  // chains are k_paths' alone
+          scene_in_cur = false;
+        }
         const uint32_t room = W - cur.paths;
         if (cur.num_groups == MAX_GROUPS || (per_pixel && scene_in_cur)) {
           close();
@@ -1724,7 +1758,7 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
         }
         if (npix <= room) {
           uint32_t k = std::min(std::min(planes, room / npix), max_planes);
-          if (per_pixel) k = 1;
+          if (per_pixel && !chain) k = 1;
           add(s, 0, npix, j, k);
           scene_in_cur = true;
           planes -= k;
@@ -1871,14 +1905,16 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
     if (waves[wv].whole) {
       // at least eight warps an SM, so that a small wave's paths spread over
       // the GPU; then 32 paths a warp
-      const uint32_t wpb = (uint32_t)r.nee_threads / 32u, paths = waves[wv].paths;
+      const uint32_t wpb = (uint32_t)r.nee_threads / 32u, items = waves[wv].items;
       const uint32_t few = (uint32_t)r.sm_count * ((8u + wpb - 1u) / wpb);
-      const uint32_t grid = std::min<uint32_t>((uint32_t)r.path_blocks, std::max<uint32_t>(few, (paths + 32u * wpb - 1u) / (32u * wpb)));
-      const uint32_t lanes = std::min<uint32_t>(32u, (paths + grid * wpb - 1u) / (grid * wpb));
+      const uint32_t grid = std::min<uint32_t>((uint32_t)r.path_blocks, std::max<uint32_t>(few, (items + 32u * wpb - 1u) / (32u * wpb)));
+      const uint32_t lanes = std::min<uint32_t>(32u, (items + grid * wpb - 1u) / (grid * wpb));
       LISA_TRY(stage(0, [&] {
         const WaveBufs bp = make_bufs(r, REFILL_PATHS);
-        if (physical) k_paths<true><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
-        else k_paths<false><<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
+        const bool chains = r.opts.rng == LISA_RNG_PER_PIXEL;
+        auto* kernel = physical ? (chains ? k_paths<true, true> : k_paths<true, false>)
+                                : (chains ? k_paths<false, true> : k_paths<false, false>);
+        kernel<<<grid, r.nee_threads, 0, r.stream>>>(bp, wd, lanes);
         return Status();
       }));
       LISA_TRY(stage(3, [&] {
@@ -2027,7 +2063,7 @@ Status renderer_render(Renderer& r, uint32_t spp_req, bool progressive, lisa_ren
     // refreshed above, outside the graph
     std::vector<uint64_t> key;
     for (const WaveLaunch& w : wb) {
-      key.push_back(w.whole ? w.paths : 0u);  // (its launch shape)
+      key.push_back(w.whole ? w.items : 0u);  // (its launch shape)
       key.push_back(((uint64_t)w.steps << 40) | ((uint64_t)w.bounces << 32) | ((uint64_t)w.scene << 3) |
                     ((uint64_t)w.guided << 2) | ((uint64_t)w.warm << 1) | w.train);
     }
@@ -2278,7 +2314,7 @@ Status configure_launch(Renderer& r) {
   bps = r.opts.blocks_per_sm ? (int)r.opts.blocks_per_sm : std::max(occ, 1);
   bps = std::min(bps, std::max(occ, 1));
   r.nee_pb_blocks = r.sm_count * bps;
-  LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_paths<false>, tthreads, 0));
+  LISA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_paths<false, false>, tthreads, 0));
   bps = r.opts.blocks_per_sm ? (int)r.opts.blocks_per_sm : std::max(occ, 1);
   r.path_blocks = r.sm_count * std::min(bps, std::max(occ, 1));
   return Status();
