@@ -984,6 +984,20 @@ static int gret(const Status& s) {
   return s.code;
 }
 
+// Runs a call's body; what host allocations throw becomes a status.
+template <class F>
+static int guarded(F&& run) {
+  Status s;
+  try {
+    s = run();
+  } catch (const std::bad_alloc&) {
+    s = Status(LISA_ERR_OOM, "host allocation failed");
+  } catch (const std::exception& e) {
+    s = Status(LISA_ERR_INVALID, e.what());
+  }
+  return gret(s);
+}
+
 // A barrier that nothing completes, waited on with an iteration limit: the
 // time-out path of the tensor-core kernels (status bit, early exit) taken
 // on purpose, with no fault and no unbounded wait.
@@ -1069,10 +1083,12 @@ int lisa_guide_set_params(lisa_guide* g, const float* params) {
 int lisa_guide_forward(lisa_guide* g, const float* features, uint32_t n, float* out) {
   if (!g || (n && (!features || !out))) return gret(Status::invalid("null argument"));
   if (n == 0) return gret(Status());
-  float *d_x = nullptr, *d_o = nullptr;
   auto run = [&]() -> Status {
-    LISA_CUDA(cudaMalloc(&d_x, sizeof(float) * 64ull * n));
-    LISA_CUDA(cudaMalloc(&d_o, sizeof(float) * 40ull * n));
+    TempDeviceBufs tmp;
+    tmp.stream = g->stream;
+    float *d_x = nullptr, *d_o = nullptr;
+    LISA_TRY(tmp.get((void**)&d_x, sizeof(float) * 64ull * n, "guide features"));
+    LISA_TRY(tmp.get((void**)&d_o, sizeof(float) * 40ull * n, "guide outputs"));
     LISA_CUDA(cudaMemcpyAsync(d_x, features, sizeof(float) * 64ull * n, cudaMemcpyHostToDevice, g->stream));
     GuideSrc src;
     std::memset(&src, 0, sizeof(src));
@@ -1082,21 +1098,20 @@ int lisa_guide_forward(lisa_guide* g, const float* features, uint32_t n, float* 
     LISA_CUDA(cudaMemcpyAsync(out, d_o, sizeof(float) * 40ull * n, cudaMemcpyDeviceToHost, g->stream));
     return guide_check_status(g->get(), g->stream);
   };
-  Status s = run();
-  if (d_x) cudaFree(d_x);
-  if (d_o) cudaFree(d_o);
-  return gret(s);
+  return guarded(run);
 }
 
 int lisa_guide_train_step(lisa_guide* g, const float* features, const float* dirs, const float* weights, uint32_t n,
                           float lr, float* loss, float* grads) {
   if (!g || (n && (!features || !dirs || !weights))) return gret(Status::invalid("null argument"));
   if (n == 0) return gret(Status::invalid("empty batch"));
-  float *d_x = nullptr, *d_d = nullptr, *d_w = nullptr;
   auto run = [&]() -> Status {
-    LISA_CUDA(cudaMalloc(&d_x, sizeof(float) * 64ull * n));
-    LISA_CUDA(cudaMalloc(&d_d, sizeof(float) * 3ull * n));
-    LISA_CUDA(cudaMalloc(&d_w, sizeof(float) * n));
+    TempDeviceBufs tmp;
+    tmp.stream = g->stream;
+    float *d_x = nullptr, *d_d = nullptr, *d_w = nullptr;
+    LISA_TRY(tmp.get((void**)&d_x, sizeof(float) * 64ull * n, "guide features"));
+    LISA_TRY(tmp.get((void**)&d_d, sizeof(float) * 3ull * n, "guide directions"));
+    LISA_TRY(tmp.get((void**)&d_w, sizeof(float) * n, "guide weights"));
     LISA_CUDA(cudaMemcpyAsync(d_x, features, sizeof(float) * 64ull * n, cudaMemcpyHostToDevice, g->stream));
     LISA_CUDA(cudaMemcpyAsync(d_d, dirs, sizeof(float) * 3ull * n, cudaMemcpyHostToDevice, g->stream));
     LISA_CUDA(cudaMemcpyAsync(d_w, weights, sizeof(float) * n, cudaMemcpyHostToDevice, g->stream));
@@ -1118,11 +1133,7 @@ int lisa_guide_train_step(lisa_guide* g, const float* features, const float* dir
     }
     return Status();
   };
-  Status s = run();
-  if (d_x) cudaFree(d_x);
-  if (d_d) cudaFree(d_d);
-  if (d_w) cudaFree(d_w);
-  return gret(s);
+  return guarded(run);
 }
 
 int lisa_guide_train_steps(lisa_guide* g, const float* features, const float* dirs, const float* weights, uint32_t n,
@@ -1131,13 +1142,15 @@ int lisa_guide_train_steps(lisa_guide* g, const float* features, const float* di
   if (n == 0 || steps == 0) return gret(Status::invalid("empty batch"));
   if (chunk == 0 || chunk % 128) return gret(Status::invalid("chunk must be a positive multiple of 128"));
   if (!(lr > 0.0f)) return gret(Status::invalid("lr must be positive"));
-  float *d_x = nullptr, *d_d = nullptr, *d_w = nullptr;
-  uint32_t* d_bar = nullptr;
   auto run = [&]() -> Status {
-    LISA_CUDA(cudaMalloc(&d_x, sizeof(float) * 64ull * n));
-    LISA_CUDA(cudaMalloc(&d_d, sizeof(float) * 3ull * n));
-    LISA_CUDA(cudaMalloc(&d_w, sizeof(float) * n));
-    LISA_CUDA(cudaMalloc(&d_bar, sizeof(uint32_t)));
+    TempDeviceBufs tmp;
+    tmp.stream = g->stream;
+    float *d_x = nullptr, *d_d = nullptr, *d_w = nullptr;
+    uint32_t* d_bar = nullptr;
+    LISA_TRY(tmp.get((void**)&d_x, sizeof(float) * 64ull * n, "guide features"));
+    LISA_TRY(tmp.get((void**)&d_d, sizeof(float) * 3ull * n, "guide directions"));
+    LISA_TRY(tmp.get((void**)&d_w, sizeof(float) * n, "guide weights"));
+    LISA_TRY(tmp.get((void**)&d_bar, sizeof(uint32_t), "grid barrier"));
     LISA_CUDA(cudaMemcpyAsync(d_x, features, sizeof(float) * 64ull * n, cudaMemcpyHostToDevice, g->stream));
     LISA_CUDA(cudaMemcpyAsync(d_d, dirs, sizeof(float) * 3ull * n, cudaMemcpyHostToDevice, g->stream));
     LISA_CUDA(cudaMemcpyAsync(d_w, weights, sizeof(float) * n, cudaMemcpyHostToDevice, g->stream));
@@ -1152,12 +1165,7 @@ int lisa_guide_train_steps(lisa_guide* g, const float* features, const float* di
     LISA_TRY(guide_check_status(g->get(), g->stream));
     return Status();
   };
-  Status s = run();
-  if (d_x) cudaFree(d_x);
-  if (d_d) cudaFree(d_d);
-  if (d_w) cudaFree(d_w);
-  if (d_bar) cudaFree(d_bar);
-  return gret(s);
+  return guarded(run);
 }
 
 }  // extern "C"
