@@ -567,7 +567,7 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
     const auto t0 = std::chrono::steady_clock::now();
     BvhDeviceInfo *d_info = nullptr, info;
     LISA_TRY(enqueue_bvh(up.v, T, r.stream, up, r.arena, &s.nodes, &s.tris, &d_info, up.leaf,
-                         r.opts.bvh_lbvh_only == 0));
+                         r.opts.bvh_lbvh_only == 0, true));
     LISA_CUDA(cudaMemcpyAsync(up.n, p.normals, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, side));
     k_pack_prims<<<r.sm_count * 8, 256, 0, side>>>(up.v, up.n, up.m, T, s.prims);
     LISA_CUDA(cudaGetLastError());

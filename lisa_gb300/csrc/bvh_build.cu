@@ -13,10 +13,12 @@
 //      Parallelism in the Construction of BVHs, Octrees, and k-d Trees",
 //      HPG 2012), equal codes ordered by index
 //   5. bottom-up AABBs with one atomic arrival counter per node
-//   6. collapse into 8-wide nodes, level by level in one cooperative launch,
-//      eight lanes per node: each node adopts up to 8 descendants by
-//      repeatedly opening the child of largest surface area
-//      (subtrees of <= 3 triangles become leaves), then stores its child
+//   6. the least-cost plan of the 8-wide collapse, bottom up (renderers)
+//   7. collapse into 8-wide nodes, level by level in one cooperative launch,
+//      eight lanes per node: each node adopts up to 8 descendants, by the
+//      plan and then, while slots are free, by opening the child of largest
+//      surface area (subtrees of <= 3 triangles become leaves, split if
+//      slots stay free), and stores its child
 //      boxes quantised to 8 bits against a per-axis power-of-two grid,
 //      rounded outward (compressed layout in the style of Ylitie, Karras,
 //      Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed
@@ -334,15 +336,12 @@ __device__ __forceinline__ void node_box(uint32_t c, const uint32_t* vals, const
 constexpr float SAH_CI = 1.2f;  // cost of a node visit relative to a triangle test
 constexpr float SAH_CT = 1.0f;
 constexpr int TL = 7;           // treelet leaves
-// Subtrees of fewer primitives keep their LBVH topology (the 8-wide
-// collapse flattens them).  Measured on the 1.31 M-triangle icosphere box
-// and the 4.48 M-triangle sphere soup: 64 against 16 builds in 3.8 instead
-// of 5.1 ms and 6.9 instead of 10.7 ms, with the same Mrays/s on the first
-// and 0.4 % fewer on the second.
-#ifndef LISA_TREELET_MIN_PRIMS
-#define LISA_TREELET_MIN_PRIMS 64
-#endif
-constexpr uint32_t TREELET_MIN_PRIMS = LISA_TREELET_MIN_PRIMS;
+// Subtrees of fewer primitives keep their LBVH topology: the planned 8-wide
+// collapse makes nearly as much of it.  Against 64, 256 takes 26.3 visits a
+// ray for 25.9 in the 4.48 M-triangle sphere soup (its frame 0.4 % longer),
+// 4.81 for 4.79 in the 1.31 M-triangle icosphere box, and builds that in
+// 0.10 ms less, 30,001 triangles in 0.05 ms (a tenth of a query of them).
+constexpr uint32_t TREELET_MIN_PRIMS = 256;
 
 __device__ __forceinline__ float4 box_min(float4 a, float4 b) {
   return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
@@ -667,6 +666,105 @@ __global__ void __launch_bounds__(SAH_THREADS) k_bottom_up_sah(SahTree t, int re
   }
 }
 
+// ---- plan of the 8-wide collapse ------------------------------------------------
+//
+// The least cost of a subtree in m slots of an 8-wide node (m = 1..7) follows
+// from its children's (the optimal collapse of Ylitie, Karras, Laine, HPG
+// 2017): in one slot it is a leaf, or a node of its own whose eight slots its
+// children share; in m slots it is that or its children share the m.  Costs
+// count a node visit 1 and a triangle test PLAN_CT, by area.  Opening the
+// largest child first instead takes 2.45 visits a ray in the Cornell box for
+// 2.07, 26.9 for 26.3 in the 4.48 M-triangle soup and 4.90 for 4.81 in the
+// icosphere box (frames 5, 3 and 2 % longer).  A third of a visit is what a
+// test costs the traversal; 0.15 and 0.6 differ by under 1 %.
+constexpr float PLAN_CT = 0.3f;
+
+// Costs o[1..7] of a node over children of costs a, b; returns its splits:
+// four bits for each m = 2..8, the slots of the left child, or 0 if m - 1
+// slots cost no more.
+__device__ __forceinline__ uint32_t plan_node(const float* a, const float* b, float area, uint32_t cnt, float* o) {
+  uint32_t d = 0;
+  float s8 = 0.0f;
+#pragma unroll
+  for (int m = 8; m >= 2; --m) {
+    float best = 3.4e38f;
+    uint32_t bk = 1;
+#pragma unroll
+    for (int k = 1; k < 8; ++k)
+      if (k < m && m - k < 8) {
+        const float v = a[k] + b[m - k];
+        if (v < best) {
+          best = v;
+          bk = (uint32_t)k;
+        }
+      }
+    d |= bk << (4 * (m - 2));
+    if (m == 8) s8 = best;
+    else o[m] = best;
+  }
+  o[1] = cnt <= 3u ? PLAN_CT * area * (float)cnt : area + s8;
+#pragma unroll
+  for (int m = 2; m < 8; ++m)
+    if (!(o[m] < o[m - 1])) {
+      o[m] = o[m - 1];
+      d &= ~(15u << (4 * (m - 2)));
+    }
+  return d;
+}
+
+// One thread for each internal node over two leaves climbs from there: past a
+// sibling that is a leaf at once, past an internal one if it comes second
+// (the arrival flags stand at 2 after the bottom-up pass).  wide: two float4
+// a node, its costs in 1..7 slots; plan: its splits.
+//
+// Bound by the latency of the climb, a dozen loads and an atomic a level, and
+// of the low nodes' scattered loads: 165 us for 1.31 M triangles (cold), as
+// much as it saves the first frame of 3.8 M rays.  On the way up in
+// k_bottom_up_sah it took 200 us or more: that kernel lives on 64 warps an
+// SM of 32 registers.  A build for a single query of some 10^5 rays (0.45 ms
+// with the query) goes without.
+__global__ void __launch_bounds__(256) k_wide_plan(SahTree t, float4* wide, uint32_t* plan) {
+  uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p + 1 >= t.n) return;
+  uint32_t l = t.left[p], r = t.right[p];
+  if (!(l & r & LEAF_BIT)) return;
+  while (true) {
+    float c[2][8], o[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t ch = h ? r : l;
+      if (ch & LEAF_BIT) {
+        const uint32_t q = t.vals[ch & ~LEAF_BIT];
+        const float a = PLAN_CT * box_half_area(t.plo[q], t.phi[q]);
+#pragma unroll
+        for (int k = 1; k < 8; ++k) c[h][k] = a;
+      } else {
+        const float4 a = __ldcg(wide + 2ull * ch), b = __ldcg(wide + 2ull * ch + 1);
+        c[h][1] = a.x;
+        c[h][2] = a.y;
+        c[h][3] = a.z;
+        c[h][4] = a.w;
+        c[h][5] = b.x;
+        c[h][6] = b.y;
+        c[h][7] = b.z;
+      }
+    }
+    const uint32_t up = t.parent_int[p];
+    plan[p] = plan_node(c[0], c[1], box_half_area(t.ilo[p], t.ihi[p]), t.count[p], o);
+    __stcg(wide + 2ull * p, make_float4(o[1], o[2], o[3], o[4]));
+    __stcg(wide + 2ull * p + 1, make_float4(o[5], o[6], o[7], 0.0f));
+    if (up == 0xffffffffu) return;
+    l = t.left[up];
+    r = t.right[up];
+    if (!((l | r) & LEAF_BIT)) {
+      uint32_t seen;
+      asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(t.flags + up) : "memory");
+      if (seen == 2u) return;
+    }
+    p = up;
+  }
+}
+
 // ---- collapse to 8-wide compressed nodes -------------------------------------
 
 struct CollapseArgs {
@@ -679,6 +777,7 @@ struct CollapseArgs {
   const uint32_t* left;
   const uint32_t* right;
   const uint32_t* count;  // primitives below each internal node
+  const uint32_t* plan;   // planned splits (plan_node), or null
   const float* verts;
   const int32_t* mats;  // material per triangle, or null
   uint4* nodes;
@@ -758,10 +857,38 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
         node_box(c, a.vals, a.plo, a.phi, a.ilo, a.ihi, lo, hi);
       };
       int nc = 0;
+      uint32_t slots = 1;  // what the plan gives the candidate
       if (active) {
         const uint32_t src = __ldcg(a.source + dst);
         nc = !(src & LEAF_BIT) && a.count[src] > 3u ? 2 : 1;
         if (k < nc) load(nc == 1 ? src : (k ? a.right[src] : a.left[src]));
+        if (nc == 2 && a.plan) {
+          const uint32_t left = a.plan[src] >> 24;
+          slots = k ? 8u - left : left;
+        }
+      }
+      // the planned splits, all candidates at once: the right child of the
+      // j-th that splits goes to lane nc + j
+      while (a.plan) {
+        uint32_t left = 0;
+        if (k < nc && slots > 1u && !(id & LEAF_BIT)) {
+          const uint32_t d = a.plan[id];
+          while (slots > 1u && !(left = (d >> (4u * (slots - 2u))) & 15u)) --slots;
+        }
+        if (!__any_sync(FULL, left != 0u)) break;
+        const uint32_t split = __ballot_sync(FULL, left != 0u) & gmask;
+        const int j = k - nc, num = __popc(split);
+        const bool take = j >= 0 && j < num;
+        const int owner = take ? (int)__fns(split, 0u, j + 1) : lane;
+        const uint32_t l = lc, r = __shfl_sync(FULL, rc, owner), rest = __shfl_sync(FULL, slots - left, owner);
+        if (left) {
+          load(l);
+          slots = left;
+        } else if (take) {
+          load(r);
+          slots = rest;
+        }
+        nc += num;
       }
       while (true) {
         // the openable candidate of largest area (its bits order as the
@@ -927,7 +1054,7 @@ inline uint64_t al256(uint64_t b) { return (std::max<uint64_t>(b, 16) + 255) & ~
 
 // Most 8-wide nodes that n triangles can give.  A node with an internal
 // child has eight children (the collapse opens candidates until there are
-// eight or none is left to open), the others (T, below F such nodes) hold at
+// eight or none is left to open, whatever was planned), the others (T, below F such nodes) hold at
 // least four triangles; the F nodes' own leaves number 8 F - (F + T - 1), so
 // n >= 4 T + 7 F - T + 1 >= 3 (F + T) + 1.
 static uint32_t max_nodes(uint32_t n) { return n / 3 + 1; }
@@ -953,7 +1080,8 @@ size_t bvh_output_bytes(uint32_t n) {
 }
 
 Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
-                   uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info, const int32_t* d_mat, bool refine) {
+                   uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info, const int32_t* d_mat, bool refine,
+                   bool plan) {
   float4 *plo, *phi, *ilo, *ihi;
   uint32_t *keys, *vals, *keys2, *vals2;
   uint32_t *left, *right, *first, *last, *par_int, *par_leaf, *counted, *source;
@@ -976,6 +1104,12 @@ Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSour
   LISA_TRY(take(tmp, &counted, counted_words(n), w));
   LISA_TRY(take(tmp, &source, max_nodes(n), w));
   LISA_TRY(take(tmp, &info, 1, w));
+  float4* wide = nullptr;
+  uint32_t* splits = nullptr;
+  if (plan) {
+    LISA_TRY(take(tmp, &wide, 2ull * n, w));
+    LISA_TRY(take(tmp, &splits, n, w));
+  }
   uint4* nodes = nullptr;
   float4* tris = nullptr;
   LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), "bvh nodes"));
@@ -1011,6 +1145,7 @@ Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSour
     // unless refine is off; first/last become count/cost
     const SahTree st{n, vals, plo, phi, par_leaf, par_int, left, right, ilo, ihi, first, (float*)last, flags};
     k_bottom_up_sah<<<cdiv(n, SAH_THREADS), SAH_THREADS, 0, s>>>(st, refine ? 1 : 0);
+    if (plan) k_wide_plan<<<cdiv(n - 1, 256), 256, 0, s>>>(st, wide, splits);
     LISA_CUDA(cudaGetLastError());
   }
   int occ = 0;
@@ -1024,7 +1159,7 @@ Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSour
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const CollapseArgs a{n, vals, plo, phi, ilo, ihi, left, right, first, d_verts, d_mat, nodes, tris, source, info};
+  const CollapseArgs a{n, vals, plo, phi, ilo, ihi, left, right, first, splits, d_verts, d_mat, nodes, tris, source, info};
   LISA_CUDA(cudaLaunchKernelEx(&cfg, k_collapse, a));
   *d_nodes = nodes;
   *d_tris = tris;
@@ -1060,7 +1195,7 @@ Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource
   uint4* nodes = nullptr;
   float4* tris = nullptr;
   BvhDeviceInfo *d_info = nullptr, h;
-  LISA_TRY(enqueue_bvh(d_verts, n, s, tmp, out, &nodes, &tris, &d_info, d_mat, refine));
+  LISA_TRY(enqueue_bvh(d_verts, n, s, tmp, out, &nodes, &tris, &d_info, d_mat, refine, true));
   LISA_CUDA(cudaMemcpyAsync(&h, d_info, sizeof(h), cudaMemcpyDeviceToHost, s));
   LISA_CUDA(cudaStreamSynchronize(s));
   LISA_TRY(bvh_result(h, n, info));

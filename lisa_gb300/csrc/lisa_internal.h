@@ -148,7 +148,8 @@ __host__ __device__ inline float ord2f(int i) {
 // the node and leaf-triangle arrays from `out`.  With d_mat (one material
 // index per triangle, device) each leaf triangle also carries its material.
 // With refine, the binary LBVH is restructured by SAH (treelets) before the
-// 8-wide collapse.
+// 8-wide collapse, which follows a plan of least cost (enqueue_bvh makes one
+// if asked to; its 36 bytes per triangle come from `tmp` as well).
 Status build_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, ScratchSource& tmp,
                  ScratchSource& out, uint4** d_nodes, float4** d_tris, BvhBuildResult* info,
                  const int32_t* d_mat = nullptr, bool refine = true);
@@ -156,9 +157,10 @@ Status build_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, 
 // unpacks *d_info once the stream has run.
 Status enqueue_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, ScratchSource& tmp,
                    ScratchSource& out, uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info,
-                   const int32_t* d_mat, bool refine);
+                   const int32_t* d_mat, bool refine, bool plan);
 Status bvh_result(const BvhDeviceInfo& h, uint32_t num_prims, BvhBuildResult* info);
-// Device bytes build_bvh takes from `tmp` and from `out` for n triangles.
+// Device bytes a build without a plan takes from `tmp`, and any from `out`,
+// for n triangles.
 size_t bvh_temp_bytes(uint32_t n);
 size_t bvh_output_bytes(uint32_t n);
 

@@ -141,7 +141,8 @@ Status trace_soup_noalloc(const float* d_vertices, uint32_t num_triangles, const
   float4* tris = nullptr;
   BvhDeviceInfo* d_info = nullptr;
   if (num_triangles)
-    LISA_TRY(enqueue_bvh(d_vertices, num_triangles, stream, region, region, &nodes, &tris, &d_info, nullptr, true));
+    LISA_TRY(enqueue_bvh(d_vertices, num_triangles, stream, region, region, &nodes, &tris, &d_info, nullptr, true,
+                         false));
   k_soup_scene<<<1, 1, 0, stream>>>(d_scene, d_ctrl, nodes, tris, num_triangles, d_info);
   LISA_CUDA(cudaGetLastError());
   return launch_trace_closest(d_scene, d_ctrl, d_rays, num_rays, d_prim, d_t, stream, sm, false, true);
