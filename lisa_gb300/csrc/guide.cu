@@ -559,7 +559,8 @@ __device__ __forceinline__ bool grid_wait(uint32_t* counter, uint32_t k, uint32_
 // A round is a serial chain: with 256 threads a tile, the work that the next
 // product does not need behind it, and only the CTAs and slots that have a
 // tile, it takes 16.9 us for one tile (24 before), 20.2 us for 152 (27).
-constexpr uint32_t ADAM_SHARE = 128;  // parameters per CTA in the Adam phase (a multiple of 4)
+constexpr uint32_t ADAM_SHARE = TRAIN_THREADS / 2;  // parameters per CTA in the Adam phase
+static_assert(NPARAM % 2 == 0, "the sums are taken two parameters at a time");
 
 template <int SRC>
 __global__ void __launch_bounds__(TRAIN_THREADS, 1)
@@ -597,10 +598,9 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
   const float inv_n = 1.0f / (float)chunk;
   // the Adam phase: for each share of 128 parameters p0.. of this CTA,
-  // thread (g, q) = (tid / 4, tid % 4) of the first 128 sums the slots
-  // j = q (mod 4) of parameters p0 + 4 g .. + 3 (one float4 a slot); the
-  // quad's sums meet by shuffles and thread (g, q) updates parameter
-  // p0 + 4 g + q
+  // thread (g, q) = (tid / 4, tid % 4) sums the slots j = q (mod 4) of
+  // parameters p0 + 2 g and + 1 (one float2 a slot); the quad's sums meet by
+  // shuffles and thread (g, q < 2) updates parameter p0 + 2 g + q
   const uint32_t qq = tid & 3;
   float* slot = part + (size_t)blockIdx.x * NPARAM;
   uint32_t phase = 0, wphase = 0, bars = 0, done = 0;
@@ -662,9 +662,9 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     // what needs nothing of the others: the next slice's features, this
     // share's parameters and moments
     features(r + 1);
-    const uint32_t i0 = blockIdx.x * ADAM_SHARE + 4u * (tid >> 2) + qq;
+    const uint32_t i0 = blockIdx.x * ADAM_SHARE + 2u * (tid >> 2) + qq;
     float m0 = 0.0f, v0 = 0.0f, w0 = 0.0f;
-    if (tid < (int)ADAM_SHARE && i0 < (uint32_t)NPARAM) {
+    if (qq < 2 && i0 < (uint32_t)NPARAM) {
       m0 = __ldcg(adam_m + i0);
       v0 = __ldcg(adam_v + i0);
       w0 = __ldcg(master + i0);
@@ -673,44 +673,40 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1)
     const float b1c = 1.0f - powf(0.9f, t), b2c = 1.0f - powf(0.999f, t);
     if (!grid_wait(grid_bar, bars++, status, &bar_ok) || failed) break;
     // Adam on this CTA's share (the step of k_guide_adam)
-    if (blockIdx.x == 0 && warp == 4) {
+    if (blockIdx.x == 0 && warp == 4 && (r + 1 == rounds || n - first <= chunk)) {  // the last round
       float l = 0.0f;
       for (uint32_t j = tid & 31; j < nslots; j += 32) l += __ldcg(loss_part + j);
 #pragma unroll
       for (int m = 16; m > 0; m >>= 1) l += __shfl_xor_sync(0xffffffffu, l, m);
       if ((tid & 31) == 0) *loss_last = l;
     }
-    for (uint32_t p0 = blockIdx.x * ADAM_SHARE; p0 < (uint32_t)NPARAM && tid < (int)ADAM_SHARE;
-         p0 += gridDim.x * ADAM_SHARE) {
-      const uint32_t pq = p0 + 4u * (tid >> 2);
-      float4 g4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t p0 = blockIdx.x * ADAM_SHARE; p0 < (uint32_t)NPARAM; p0 += gridDim.x * ADAM_SHARE) {
+      const uint32_t pq = p0 + 2u * (tid >> 2);
+      float2 g2 = make_float2(0.0f, 0.0f);
       if (pq < (uint32_t)NPARAM) {
-        // (up to 19 slots in flight per thread: the sum is latency-bound)
-        for (uint32_t j0 = qq; j0 < nslots; j0 += 76) {
-          float4 x[19];
+        // (up to 38 slots in flight per thread, a slot of every SM at once:
+        // the sum is latency-bound)
+        for (uint32_t j0 = qq; j0 < nslots; j0 += 152) {
+          float2 x[38];
 #pragma unroll
-          for (uint32_t k = 0; k < 19; ++k)
-            if (j0 + 4 * k < nslots) x[k] = __ldcg(reinterpret_cast<const float4*>(part + (size_t)(j0 + 4 * k) * NPARAM + pq));
+          for (uint32_t k = 0; k < 38; ++k)
+            if (j0 + 4 * k < nslots) x[k] = __ldcg(reinterpret_cast<const float2*>(part + (size_t)(j0 + 4 * k) * NPARAM + pq));
 #pragma unroll
-          for (uint32_t k = 0; k < 19; ++k)
+          for (uint32_t k = 0; k < 38; ++k)
             if (j0 + 4 * k < nslots) {
-              g4.x += x[k].x;
-              g4.y += x[k].y;
-              g4.z += x[k].z;
-              g4.w += x[k].w;
+              g2.x += x[k].x;
+              g2.y += x[k].y;
             }
         }
       }
 #pragma unroll
       for (int m = 1; m <= 2; m <<= 1) {
-        g4.x += __shfl_xor_sync(0xffffffffu, g4.x, m);
-        g4.y += __shfl_xor_sync(0xffffffffu, g4.y, m);
-        g4.z += __shfl_xor_sync(0xffffffffu, g4.z, m);
-        g4.w += __shfl_xor_sync(0xffffffffu, g4.w, m);
+        g2.x += __shfl_xor_sync(0xffffffffu, g2.x, m);
+        g2.y += __shfl_xor_sync(0xffffffffu, g2.y, m);
       }
       const uint32_t i = pq + qq;
-      const float gi = qq == 0 ? g4.x : qq == 1 ? g4.y : qq == 2 ? g4.z : g4.w;
-      if (i < (uint32_t)NPARAM) {
+      const float gi = qq == 0 ? g2.x : g2.y;
+      if (qq < 2 && i < (uint32_t)NPARAM) {
         if (!isfinite(gi)) atomicOr(status, ST_GUIDE_NONFINITE);
         else {
           const bool own = i == i0;  // loaded before the grid met
