@@ -280,7 +280,7 @@ __device__ __forceinline__ bool train_tile(const GuideSrc& src, uint32_t i, uint
   };
   const bool valid = i < n;
   float wx = 0.0f, wy = 0.0f, wz = 1.0f, wt = 0.0f;
-  if (valid && h == 0) {
+  if (valid) {
     if (SRC == SRC_RAW) {
       wx = __ldg(src.dirs + 3ull * i);
       wy = __ldg(src.dirs + 3ull * i + 1);
@@ -316,34 +316,38 @@ __device__ __forceinline__ bool train_tile(const GuideSrc& src, uint32_t i, uint
         q.w = bias_relu_bf16x2(v[8 * c + 6], v[8 * c + 7], x.z, x.w);
         *(uint4*)(act + (l + 1) * TILE + row * 128 + (((4 * h + c) ^ (row & 7)) << 4)) = q;
       }
-    } else if (h == 0) {
+    } else {
       tc::tmem_ld16x<3>(tmem + TM_FWD + lane_off, g);
     }
   }
-  // loss gradient at the output (40 values, padded with zeros to 64): one
-  // thread per sample; the other half writes the padding
+  // loss gradient at the output (40 values, padded with zeros to 64): four
+  // lobes for each of the sample's two threads
   float lsum = 0.0f;
-  if (h == 0) {
+  {
     float o[40];
 #pragma unroll
     for (int k = 0; k < 40; ++k) o[k] = g[k] + s_b[4 * 64 + k];
     if (valid && wt != 0.0f) {
       const float il = rsqrtf(fmaxf(wx * wx + wy * wy + wz * wz, 1e-30f));
-      lsum = guide::loss_grad(o, wx * il, wy * il, wz * il, wt * inv_n, g);
+      lsum = guide::loss_grad(o, h, wx * il, wy * il, wz * il, wt * inv_n, g);
     } else {
 #pragma unroll
       for (int k = 0; k < 40; ++k) g[k] = 0.0f;
     }
-    store_half_row_bf16(act + 5 * TILE, row, 0, g);
-    uint4 q;
-    q.x = pack_bf16x2(g[32], g[33]);
-    q.y = pack_bf16x2(g[34], g[35]);
-    q.z = pack_bf16x2(g[36], g[37]);
-    q.w = pack_bf16x2(g[38], g[39]);
-    *(uint4*)(act + 5 * TILE + row * 128 + ((4 ^ (row & 7)) << 4)) = q;
-  } else {
 #pragma unroll
-    for (int c = 5; c < 8; ++c) *(uint4*)(act + 5 * TILE + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < 32; ++k) g[k] = k < 20 ? (h ? g[20 + k] : g[k]) : 0.0f;
+    // columns 20 h .. + 19, four at a time
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const int col = 20 * h + 4 * j;
+      uint2 q;
+      q.x = pack_bf16x2(g[4 * j], g[4 * j + 1]);
+      q.y = pack_bf16x2(g[4 * j + 2], g[4 * j + 3]);
+      *(uint2*)(act + 5 * TILE + row * 128 + (((col >> 3) ^ (row & 7)) << 4) + (col & 4) * 2) = q;
+    }
+    if (h)
+#pragma unroll
+      for (int c = 5; c < 8; ++c) *(uint4*)(act + 5 * TILE + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
   }
   float* const s_dbw = s_db + rows32 * DB_WORDS;  // the sums of these 32 rows
   // backward, layer 5 (index 4) down to layer 1 (index 0): dZ_l is in tile
@@ -376,11 +380,8 @@ __device__ __forceinline__ bool train_tile(const GuideSrc& src, uint32_t i, uint
     }
     // meanwhile: the bias gradients of layer l and dW of the layer above
     if (l == 4) {
+      add_bias_grad(s_dbw + 4 * 64 + 20 * h, g, 20);
       if (h == 0) {
-        add_bias_grad(s_dbw + 4 * 64, g, 32);
-#pragma unroll
-        for (int k = 40; k < 64; ++k) g[k] = 0.0f;
-        add_bias_grad(s_dbw + 4 * 64 + 32, g + 32, 8);
 #pragma unroll
         for (int o2 = 16; o2 > 0; o2 >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o2);
         if ((tid & 31) == 0) s_loss[rows32] += lsum;

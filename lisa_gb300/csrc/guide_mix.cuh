@@ -164,9 +164,12 @@ __device__ __forceinline__ float hemi_pdf(float nx, float ny, float nz, float wx
   return __fdividef(1.0f, 12.0f * m * m * m);
 }
 
-// Gradient of  -wt * log q(w)  with respect to the 40 raw outputs o; also
-// returns the loss term.  wt already includes any batch normalisation.
-__device__ __forceinline__ float loss_grad(const float* o, float wx, float wy, float wz, float wt, float* g) {
+// Gradient of  -wt * log q(w)  with respect to the 40 raw outputs o, the 20
+// of the first (h = 0) or last four lobes; also returns the loss term.  wt
+// already includes any batch normalisation.  Two threads of different warps
+// share a sample: the derivatives, with their exponentials and divisions,
+// take longer than the lobes, which both decode.
+__device__ __forceinline__ float loss_grad(const float* o, int h, float wx, float wy, float wz, float wt, float* g) {
   Lobe L[LOBES];
   decode(o, L);
   float f[LOBES];
@@ -180,6 +183,7 @@ __device__ __forceinline__ float loss_grad(const float* o, float wx, float wy, f
   const float iq = 1.0f / q;
 #pragma unroll
   for (int k = 0; k < LOBES; ++k) {
+    if ((k < LOBES / 2) != (h == 0)) continue;
     const float r = L[k].w * f[k] * iq;  // responsibility
     const float kap = L[k].kappa;
     const float c = L[k].mx * wx + L[k].my * wy + L[k].mz * wz;
