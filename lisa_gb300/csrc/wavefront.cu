@@ -448,18 +448,22 @@ __device__ __forceinline__ uint32_t queue_vertex(const WaveBufs& b, bool vertex,
 // (probability c) and the guide's vMF mixture.  The path continues with
 // weight p_hemi(w) / (c p_hemi(w) + (1-c) q_guide(w)), so the estimator's
 // expectation is unchanged; directions below the surface get weight 0.
+//
+// Without NET, c = 1: the mixture is neither sampled nor weighed (its
+// density times 0 adds nothing), so o is not read.
+template <bool NET>
 __device__ __forceinline__ V3 guided_bounce(const float* o, V3 N, uint32_t& seed, float c, float& weight) {
   guide::Lobe L[guide::LOBES];
-  guide::decode(o, L);
+  if (NET) guide::decode(o, L);
   V3 w;
-  if (rnd(seed) < c) {
+  if (rnd(seed) < c || !NET) {
     w = bsdf::shoot_ray_hemisphere(N, seed);
   } else {
     const float u0 = rnd(seed), u1 = rnd(seed), u2 = rnd(seed);
     guide::mix_sample(L, u0, u1, u2, w.x, w.y, w.z);
   }
   const float ph = guide::hemi_pdf(N.x, N.y, N.z, w.x, w.y, w.z);
-  const float q = c * ph + (1.0f - c) * guide::mix_pdf(L, w.x, w.y, w.z);
+  const float q = NET ? c * ph + (1.0f - c) * guide::mix_pdf(L, w.x, w.y, w.z) : ph;
   weight = (ph > 0.0f && q > 0.0f && isfinite(q)) ? ph / q : 0.0f;
   return w;
 }
@@ -728,11 +732,16 @@ __global__ void __launch_bounds__(128, LISA_NEE_MIN_BLOCKS) k_nee(const __grid_c
 // depth and the wave's salt, not by the path's stream; drop =
 // ctrl->drop_prob, read once per launch), warp-aggregated over the lanes
 // that call it, and returns the record index or ~0u; record_write fills it.
+__device__ __forceinline__ bool record_keep(const WaveBufs& b, int depth, float drop, uint32_t slot, bool want) {
+  if (b.rec_cap == 0) return false;  // a wave that does not train keeps no records
+  const float u = (float)(tea<4>(slot * 16u + (uint32_t)depth, b.rec_salt) >> 8) * (1.0f / 16777216.0f);
+  return want && u >= drop;
+}
+
 __device__ __forceinline__ uint32_t record_reserve(const WaveBufs& b, int depth, float drop, uint32_t slot,
                                                    bool want) {
-  if (b.rec_cap == 0) return ~0u;  // a wave that does not train keeps no records
-  const float u = (float)(tea<4>(slot * 16u + (uint32_t)depth, b.rec_salt) >> 8) * (1.0f / 16777216.0f);
-  const bool keep = want && u >= drop;
+  if (b.rec_cap == 0) return ~0u;
+  const bool keep = record_keep(b, depth, drop, slot, want);
   const uint32_t active = __activemask();
   const uint32_t mask = __ballot_sync(active, keep);
   if (!mask) return ~0u;
@@ -745,15 +754,22 @@ __device__ __forceinline__ uint32_t record_reserve(const WaveBufs& b, int depth,
   return keep && k < b.rec_cap ? k : ~0u;
 }
 
-__device__ __forceinline__ void record_write(const WaveBufs& b, uint32_t k, uint32_t slot, float flag, float4 r0,
-                                             float4 r1, float4 r2, float4 r3, V3 c0) {
+struct Record {
+  float4 r[4];
+  float4 col;  // see WaveBufs
+};
+__device__ __forceinline__ void record_fill(Record& rec, uint32_t slot, float flag, float4 r0, float4 r1, float4 r2,
+                                            float4 r3, V3 c0) {
+  rec.r[0] = r0;
+  rec.r[1] = r1;
+  rec.r[2] = r2;
+  rec.r[3] = r3;
+  rec.col = make_float4(c0.x, c0.y, c0.z, __uint_as_float((slot << 1) | (flag != 0.0f ? 1u : 0u)));
+}
+__device__ __forceinline__ void record_write(const WaveBufs& b, uint32_t k, const Record& rec) {
   if (k == ~0u) return;
-  float4* rec = b.rec_list + 4ull * k;
-  rec[0] = r0;
-  rec[1] = r1;
-  rec[2] = r2;
-  rec[3] = r3;
-  b.rec_col[k] = make_float4(c0.x, c0.y, c0.z, __uint_as_float((slot << 1) | (flag != 0.0f ? 1u : 0u)));
+  for (int j = 0; j < 4; ++j) b.rec_list[4ull * k + j] = rec.r[j];
+  b.rec_col[k] = rec.col;
 }
 
 // ---------------------------------------------------------------------------
@@ -766,15 +782,17 @@ __device__ __forceinline__ void record_write(const WaveBufs& b, uint32_t k, uint
 // with a training record per vertex (the radiance later gathered along the
 // new direction, over the throughput after the bounce, is the incident
 // radiance).  Returns whether a continuation ray (p, nd) is wanted.
+template <bool NET>
 __device__ __forceinline__ bool guided_compat_vertex(const WaveBufs& b, int depth, float drop, uint32_t i,
                                                      const float* o, V3& p, V3& nd, uint32_t& slot, uint32_t& scene,
-                                                     uint32_t& guided_n) {
+                                                     uint32_t& guided_n, Record& rec, bool& keep) {
   const float4 a4 = b.nee_a[i], b4 = b.nee_b[i], c4 = b.nee_c[i];
   slot = __float_as_uint(a4.w);
   scene = __float_as_uint(c4.w);
   const SceneDev& sc = b.scenes[scene];
   if (sc.mats[__float_as_int(b4.w)].roughness != 1.0f) return false;  // bounced in k_nee
-  const uint32_t rk = record_reserve(b, depth, drop, slot, true);
+  keep = !NET && record_keep(b, depth, drop, slot, true);
+  const uint32_t rk = NET ? record_reserve(b, depth, drop, slot, true) : ~0u;
   const float4 cw = b.ps_col[slot];
   p = ld3(a4);
   const V3 N = ld3(b4);
@@ -783,12 +801,13 @@ __device__ __forceinline__ bool guided_compat_vertex(const WaveBufs& b, int dept
   const float4 at = b.ps_att[slot];
   const int stale = __float_as_int(at.w);
   float weight;
-  nd = guided_bounce(o, N, seed, b.bsdf_fraction, weight);
+  nd = guided_bounce<NET>(o, N, seed, b.bsdf_fraction, weight);
   const V3 att = ld3(at) * weight;
   const float il = rsqrtf(fmaxf(dot(D, D), 1e-30f));
-  record_write(b, rk, slot, stale >= 0 ? 1.0f : 0.0f, make_float4(p.x, p.y, p.z, weight),
+  record_fill(rec, slot, stale >= 0 ? 1.0f : 0.0f, make_float4(p.x, p.y, p.z, weight),
               make_float4(N.x, N.y, N.z, nd.x), make_float4(-D.x * il, -D.y * il, -D.z * il, nd.y),
               make_float4(att.x, att.y, att.z, nd.z), ld3(cw));
+  record_write(b, rk, rec);
   b.ps_rng[slot] = seed;
   b.ps_att[slot] = make_float4(att.x, att.y, att.z, at.w);
   ++guided_n;
@@ -1007,8 +1026,10 @@ __global__ void __launch_bounds__(128, LISA_NEE_PB_MIN_BLOCKS) k_nee_pb(const __
 // one-sample MIS between cosine sampling (probability c) and the guide's
 // mixture, q = c cos/pi + (1-c) q_guide, throughput x (cos/pi) / q -- with a
 // training record per diffuse bounce.
+template <bool NET>
 __device__ __forceinline__ bool guided_pb_vertex(const WaveBufs& b, int depth, float drop, uint32_t i, const float* o,
-                                                 V3& p, V3& nd, uint32_t& slot, uint32_t& scene, uint32_t& guided_n) {
+                                                 V3& p, V3& nd, uint32_t& slot, uint32_t& scene, uint32_t& guided_n,
+                                                 Record& rec, bool& keep) {
   const float c = b.bsdf_fraction;
   const float4 a4 = b.nee_a[i], b4 = b.nee_b[i], c4 = b.nee_c[i];
   p = ld3(a4);
@@ -1027,9 +1048,10 @@ __device__ __forceinline__ bool guided_pb_vertex(const WaveBufs& b, int depth, f
   // bounce is drawn in k_nee_pb; decided first so that the training
   // record's slot is reserved while the mixture is evaluated
   const bool diffuse = r >= 1.0f || (r > 0.0f && rnd(seed) < r);
-  const uint32_t rk = record_reserve(b, depth, drop, slot, diffuse);
+  keep = !NET && record_keep(b, depth, drop, slot, diffuse);
+  const uint32_t rk = NET ? record_reserve(b, depth, drop, slot, diffuse) : ~0u;
   guide::Lobe L[guide::LOBES];
-  guide::decode(o, L);
+  if (NET) guide::decode(o, L);
   const float4 l0 = b.nee_light[2ull * i], l1 = b.nee_light[2ull * i + 1];
   if (l1.z != 0.0f) {
     const float pl = l0.w, cos_x = l1.x;
@@ -1037,14 +1059,15 @@ __device__ __forceinline__ bool guided_pb_vertex(const WaveBufs& b, int depth, f
     // (fast reciprocals: the guided bounce's densities need no bit-exact
     // agreement with the oracle, only the same values for sampling and weight)
     const float fcos = r * cos_x * (1.0f / PI_F);
-    const float pb = r * (c * (cos_x * (1.0f / PI_F)) + (1.0f - c) * guide::mix_pdf(L, l0.x, l0.y, l0.z));
+    const float px = cos_x * (1.0f / PI_F);
+    const float pb = r * (NET ? c * px + (1.0f - c) * guide::mix_pdf(L, l0.x, l0.y, l0.z) : px);
     const float wl = __fdividef(pl * pl, pl * pl + pb * pb);
     col = col + ((att * v3(em.emission[0], em.emission[1], em.emission[2])) * __fdividef(fcos, pl)) * wl;
   }
   float prev = 0.0f;
   bool want;
   if (diffuse) {
-    if (rnd(seed) < c) {
+    if (rnd(seed) < c || !NET) {
       nd = cosine_dir(Ns, seed);
     } else {
       const float u0 = rnd(seed), u1 = rnd(seed), u2 = rnd(seed);
@@ -1052,14 +1075,15 @@ __device__ __forceinline__ bool guided_pb_vertex(const WaveBufs& b, int depth, f
     }
     const float cs = dot(Ns, nd);
     const float pc = cs > 0.0f ? cs * (1.0f / PI_F) : 0.0f;
-    const float qm = c * pc + (1.0f - c) * guide::mix_pdf(L, nd.x, nd.y, nd.z);
+    const float qm = NET ? c * pc + (1.0f - c) * guide::mix_pdf(L, nd.x, nd.y, nd.z) : pc;
     const float weight = (pc > 0.0f && qm > 0.0f && isfinite(qm)) ? __fdividef(pc, qm) : 0.0f;
     att = att * weight;
     prev = r * qm;
     want = weight > 0.0f;
     const float il = rsqrtf(fmaxf(dot(D, D), 1e-30f));
-    record_write(b, rk, slot, 0.0f, make_float4(p.x, p.y, p.z, weight), make_float4(N.x, N.y, N.z, nd.x),
+    record_fill(rec, slot, 0.0f, make_float4(p.x, p.y, p.z, weight), make_float4(N.x, N.y, N.z, nd.x),
                 make_float4(-D.x * il, -D.y * il, -D.z * il, nd.y), make_float4(att.x, att.y, att.z, nd.z), col);
+    record_write(b, rk, rec);
     ++guided_n;
   } else {
     nd = reflect(D, Ns);
@@ -1098,9 +1122,11 @@ __global__ void __launch_bounds__(INFER_THREADS, INFER_BLOCKS_PER_SM) k_guided_i
     bool want = false;
     V3 p = v3(0.0f), nd = v3(0.0f);
     uint32_t slot = 0, scene = 0;
+    Record rec;
+    bool keep;
     if (valid) {
-      if (PHYS) want = guided_pb_vertex(b, depth, drop, i, o, p, nd, slot, scene, guided_n);
-      else want = guided_compat_vertex(b, depth, drop, i, o, p, nd, slot, scene, guided_n);
+      if (PHYS) want = guided_pb_vertex<true>(b, depth, drop, i, o, p, nd, slot, scene, guided_n, rec, keep);
+      else want = guided_compat_vertex<true>(b, depth, drop, i, o, p, nd, slot, scene, guided_n, rec, keep);
     }
     const uint32_t ri = warp_reserve(&b.ctrl->qcount[q ^ 1], want);
     if (want && queue_fits(b, ri)) {
@@ -1108,6 +1134,65 @@ __global__ void __launch_bounds__(INFER_THREADS, INFER_BLOCKS_PER_SM) k_guided_i
       b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(scene));
     }
   });
+  warp_add32(&b.ctrl->guided_count, guided_n);
+  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->infer_rows += *(volatile uint32_t*)&b.ctrl->nee_count;
+}
+
+// The same vertices where the BSDF draws every bounce (bsdf_fraction 1: a
+// warm-up wave, whose records train the guide): the guide's density has no
+// weight, so its network does not run.  Bound by the gathers of path state
+// and by the atomics on the queue and record counters, one each for a block
+// of 256: 0.91 ms for 14.2 M vertices of eight depths (1.22 with a warp's
+// atomics), 2.02 with the network.  Resident blocks only: eight an SM in
+// turn took 0.1 ms more, 32 0.7.
+constexpr int BOUNCE_BLOCKS_PER_SM = 4;
+
+template <bool PHYS>
+__global__ void __launch_bounds__(256, BOUNCE_BLOCKS_PER_SM) k_bsdf_bounce(WaveBufs b, int depth) {
+  const int q = depth & 1;
+  const uint32_t count = min(*(volatile uint32_t*)&b.ctrl->nee_count, b.capacity);
+  const float drop = b.ctrl->drop_prob;
+  uint32_t guided_n = 0;
+  __shared__ uint2 s_n[8];  // per warp: rays for the next queue, records
+  __shared__ uint32_t s_ray, s_rec;
+  const uint32_t warp = threadIdx.x >> 5;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += gridDim.x * blockDim.x) {
+    const uint32_t i = base + threadIdx.x;
+    bool want = false, keep = false;
+    V3 p = v3(0.0f), nd = v3(0.0f);
+    uint32_t slot = 0, scene = 0;
+    Record rec;
+    if (i < count) {
+      if (PHYS) want = guided_pb_vertex<false>(b, depth, drop, i, nullptr, p, nd, slot, scene, guided_n, rec, keep);
+      else want = guided_compat_vertex<false>(b, depth, drop, i, nullptr, p, nd, slot, scene, guided_n, rec, keep);
+    }
+    // places in both lists, one atomic each for the block
+    const uint32_t rays = __ballot_sync(FULL, want), recs = __ballot_sync(FULL, keep);
+    if ((threadIdx.x & 31u) == 0) s_n[warp] = make_uint2(__popc(rays), __popc(recs));
+    __syncthreads();
+    uint2 before = make_uint2(0u, 0u), all = before;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      const uint2 v = s_n[k];
+      if (k == warp) before = all;
+      all.x += v.x;
+      all.y += v.y;
+    }
+    if (threadIdx.x == 0) s_ray = atomicAdd(&b.ctrl->qcount[q ^ 1], all.x);
+    if (threadIdx.x == 32 && all.y) s_rec = atomicAdd(&b.ctrl->rec_count, all.y);
+    __syncthreads();
+    if (want) {
+      const uint32_t ri = s_ray + before.x + __popc(rays & lanemask_lt());
+      if (queue_fits(b, ri)) {
+        b.ro[q ^ 1][ri] = make_float4(p.x, p.y, p.z, __uint_as_float(slot));
+        b.rd[q ^ 1][ri] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(scene));
+      }
+    }
+    if (keep) {
+      const uint32_t k = s_rec + before.y + __popc(recs & lanemask_lt());
+      if (k < b.rec_cap) record_write(b, k, rec);
+    }
+  }
   warp_add32(&b.ctrl->guided_count, guided_n);
   if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->infer_rows += *(volatile uint32_t*)&b.ctrl->nee_count;
 }
@@ -1969,7 +2054,11 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
           bw.rec_salt = (uint32_t)(r.guide_waves_done + wv) * 2654435761u + 17u;
           if (!waves[wv].train) bw.rec_cap = 0;
           const uint32_t grid = std::min<uint32_t>((r.capacity + 255) / 256, (uint32_t)(r.sm_count * INFER_BLOCKS_PER_SM));
-          if (physical)
+          if (bw.bsdf_fraction == 1.0f) {
+            const uint32_t g = std::min<uint32_t>((r.capacity + 255) / 256, (uint32_t)(r.sm_count * BOUNCE_BLOCKS_PER_SM));
+            if (physical) k_bsdf_bounce<true><<<g, 256, 0, r.stream>>>(bw, (int)d);
+            else k_bsdf_bounce<false><<<g, 256, 0, r.stream>>>(bw, (int)d);
+          } else if (physical)
             k_guided_infer<true><<<grid, INFER_THREADS, INFER_SMEM, r.stream>>>(net->w_bf16, net->master, infer_src, net->status,
                                                                        bw, (int)d);
           else
