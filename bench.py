@@ -216,16 +216,18 @@ def make_scene(level=8, res=1024):
 
 
 # Algorithmic bytes.  Closest-hit kernel (k_trace), per radiance ray: the
-# queued ray read (32 B) and its hit written (8 B); per node visit 80 B; per
-# triangle test 48 B.  Emitter-search kernel (k_nee), per opaque vertex: the
-# queue entry (48 B) + path state read and written back (36 + 36 B) + the
+# queued ray read (32 B) and its hit written (8 B); per node visit 96 B; per
+# triangle test 48 B.  Emitter-search kernel (k_nee), which also shades: per
+# radiance ray the ray and its hit (32 + 8 B); per opaque vertex its shading
+# record (80 B) + path state read and written back (36 + 36 B) + the
 # continuation ray (32 B); per shadow ray that walks a BVH the material
 # look-up of its hit (16 B); node visits and triangle tests as above.  (A try
 # that cannot change the search's result moves no bytes.)
 TRACE_B_RAY = 32 + 8
-NEE_B_VERTEX = 48 + 36 + 36 + 32
+NEE_B_SHADE = 32 + 8
+NEE_B_VERTEX = 80 + 36 + 36 + 32
 NEE_B_RAY = 16
-B_NODE = 80
+B_NODE = 96
 B_TRI = 48
 
 
@@ -493,12 +495,12 @@ def run_ours(args, rank, ws, local):
              "counts_per_step": {"rays": radiance, "node_visits": cs.node_visits_trace,
                                  "tri_tests": cs.tri_tests_trace}}),
         "k_nee": kernel_roofline(
-            "k_nee (30-try emitter search + bounce)", nee_ms, nee_launches,
-            cs.nee_vertices * NEE_B_VERTEX + cs.shadow_traversals * NEE_B_RAY + cs.node_visits_nee * B_NODE +
-            cs.tri_tests_nee * B_TRI, cs.launches_nee, peak, peak_kind,
+            "k_nee (shading + 30-try emitter search + bounce)", nee_ms, nee_launches,
+            radiance * NEE_B_SHADE + cs.nee_vertices * NEE_B_VERTEX + cs.shadow_traversals * NEE_B_RAY +
+            cs.node_visits_nee * B_NODE + cs.tri_tests_nee * B_TRI, cs.launches_nee, peak, peak_kind,
             dram.get("k_nee_dram_bytes_per_vertex"), cs.nee_vertices, dram.get("k_nee_limiter"),
-            {"per_unit": {"vertex_B": NEE_B_VERTEX, "walked_shadow_ray_B": NEE_B_RAY, "node_B": B_NODE,
-                          "tri_B": B_TRI},
+            {"per_unit": {"shaded_ray_B": NEE_B_SHADE, "vertex_B": NEE_B_VERTEX, "walked_shadow_ray_B": NEE_B_RAY,
+                          "node_B": B_NODE, "tri_B": B_TRI},
              "counts_per_step": {"nee_vertices": cs.nee_vertices, "shadow_rays": cs.rays_shadow,
                                  "shadow_traversals": cs.shadow_traversals, "node_visits": cs.node_visits_nee,
                                  "tri_tests": cs.tri_tests_nee}}),

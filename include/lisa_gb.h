@@ -183,9 +183,9 @@ typedef struct lisa_render_stats {
                                 * unset), so only their count was kept      */
   double ms_guide_infer;       /* guide stage split (stage_timing): inference */
   double ms_guide_train;       /* and training (collection, steps, Adam)      */
-  uint64_t guide_infer_rows;   /* emitter-queue entries of the guided depths (the
-                                * inference runs on them, but in waves whose
-                                * bounces are all the BSDF's)                 */
+  uint64_t guide_infer_rows;   /* emitter-queue entries the inference ran on
+                                * (none in waves whose bounces are all the
+                                * BSDF's, the warm-up)                        */
   uint64_t guide_train_samples;/* samples of the training steps               */
 } lisa_render_stats;
 

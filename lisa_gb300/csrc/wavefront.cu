@@ -1194,7 +1194,6 @@ __global__ void __launch_bounds__(256, BOUNCE_BLOCKS_PER_SM) k_bsdf_bounce(WaveB
     }
   }
   warp_add32(&b.ctrl->guided_count, guided_n);
-  if (blockIdx.x == 0 && threadIdx.x == 0) b.ctrl->infer_rows += *(volatile uint32_t*)&b.ctrl->nee_count;
 }
 
 // With one stream per pixel: the first path of the wave's pixel `item`, and
