@@ -279,9 +279,8 @@ Status autotune(const lisa_renderer_params* scenes, int n, const lisa_options* b
   LISA_CUDA(cudaMemGetInfo(&free_b, &total_b));
   uint32_t maxd = 1;
   for (int i = 0; i < n; ++i) maxd = std::max(maxd, scenes[i].num_bounces);
-  // queue bytes per path: rays (2 x 32), hit 8, path state 36, emitter queue
-  // 48; guided mode adds 160 B of network outputs and 80 B per depth of
-  // training records
+  // queue bytes per path, bounded from above: rays (2 x 32), hit 8, path
+  // state 36, and, guided, vertices (48), emitter samples (32) and records
   const uint64_t per_path = 156 + (o.mode == LISA_MODE_GUIDED ? 160ull + 80ull * maxd : 0ull);
   std::vector<uint32_t> Ws;
   for (uint32_t w = 1u << 20; w <= (1u << 24); w <<= 1) {
