@@ -418,8 +418,9 @@ __constant__ uint8_t c_subset[119] = {
 // largest; and each rebuilds one node when the best topology is cheaper.
 // What bounds the kernel is the chain of treelets from a leaf to the root:
 // with the growth, the boxes and the rebuilding on one lane it took 351 us
-// for 30,001 triangles and 2.4 ms for 1.31 M, now 180 us and 0.51 ms.  All
-// 32 lanes call it with the same root.
+// for 30,001 triangles and 2.4 ms for 1.31 M; so 180 us and 0.51 ms, and from
+// 256 triangles on 125 us and 0.39 ms.  All 32 lanes call it with the same
+// root.
 __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSmem& s) {
   const int lane = threadIdx.x & 31;
   __syncwarp();  // the root's box, count and cost, just written by its lane, are visible
@@ -828,8 +829,9 @@ __device__ __forceinline__ bool collapse_barrier(BvhDeviceInfo* info, uint32_t k
 // Eight lanes collapse one node: lane k holds candidate k, its children's
 // indices loaded ahead (a step of the growth costs one memory latency), and
 // then quantises and writes child k.  Bound by those latencies, level after
-// level: 70 us for 30,001 triangles and 269 for 1.31 M, where 24 launches
-// with a thread per node and the grid in FP64 took 589 and 1,200 (cold).
+// level: 70 us for 30,001 triangles and 269 for 1.31 M (295 with a plan to
+// look up), where 24 launches with a thread per node and the grid in FP64
+// took 589 and 1,200 (cold).
 __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, k = lane & 7, g0 = lane & 24;  // candidate, first lane of the group
