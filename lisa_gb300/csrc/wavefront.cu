@@ -1221,7 +1221,7 @@ __device__ __forceinline__ uint32_t next_of_pixel(const WaveDesc& w, uint32_t sl
 // throughput: each stage launch ends with the wave's longest ray (up to a
 // hundred node visits of about a microsecond), and a frame is a chain of
 // three such launches per depth.  Here a path waits only for itself: a
-// 160 x 90 preview of the Cornell box takes 182 us instead of 397, a
+// 160 x 90 preview of the Cornell box takes 163 us instead of 397, a
 // 333 x 217 frame of eight samples with one stream per pixel 1.9 instead of 8.3.  It is
 // bound by issue (58 % of the slots) and by instruction fetch: the loop is
 // 42 KB of code, so a routine is written once and shared by the ray kinds
@@ -2012,11 +2012,17 @@ Status launch_wave_sequence(Renderer& r, const std::vector<WaveLaunch>& waves, l
       train_src.n = r.guide_batch_cap;
     }
     if (waves[wv].whole) {
-      // at least eight warps an SM, so that a small wave's paths spread over
-      // the GPU; then 32 paths a warp
+      // All resident warps share a wave of up to ten paths each: it takes as
+      // long as its longest path, and a warp of few paths steps that one faster.  (160 x 90 paths over 20 warps an SM against
+      // eight: Cornell box 112 / 132 us, icosphere box 207 / 230, hard
+      // indirect 273 / 315.)  Then warps of 32, at least eight an SM: with
+      // more paths the warps' own bookkeeping weighs more (250 x 150 paths
+      // over 20 warps an SM against eight: 281 / 275 and 380 / 370).
       const uint32_t wpb = (uint32_t)r.nee_threads / 32u, items = waves[wv].items;
-      const uint32_t few = (uint32_t)r.sm_count * ((8u + wpb - 1u) / wpb);
-      const uint32_t grid = std::min<uint32_t>((uint32_t)r.path_blocks, std::max<uint32_t>(few, (items + 32u * wpb - 1u) / (32u * wpb)));
+      const uint32_t all = (uint32_t)r.path_blocks, few = (uint32_t)r.sm_count * ((8u + wpb - 1u) / wpb);
+      const uint32_t grid = items <= 10u * wpb * all
+                                ? all
+                                : std::min(all, std::max(few, (items + 32u * wpb - 1u) / (32u * wpb)));
       const uint32_t lanes = std::min<uint32_t>(32u, (items + grid * wpb - 1u) / (grid * wpb));
       LISA_TRY(stage(0, [&] {
         const WaveBufs bp = make_bufs(r, REFILL_PATHS);
