@@ -488,16 +488,19 @@ __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSm
   }
   __syncwarp();
   // Best partition (P, S \ P) of a subset with its lowest member in P, each
-  // once: P = low + fixed + a subset of `rest`; P = S is skipped.
+  // once: P = low + fixed + a subset of `rest`; P = S is skipped.  The first
+  // is taken whatever it costs: costs that overflow (thousands of triangles
+  // that overlap, 1e17 across) must still leave a partition, or a subset
+  // would be split into nothing and itself.
   auto best_partition = [&](uint32_t sset, uint32_t fixed, uint32_t rest, float& best, uint32_t& bp) {
     uint32_t q = rest;
-    best = 3.4e38f;
+    best = INFINITY;
     bp = 0;
     while (true) {
       const uint32_t pset = q | fixed;
       if (pset != sset) {
         const float c = s.opt[pset] + s.opt[sset ^ pset];
-        if (c < best) {
+        if (bp == 0u || c < best) {
           best = c;
           bp = pset;
         }
@@ -526,7 +529,7 @@ __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSm
     // highest members
     const int i = lane >> 2;
     const uint32_t sset = i < 7 ? c_subset[112 + i] : 0xffu;
-    float best = 3.4e38f;
+    float best = INFINITY;
     uint32_t bp = 0;
     if (sset <= full) {
       const uint32_t low = sset & (0u - sset);
