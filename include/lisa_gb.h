@@ -412,6 +412,12 @@ int lisa_renderer_guide(lisa_renderer* r, int32_t scene, lisa_guide** out);
 #define LISA_STATUS_WAIT_TIMEOUT 16u
 int lisa_selftest_wait_timeout(uint32_t limit, uint32_t* status_word);
 
+/* Builds the BVH of num_triangles triangles with its sort marked as failed,
+ * as a bounded wait that ran out leaves it.  Returns the build's status
+ * (LISA_ERR_DEVICE); *written receives the number of 4-byte words that the
+ * kernels after the sort wrote (0: they returned at once). */
+int lisa_selftest_bvh_failed(uint32_t num_triangles, uint32_t* written);
+
 #ifdef __cplusplus
 }
 #endif

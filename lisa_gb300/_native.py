@@ -147,6 +147,7 @@ SIGNATURES = {
     "lisa_tuning_cache_store": (C.c_int, [C.c_char_p, _P]),
     "lisa_guide_create": (C.c_int, [C.c_uint32, C.POINTER(_P)]),
     "lisa_selftest_wait_timeout": (C.c_int, [C.c_uint32, C.POINTER(C.c_uint32)]),
+    "lisa_selftest_bvh_failed": (C.c_int, [C.c_uint32, C.POINTER(C.c_uint32)]),
     "lisa_guide_destroy": (None, [_P]),
     "lisa_guide_get_params": (C.c_int, [_P, _P]),
     "lisa_guide_set_params": (C.c_int, [_P, _P]),

@@ -1094,4 +1094,17 @@ int lisa_bvh_info(lisa_renderer* r, int32_t scene, uint32_t* nodes, uint32_t* tr
   })
 }
 
+int lisa_selftest_bvh_failed(uint32_t num_triangles, uint32_t* written) {
+  API_GUARD({
+    if (!written || num_triangles == 0 || num_triangles > 65536u)
+      return ret(Status::invalid("null argument, no triangles or more than 65536"));
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+      cudaGetLastError();
+      return ret(Status(LISA_ERR_UNSUPPORTED, "no CUDA device"));
+    }
+    return ret(selftest_bvh_failed(num_triangles, written));
+  })
+}
+
 }  // extern "C"

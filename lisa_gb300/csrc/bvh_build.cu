@@ -267,6 +267,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const uint32_t* __restri
   }
 }
 
+// A sort whose wait ran out leaves places of its output unwritten and keys
+// out of order, so the kernels behind it, which take indices from there,
+// return at once: the build then ends with its status alone.
+
 // ---- Karras radix tree ------------------------------------------------------
 __device__ __forceinline__ int kdelta(const uint32_t* keys, int64_t n, int64_t i, int64_t j) {
   if (j < 0 || j >= n) return -1;
@@ -277,7 +281,9 @@ __device__ __forceinline__ int kdelta(const uint32_t* keys, int64_t n, int64_t i
 
 __global__ void k_karras(const uint32_t* __restrict__ keys, uint32_t n, uint32_t* __restrict__ left,
                          uint32_t* __restrict__ right, uint32_t* __restrict__ first, uint32_t* __restrict__ last,
-                         uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf) {
+                         uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf,
+                         const uint32_t* __restrict__ failed) {
+  if (*failed != 0u) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n - 1) return;
   const int64_t N = n;
@@ -368,6 +374,7 @@ struct SahTree {
   uint32_t* count;  // per internal node: primitives below
   float* cost;      // per internal node: SAH cost of its subtree
   uint32_t* flags;
+  const uint32_t* failed;  // the sort's
 };
 
 // box, count and cost of a child (leaf or internal node, already complete)
@@ -631,6 +638,7 @@ __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSm
 constexpr int SAH_THREADS = 256;
 
 __global__ void __launch_bounds__(SAH_THREADS) k_bottom_up_sah(SahTree t, int refine) {
+  if (*t.failed != 0u) return;
   __shared__ TreeletSmem tls[SAH_THREADS / 32];
   TreeletSmem& tl = tls[threadIdx.x >> 5];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -729,7 +737,7 @@ __device__ __forceinline__ uint32_t plan_node(const float* a, const float* b, fl
 // with the query) goes without.
 __global__ void __launch_bounds__(256) k_wide_plan(SahTree t, float4* wide, uint32_t* plan) {
   uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p + 1 >= t.n) return;
+  if (p + 1 >= t.n || *t.failed != 0u) return;
   uint32_t l = t.left[p], r = t.right[p];
   if (!(l & r & LEAF_BIT)) return;
   while (true) {
@@ -841,7 +849,8 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
   const uint32_t gmask = 0xffu << g0, glt = ((1u << lane) - 1u) & gmask;
   const uint32_t groups = gridDim.x * (COLLAPSE_THREADS / 8);
   const uint32_t group = (blockIdx.x * COLLAPSE_THREADS + threadIdx.x) >> 3;
-  uint32_t begin = 0, end = 1;
+  // (nothing to do after a failed sort: the first barrier then says so)
+  uint32_t begin = 0, end = *(volatile uint32_t*)&a.info->failed ? 0u : 1u;
   for (uint32_t level = 0;; ++level) {
     // (whole warps run each round: the groups of a warp are consecutive)
     for (uint32_t w0 = begin + (group & ~3u); w0 < end; w0 += groups) {
@@ -1029,11 +1038,13 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
 
 // Start values of a build: the tables that count up, the bounds, node 0 (the
 // root).
-__global__ void k_build_init(uint32_t* zero, uint64_t words, BvhDeviceInfo* info, uint32_t* source, uint32_t root) {
+__global__ void k_build_init(uint32_t* zero, uint64_t words, BvhDeviceInfo* info, uint32_t* source, uint32_t root,
+                             uint32_t failed) {
   for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0u;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     BvhDeviceInfo b;
-    b.nodes = b.tris = b.depth = b.failed = b.barrier = 0u;
+    b.nodes = b.tris = b.depth = b.barrier = 0u;
+    b.failed = failed;
     for (int k = 0; k < 3; ++k) b.level[k] = 0u;
     for (int k = 0; k < 12; ++k) b.bounds[k] = (k / 3) & 1 ? (int)0x80000000 : 0x7fffffff;  // max, min
     for (int k = 0; k < RS_PASSES; ++k) b.ticket[k] = 0u;
@@ -1084,48 +1095,51 @@ size_t bvh_output_bytes(uint32_t n) {
   return (size_t)(al256((uint64_t)NODE_BYTES * max_nodes(n)) + al256((uint64_t)TRI_BYTES * n));
 }
 
+// what the kernels after the sort write
+static const char *const BVH_TREE = "bvh tree", *const BVH_NODES = "bvh nodes", *const BVH_TRIS = "bvh triangles";
+
 Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
                    uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info, const int32_t* d_mat, bool refine,
-                   bool plan) {
+                   bool plan, bool sort_failed) {
   float4 *plo, *phi, *ilo, *ihi;
   uint32_t *keys, *vals, *keys2, *vals2;
   uint32_t *left, *right, *first, *last, *par_int, *par_leaf, *counted, *source;
   BvhDeviceInfo* info;
-  const char* w = "bvh build scratch";
+  const char *w = "bvh build scratch", *wt = BVH_TREE;
   LISA_TRY(take(tmp, &plo, n, w));
   LISA_TRY(take(tmp, &phi, n, w));
-  LISA_TRY(take(tmp, &ilo, n, w));
-  LISA_TRY(take(tmp, &ihi, n, w));
+  LISA_TRY(take(tmp, &ilo, n, wt));
+  LISA_TRY(take(tmp, &ihi, n, wt));
   LISA_TRY(take(tmp, &keys, n, w));
   LISA_TRY(take(tmp, &vals, n, w));
   LISA_TRY(take(tmp, &keys2, n, w));
   LISA_TRY(take(tmp, &vals2, n, w));
-  LISA_TRY(take(tmp, &left, n, w));
-  LISA_TRY(take(tmp, &right, n, w));
-  LISA_TRY(take(tmp, &first, n, w));
-  LISA_TRY(take(tmp, &last, n, w));
-  LISA_TRY(take(tmp, &par_int, n, w));
-  LISA_TRY(take(tmp, &par_leaf, n, w));
+  LISA_TRY(take(tmp, &left, n, wt));
+  LISA_TRY(take(tmp, &right, n, wt));
+  LISA_TRY(take(tmp, &first, n, wt));
+  LISA_TRY(take(tmp, &last, n, wt));
+  LISA_TRY(take(tmp, &par_int, n, wt));
+  LISA_TRY(take(tmp, &par_leaf, n, wt));
   LISA_TRY(take(tmp, &counted, counted_words(n), w));
   LISA_TRY(take(tmp, &source, max_nodes(n), w));
   LISA_TRY(take(tmp, &info, 1, w));
   float4* wide = nullptr;
   uint32_t* splits = nullptr;
   if (plan) {
-    LISA_TRY(take(tmp, &wide, 2ull * n, w));
-    LISA_TRY(take(tmp, &splits, n, w));
+    LISA_TRY(take(tmp, &wide, 2ull * n, wt));
+    LISA_TRY(take(tmp, &splits, n, wt));
   }
   uint4* nodes = nullptr;
   float4* tris = nullptr;
-  LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), "bvh nodes"));
-  LISA_TRY(take(out, &tris, (uint64_t)(TRI_BYTES / 16) * n, "bvh triangles"));
+  LISA_TRY(take(out, &nodes, (uint64_t)(NODE_BYTES / 16) * max_nodes(n), BVH_NODES));
+  LISA_TRY(take(out, &tris, (uint64_t)(TRI_BYTES / 16) * n, BVH_TRIS));
   int dev = 0, sms = 0;
   LISA_CUDA(cudaGetDevice(&dev));
   LISA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
 
   const uint32_t root = n > 1 ? 0u : LEAF_BIT;
   k_build_init<<<std::min<uint32_t>(cdiv(counted_words(n), 1024), (uint32_t)sms * 8u), 256, 0, s>>>(
-      counted, counted_words(n), info, source, root);
+      counted, counted_words(n), info, source, root, sort_failed ? 1u : 0u);
   k_prim_bounds<<<std::min<uint32_t>(cdiv(n, 256), (uint32_t)sms * 8u), 256, 0, s>>>(d_verts, n, plo, phi, info->bounds);
   k_morton<<<cdiv(n, 256), 256, 0, s>>>(plo, phi, n, info->bounds, keys, vals);
   const uint32_t tiles = sort_tiles(n);
@@ -1145,10 +1159,12 @@ Status enqueue_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSour
   }
   LISA_CUDA(cudaGetLastError());
   if (n > 1) {
-    k_karras<<<cdiv(n - 1, 256), 256, 0, s>>>(keys, n, left, right, first, last, par_int, par_leaf);
+    k_karras<<<cdiv(n - 1, 256), 256, 0, s>>>(keys, n, left, right, first, last, par_int, par_leaf,
+                                             &info->failed);
     // boxes, counts and SAH costs bottom up, with treelet restructuring
     // unless refine is off; first/last become count/cost
-    const SahTree st{n, vals, plo, phi, par_leaf, par_int, left, right, ilo, ihi, first, (float*)last, flags};
+    const SahTree st{n, vals, plo, phi, par_leaf, par_int, left, right, ilo, ihi, first, (float*)last, flags,
+                     &info->failed};
     k_bottom_up_sah<<<cdiv(n, SAH_THREADS), SAH_THREADS, 0, s>>>(st, refine ? 1 : 0);
     if (plan) k_wide_plan<<<cdiv(n - 1, 256), 256, 0, s>>>(st, wide, splits);
     LISA_CUDA(cudaGetLastError());
@@ -1183,6 +1199,37 @@ Status bvh_result(const BvhDeviceInfo& h, uint32_t n, BvhBuildResult* info) {
     info->bmax[k] = ord2f(h.bounds[3 + k]);
   }
   return Status();
+}
+
+// A build whose sort is marked as failed from the start: its status, and how
+// many words the kernels after the sort wrote.
+Status selftest_bvh_failed(uint32_t n, uint32_t* written) {
+  struct Spy : TempDeviceBufs {
+    std::vector<std::pair<void*, size_t>> watched;
+    Status get(void** p, size_t bytes, const char* what) override {
+      bytes = (bytes + 3) & ~(size_t)3;
+      LISA_TRY(TempDeviceBufs::get(p, bytes, what));
+      LISA_CUDA(cudaMemset(*p, 0xa5, bytes));
+      if (what == BVH_TREE || what == BVH_NODES || what == BVH_TRIS) watched.push_back({*p, bytes});
+      return Status();
+    }
+  } spy;
+  float* d_verts = nullptr;
+  LISA_TRY(spy.get((void**)&d_verts, sizeof(float) * 9ull * n, "vertices"));
+  LISA_CUDA(cudaMemset(d_verts, 0, sizeof(float) * 9ull * n));
+  uint4* nodes = nullptr;
+  float4* tris = nullptr;
+  BvhDeviceInfo *d_info = nullptr, h;
+  LISA_TRY(enqueue_bvh(d_verts, n, nullptr, spy, spy, &nodes, &tris, &d_info, nullptr, true, true, true));
+  LISA_CUDA(cudaMemcpy(&h, d_info, sizeof(h), cudaMemcpyDeviceToHost));
+  *written = h.nodes + h.tris + h.depth;
+  for (const auto& b : spy.watched) {
+    std::vector<uint32_t> words(b.second / 4);
+    LISA_CUDA(cudaMemcpy(words.data(), b.first, b.second, cudaMemcpyDeviceToHost));
+    for (uint32_t x : words) *written += x != 0xa5a5a5a5u;
+  }
+  BvhBuildResult info;
+  return bvh_result(h, n, &info);
 }
 
 Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,

@@ -157,8 +157,9 @@ Status build_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, 
 // unpacks *d_info once the stream has run.
 Status enqueue_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream, ScratchSource& tmp,
                    ScratchSource& out, uint4** d_nodes, float4** d_tris, BvhDeviceInfo** d_info,
-                   const int32_t* d_mat, bool refine, bool plan);
+                   const int32_t* d_mat, bool refine, bool plan, bool sort_failed = false);
 Status bvh_result(const BvhDeviceInfo& h, uint32_t num_prims, BvhBuildResult* info);
+Status selftest_bvh_failed(uint32_t n, uint32_t* written);
 // Device bytes a build without a plan takes from `tmp`, and any from `out`,
 // for n triangles.
 size_t bvh_temp_bytes(uint32_t n);
