@@ -295,7 +295,8 @@ int lisa_write_ppm(const char* path, const uint8_t* rgba8, uint32_t width, uint3
 /* ---- traversal hooks (closest hit) ------------------------------------ */
 
 /* Closest hit of n rays against scene 0 of r.  rays: n x 8 floats
- * (ox oy oz tmin dx dy dz tmax).  prim: original triangle index or -1;
+ * (ox oy oz tmin dx dy dz tmax); a hit has tmin < t < tmax, and tmin may be
+ * negative.  prim: original triangle index or -1;
  * t: hit distance (+inf on a miss).  Ties go to the lowest triangle index.
  * Replaces optixTrace with OPTIX_RAY_FLAG_NONE (shader.cu:77-98).
  * Host buffers. */

@@ -251,7 +251,9 @@ __device__ __forceinline__ float intersect_tri(const RayShear& h, V3 va, V3 vb, 
 // 2^-24 (11 |c| + 4343 |s|) against 2^-24 (16 |c| + 8192 |s|) -- so the
 // traversal never culls a box the exact ray enters.  (An overflow makes the
 // axis NaN, which the minima and maxima drop: the box is kept.)  Candidates
-// are culled against best_t*(1+2^-16) + slack.
+// are culled against best_t + 2^-16 |best_t| + slack.  (A negative entry
+// distance, of a ray with tmin < 0, is rounded towards zero by up to 2^-20 of
+// it, which this margin covers; it orders the children last, not wrongly.)
 // Together with the lowest-index tie rule the result equals a brute-force
 // scan with the same triangle test.
 //
@@ -511,16 +513,31 @@ __device__ __forceinline__ float test_tri(const char* p, float4 r0, float4 r1, i
   return intersect_tri(h, v3(x.x, y.x, z.x), v3(x.y, y.y, z.y), v3(x.z, y.z, z.z), r0.w);
 }
 
+// A distance as an integer in the same order, and back.  The path tracer's are
+// positive, so their bits will do; given rays (SIGNED) may start behind their
+// origin (tmin < 0), where -0 and +0 are one distance.
+template <bool SIGNED>
+__device__ __forceinline__ uint32_t dist_key(float t) {
+  if (!SIGNED) return __float_as_uint(t);
+  const int i = __float_as_int(fadd(t, 0.0f));
+  return (uint32_t)(i ^ ((i >> 31) & 0x7fffffff)) ^ 0x80000000u;
+}
+template <bool SIGNED>
+__device__ __forceinline__ float key_dist(uint32_t k) {
+  if (!SIGNED) return __uint_as_float(k);
+  const int i = (int)(k ^ 0x80000000u);
+  return __int_as_float(i ^ ((i >> 31) & 0x7fffffff));
+}
+
 // Tests the triangles of all lanes of the warp, up to 32 at a time.  Either
 // each lane its own, one per pass (when that takes no more passes), or the
 // lanes' triangles laid end to end (a prefix sum of their counts): each lane
 // writes the addresses of its own into the pass's list, and lane j takes the
 // j-th with the asking lane's ray.  A lane's best hit is the minimum of the
-// 64-bit keys (t, triangle id) -- t is positive, so its bits order as the
-// float -- which is the brute-force tie rule.  Called by all 32 lanes; lanes
+// 64-bit keys (t, triangle id), which is the brute-force tie rule.  Called by all 32 lanes; lanes
 // without a ray pass w.tmask = 0.  MAT: the hit's emitter material is wanted
 // too.
-template <bool COUNT, bool MAT>
+template <bool COUNT, bool MAT, bool SIGNED>
 __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& sc, NodeWork w, uint32_t& tests,
                                                TriPass& tp) {
   const int lane = threadIdx.x & 31;
@@ -539,7 +556,7 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
   const bool own = most <= 1 || most <= ((total + 31u) >> 5);
   uint32_t pos = incl - cnt;
   const unsigned long long key0 =
-      ((unsigned long long)__float_as_uint(s.best_t) << 32) | (uint32_t)s.best_prim;
+      ((unsigned long long)dist_key<SIGNED>(s.best_t) << 32) | (uint32_t)s.best_prim;
   tp.key[lane] = key0;
   const uint32_t passes = own ? most : (total + 31u) >> 5;
 #pragma unroll 1
@@ -569,10 +586,10 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
       const float t = test_tri((const char*)(e & ~31ull), tp.ray0[o], tp.ray1[o], prim);
       if (COUNT) ++tests;
       const unsigned long long okey = *(volatile unsigned long long*)&tp.key[o];
-      const float bt = __uint_as_float((uint32_t)(okey >> 32));
+      const float bt = key_dist<SIGNED>((uint32_t)(okey >> 32));
       if (t < bt || (t == bt && prim < (int)(uint32_t)okey)) {
         better = true;
-        key = ((unsigned long long)__float_as_uint(t) << 32) | (uint32_t)prim;
+        key = ((unsigned long long)dist_key<SIGNED>(t) << 32) | (uint32_t)prim;
         atomicMin(&tp.key[o], key);
       }
     }
@@ -584,10 +601,10 @@ __device__ __forceinline__ void trav_tris_warp(TravState& s, const TraceScene& s
   }
   const unsigned long long best = tp.key[lane];
   if (best != key0) {
-    s.best_t = __uint_as_float((uint32_t)(best >> 32));
+    s.best_t = key_dist<SIGNED>((uint32_t)(best >> 32));
     s.best_prim = (int)(uint32_t)best;
     if (MAT) s.best_mat = tp.mat[lane];
-    s.cull = fmaf(s.best_t, 1.52587890625e-5f, s.best_t) + s.r.slack;
+    s.cull = fmaf(SIGNED ? fabsf(s.best_t) : s.best_t, 1.52587890625e-5f, s.best_t) + s.r.slack;
   }
   __syncwarp();
 }
@@ -733,12 +750,12 @@ __device__ __forceinline__ bool trav_pop(TravState& s, uint2* stack, const NodeW
 // Returns true for an active lane whose traversal is finished (s.best_prim /
 // s.best_t hold the result, best_prim -1 on a miss); inactive lanes get
 // false.
-template <bool COUNT, bool MAT>
+template <bool COUNT, bool MAT, bool SIGNED = false>
 __device__ __forceinline__ bool trav_step_warp(bool active, TravState& s, const TraceScene& sc, uint2* stack,
                                                uint32_t& visits, uint32_t& tests, uint32_t* status, TriPass& tp) {
   NodeWork w{0u, 0u, 0u, 0u, 0.0f};
   if (active) w = trav_node<COUNT>(s, sc, stack, visits, status);
-  trav_tris_warp<COUNT, MAT>(s, sc, w, tests, tp);
+  trav_tris_warp<COUNT, MAT, SIGNED>(s, sc, w, tests, tp);
   return active && trav_pop(s, stack, w);
 }
 
@@ -766,7 +783,7 @@ __device__ __forceinline__ void brute_hit(const SceneDev& sc, V3 o, V3 d, float 
   }
   if (best >= 0) {
     out_prim = best;
-    out_t = best_t;
+    out_t = fadd(best_t, 0.0f);  // (+0 for -0, as dist_key has it)
   }
 }
 

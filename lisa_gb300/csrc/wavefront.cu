@@ -1709,6 +1709,16 @@ __global__ void k_moments(const float4* __restrict__ sum, const double* __restri
 // ---------------------------------------------------------------------------
 // traversal hooks: closest hit / brute force / counting pass of given rays
 
+// Ray i of `rays` (ox oy oz tmin dx dy dz tmax).  A negative tmax gets the
+// margin of a best hit (a positive one needs none: its entry distances are
+// rounded down).
+__device__ __forceinline__ bool begin_given(TravState& s, const TraceScene& ts, const float* rays, uint32_t i, TriPass& tp) {
+  const float* r = rays + 8ull * i;
+  const bool active = trav_begin(s, ts, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), r[3], r[7], tp);
+  if (r[7] < 0.0f) s.cull = fmaf(-r[7], 1.52587890625e-5f, r[7]);
+  return active;
+}
+
 template <bool COUNT>
 __global__ void __launch_bounds__(128) k_trace_rays(const SceneDev* __restrict__ scd, const float* __restrict__ rays,
                                                    uint32_t n, int32_t* prim, float* tout, WaveCtrl* ctrl) {
@@ -1723,12 +1733,9 @@ __global__ void __launch_bounds__(128) k_trace_rays(const SceneDev* __restrict__
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     TravState s;
     bool active = false;
-    if (i < n) {
-      const float* r = rays + 8ull * i;
-      active = trav_begin(s, ts, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), r[3], r[7], tp);
-    }
+    if (i < n) active = begin_given(s, ts, rays, i, tp);
     while (__any_sync(FULL, active))
-      if (trav_step_warp<COUNT, false>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) active = false;
+      if (trav_step_warp<COUNT, false, true>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) active = false;
     if (i < n) {
       if (prim) prim[i] = s.best_prim;
       if (tout) tout[i] = s.best_prim >= 0 ? s.best_t : __int_as_float(0x7f800000);
@@ -1776,8 +1783,7 @@ __global__ void __launch_bounds__(128, LISA_TRACE_MIN_BLOCKS) k_trace_rays_share
       const uint32_t at = next + __popc(idle & lanemask_lt());
       if (!active && at < end) {
         i = at;
-        const float* r = rays + 8ull * i;
-        active = trav_begin(s, ts, v3(r[0], r[1], r[2]), v3(r[4], r[5], r[6]), r[3], r[7], tp);
+        active = begin_given(s, ts, rays, i, tp);
         if (!active) done();
       }
       next = min(end, next + __popc(idle));
@@ -1786,7 +1792,7 @@ __global__ void __launch_bounds__(128, LISA_TRACE_MIN_BLOCKS) k_trace_rays_share
       if (next >= end) break;
       continue;
     }
-    if (trav_step_warp<COUNT, false>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) {
+    if (trav_step_warp<COUNT, false, true>(active, s, ts, stack, visits, tests, &ctrl->status, tp)) {
       active = false;
       done();
     }
