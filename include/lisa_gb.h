@@ -329,7 +329,8 @@ int lisa_trace_soup_noalloc(const float* d_vertices, uint32_t num_triangles, con
  * runs the closest-hit kernel on the rays with counters enabled. */
 int lisa_trace_count(lisa_renderer* r, const float* rays, uint32_t n, uint64_t* node_visits,
                      uint64_t* tri_tests);
-/* BVH statistics: 8-wide node count, leaf triangle slots, depth. */
+/* BVH statistics: 8-wide node count, leaf triangle slots, depth, and the GPU
+ * time of its construction (not of the copies around it). */
 int lisa_bvh_info(lisa_renderer* r, int32_t scene, uint32_t* nodes, uint32_t* tri_slots,
                   uint32_t* depth, double* build_ms);
 

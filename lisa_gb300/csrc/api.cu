@@ -8,7 +8,6 @@
 #include <cuda.h>
 
 #include <algorithm>
-#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -508,13 +507,14 @@ struct SceneUpload : TempDeviceBufs {
   uint32_t* mask = nullptr;
   PrimScan* scan = nullptr;
   cudaStream_t side = nullptr;
-  cudaEvent_t ready = nullptr;
+  cudaEvent_t ready = nullptr, build0 = nullptr, build1 = nullptr;
   ~SceneUpload() {
     if (side) {
       cudaStreamSynchronize(side);
       cudaStreamDestroy(side);
     }
-    if (ready) cudaEventDestroy(ready);
+    for (cudaEvent_t e : {ready, build0, build1})
+      if (e) cudaEventDestroy(e);
   }
 };
 }  // namespace
@@ -564,10 +564,14 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
       LISA_CUDA(cudaEventRecord(up.ready, r.stream));
       LISA_CUDA(cudaStreamWaitEvent(side, up.ready, 0));
     }
-    const auto t0 = std::chrono::steady_clock::now();
+    // (the build's time is its own on the GPU, without the copies around it)
+    LISA_CUDA(cudaEventCreate(&up.build0));
+    LISA_CUDA(cudaEventCreate(&up.build1));
+    LISA_CUDA(cudaEventRecord(up.build0, r.stream));
     BvhDeviceInfo *d_info = nullptr, info;
     LISA_TRY(enqueue_bvh(up.v, T, r.stream, up, r.arena, &s.nodes, &s.tris, &d_info, up.leaf,
                          r.opts.bvh_lbvh_only == 0, true));
+    LISA_CUDA(cudaEventRecord(up.build1, r.stream));
     LISA_CUDA(cudaMemcpyAsync(up.n, p.normals, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, side));
     k_pack_prims<<<r.sm_count * 8, 256, 0, side>>>(up.v, up.n, up.m, T, s.prims);
     LISA_CUDA(cudaGetLastError());
@@ -575,7 +579,9 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
     LISA_CUDA(cudaMemcpyAsync(&scan, up.scan, sizeof(scan), cudaMemcpyDeviceToHost, r.stream));
     LISA_CUDA(cudaStreamSynchronize(r.stream));
     LISA_TRY(bvh_result(info, T, &s.bvh));
-    s.bvh.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    float build_ms = 0.0f;
+    LISA_CUDA(cudaEventElapsedTime(&build_ms, up.build0, up.build1));
+    s.bvh.build_ms = build_ms;
     if (scan.bad != 0xffffffffu)
       return Status::invalid("material index out of range at triangle " + std::to_string(scan.bad));
     // the host's own work on emitters: their list for the physically based

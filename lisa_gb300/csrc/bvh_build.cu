@@ -24,7 +24,6 @@
 //      Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed
 //      Wide BVHs", HPG 2017).  Leaf triangles are copied into leaf order.
 #include <algorithm>
-#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -1234,7 +1233,6 @@ Status selftest_bvh_failed(uint32_t n, uint32_t* written) {
 
 Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource& tmp, ScratchSource& out,
                  uint4** d_nodes, float4** d_tris, BvhBuildResult* info, const int32_t* d_mat, bool refine) {
-  auto t0 = std::chrono::steady_clock::now();
   *d_nodes = nullptr;
   *d_tris = nullptr;
   if (n == 0) {
@@ -1253,7 +1251,6 @@ Status build_bvh(const float* d_verts, uint32_t n, cudaStream_t s, ScratchSource
   LISA_TRY(bvh_result(h, n, info));
   *d_nodes = nodes;
   *d_tris = tris;
-  info->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   return Status();
 }
 
