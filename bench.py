@@ -442,6 +442,7 @@ def run_ours(args, rank, ws, local):
         with tempfile.TemporaryDirectory() as td:
             tuning = L.autotune(params, base, cache=os.path.join(td, "tune.json"))
         base = L.apply_tuning(tuning, base)
+        base.refill_idle = 0  # each kernel's own threshold (the tuner tries one for all)
     tuned = {k: getattr(base, k) for k in ("paths_in_flight", "threads_per_block", "blocks_per_sm", "refill_idle")}
     opts = L.default_options(stage_timing=1, **tuned)
     r = L.Renderer(params, opts)

@@ -134,9 +134,9 @@ typedef struct lisa_options {
                                 waves (0 = fill the wavefront)                */
   uint32_t refill_idle;      /* persistent traversal kernels take new work once
                                 this many of a warp's 32 lanes are idle
-                                (1..32; 0 = 12; the closest-hit kernel four
-                                fewer, the emitter search four more, whole
-                                paths eight more)                             */
+                                (1..32, in every kernel; 0 = 8 in the
+                                closest-hit kernel, 16 in the emitter search,
+                                20 where it runs whole paths)                 */
   uint32_t estimator;        /* LISA_ESTIMATOR_*                               */
   uint32_t bvh_lbvh_only;    /* 1 = keep the plain LBVH: skip its SAH treelet
                                 restructuring before the 8-wide collapse      */

@@ -26,6 +26,7 @@
 #include "guide_mix.cuh"
 #include "lisa_device.cuh"
 #include "lisa_internal.h"
+#include "refill.h"
 #include "wavefront.cuh"
 
 #ifndef LISA_BSDF_HEADER
@@ -56,13 +57,6 @@ constexpr uint32_t FULL = 0xffffffffu;
 #ifndef LISA_PATHS_MIN_BLOCKS
 #define LISA_PATHS_MIN_BLOCKS 5  // whole paths: 96 registers, best of 4..6
 #endif
-// Idle lanes (of 32) that trigger a refill round: the option (default 12)
-// plus this much for each kind of kernel, whose rounds differ in length.
-// Measured by default: closest hit 8 (4, 8, 10, 12, 16 tried: 14.05 ms a step
-// of the 1.31 M-triangle icosphere box at 8, 14.19 at 12), emitter search 16
-// (12.1 ms against 12.4 at 12 and 12.7 at 8), whole paths 20 (5.15 ms of 4 Mi
-// Cornell box paths against 5.26 at 16 and 5.61 at 12).
-constexpr int REFILL_DEFAULT = 12, REFILL_TRACE = -4, REFILL_NEE = 4, REFILL_PATHS = 8;
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
@@ -1970,8 +1964,8 @@ void plan_waves(Renderer& r, const std::vector<uint32_t>& spp, const std::vector
   }
 }
 
-// kind: REFILL_*, of the kernel the buffers go to
-WaveBufs make_bufs(Renderer& r, int kind = 0) {
+// own: REFILL_*, of the kernel the buffers go to (0: it does not traverse)
+WaveBufs make_bufs(Renderer& r, uint32_t own = 0) {
   WaveBufs b;
   std::memset(&b, 0, sizeof(b));
   b.ro[0] = r.ro[0];
@@ -1988,8 +1982,7 @@ WaveBufs make_bufs(Renderer& r, int kind = 0) {
   b.ctrl = r.ctrl;
   b.scenes = r.d_scenes;
   b.capacity = r.capacity;
-  const int idle = (r.opts.refill_idle ? (int)std::min<uint32_t>(r.opts.refill_idle, 32u) : REFILL_DEFAULT) + kind;
-  b.refill_busy_max = (uint32_t)(32 - std::min(std::max(idle, 1), 32));
+  b.refill_busy_max = 32u - refill_idle_lanes(r.opts.refill_idle, own);
   b.physical = r.opts.estimator == LISA_ESTIMATOR_PHYSICAL;
   b.rec_list = r.rec_list;
   b.rec_col = r.rec_list ? r.rec_list + 4ull * r.rec_cap : nullptr;
