@@ -519,8 +519,25 @@ struct SceneUpload : TempDeviceBufs {
 };
 }  // namespace
 
+static Status bad_material(uint32_t t) {
+  return Status::invalid("material index out of range at triangle " + std::to_string(t));
+}
+
+static Status upload_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s);
+
+// The device's scan of the triangles finds a bad material index, behind
+// allocations and a build that may fail for reasons of their own.  Then the
+// host looks, so that a bad scene is refused as one whatever else went wrong.
 Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
   LISA_TRY(validate(p));
+  const Status st = upload_scene(r, p, s);
+  if (!st.ok())
+    for (uint32_t t = 0; t < (uint32_t)(p.num_vertices / 3); ++t)
+      if ((uint32_t)p.mat_indices[t] >= (uint32_t)p.num_materials) return bad_material(t);
+  return st;
+}
+
+static Status upload_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
   s.params = p;
   s.output_image = p.output_image ? p.output_image : "";
   s.params.output_image = nullptr;
@@ -582,8 +599,7 @@ Status create_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu& s) {
     float build_ms = 0.0f;
     LISA_CUDA(cudaEventElapsedTime(&build_ms, up.build0, up.build1));
     s.bvh.build_ms = build_ms;
-    if (scan.bad != 0xffffffffu)
-      return Status::invalid("material index out of range at triangle " + std::to_string(scan.bad));
+    if (scan.bad != 0xffffffffu) return bad_material(scan.bad);
     // the host's own work on emitters: their list for the physically based
     // estimator, their BVH for the other (its search would not use a small one)
     if (r.opts.estimator == LISA_ESTIMATOR_PHYSICAL ? scan.emissive > 0 : scan.emissive >= EMIT_BVH_MIN_TRIS) {
