@@ -137,13 +137,7 @@ __global__ void k_morton(const float4* __restrict__ lo, const float4* __restrict
 }
 
 // ---- radix sort -----------------------------------------------------------
-constexpr int RS_THREADS = 256;
-constexpr int RS_PASSES = 4;  // 8 bits each (BvhDeviceInfo has a ticket per pass)
 constexpr uint32_t RS_POLLS = 1u << 22;  // of a look-back wait, then the build fails
-
-// Keys per thread of a tile: 16, but 4 for up to 256 Ki keys, which would
-// otherwise make too few tiles (8 of them at 30,000) to fill the GPU.
-inline int rs_rounds(uint32_t n) { return n <= (1u << 18) ? 4 : 16; }
 
 // Histograms of the four digits (hist: 4 x 256, zeroed before).
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const uint32_t* __restrict__ keys, uint32_t n,
@@ -1064,35 +1058,7 @@ Status take(ScratchSource& src, T** p, uint64_t count, const char* what) {
   *p = (T*)q;
   return Status();
 }
-inline uint64_t al256(uint64_t b) { return (std::max<uint64_t>(b, 16) + 255) & ~255ull; }
 }  // namespace
-
-// Most 8-wide nodes that n triangles can give.  A node with an internal
-// child has eight children (the collapse opens candidates until there are
-// eight or none is left to open, whatever was planned), the others (T, below F such nodes) hold at
-// least four triangles; the F nodes' own leaves number 8 F - (F + T - 1), so
-// n >= 4 T + 7 F - T + 1 >= 3 (F + T) + 1.
-static uint32_t max_nodes(uint32_t n) { return n / 3 + 1; }
-
-static uint32_t sort_tiles(uint32_t n) { return cdiv(n, (uint64_t)RS_THREADS * rs_rounds(n)); }
-// Words of the tables that a build counts up in: look-back states and digit
-// histograms of the sort, arrival flags of the bottom-up pass.
-static uint64_t counted_words(uint32_t n) { return (uint64_t)RS_PASSES * 256 * (sort_tiles(n) + 1) + n; }
-
-size_t bvh_temp_bytes(uint32_t n) {
-  uint64_t b = 0;
-  b += 4 * al256(16ull * n);                // plo phi ilo ihi
-  b += 4 * al256(4ull * n);                 // keys vals keys2 vals2
-  b += 6 * al256(4ull * n);                 // tree links, counts and costs
-  b += al256(4ull * counted_words(n));
-  b += al256(4ull * max_nodes(n));          // collapse work list
-  b += al256(sizeof(BvhDeviceInfo));
-  return (size_t)b;
-}
-
-size_t bvh_output_bytes(uint32_t n) {
-  return (size_t)(al256((uint64_t)NODE_BYTES * max_nodes(n)) + al256((uint64_t)TRI_BYTES * n));
-}
 
 // what the kernels after the sort write
 static const char *const BVH_TREE = "bvh tree", *const BVH_NODES = "bvh nodes", *const BVH_TRIS = "bvh triangles";

@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "bvh_sizes.h"
 #include "device_math.cuh"
 
 namespace lisa {
@@ -306,9 +307,6 @@ __device__ __forceinline__ TraceScene trace_scene_emit(const SceneDev& sc) {
 #endif
   return t;
 }
-
-constexpr int NODE_BYTES = 96;
-constexpr int TRI_BYTES = 64;
 
 // 32 bytes of read-only global memory, 32-byte aligned, in one load.
 struct Words8 {

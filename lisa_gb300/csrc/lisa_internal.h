@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/lisa_gb.h"
+#include "bvh_sizes.h"
 
 namespace lisa {
 
@@ -117,19 +118,6 @@ struct BvhBuildResult {
   float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};
 };
 
-// What a build leaves on the device, for the host and for kernels that
-// follow it on the stream.
-struct BvhDeviceInfo {
-  uint32_t nodes;      // 8-wide nodes
-  uint32_t tris;       // leaf triangles written
-  uint32_t depth;
-  uint32_t failed;     // a bounded wait ran out
-  int bounds[12];      // scene min, max and centroid min, max, as order-preserving ints
-  uint32_t level[3];   // nodes taken by the collapse's current level (in turn)
-  uint32_t barrier;    // arrivals of the collapse's blocks
-  uint32_t ticket[4];  // tiles started, per sort pass
-};
-
 // Order-preserving ints of floats.
 __host__ __device__ inline int f2ord(float f) {
   int i;
@@ -160,10 +148,6 @@ Status enqueue_bvh(const float* d_verts, uint32_t num_prims, cudaStream_t stream
                    const int32_t* d_mat, bool refine, bool plan, bool sort_failed = false);
 Status bvh_result(const BvhDeviceInfo& h, uint32_t num_prims, BvhBuildResult* info);
 Status selftest_bvh_failed(uint32_t n, uint32_t* written);
-// Device bytes a build without a plan takes from `tmp`, and any from `out`,
-// for n triangles.
-size_t bvh_temp_bytes(uint32_t n);
-size_t bvh_output_bytes(uint32_t n);
 
 // ---- renderer ---------------------------------------------------------------
 struct SceneDev;

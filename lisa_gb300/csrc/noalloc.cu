@@ -38,10 +38,15 @@ namespace lisa {
 namespace {
 
 constexpr uint32_t NOALLOC_MAX_TRIANGLES = 65536;
-// BVH build temporaries (~172 B per triangle) + 8-wide nodes and leaf
-// triangles (~128 B per triangle) + the scene record and status word, with
-// room for alignment.
+// The size is part of the interface.  A build takes 113 B a triangle of it for
+// temporaries and 96 B for 8-wide nodes and leaf triangles.
 constexpr size_t NOALLOC_SCRATCH_BYTES = (size_t)NOALLOC_MAX_TRIANGLES * 320 + (1u << 20);
+static_assert(al256(sizeof(SceneDev)) + al256(sizeof(WaveCtrl)) + bvh_temp_bytes(NOALLOC_MAX_TRIANGLES) +
+                      bvh_output_bytes(NOALLOC_MAX_TRIANGLES) <=
+                  NOALLOC_SCRATCH_BYTES,
+              "the scene record, the status word and the build of the largest soup fit the scratch");
+static_assert((bvh_temp_bytes(NOALLOC_MAX_TRIANGLES) >> 16) == 113 && (bvh_output_bytes(NOALLOC_MAX_TRIANGLES) >> 16) == 96,
+              "the figures above");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
