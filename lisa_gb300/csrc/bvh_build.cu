@@ -968,7 +968,11 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
 #pragma unroll
       for (int ax = 0; ax < 3; ++ax) {
         e[ax] = grid_exponent(__fsub_ru(q[ax], p[ax]));
-        // rounded outward: p + 2^e * ql <= lo and p + 2^e * qh >= hi exactly
+        // rounded outward: p + 2^e * ql <= lo and p + 2^e * qh >= hi exactly.
+        // (Every whole number of steps up to 255 is a float, so a difference
+        // rounded down has the floor of the exact one, and rounded up its
+        // ceiling; likewise 255 * 2^e for the exponent.  FP64 would find no
+        // tighter box.)
         uint32_t ql = 0, qh = 0;
         if (k < nc) {
           ql = (uint32_t)fminf(fmaxf(floorf(ldexpf(__fsub_rd(clo[ax], p[ax]), -e[ax])), 0.0f), 255.0f);
