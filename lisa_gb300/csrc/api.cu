@@ -507,14 +507,13 @@ struct SceneUpload : TempDeviceBufs {
   uint32_t* mask = nullptr;
   PrimScan* scan = nullptr;
   cudaStream_t side = nullptr;
-  cudaEvent_t ready = nullptr, build0 = nullptr, build1 = nullptr;
+  cudaEvent_t ready = nullptr;
   ~SceneUpload() {
     if (side) {
       cudaStreamSynchronize(side);
       cudaStreamDestroy(side);
     }
-    for (cudaEvent_t e : {ready, build0, build1})
-      if (e) cudaEventDestroy(e);
+    if (ready) cudaEventDestroy(ready);
   }
 };
 }  // namespace
@@ -581,14 +580,9 @@ static Status upload_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu&
       LISA_CUDA(cudaEventRecord(up.ready, r.stream));
       LISA_CUDA(cudaStreamWaitEvent(side, up.ready, 0));
     }
-    // (the build's time is its own on the GPU, without the copies around it)
-    LISA_CUDA(cudaEventCreate(&up.build0));
-    LISA_CUDA(cudaEventCreate(&up.build1));
-    LISA_CUDA(cudaEventRecord(up.build0, r.stream));
     BvhDeviceInfo *d_info = nullptr, info;
     LISA_TRY(enqueue_bvh(up.v, T, r.stream, up, r.arena, &s.nodes, &s.tris, &d_info, up.leaf,
                          r.opts.bvh_lbvh_only == 0, true));
-    LISA_CUDA(cudaEventRecord(up.build1, r.stream));
     LISA_CUDA(cudaMemcpyAsync(up.n, p.normals, sizeof(float) * 9ull * T, cudaMemcpyHostToDevice, side));
     k_pack_prims<<<r.sm_count * 8, 256, 0, side>>>(up.v, up.n, up.m, T, s.prims);
     LISA_CUDA(cudaGetLastError());
@@ -596,9 +590,6 @@ static Status upload_scene(Renderer& r, const lisa_renderer_params& p, SceneGpu&
     LISA_CUDA(cudaMemcpyAsync(&scan, up.scan, sizeof(scan), cudaMemcpyDeviceToHost, r.stream));
     LISA_CUDA(cudaStreamSynchronize(r.stream));
     LISA_TRY(bvh_result(info, T, &s.bvh));
-    float build_ms = 0.0f;
-    LISA_CUDA(cudaEventElapsedTime(&build_ms, up.build0, up.build1));
-    s.bvh.build_ms = build_ms;
     if (scan.bad != 0xffffffffu) return bad_material(scan.bad);
     // the host's own work on emitters: their list for the physically based
     // estimator, their BVH for the other (its search would not use a small one)

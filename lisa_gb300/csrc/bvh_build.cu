@@ -801,6 +801,12 @@ __device__ __forceinline__ int grid_exponent(float ext) {
 
 constexpr int COLLAPSE_THREADS = 128;
 
+__device__ __forceinline__ uint64_t gpu_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // All blocks of the cooperative grid meet; false once a wait (bounded) has
 // run out in some block.  Memory written before is visible after it to loads
 // that bypass L1.
@@ -1027,6 +1033,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(CollapseArgs a) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.info->nodes = end;
         a.info->depth = level + 1u;
+        a.info->end_ns = gpu_ns();
       }
       return;
     }
@@ -1042,6 +1049,8 @@ __global__ void k_build_init(uint32_t* zero, uint64_t words, BvhDeviceInfo* info
     BvhDeviceInfo b;
     b.nodes = b.tris = b.depth = b.barrier = 0u;
     b.failed = failed;
+    b.begin_ns = gpu_ns();
+    b.end_ns = 0u;
     for (int k = 0; k < 3; ++k) b.level[k] = 0u;
     for (int k = 0; k < 12; ++k) b.bounds[k] = (k / 3) & 1 ? (int)0x80000000 : 0x7fffffff;  // max, min
     for (int k = 0; k < RS_PASSES; ++k) b.ticket[k] = 0u;
@@ -1163,6 +1172,7 @@ Status bvh_result(const BvhDeviceInfo& h, uint32_t n, BvhBuildResult* info) {
   info->num_nodes = h.nodes;
   info->num_tri_slots = h.tris;
   info->depth = h.depth;
+  info->build_ms = 1e-6 * (double)(h.end_ns - h.begin_ns);
   for (int k = 0; k < 3; ++k) {
     info->bmin[k] = ord2f(h.bounds[k]);
     info->bmax[k] = ord2f(h.bounds[3 + k]);

@@ -22,6 +22,7 @@ struct BvhDeviceInfo {
   uint32_t level[3];   // nodes taken by the collapse's current level (in turn)
   uint32_t barrier;    // arrivals of the collapse's blocks
   uint32_t ticket[4];  // tiles started, per sort pass
+  uint64_t begin_ns, end_ns;  // the GPU's clock in the first kernel and at the end of the last
 };
 
 constexpr int RS_THREADS = 256;

@@ -114,7 +114,7 @@ struct BvhBuildResult {
   uint32_t num_nodes = 0;
   uint32_t num_tri_slots = 0;
   uint32_t depth = 0;
-  double build_ms = 0.0;  // GPU time of the kernels, first to last (a scene's own BVH)
+  double build_ms = 0.0;  // GPU time of the kernels, first to last
   float bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0};
 };
 
