@@ -52,13 +52,13 @@ constexpr int NEE_TRIES = 30;      // shader.cu:199
 // fewer, the bounds test of the emitter search is as selective)
 constexpr uint32_t EMIT_BVH_MIN_TRIS = 32;
 // Entries of a ray's traversal stack.  A node pushes up to seven of its
-// children, so a tree of depth d takes at most 7 (d - 1): none of up to 28
+// children, so a tree of depth d takes at most 7 (d - 1): none of up to 33
 // levels overflows it (a deeper one may, which sets ST_STACK_OVERFLOW).  The
-// scenes here have 6 to 12 levels and use up to 20 entries; soups of a million
-// triangles of sizes that span 2^60, or that all overlap, 17 to 26 levels and
-// up to 102, where 64 entries failed.  Its unused part costs no time, only
-// local memory that the driver reserves (1.5 KB a resident thread).
-constexpr int TRAV_STACK = 192;
+// scenes here have 6 to 12 levels and use up to 20 entries; soups of six
+// million triangles of sizes that span 2^120, or that all overlap, 17 to 29
+// levels and up to 110, where 64 entries failed.  Its unused part costs no
+// time, only local memory that the driver reserves (1.75 KB a resident thread).
+constexpr int TRAV_STACK = 224;
 
 enum StatusBits : uint32_t {
   ST_STACK_OVERFLOW = 1u,
