@@ -262,7 +262,9 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_pass(const uint32_t* __restri
 
 // A sort whose wait ran out leaves places of its output unwritten and keys
 // out of order, so the kernels behind it, which take indices from there,
-// return at once: the build then ends with its status alone.
+// do nothing: the build then ends with its status alone.  (They look at the
+// mark beside their first loads; waiting for it before those would add its
+// latency to each.)
 
 // ---- Karras radix tree ------------------------------------------------------
 __device__ __forceinline__ int kdelta(const uint32_t* keys, int64_t n, int64_t i, int64_t j) {
@@ -276,10 +278,10 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, uint32_t n, uint32_t
                          uint32_t* __restrict__ right, uint32_t* __restrict__ first, uint32_t* __restrict__ last,
                          uint32_t* __restrict__ parent_int, uint32_t* __restrict__ parent_leaf,
                          const uint32_t* __restrict__ failed) {
-  if (*failed != 0u) return;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)n - 1) return;
-  const int64_t N = n;
+  const uint32_t bad = *failed;
+  const int64_t N = n;  // (keys in any order: every index below stays inside)
   const int d = (kdelta(keys, N, i, i + 1) - kdelta(keys, N, i, i - 1)) >= 0 ? 1 : -1;
   const int dmin = kdelta(keys, N, i, i - d);
   int64_t lmax = 2;
@@ -298,6 +300,7 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, uint32_t n, uint32_t
   const int64_t lo = i < j ? i : j, hi = i < j ? j : i;
   const uint32_t lc = (lo == gamma) ? (LEAF_BIT | (uint32_t)gamma) : (uint32_t)gamma;
   const uint32_t rc = (hi == gamma + 1) ? (LEAF_BIT | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
+  if (bad != 0u) return;
   left[i] = lc;
   right[i] = rc;
   first[i] = (uint32_t)lo;
@@ -631,12 +634,11 @@ __device__ void treelet_optimize_warp(const SahTree& t, uint32_t root, TreeletSm
 constexpr int SAH_THREADS = 256;
 
 __global__ void __launch_bounds__(SAH_THREADS) k_bottom_up_sah(SahTree t, int refine) {
-  if (*t.failed != 0u) return;
   __shared__ TreeletSmem tls[SAH_THREADS / 32];
   TreeletSmem& tl = tls[threadIdx.x >> 5];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t p = (i < t.n && t.n >= 2) ? t.parent_leaf[i] : 0xffffffffu;
-  bool active = p != 0xffffffffu;
+  bool active = p != 0xffffffffu && *t.failed == 0u;
   while (__any_sync(0xffffffffu, active)) {
     bool want = false;
     if (active) {
@@ -730,9 +732,9 @@ __device__ __forceinline__ uint32_t plan_node(const float* a, const float* b, fl
 // with the query) goes without.
 __global__ void __launch_bounds__(256) k_wide_plan(SahTree t, float4* wide, uint32_t* plan) {
   uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p + 1 >= t.n || *t.failed != 0u) return;
+  if (p + 1 >= t.n) return;
   uint32_t l = t.left[p], r = t.right[p];
-  if (!(l & r & LEAF_BIT)) return;
+  if (!(l & r & LEAF_BIT) || *t.failed != 0u) return;
   while (true) {
     float c[2][8], o[8];
 #pragma unroll
