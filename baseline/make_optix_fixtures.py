@@ -3,7 +3,7 @@
 Run on a machine with the GPU, after baseline/stage_optix.py staged the
 reference sources (they travel in baseline/_ref):
 
-    python baseline/make_optix_fixtures.py gpurun_out/optix_fixtures
+    python baseline/make_optix_fixtures.py out/optix_fixtures
 
 For each scene of tests/golden/shader_scenes.py it runs the reference's own
 OptiX pipeline (baseline/optix_harness.cc) on the scene written as .rto +
